@@ -4,7 +4,9 @@
 #include <cmath>
 #include <cstdio>
 #include <algorithm>
+#include <array>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -64,7 +66,8 @@ struct plum_ctx {
   double* d_out = nullptr;     // small result block
   double* d_obs_per = nullptr;  // [n_mol * 5] per-molecule Rg / Ree sums
   double* d_press = nullptr;    // wall-force pressure partials and sums
-  int press_cap = 0;
+  double* d_gtab64 = nullptr;   // FP64 g(u) table of its real-space force
+  long long press_cap = 0;
   unsigned* d_rhoz = nullptr;   // [3 * rhoz_bins] rho(z) counts
   int rhoz_bins = 0;
   // surrogate training data: descriptor accumulator and device copies of
@@ -121,7 +124,8 @@ namespace {
 // PotentialEwaldCoul::ReadParameters (potential_ewald_coul.cc:38-115):
 // padded z for the dipole correction, real-space cut-off and cells, k^2
 // cut-off and cells; then the half-space k-set {k : 0 < k^2 <= kc^2}.
-int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw) {
+int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
+                std::vector<KUnit>* ku) {
   Input& in = c->in;
   DevParams& P = c->P;
   EwaldSetup E;
@@ -160,6 +164,20 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw) {
     kw->push_back(E.kw[k]);
   }
   P.n_k = (int)kn->size();
+  // the list as +-nz pairs, in list order (a column's vectors are consecutive)
+  std::map<std::array<int, 3>, int> at;
+  for (int k = 0; k < P.n_k; k++) at[{(*kn)[k].x, (*kn)[k].y, (*kn)[k].z}] = k;
+  ku->clear();
+  for (int k = 0; k < P.n_k; k++) {
+    const short4 v = (*kn)[k];
+    const auto mate = at.find({v.x, v.y, -v.z});
+    const int m = v.z == 0 || mate == at.end() ? -1 : mate->second;
+    if (v.z >= 0)
+      ku->push_back(KUnit{v.x, v.y, v.z, 0, k, m});
+    else if (m < 0)
+      ku->push_back(KUnit{v.x, v.y, (short)-v.z, 0, -1, k});
+  }
+  P.n_ku = (int)ku->size();
   c->in.x_kcut2 = E.kc2;  // effective k^2 cut-off, reported by plum_ctx_info
   return PLUM_OK;
 }
@@ -570,12 +588,13 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   P.n_ion_total = (int)ions.size();
   std::vector<short4> kn;
   std::vector<double> kw;
+  std::vector<KUnit> ku;
   if (form == PLUM_FORM_FP32 && in.npbc == 3 && in.dipole) {
     delete c;
     return fail(PLUM_ERR_INPUT, "the precision form needs npbc = 2 when the dipole correction is on");
   }
   if (in.use_ewald) {
-    int rc = setup_ewald(c, &kn, &kw);
+    int rc = setup_ewald(c, &kn, &kw, &ku);
     if (rc) {
       delete c;
       return rc;
@@ -627,6 +646,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   rc |= dalloc(&B.ion_ids, ions.size());
   rc |= dalloc(&B.kn, kn.size());
   rc |= dalloc(&B.kw, kw.size());
+  rc |= dalloc(&B.ku, ku.size());
   rc |= dalloc(&B.sk, kn.size());
   rc |= dalloc(&B.dsk, 2 * kn.size());
   rc |= dalloc(&B.done_count, 1);
@@ -657,8 +677,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   if (P.use_ewald) {
     rc |= dalloc(&c->d_htab64, (size_t)kH64Bins * kH64Stride);
     if (!rc) {
-      std::vector<double> h((size_t)kH64Bins * kH64Stride);
-      build_h64_table(h.data());
+      const std::vector<double>& h = h64_table();
       cudaMemcpy(c->d_htab64, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice);
       P.htab64 = c->d_htab64;
     }
@@ -702,6 +721,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   if (!kn.empty()) {
     cudaMemcpy(B.kn, kn.data(), sizeof(short4) * kn.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(B.kw, kw.data(), sizeof(double) * kw.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(B.ku, ku.data(), sizeof(KUnit) * ku.size(), cudaMemcpyHostToDevice);
   }
   cudaMemset(B.state, 0, sizeof(DevState));
   cudaMemset(B.ktile_count, 0, sizeof(int) * std::max(1, ktile_count(P)));
@@ -734,7 +754,7 @@ int plum_ctx_destroy(plum_ctx* c) {
                   c->d_rp1,      c->d_rb1,     c->desc_fine, c->cb_part32, c->cb_ticket,
                   c->d_stream,   c->d_mt,      c->d_log_type, c->d_log_acc, c->d_log_e,
                   c->d_press,    c->d_sk_part, c->d_log_de, c->d_htab, c->d_htab64,
-                  c->B.fpos64};
+                  c->B.fpos64,   c->B.ku,      c->d_gtab64};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
@@ -1478,23 +1498,24 @@ int plum_pressure_slit(plum_ctx* c, double* out6) {
   }
   if (S.phantom < 0 || S.phantom > S.n_mol) return fail(PLUM_ERR_INPUT, "bad number of wall sites");
   const int* ms = in.mol_start.data();
-  const long long n_pair = slit_pair_items(S, ms);
-  const long long n_wall = slit_wall_items(S, ms);
-  const int n_k = (S.use_ewald && S.phantom > 0) ? P.n_k : 0;
-  int n1 = 0, n2 = 0;
-  const int need = slit_partials_count(n_pair + n_wall, n_k, &n1, &n2);
-  if (need > c->press_cap) {
+  const SlitGrid G = slit_grid(S, P, slit_pair_items(S, ms), ms[S.phantom / 2]);
+  if (G.total > c->press_cap) {
     if (c->d_press) cudaFree(c->d_press);
     c->d_press = nullptr;
     c->press_cap = 0;
-    if (dalloc(&c->d_press, need)) return PLUM_ERR_CUDA;
-    c->press_cap = need;
+    if (dalloc(&c->d_press, G.total)) return PLUM_ERR_CUDA;
+    c->press_cap = G.total;
   }
-  launch_slit_pressure(S, c->B, n_pair, n_wall, ms[S.phantom], n_k, P.kunit, c->d_press, n1, n2,
-                       c->s);
+  if (!c->d_gtab64) {
+    const std::vector<double>& g = g64_table();
+    if (dalloc(&c->d_gtab64, g.size())) return PLUM_ERR_CUDA;
+    CK(cudaMemcpyAsync(c->d_gtab64, g.data(), sizeof(double) * g.size(), cudaMemcpyHostToDevice,
+                       c->s));
+  }
+  launch_slit_pressure(S, P, c->B, G, ms[S.phantom], c->d_gtab64, c->d_press, c->s);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(c->h_out, c->d_press + 6 * (size_t)n1 + 3 * (size_t)n2, sizeof(double) * 6,
-                     cudaMemcpyDeviceToHost, c->s));
+  CK(cudaMemcpyAsync(c->h_out, c->d_press + G.out_off, sizeof(double) * 6, cudaMemcpyDeviceToHost,
+                     c->s));
   CK(cudaStreamSynchronize(c->s));
   std::memcpy(out6, c->h_out, sizeof(double) * 6);
   return PLUM_OK;
@@ -2669,8 +2690,7 @@ int plum_batch_set_real_term(plum_batch* b, int table) {
 int plum_batch_real_term(const plum_batch* b) { return b ? b->tune.htab : -1; }
 
 int plum_h64_table(double* out, int cap) {
-  std::vector<double> h((size_t)kH64Bins * kH64Stride);
-  build_h64_table(h.data());
+  const std::vector<double>& h = h64_table();
   for (int i = 0; i < std::min(cap, kH64Bins); i++)
     for (int q = 0; q < kH64Stride; q++) out[(size_t)i * kH64Stride + q] = h[(size_t)i * kH64Stride + q];
   return kH64Bins;

@@ -21,6 +21,7 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 namespace plum {
@@ -59,7 +60,7 @@ struct DevParams {
   double lB, sqrt_alpha, real_cut;
   int real_cell[3];
   int single_image;  // real_cut <= half of every Ewald box length
-  int n_k, kmax[3];
+  int n_k, n_ku, kmax[3];
   int koff[3], kper;  // per-bead table: axis a at koff[a], n = 0..kmax[a]; kper entries
   int kchunk_delta, kchunk_sk;  // beads per table chunk (fits kKTableBytes)
   double kunit[3];   // 2 kPi / ebox[a]
@@ -152,6 +153,17 @@ __host__ __device__ inline bool fix_pairs(const DevParams& P) {
          P.pair_kind == 0 && P.ebox[0] == P.ebox[1] && P.ebox[1] == P.ebox[2];
 }
 
+// Two half-space k-vectors (nx, ny, +nz) and (nx, ny, -nz), nz >= 0, at places
+// kp and km of the k list (-1: not in the k-set, as for nz = 0 or in the
+// nx = ny = 0 column, which has one of the two only). With c = q e^{i(kx x + ky
+// y)} their sums over beads are A + iB and A - iB, A = sum c cos(kz z), B = sum
+// c sin(kz z): four multiply-adds per bead serve both vectors. Units of one
+// (nx, ny) column are consecutive.
+struct alignas(16) KUnit {
+  short nx, ny, nz, pad;
+  int kp, km;
+};
+
 struct DevBuffers {  // all pointers: copied word-wise into shared memory by the batch kernels
   double4_32a* pos;
   double4_32a* trial;
@@ -160,6 +172,7 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   int* chain_ids;
   int* ion_ids;
   short4* kn;
+  KUnit* ku;         // [n_ku] the k list as +-nz pairs
   double* kw;
   double2* sk;
   double2* dsk;      // [2][n_k] double-buffered dS(k)
@@ -205,15 +218,21 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   int4* cell_extra;  // [cell_cap]
 };
 
-// Wall-force pressure of slit systems (kern_pressure.cu, slit_pressure.h):
-// partial-sum block counts for n_items pair + wall items and n_k k vectors
-// (returns the scratch doubles needed), and the three launches; the six sums
-// land at scratch[6 n1 + 3 n2 ..].
+// Wall-force pressure of slit systems (kern_pressure.cu, slit_pressure.h): the
+// six sums land at scratch[out_off ..].
 struct SlitPressParams;
-int slit_partials_count(long long n_items, int n_k, int* n1, int* n2);
-void launch_slit_pressure(const SlitPressParams& S, const DevBuffers& B, long long n_pair,
-                          long long n_wall, int wall_b0, int n_k, const double* kunit,
-                          double* scratch, int n1, int n2, cudaStream_t s);
+// Launch sizes and scratch layout (doubles) of one pressure evaluation.
+struct SlitGrid {
+  // pair kernel: `per` beads from bead0 on per tile, 32-site groups (groups1 of
+  // them the first wall's), n1 = tiles x groups blocks
+  int bead0, per, tiles, sites, groups1, groups, n1;
+  int ktiles, kgroups, n2;              // k kernel: unit tiles x bead groups; blocks of the k sums
+  long long sk_off, part3_off, mask_off, out_off, total;
+};
+SlitGrid slit_grid(const SlitPressParams& S, const DevParams& P, long long n_pair, int bead0);
+void launch_slit_pressure(const SlitPressParams& S, const DevParams& P, const DevBuffers& B,
+                          const SlitGrid& G, int wall_b0, const double* gtab, double* scratch,
+                          cudaStream_t s);
 
 // Launch helpers (kern_energy.cu / kern_moves.cu). All enqueue on `s`.
 int pair_grid();
@@ -316,7 +335,11 @@ void build_h32_table(float4* out, double scale = 1.0, double cut = 0.0);  // kH3
 // stays below 1e-17. u below the table takes erfc / r directly.
 constexpr int kH64ELo = -12, kH64EHi = 5, kH64Per = 32, kH64Stride = 10;
 constexpr int kH64Bins = (kH64EHi - kH64ELo) * kH64Per;
-void build_h64_table(double* out);  // kH64Bins * kH64Stride entries
+const std::vector<double>& h64_table();  // kH64Bins * kH64Stride entries
+// The same bins of g(u) = (h(u) + 2 e^{-u} / sqrt(kPi)) / u, the real-space
+// force: (erfc(sqrt(alpha) r) / r + 2 sqrt(alpha / kPi) e^{-alpha r^2}) / r^2 =
+// alpha^{3/2} g(alpha r^2) (kPi the reference's constant).
+const std::vector<double>& g64_table();
 constexpr int kMinItemPairs = 1024;  // smallest item the slot buffers are sized for
 constexpr int kMinKTile = 64;
 // Pair items of the batched energy change: up to kPairGroup moved beads

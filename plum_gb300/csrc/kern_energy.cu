@@ -26,6 +26,7 @@
 
 #include "engine.h"
 #include "device_common.cuh"
+#include "kspace64.cuh"
 
 namespace plum {
 
@@ -111,29 +112,6 @@ __device__ __forceinline__ void pair64(const DevParams& P, double4_32a a, int ta
       re += P.lB * qq * real_images64(P, x, y, z);
     }
   }
-}
-
-// e^{i n theta} tables for one bead: tab[koff[axis] + n], n = 0..kmax[axis];
-// q folded into the x table.
-__device__ __forceinline__ void build_axis_table(const DevParams& P, double4_32a p,
-                                                 int axis, double2* tab) {
-  double w = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
-  if (axis < P.npbc) w -= P.ebox[axis] * floor(w * P.inv_ebox[axis]);
-  double s, c;
-  sincos(P.kunit[axis] * w, &s, &c);
-  double2 e = axis == 0 ? make_double2(p.w, 0.0) : make_double2(1.0, 0.0);
-  double2* t = tab + P.koff[axis];
-  t[0] = e;
-  for (int n = 1; n <= P.kmax[axis]; n++) {
-    double re = e.x * c - e.y * s;
-    double im = e.x * s + e.y * c;
-    e = make_double2(re, im);
-    t[n] = e;
-  }
-}
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
 // q e^{i k.r} from a bead's tables for k = (nx >= 0, ny, nz).
@@ -779,10 +757,11 @@ void launch_rhoz(const DevParams& P, const DevBuffers& B, double res, int n_bins
 }
 
 
-// The FP64 h(u) table: per bin the degree-8 Chebyshev interpolant of
-// h(u) = erfc(sqrt u) / sqrt u at the 9 Chebyshev nodes of y in [-1/2, 1/2]
-// (u = lo + (y + 1/2) w), in long double, then rewritten in powers of y.
-void build_h64_table(double* out) {
+// An FP64 table over u: per bin the degree-8 Chebyshev interpolant of f at the
+// 9 Chebyshev nodes of y in [-1/2, 1/2] (u = lo + (y + 1/2) w), in long double,
+// then rewritten in powers of y.
+template <class F>
+static std::vector<double> build_table64(F f_of) {
   constexpr int n = 9;
   const long double pi = 3.141592653589793238462643383279503L;
   long double T[n][n] = {};  // T_j(t) coefficients in powers of t
@@ -791,27 +770,48 @@ void build_h64_table(double* out) {
   for (int j = 2; j < n; j++)
     for (int q = 0; q < n; q++)
       T[j][q] = (q ? 2.0L * T[j - 1][q - 1] : 0.0L) - T[j - 2][q];
+  long double tk[n], cs[n][n];  // nodes t = 2 y in [-1, 1], cos(j arccos t)
+  for (int k = 0; k < n; k++) {
+    tk[k] = std::cos(pi * (k + 0.5L) / n);
+    for (int j = 0; j < n; j++) cs[j][k] = std::cos(pi * j * (k + 0.5L) / n);
+  }
+  std::vector<double> out((size_t)kH64Bins * kH64Stride, 0.0);
   int b = 0;
   for (int e = kH64ELo; e < kH64EHi; e++)
     for (int j = 0; j < kH64Per; j++, b++) {
       const long double lo = std::ldexp(1.0L + (long double)j / kH64Per, e);
       const long double w = std::ldexp(1.0L / kH64Per, e);
-      long double f[n], tk[n];
-      for (int k = 0; k < n; k++) {
-        tk[k] = std::cos(pi * (k + 0.5L) / n);  // t = 2 y in [-1, 1]
-        const long double u = lo + (0.5L * tk[k] + 0.5L) * w;
-        const long double r = std::sqrt(u);
-        f[k] = std::erfc(r) / r;
-      }
+      long double f[n];
+      for (int k = 0; k < n; k++) f[k] = f_of(lo + (0.5L * tk[k] + 0.5L) * w);
       long double mono[n] = {};  // powers of y
       for (int jj = 0; jj < n; jj++) {
         long double a = 0.0L;
-        for (int k = 0; k < n; k++) a += f[k] * std::cos(pi * jj * (k + 0.5L) / n);
+        for (int k = 0; k < n; k++) a += f[k] * cs[jj][k];
         a *= (jj ? 2.0L : 1.0L) / n;
         for (int q = 0; q < n; q++) mono[q] += a * T[jj][q] * std::ldexp(1.0L, q);
       }
-      for (int q = 0; q < kH64Stride; q++) out[(size_t)b * kH64Stride + q] = q < n ? (double)mono[q] : 0.0;
+      for (int q = 0; q < n; q++) out[(size_t)b * kH64Stride + q] = (double)mono[q];
     }
+  return out;
+}
+
+// The tables hold constants, so a process makes each once (5,000 long-double
+// erfcs; on aarch64, where long double is done in software, tens of
+// milliseconds that every context used to spend).
+const std::vector<double>& h64_table() {
+  static const std::vector<double> t = build_table64([](long double u) {
+    const long double r = std::sqrt(u);
+    return std::erfc(r) / r;
+  });
+  return t;
+}
+
+const std::vector<double>& g64_table() {
+  static const std::vector<double> t = build_table64([](long double u) {
+    const long double r = std::sqrt(u);
+    return (std::erfc(r) / r + 2.0L / std::sqrt(3.14159265359L) * std::exp(-u)) / u;
+  });
+  return t;
 }
 
 }  // namespace plum

@@ -1,21 +1,30 @@
 // Wall-force pressure of slit systems (ForceField::CalcPressureForceLJELSlit,
 // pressure.cc:404-488) on the device: the per-item arithmetic of
-// slit_pressure.h in three launches.
+// slit_pressure.h in four launches.
 //
-//  k_slit_pairs  (site, bead) pair items -- LJ and real-space Ewald z forces --
-//                then the wall items (the external force of every system
-//                bead), dealt grid-stride; each block writes six partial sums
-//  k_slit_recip  one thread per half-space k vector: the five group structure
-//                factors over all beads (staged through shared memory in tiles
-//                of 256) and the k vector's reciprocal z forces; each block
-//                writes three partial sums
+//  k_slit_pairs  (site, bead) pairs -- LJ and real-space Ewald z forces -- a
+//                thread per bead against a chunk of sites staged in shared
+//                memory, so a bead's molecule, kind and type mix are found once
+//                and not per pair; then the wall force of every system bead;
+//                each block writes six partial sums
+//  k_slit_sk     the five group structure factors over (k unit tile) x (bead
+//                group) blocks from per-axis phase tables, two vectors (+-nz)
+//                per four multiply-adds
+//  k_slit_recip  the bead groups' parts added in order, and the reciprocal z
+//                forces of every k; each block writes three partial sums
 //  k_slit_sum    one block adds the partials in a fixed order: the result is
 //                run-to-run identical
 //
-// Cost: pairs are sites x (beads of the second wall and the system), each
-// with the real-space image loop; the k part is n_k x n_bead sincos, in place
-// of the reference's sites x beads x n_k.
+// Bound: the FP64 pipe (about 75 operations per pair within r_c, 5 per unit
+// and charged bead), spread over every SM. A thread per k over all beads with
+// a sincos each kept 6 of 152 SMs busy for 6.6 ms on a 1,391-vector,
+// 3,200-bead brush; the tables need one sincos per bead and axis. The whole
+// evaluation takes 0.18 ms there (7.1 ms before).
+#include <algorithm>
+
+#include "device_common.cuh"
 #include "engine.h"
+#include "kspace64.cuh"
 #include "slit_pressure.h"
 
 namespace plum {
@@ -42,74 +51,198 @@ __device__ __forceinline__ void block_sums(double* v, double* out) {
   }
 }
 
-__global__ void __launch_bounds__(kSlitThreads)
-    k_slit_pairs(const SlitPressParams S, const double* xyzq, const int* type,
-                 const int* mol_start, long long n_pair, long long n_wall, int wall_b0,
-                 double* part) {
-  double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const long long n = n_pair + n_wall;
-  const long long stride = (long long)gridDim.x * kSlitThreads;
-  for (long long it = (long long)blockIdx.x * kSlitThreads + threadIdx.x; it < n; it += stride) {
-    if (it < n_pair)
-      slit_pair_item(S, xyzq, type, mol_start, it, acc);
-    else
-      slit_wall_item(S, xyzq, type, mol_start, wall_b0 + (int)(it - n_pair), acc);
+// The real-space force factor from the FP64 g(u) table (directly below it).
+struct SlitTab {
+  const double* tab;
+  double alpha, scale;  // scale = alpha^{3/2}
+  __device__ __forceinline__ double operator()(double d2) const {
+    const long long bits = __double_as_longlong(alpha * d2);
+    return bits >= kH64LoBits ? scale * h64_tab(tab, bits) : SlitErfc{alpha}(d2);
   }
-  block_sums<6>(acc, part + 6 * (size_t)blockIdx.x);
+};
+
+// A warp takes 32 sites of one wall (a lane each) against the beads of its
+// block's tile, one at a time: the bead's kind is the same for every lane, and
+// as the sites of a wall share their z, so is the test that drops images
+// beyond r_c along z (half the pairs of a slit wider than r_c). With a bead
+// per lane the lanes' z differ and a warp ran nearly every image: 207 us
+// against 89 us on 128 sites x 3,200 beads (with the force's one table load in
+// place of an exponential, an erfc and two divisions).
+// Block (x, y): beads bead0 + x per .. of 32-site group y. The second wall's
+// sites meet system beads only (pressure.cc:419-455).
+__global__ void __launch_bounds__(kSlitThreads)
+    k_slit_pairs(const SlitPressParams S, const DevBuffers B, SlitGrid G, int wall_b0,
+                 const double* __restrict__ gtab, double* part) {
+  __shared__ double s_b[kSlitThreads][4];
+  __shared__ int s_kid[kSlitThreads], s_t[kSlitThreads];
+  __shared__ SlitMix s_mix[kSlitMaxTypes][kSlitMaxTypes];
+  for (int i = threadIdx.x; i < S.n_type * S.n_type; i += kSlitThreads)
+    s_mix[i / S.n_type][i % S.n_type] = slit_mix(S, i / S.n_type, i % S.n_type);
+  double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const int c0 = G.bead0 + blockIdx.x * G.per, cn = min(G.per, S.n_bead - c0);
+  if ((int)threadIdx.x < cn) {
+    const int b = c0 + threadIdx.x;
+    const double4_32a p = B.pos[b];
+    s_b[threadIdx.x][0] = p.x, s_b[threadIdx.x][1] = p.y;
+    s_b[threadIdx.x][2] = p.z, s_b[threadIdx.x][3] = p.w;
+    s_t[threadIdx.x] = B.type[b];
+    const int j = slit_mol_of(B.mol_start, S.n_mol, b);
+    const int kid = j >= S.phantom ? (B.mol_start[j + 1] - B.mol_start[j] > 1 ? 1 : 0) : 2;
+    s_kid[threadIdx.x] = kid;
+    if (blockIdx.y == 0 && S.use_ext && b >= wall_b0)
+      slit_add(acc, 0, kid, 0.5 * slit_wall_force(S, p.z, B.type[b]));
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, half = S.phantom / 2;
+  const bool second = (int)blockIdx.y >= G.groups1;
+  const int w = (second ? half + 32 * ((int)blockIdx.y - G.groups1) : 32 * (int)blockIdx.y) + lane;
+  if (w < G.sites && (second || w < half)) {
+    const double4_32a p = B.pos[B.mol_start[w]];
+    const double pw[4] = {p.x, p.y, p.z, p.w};
+    const int tw = B.type[B.mol_start[w]];
+    const SlitTab term{gtab, S.alpha, S.alpha * sqrt(S.alpha)};
+    for (int i = threadIdx.x >> 5; i < cn; i += kSlitThreads / 32) {
+      const int kid = s_kid[i];
+      if (second && kid == 2) continue;
+      double v[2] = {0.0, 0.0};
+      slit_site_force(S, pw, s_b[i], s_mix[s_t[i]][tw], term, v);
+      const double C = kid == 2 ? -1.0 : (second ? 0.5 : -0.5);
+      slit_add(acc, 0, kid, C * v[0]);
+      slit_add(acc, 3, kid, C * v[1]);
+    }
+  }
+  block_sums<6>(acc, part + 6 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x));
 }
 
-__global__ void __launch_bounds__(kSlitThreads)
-    k_slit_recip(const SlitPressParams S, const double* xyzq, const int* mol_start,
-                 const short4* kn, const double* kw, int n_k, double3 kunit, double* part) {
-  __shared__ double4_32a s_p[kSlitThreads];
-  __shared__ int s_g[kSlitThreads];
-  const int k = blockIdx.x * kSlitThreads + threadIdx.x;
-  const bool on = k < n_k;
-  double kx = 0.0, ky = 0.0, kz = 0.0, w = 0.0;
-  if (on) {
-    const short4 v = kn[k];
-    kx = v.x * kunit.x;
-    ky = v.y * kunit.y;
-    kz = v.z * kunit.z;
-    w = kw[k];
-  }
-  double re[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, im[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int t0 = 0; t0 < S.n_bead; t0 += kSlitThreads) {
-    const int b = t0 + threadIdx.x;
-    __syncthreads();  // the previous tile is consumed
-    if (b < S.n_bead) {
-      const double* p = xyzq + 4 * (size_t)b;
-      double x = p[0], y = p[1], z = p[2];
-      // the periodic axes into the primary cell (e^{i k.r} is periodic there)
-      if (S.npbc > 0) x -= S.ebox[0] * floor(x / S.ebox[0]);
-      if (S.npbc > 1) y -= S.ebox[1] * floor(y / S.ebox[1]);
-      if (S.npbc > 2) z -= S.ebox[2] * floor(z / S.ebox[2]);
-      s_p[threadIdx.x] = make_double4_32a(x, y, z, p[3]);
-      s_g[threadIdx.x] = p[3] != 0.0 ? slit_bead_groups(S, mol_start, b) : 0;
-    } else {
-      s_g[threadIdx.x] = 0;
-    }
-    __syncthreads();
-    const int nt = min(kSlitThreads, S.n_bead - t0);
-    if (on)
-      for (int u = 0; u < nt; u++) {
-        const int g = s_g[u];  // the same for every thread: no divergence
-        if (!g) continue;
-        const double4_32a p = s_p[u];
-        double s, c;
-        sincos(kx * p.x + ky * p.y + kz * p.z, &s, &c);
-        s *= p.w;
-        c *= p.w;
+// The group sums (KUnit's A, B) of kSlitPer units per thread over one part of
+// the beads, written as S(k) parts [bead part][5][n_k], and which groups the
+// part has (mask[bead part]; the other groups' slots are neither written nor
+// read). A bead's group is the same for every thread and beads of a kind are
+// consecutive, so one pair of sums runs until the group changes and is then
+// added to the group's slots: five predicated sums per unit kept the FP64 pipe
+// on four idle ones (21 operations per unit and bead instead of 5, 131 us
+// against 52 us). A block takes 768 units, so that a usual brush's k-set
+// is one tile and each bead's phase tables are built once; the tables' tasks
+// run axis by axis, so that a warp's lanes share the length of their recursion.
+constexpr int kSlitPer = 2;
+constexpr int kSlitSkThreads = 384;
+
+__global__ void __launch_bounds__(kSlitSkThreads, 1)
+    k_slit_sk(const SlitPressParams S, const DevParams P, const DevBuffers B, int groups,
+              double2* part, int* mask) {
+  extern __shared__ __align__(32) unsigned char smem[];
+  double2* tabs = reinterpret_cast<double2*>(smem);
+  __shared__ int s_g[32];
+  const int per_g = (S.n_bead + groups - 1) / groups;
+  const int b0 = blockIdx.y * per_g, b1 = min(S.n_bead, b0 + per_g);
+  KUnit un[kSlitPer];
+  bool mine[kSlitPer], col[kSlitPer];
+  double2 A[kSlitPer], Bs[kSlitPer];
 #pragma unroll
-        for (int q = 0; q < 5; q++)
-          if (g >> q & 1) {
-            re[q] += c;
-            im[q] += s;
-          }
-      }
+  for (int q = 0; q < kSlitPer; q++) {
+    const int u = (blockIdx.x * kSlitSkThreads + threadIdx.x) * kSlitPer + q;
+    mine[q] = u < P.n_ku;
+    un[q] = mine[q] ? B.ku[u] : KUnit{0, 0, 0, 0, -1, -1};
+    col[q] = q == 0 || un[q].nx != un[q - 1].nx || un[q].ny != un[q - 1].ny;
+    A[q] = Bs[q] = make_double2(0.0, 0.0);
   }
+  int run = 0, seen = 0;  // the current beads' groups, the groups written so far
+  double2* const out = part + (size_t)blockIdx.y * 5 * P.n_k;
+  auto flush = [&]() {
+    if (run == 0) return;
+#pragma unroll
+    for (int q = 0; q < kSlitPer; q++) {
+      const double2 v[2] = {unit_plus(A[q], Bs[q]), unit_minus(A[q], Bs[q])};
+      const int at[2] = {un[q].kp, un[q].km};
+      for (int r = 0; r < 5; r++)
+        if (run >> r & 1)
+          for (int h = 0; h < 2; h++)
+            if (at[h] >= 0) {
+              double2* o = out + (size_t)r * P.n_k + at[h];
+              const double2 old = seen >> r & 1 ? *o : make_double2(0.0, 0.0);
+              *o = make_double2(old.x + v[h].x, old.y + v[h].y);
+            }
+      A[q] = Bs[q] = make_double2(0.0, 0.0);
+    }
+    seen |= run;
+  };
+  for (int c0 = b0; c0 < b1; c0 += P.kchunk_sk) {
+    const int cnt = min(P.kchunk_sk, b1 - c0);
+    __syncthreads();  // the previous chunk is consumed
+    if (threadIdx.x < cnt)
+      s_g[threadIdx.x] =
+          B.pos[c0 + threadIdx.x].w != 0.0 ? slit_bead_groups(S, B.mol_start, c0 + threadIdx.x) : 0;
+    for (int t = threadIdx.x; t < 3 * 32; t += kSlitSkThreads)
+      if ((t & 31) < cnt)
+        build_axis_table(P, B.pos[c0 + (t & 31)], t >> 5, tabs + (t & 31) * P.kper);
+    __syncthreads();
+    for (int i = 0; i < cnt; i++) {
+      const int g = s_g[i];
+      if (!g) continue;
+      if (g != run) {
+        flush();
+        run = g;
+      }
+      const double2* tab = tabs + i * P.kper;
+      double2 xy = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < kSlitPer; q++) {
+        if (!mine[q]) continue;
+        if (col[q]) xy = unit_xy(P, tab, un[q].nx, un[q].ny);
+        unit_add(xy, tab[P.koff[2] + un[q].nz], A[q], Bs[q]);
+      }
+    }
+  }
+  flush();
+  if (blockIdx.x == 0 && threadIdx.x == 0) mask[blockIdx.y] = seen;
+}
+
+constexpr int kSlitK = 8;  // k vectors per block, 32 threads each
+
+__global__ void __launch_bounds__(kSlitThreads)
+    k_slit_recip(const SlitPressParams S, const DevParams P, const DevBuffers B, int groups,
+                 const double2* sk_part, const int* mask, double* part) {
+  __shared__ double2 s_sum[kSlitThreads / kSlitK][5][kSlitK];
+  const int l = threadIdx.x % kSlitK, sl = threadIdx.x / kSlitK;
+  const int k = blockIdx.x * kSlitK + l;
+  const bool on = k < P.n_k;
+  double2 s[5];
+#pragma unroll
+  for (int r = 0; r < 5; r++) s[r] = make_double2(0.0, 0.0);
+  if (on)
+    for (int g = sl; g < groups; g += kSlitThreads / kSlitK) {
+      const int m = mask[g];
+#pragma unroll
+      for (int r = 0; r < 5; r++)
+        if (m >> r & 1) {
+          const double2 v = sk_part[((size_t)g * 5 + r) * P.n_k + k];
+          s[r].x += v.x;
+          s[r].y += v.y;
+        }
+    }
+#pragma unroll
+  for (int r = 0; r < 5; r++) s_sum[sl][r][l] = s[r];
+  __syncthreads();
+  // the 32 slices of each (group, vector), added in order by a thread each
+  if (threadIdx.x < 5 * kSlitK) {
+    const int r = threadIdx.x / kSlitK, v = threadIdx.x % kSlitK;
+    double2 t = s_sum[0][r][v];
+    for (int q = 1; q < kSlitThreads / kSlitK; q++) {
+      t.x += s_sum[q][r][v].x;
+      t.y += s_sum[q][r][v].y;
+    }
+    s_sum[0][r][v] = t;
+  }
+  __syncthreads();
   double o[3] = {0.0, 0.0, 0.0};
-  if (on) slit_k_terms(kz, w, re, im, o);
+  if (on && sl == 0) {
+    double re[5], im[5];
+    for (int r = 0; r < 5; r++) {
+      re[r] = s_sum[0][r][l].x;
+      im[r] = s_sum[0][r][l].y;
+    }
+    slit_k_terms(B.kn[k].z * P.kunit[2], B.kw[k], re, im, o);
+  }
   const double pre = slit_recip_prefactor(S);
   for (int q = 0; q < 3; q++) o[q] *= pre;
   block_sums<3>(o, part + 3 * (size_t)blockIdx.x);
@@ -130,27 +263,55 @@ __global__ void __launch_bounds__(kSlitThreads)
 
 }  // namespace
 
-int slit_partials_count(long long n_items, int n_k, int* n1, int* n2) {
-  const long long blocks = (n_items + kSlitThreads - 1) / kSlitThreads;
-  *n1 = (int)(blocks < 1 ? 1 : (blocks > 152 * 8 ? 152 * 8 : blocks));
-  *n2 = (n_k + kSlitThreads - 1) / kSlitThreads;
-  return 6 * *n1 + 3 * *n2 + 6;
+// Pair kernel: bead tiles x 32-site groups of each wall, about two blocks per
+// SM (a tile is a multiple of the block's eight warps). k kernel: unit tiles x
+// bead groups, one block per SM; fewer groups where that would leave a group
+// under 8 beads (its tables then cost more than its sums).
+SlitGrid slit_grid(const SlitPressParams& S, const DevParams& P, long long n_pair, int bead0) {
+  SlitGrid G;
+  G.bead0 = bead0;
+  G.sites = n_pair > 0 ? S.phantom : 0;
+  G.groups1 = (G.sites / 2 + 31) / 32;
+  G.groups = std::max(1, G.groups1 + (G.sites - G.sites / 2 + 31) / 32);
+  const int nb = std::max(1, S.n_bead - bead0);
+  const long long per = ((long long)nb * G.groups + pair_grid() - 1) / pair_grid();
+  G.per = (int)std::min<long long>(kSlitThreads, (per + 7) / 8 * 8);
+  G.tiles = (nb + G.per - 1) / G.per;
+  G.n1 = G.tiles * G.groups;
+  G.ktiles = G.kgroups = G.n2 = 0;
+  if (S.use_ewald && S.phantom > 0 && P.n_k > 0) {
+    const int units = kSlitSkThreads * kSlitPer;
+    G.ktiles = (P.n_ku + units - 1) / units;
+    G.kgroups = std::max(1, std::min((S.n_bead + 7) / 8, pair_grid() / 2 / G.ktiles));
+    G.n2 = (P.n_k + kSlitK - 1) / kSlitK;
+  }
+  G.sk_off = 6LL * G.n1;  // even: the S(k) parts are double2
+  G.part3_off = G.sk_off + 10LL * G.kgroups * P.n_k;
+  G.mask_off = G.part3_off + 3LL * G.n2;
+  G.out_off = G.mask_off + G.kgroups;  // room for kgroups ints
+  G.total = G.out_off + 6;
+  return G;
 }
 
-void launch_slit_pressure(const SlitPressParams& S, const DevBuffers& B, long long n_pair,
-                          long long n_wall, int wall_b0, int n_k, const double* kunit,
-                          double* scratch, int n1, int n2, cudaStream_t s) {
-  const double* xyzq = reinterpret_cast<const double*>(B.pos);
-  double* part = scratch;
-  double* part3 = scratch + 6 * (size_t)n1;
-  double* out6 = part3 + 3 * (size_t)n2;
-  k_slit_pairs<<<n1, kSlitThreads, 0, s>>>(S, xyzq, B.type, B.mol_start, n_pair, n_wall,
-                                           wall_b0, part);
-  if (n2 > 0)
-    k_slit_recip<<<n2, kSlitThreads, 0, s>>>(S, xyzq, B.mol_start, B.kn, B.kw, n_k,
-                                             make_double3(kunit[0], kunit[1], kunit[2]),
-                                             part3);
-  k_slit_sum<<<1, kSlitThreads, 0, s>>>(part, n1, part3, n2, out6);
+void launch_slit_pressure(const SlitPressParams& S, const DevParams& P, const DevBuffers& B,
+                          const SlitGrid& G, int wall_b0, const double* gtab, double* scratch,
+                          cudaStream_t s) {
+  k_slit_pairs<<<dim3(G.tiles, G.groups), kSlitThreads, 0, s>>>(S, B, G, wall_b0, gtab, scratch);
+  if (G.n2 > 0) {
+    static bool attr = false;
+    if (!attr) {
+      cudaFuncSetAttribute(k_slit_sk, cudaFuncAttributeMaxDynamicSharedMemorySize, kKTableBytes);
+      attr = true;
+    }
+    double2* sk = reinterpret_cast<double2*>(scratch + G.sk_off);
+    int* mask = reinterpret_cast<int*>(scratch + G.mask_off);
+    k_slit_sk<<<dim3(G.ktiles, G.kgroups), kSlitSkThreads,
+                (size_t)P.kchunk_sk * P.kper * sizeof(double2), s>>>(S, P, B, G.kgroups, sk, mask);
+    k_slit_recip<<<G.n2, kSlitThreads, 0, s>>>(S, P, B, G.kgroups, sk, mask,
+                                               scratch + G.part3_off);
+  }
+  k_slit_sum<<<1, kSlitThreads, 0, s>>>(scratch, G.n1, scratch + G.part3_off, G.n2,
+                                        scratch + G.out_off);
 }
 
 }  // namespace plum

@@ -76,59 +76,100 @@ PLUM_HD int slit_mol_of(const int* mol_start, int n_mol, int b) {
 }
 
 // Nearest-image component on a periodic axis (GetDistVector, misc.cc:43-56).
-PLUM_HD double slit_wrap(double d, double L) { return d - L * round(d / L); }
+PLUM_HD double slit_wrap(double d, double L) { return d - L * rint(d * (1.0 / L)); }
 
-// PotentialTruncatedLJ::PairForce (potential_truncated_lj.cc:87-122) at
-// distance r between types ta and tb. Beyond a positive cut-off it is the
-// cut-off's r^-6 term evaluated at r, as the reference writes it. The
-// reference's own function tests an uninitialised local against -1 first
-// (potential_truncated_lj.cc:95-100); this follows the evident intent, the
-// overlap value only for r <= 0. Hard spheres exert none
-// (potential_hard_sphere.cc:51-56).
-PLUM_HD double slit_lj_force(const SlitPressParams& S, int ta, int tb, double r) {
-  if (S.pair_kind == 1) return 0.0;
+// PotentialTruncatedLJ::PairForce (potential_truncated_lj.cc:87-122) between
+// two types. Beyond a positive cut-off it is the cut-off's r^-6 term evaluated
+// at r, as the reference writes it. The reference's own function tests an
+// uninitialised local against -1 first (potential_truncated_lj.cc:95-100);
+// this follows the evident intent, the overlap value only for r <= 0. Hard
+// spheres exert none (potential_hard_sphere.cc:51-56). The pressure needs its
+// z component (r_z / r) F(r) alone: F's powers and the direction then take
+// 1 / r^2 only, so a pair costs one division and no square root. SlitMix holds
+// what depends on the two types.
+struct SlitMix {
+  double sig2, eps4, rc2, irc2;
+};
+PLUM_HD SlitMix slit_mix(const SlitPressParams& S, int ta, int tb) {
+  SlitMix M;
   const double sigma = (S.lj_sig[ta] + S.lj_sig[tb]) / 2;
-  const double eps = sqrt(S.lj_eps[ta] * S.lj_eps[tb]);
-  if (r <= 0) return kSlitVeryLarge;
-  double x;
-  if (S.lj_cut < 0) {
-    if (!(r < kSlit216 * sigma)) return 0.0;
-    x = sigma / r;
-  } else {
-    x = sigma / (r < S.lj_cut ? r : S.lj_cut);
-  }
-  const double x2 = x * x;
-  const double r6 = x2 * x2 * x2;
-  return 4 * eps * (r6 * r6 * 12 / r - r6 * 6 / r);
+  const double rc = S.lj_cut < 0 ? kSlit216 * sigma : S.lj_cut;
+  M.sig2 = sigma * sigma;
+  M.eps4 = 4 * sqrt(S.lj_eps[ta] * S.lj_eps[tb]);
+  M.rc2 = rc * rc;
+  M.irc2 = 1 / M.rc2;
+  return M;
 }
+PLUM_HD double slit_lj_z(const SlitPressParams& S, const SlitMix& M, double rz, double r2) {
+  if (!(r2 > 0)) {  // coincident: the undefined direction, as r_z / r has it
+    const double r = sqrt(r2);
+    return (rz / r) * (S.pair_kind == 1 ? 0.0 : kSlitVeryLarge);
+  }
+  if (S.pair_kind == 1 || (S.lj_cut < 0 && !(r2 < M.rc2))) return 0.0;
+  const double ir2 = 1 / r2;
+  const double x2 = M.sig2 * (r2 < M.rc2 ? ir2 : M.irc2);
+  const double r6 = x2 * x2 * x2;
+  return M.eps4 * (r6 * r6 * 12 - r6 * 6) * (rz * ir2);
+}
+
+// (erfc(sqrt(alpha) d) / d + 2 sqrt(alpha / kPi) e^{-alpha d^2}) / d^2 at d^2 >
+// 0; the device passes its table's.
+struct SlitErfc {
+  double alpha;
+  PLUM_HD double operator()(double d2) const {
+    const double d = sqrt(d2);
+    return (erfc(sqrt(alpha) * d) / d + 2 * sqrt(alpha / kSlitPi) * exp(-alpha * d2)) / d2;
+  }
+};
 
 // PotentialEwaldCoul::PairForceZReal (potential_ewald_coul.cc:261-293): z
 // force on a wall charge from a bead at (rx, ry, rz) = r_site - r_bead
 // (nearest image on the periodic axes of the Ewald box), summed over the
-// image cells within the real-space cut-off. qq = q_site q_bead.
+// image cells within the real-space cut-off. qq = q_site q_bead; term: see
+// SlitErfc.
+template <class Term>
 PLUM_HD double slit_ew_real_z(const SlitPressParams& S, double rx, double ry, double rz,
-                              double qq) {
+                              double qq, const Term& term) {
   if (qq == 0) return 0.0;
-  const double pre = S.lB * qq;
-  const double pre2 = 2 * sqrt(S.alpha / kSlitPi);
-  const double sa = sqrt(S.alpha), rc = S.real_cut;
+  const double rc = S.real_cut, rc2 = rc * rc;
   double f = 0.0;
-  for (int a = -S.real_cell[0]; a <= S.real_cell[0]; a++) {
-    const double x = rx + a * S.ebox[0];
-    if (fabs(x) > rc) continue;  // no image of this shift is inside the cut-off
+  if (S.real_cell[0] == 1 && S.real_cell[1] == 1 && S.real_cell[2] == 1) {
+    // r_c <= L on every axis: of an axis' images only the nearest to zero and
+    // the one a box length to its other side can lie within r_c
+    const double x1 = rx - copysign(S.ebox[0], rx), y1 = ry - copysign(S.ebox[1], ry);
+    const double z1 = rz - copysign(S.ebox[2], rz);
+    const bool mx = fabs(x1) <= rc, my = fabs(y1) <= rc, mz = fabs(z1) <= rc;
+    for (int c = 0; c < 2; c++) {
+      const double z = c ? z1 : rz;
+      if (c ? !mz : fabs(rz) > rc) continue;
+      for (int b = 0; b < 2; b++) {
+        if (b && !my) continue;
+        const double y = b ? y1 : ry, yz = y * y + z * z;
+        for (int a = 0; a < 2; a++) {
+          if (a && !mx) continue;
+          const double x = a ? x1 : rx;
+          const double d2 = x * x + yz;
+          if (d2 > 0 && d2 <= rc2) f += term(d2) * z;
+        }
+      }
+    }
+    return S.lB * qq * f;
+  }
+  for (int c = -S.real_cell[2]; c <= S.real_cell[2]; c++) {
+    const double z = rz + c * S.ebox[2];
+    if (fabs(z) > rc) continue;  // no image of this shift is inside the cut-off
     for (int b = -S.real_cell[1]; b <= S.real_cell[1]; b++) {
       const double y = ry + b * S.ebox[1];
       if (fabs(y) > rc) continue;
-      for (int c = -S.real_cell[2]; c <= S.real_cell[2]; c++) {
-        const double z = rz + c * S.ebox[2];
-        if (fabs(z) > rc) continue;
-        const double d = sqrt(x * x + y * y + z * z);
-        if (d > 0 && d <= rc)
-          f += pre * ((pre2 * exp(-S.alpha * d * d)) + (erfc(sa * d) / d)) * z / (d * d);
+      for (int a = -S.real_cell[0]; a <= S.real_cell[0]; a++) {
+        const double x = rx + a * S.ebox[0];
+        if (fabs(x) > rc) continue;
+        const double d2 = x * x + y * y + z * z;
+        if (d2 > 0 && d2 <= rc2) f += term(d2) * z;
       }
     }
   }
-  return f;
+  return S.lB * qq * f;
 }
 
 // One 9-3 wall term of the force: k93 eps ((s/h)^6 6/h - (s/h)^3 3/h) with
@@ -197,6 +238,24 @@ PLUM_HD long long slit_wall_items(const SlitPressParams& S, const int* mol_start
   return S.n_bead - mol_start[S.phantom];
 }
 
+// LJ (v[0]) and real-space Ewald (v[1]) z force of one (site, bead) pair;
+// pw, pb: x, y, z, q.
+template <class Term>
+PLUM_HD void slit_site_force(const SlitPressParams& S, const double* pw, const double* pb,
+                             const SlitMix& M, const Term& term, double* v) {
+  // the Ewald box differs from the box along z only (its padding)
+  const double x = slit_wrap(pw[0] - pb[0], S.box[0]), y = slit_wrap(pw[1] - pb[1], S.box[1]);
+  const double dz = pw[2] - pb[2];
+  if (S.use_pair) {
+    const double z = S.npbc > 2 ? slit_wrap(dz, S.box[2]) : dz;
+    v[0] = slit_lj_z(S, M, z, x * x + y * y + z * z);
+  }
+  if (S.use_ewald) {
+    const double z = S.npbc > 2 ? slit_wrap(dz, S.ebox[2]) : dz;
+    v[1] = slit_ew_real_z(S, x, y, z, pw[3] * pb[3], term);
+  }
+}
+
 // Pair item `item` (site i = item / nb, bead b0 + item % nb): adds its LJ and
 // real-space z forces, weighted as pressure.cc:421-428 weights them, into
 // acc[0..2] (LJ: ion, polymer, wall-wall) and acc[3..5] (Ewald real space).
@@ -215,23 +274,10 @@ PLUM_HD void slit_pair_item(const SlitPressParams& S, const double* xyzq, const 
   const int w = mol_start[i];
   const double* pw = xyzq + 4 * (long long)w;
   const double* pb = xyzq + 4 * (long long)b;
-  if (S.use_pair) {
-    double r[3];
-    for (int a = 0; a < 3; a++) {
-      const double d = pw[a] - pb[a];
-      r[a] = a < S.npbc ? slit_wrap(d, S.box[a]) : d;
-    }
-    const double rr = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-    slit_add(acc, 0, kid, C * (r[2] / rr) * slit_lj_force(S, type[b], type[w], rr));
-  }
-  if (S.use_ewald) {
-    double r[3];
-    for (int a = 0; a < 3; a++) {
-      const double d = pw[a] - pb[a];
-      r[a] = a < S.npbc ? slit_wrap(d, S.ebox[a]) : d;
-    }
-    slit_add(acc, 3, kid, C * slit_ew_real_z(S, r[0], r[1], r[2], pw[3] * pb[3]));
-  }
+  double v[2] = {0.0, 0.0};
+  slit_site_force(S, pw, pb, slit_mix(S, type[b], type[w]), SlitErfc{S.alpha}, v);
+  slit_add(acc, 0, kid, C * v[0]);
+  slit_add(acc, 3, kid, C * v[1]);
 }
 
 // Wall item for system bead b: half its external force on the wall into
