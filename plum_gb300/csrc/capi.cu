@@ -7,6 +7,7 @@
 #include <array>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -67,6 +68,7 @@ struct plum_ctx {
   double* d_obs_per = nullptr;  // [n_mol * 5] per-molecule Rg / Ree sums
   double* d_press = nullptr;    // wall-force pressure partials and sums
   double* d_gtab64 = nullptr;   // FP64 g(u) table of its real-space force
+  unsigned char* d_fx = nullptr;  // the integer pair form's table
   long long press_cap = 0;
   unsigned* d_rhoz = nullptr;   // [3 * rhoz_bins] rho(z) counts
   int rhoz_bins = 0;
@@ -154,6 +156,7 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
   P.sqrt_alpha = std::sqrt(in.alpha);
   P.alpha = in.alpha;
   P.kpref = in.lB / (kPiRef * vol) * (4 * kPiRef * kPiRef);
+  P.turn_eps = (double)((kPiRef / 3.141592653589793238462643383279503L - 1.0L) * 0x1p64L);
   P.self_coef = -in.lB * std::sqrt(in.alpha / kPiRef);
   P.dip_coef = in.lB * 2 * kPiRef / (vol / 1.0);
   P.dipole = in.dipole;
@@ -195,8 +198,14 @@ int dalloc(T** p, size_t n) {
 // compared first: drift[0..3] = running - recomputed per term, drift[4] =
 // the largest |total drift| seen (kept across calls), drift[5] += 1.
 __global__ void k_assemble_total(const DevParams P, const DevBuffers B, const double* tot_part,
-                                 int n_part, const double* misc, double* out, double* drift) {
-  __shared__ double red[8];
+                                 int n_part, const double* misc_part, double* out,
+                                 double* drift) {
+  __shared__ double red[32], misc[5];
+  if (threadIdx.x < 5) {
+    double t = 0.0;
+    for (int b = 0; b < kMiscBlocks; b++) t += misc_part[5 * b + threadIdx.x];
+    misc[threadIdx.x] = t;
+  }
   double lj = 0.0, re = 0.0, ek = 0.0;
   for (int i = threadIdx.x; i < n_part; i += blockDim.x) {
     lj += tot_part[2 * i];
@@ -273,9 +282,9 @@ int enqueue_total(plum_ctx* c, cudaStream_t s, double* drift) {
     launch_sk_full64(P, c->B, c->d_sk_part, s);
     k += 2;
   }
-  launch_misc_total64(P, c->B, c->d_out + 16, s);
-  k_assemble_total<<<1, 256, 0, s>>>(P, c->B, c->d_tot_part, c->n_tot_part, c->d_out + 16,
-                                     c->d_out, drift);
+  launch_misc_total64(P, c->B, c->d_out + 64, s);
+  k_assemble_total<<<1, 1024, 0, s>>>(P, c->B, c->d_tot_part, c->n_tot_part, c->d_out + 64,
+                                      c->d_out, drift);
   k += 2;
   if (c->form == PLUM_FORM_FP32) {
     launch_fix_all(P, c->B, s);
@@ -656,17 +665,14 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   rc |= dalloc(&B.ftrial, c->max_len);
   {
     int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
-    rc |= dalloc(&B.dsk_part, (size_t)groups * std::max(1, P.n_k));
     rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
     rc |= dalloc(&B.ktile_count, ktile_count(P));
     rc |= dalloc(&B.kpartial, ktile_count(P));
   }
   rc |= dalloc(&B.bond_mol, in.n_mol);
   rc |= dalloc(&B.state, 1);
-  c->n_tot_part = total_partials_count(P);
-  rc |= dalloc(&c->d_tot_part, 2 * (size_t)c->n_tot_part);
   rc |= dalloc(&c->d_sk_part, (size_t)sk_full_groups(P) * std::max(1, P.n_k));
-  rc |= dalloc(&c->d_out, 64);
+  rc |= dalloc(&c->d_out, 64 + 5 * kMiscBlocks);
   rc |= dalloc(&c->d_obs_per, 5 * (size_t)std::max(1, in.n_mol));
   c->rhoz_bins = (int)std::ceil(in.box[2] / kRhoZRes);
   rc |= dalloc(&c->d_rhoz, 3 * (size_t)std::max(1, c->rhoz_bins));
@@ -682,8 +688,31 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
       P.htab64 = c->d_htab64;
     }
   }
-  // the plain form's 64-bit position mirror for its fixed-point pair loop
-  if (form == PLUM_FORM_FP64 && fix_pairs(P)) rc |= dalloc(&c->B.fpos64, nb);
+  // the integer pair form's table, for every form's from-scratch energies
+  {
+    P.fx = FixTab{};
+    const bool cubic = P.ebox[0] == P.ebox[1] && P.ebox[1] == P.ebox[2];
+    std::shared_ptr<const FixTable> t;
+    if (P.use_ewald && P.same_wrap && P.npbc == 3 && P.pair_kind == 0 && cubic)
+      t = fix_table(FixSystem{P.alpha, P.ebox[0], P.real_cut, P.use_pair ? P.lj_max2 : 0.0});
+    if (t && !rc) {
+      const size_t n = t->c01.size(), b16 = n * sizeof(FixPair64), b8 = n * sizeof(FixPair32);
+      rc |= dalloc(&c->d_fx, 2 * b16 + b8);
+      if (!rc) {
+        cudaMemcpy(c->d_fx, t->c01.data(), b16, cudaMemcpyHostToDevice);
+        cudaMemcpy(c->d_fx + b16, t->c23.data(), b16, cudaMemcpyHostToDevice);
+        cudaMemcpy(c->d_fx + 2 * b16, t->c45.data(), b8, cudaMemcpyHostToDevice);
+        P.fx = t->t;
+        P.fx.c01 = reinterpret_cast<const FixPair64*>(c->d_fx);
+        P.fx.c23 = reinterpret_cast<const FixPair64*>(c->d_fx + b16);
+        P.fx.c45 = reinterpret_cast<const FixPair32*>(c->d_fx + 2 * b16);
+      }
+    }
+  }
+  // the plain form's 64-bit position mirror for its integer pair loop
+  if (form == PLUM_FORM_FP64 && P.fx.mode) rc |= dalloc(&c->B.fpos64, nb);
+  c->n_tot_part = total_partials_count(P);
+  rc |= dalloc(&c->d_tot_part, 2 * (size_t)c->n_tot_part);
   // the precision form's real-space term from the h(u) table where the
   // cut-off lies inside it (alpha r_c^2 < 2^kH32EHi)
   P.htab = nullptr;
@@ -748,13 +777,14 @@ int plum_ctx_destroy(plum_ctx* c) {
   void* ptrs[] = {c->B.pos,      c->B.trial,   c->B.type,  c->B.mol_start, c->B.chain_ids,
                   c->B.ion_ids,  c->B.kn,      c->B.kw,    c->B.sk,        c->B.dsk,
                   c->B.partial,  c->B.bond_mol, c->B.state, c->d_tot_part,  c->d_out,
-                  c->B.dsk_part, c->B.ktile_count, c->B.kpartial, c->B.fpos, c->B.done_count,
+                  c->B.ktile_count, c->B.kpartial, c->B.fpos, c->B.done_count,
                   c->B.fq,       c->B.ftrial,  c->B.dsk_part32, c->cb_b, c->cb_c, c->cb_so,
                   c->cb_part,    c->cb_u,      c->d_obs_per, c->d_rhoz, c->desc_acc,
                   c->d_rp1,      c->d_rb1,     c->desc_fine, c->cb_part32, c->cb_ticket,
                   c->d_stream,   c->d_mt,      c->d_log_type, c->d_log_acc, c->d_log_e,
                   c->d_press,    c->d_sk_part, c->d_log_de, c->d_htab, c->d_htab64,
-                  c->B.fpos64,   c->B.ku,      c->d_gtab64};
+                  c->B.fpos64,   c->B.ku,      c->d_gtab64,
+                  c->d_fx};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
@@ -886,7 +916,7 @@ int rebuild_system(plum_ctx* c) {
   P.n_ion_total = (int)ions.size();
   const bool mirror64 = B.fpos64 != nullptr;
   void* old[] = {B.pos,      B.trial,      B.type,     B.mol_start, B.chain_ids, B.ion_ids,
-                 B.fpos,     B.fq,         B.ftrial,   B.dsk_part,  B.dsk_part32, B.bond_mol,
+                 B.fpos,     B.fq,         B.ftrial,   B.dsk_part32, B.bond_mol,
                  c->d_tot_part, c->d_obs_per, c->cb_b, c->cb_c,    c->cb_part,  c->cb_u,
                  B.fpos64};
   for (void* q : old)
@@ -896,7 +926,6 @@ int rebuild_system(plum_ctx* c) {
   B.type = B.mol_start = B.chain_ids = B.ion_ids = nullptr;
   B.fpos = B.ftrial = nullptr;
   B.fq = nullptr;
-  B.dsk_part = nullptr;
   B.dsk_part32 = nullptr;
   B.bond_mol = nullptr;
   c->d_tot_part = c->d_obs_per = nullptr;
@@ -909,7 +938,6 @@ int rebuild_system(plum_ctx* c) {
            dalloc(&B.ftrial, c->max_len) | dalloc(&B.bond_mol, in.n_mol);
   if (mirror64) rc |= dalloc(&B.fpos64, nb);
   const int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
-  rc |= dalloc(&B.dsk_part, (size_t)groups * std::max(1, P.n_k));
   rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
   c->n_tot_part = total_partials_count(P);
   rc |= dalloc(&c->d_tot_part, 2 * (size_t)c->n_tot_part);

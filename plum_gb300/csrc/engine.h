@@ -13,7 +13,8 @@
 //                           an accepted change is added to sk by the next
 //                           delta kernel)
 //   partial double[grid*4]  per-block partial sums of the pending move
-//   dsk_part double2[groups*n_k], kpartial double[k tiles]: k-space parts
+//   dsk_part32 float2[groups*n_k], kpartial double[k tiles]: the precision
+//                           form's k-space parts
 //   state  DevState         running energies, the pending move, stream cursor
 // Everything here is a few MB even at 20,000 beads and 15,624 k-vectors, so
 // it stays L2-resident across moves; the pair sweeps are FP64/FP32-pipe
@@ -21,8 +22,10 @@
 #pragma once
 
 #include <cstdint>
-#include <vector>
 #include <cuda_runtime.h>
+
+#include "fix_pair.h"
+#include "real_tables.h"
 
 namespace plum {
 
@@ -105,6 +108,10 @@ struct DevParams {
   double alpha;
   int same_wrap;
   double lj_max2;  // largest lj_rc2 over the type pairs in use
+  // the integer pair form (fix_pair.h): LJ + Ewald in a cubic box periodic on
+  // every axis, r_c <= L, one box for both terms; mode 0 where it does not apply
+  FixTab fx;
+  double turn_eps;  // (kPi / pi - 1) 2^64: phases count turns of the reference's 2 kPi
 };
 
 // The pending move: beads [b_lo, b_hi) of molecule `mol` hold trial
@@ -145,14 +152,6 @@ struct DevState {
   int log_n, log_cap;
 };
 
-// The fixed-point pair form of the FP64 kernels (k_delta64, k_total64):
-// LJ + Ewald in a cubic box periodic on every axis, one image (r_c <= L/2),
-// one box for both terms, the FP64 h(u) table.
-__host__ __device__ inline bool fix_pairs(const DevParams& P) {
-  return P.use_ewald && P.htab64 && P.same_wrap && P.npbc == 3 && P.single_image &&
-         P.pair_kind == 0 && P.ebox[0] == P.ebox[1] && P.ebox[1] == P.ebox[2];
-}
-
 // Two half-space k-vectors (nx, ny, +nz) and (nx, ny, -nz), nz >= 0, at places
 // kp and km of the k list (-1: not in the k-set, as for nz = 0 or in the
 // nx = ny = 0 column, which has one of the two only). With c = q e^{i(kx x + ky
@@ -177,7 +176,7 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   double2* sk;
   double2* dsk;      // [2][n_k] double-buffered dS(k)
   double* partial;   // [grid][4]
-  // plain form mirror (fix_pairs systems; null otherwise): 64-bit
+  // plain form mirror (where P.fx applies; null otherwise): 64-bit
   // fixed-point fractions of the box (X, Y, Z) and the charge's bits
   ulonglong4_32a* fpos64;  // [n_bead] current positions
   // precision form mirrors: 32-bit fixed-point fractions of the Ewald box
@@ -185,7 +184,6 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   float* fq;         // [n_bead] charges
   int4* ftrial;      // [max molecule length] trial of the pending move's beads
   float2* dsk_part32;  // [groups][n_k]
-  double2* dsk_part; // [groups][n_k] dS(k) parts of the pending move
   int* ktile_count;  // [k tiles] arrival tickets (reset by the last arrival)
   int* done_count;   // [1] block arrival ticket of the delta kernel
   double* kpartial;  // [k tiles] energy change per k tile
@@ -245,8 +243,8 @@ int total_partials_count(const DevParams& P);
 // the caller (one per context, so contexts on different streams never share it)
 int sk_full_groups(const DevParams& P);
 void launch_sk_full64(const DevParams& P, const DevBuffers& B, double2* part, cudaStream_t s);
-void launch_misc_total64(const DevParams& P, const DevBuffers& B, double* out6,
-                         cudaStream_t s);
+constexpr int kMiscBlocks = 64;  // five sums each
+void launch_misc_total64(const DevParams& P, const DevBuffers& B, double* out, cudaStream_t s);
 
 // Serial step: mode bits
 constexpr int kModeFinish = 1;   // reduce partials, compose dE
@@ -327,19 +325,6 @@ constexpr int kH32ELo = -14, kH32EHi = 5, kH32Per = 32;
 constexpr int kH32Bins = (kH32EHi - kH32ELo) * kH32Per;
 constexpr double kH32Cut = 16.0;
 void build_h32_table(float4* out, double scale = 1.0, double cut = 0.0);  // kH32Bins entries
-// The FP64 table of h(u): kH64Per bins per octave of u for octaves
-// 2^kH64ELo .. 2^(kH64EHi - 1), a degree-8 polynomial in y = f - 1/2 per bin
-// (kH64Stride doubles per bin, the last zero, for 16-byte loads): Chebyshev
-// interpolation of erfcl at 9 nodes in long double, converted to powers of y.
-// About 2e-16 relative below u = 8; above it h < 3e-5 and the absolute error
-// stays below 1e-17. u below the table takes erfc / r directly.
-constexpr int kH64ELo = -12, kH64EHi = 5, kH64Per = 32, kH64Stride = 10;
-constexpr int kH64Bins = (kH64EHi - kH64ELo) * kH64Per;
-const std::vector<double>& h64_table();  // kH64Bins * kH64Stride entries
-// The same bins of g(u) = (h(u) + 2 e^{-u} / sqrt(kPi)) / u, the real-space
-// force: (erfc(sqrt(alpha) r) / r + 2 sqrt(alpha / kPi) e^{-alpha r^2}) / r^2 =
-// alpha^{3/2} g(alpha r^2) (kPi the reference's constant).
-const std::vector<double>& g64_table();
 constexpr int kMinItemPairs = 1024;  // smallest item the slot buffers are sized for
 constexpr int kMinKTile = 64;
 // Pair items of the batched energy change: up to kPairGroup moved beads

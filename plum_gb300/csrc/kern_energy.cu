@@ -6,18 +6,18 @@
 //                             space (potential_ewald_coul.cc:134-164) at trial
 //                             minus current positions; moved x moved pairs once
 //                             (potential_pair.cc:156-175, potential_ewald.cc:436-476)
-//                k items      half-space k tiles x moved-bead groups: dS(k) and
-//                             the |S|^2 change, which equals the reference's
+//                k blocks     dS(k) and the |S|^2 change of a run of k units over
+//                             all moved beads, which equals the reference's
 //                             pairwise PairEnergyRepl sum
 //                             (potential_ewald_coul.cc:198-225) on the same k-set
-//              Every block writes its own partial sums; the serial kernel adds
-//              them in a fixed order, so results are run-to-run identical.
-//  k_total64   all i<j pairs from scratch (tile pairs of 128 x 128)
-//  k_sk64      S(k) from scratch (k tile x bead group partials)
+//              Every block writes its own partial sums; the last one adds them in
+//              a fixed order, so results are run-to-run identical.
+//  k_total64*  all i<j pairs from scratch (tile pairs)
+//  k_sk64      S(k) from scratch (k unit tile x bead group partials)
 //  k_misc64    bonds, walls, self energy, self images, sum q z
 //
 // Phases e^{i k.r} come from per-axis tables e^{i n theta_a}, n = 0..kmax,
-// built by complex recursion from one sincos per bead and axis, with theta_a
+// built by complex recursion from one exponential per bead and axis, with theta_a
 // = 2 kPi w_a / L_a on coordinates wrapped into the primary cell (periodic
 // axes). This replaces the reference's cos(k.r) per pair and k.
 #include <algorithm>
@@ -114,16 +114,6 @@ __device__ __forceinline__ void pair64(const DevParams& P, double4_32a a, int ta
   }
 }
 
-// q e^{i k.r} from a bead's tables for k = (nx >= 0, ny, nz).
-__device__ __forceinline__ double2 phase_from(const DevParams& P, const double2* tab, short4 k) {
-  double2 ex = tab[P.koff[0] + k.x];
-  double2 ey = tab[P.koff[1] + (k.y >= 0 ? k.y : -k.y)];
-  if (k.y < 0) ey.y = -ey.y;
-  double2 ez = tab[P.koff[2] + (k.z >= 0 ? k.z : -k.z)];
-  if (k.z < 0) ez.y = -ez.y;
-  return cmul(cmul(ex, ey), ez);
-}
-
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double* sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -137,13 +127,13 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return t;  // valid in thread 0
 }
 
-// Constants of the fixed-point pair form: squared distances in units of
-// (L / 2^64)^2 ("raw"). A non-negative double orders like its bit pattern
-// read as an integer, so the cut-off tests are integer compares (off the
-// FP64 pipe).
+// Constants of the integer pair form's FP64 path (near pairs): squared distances
+// in units of (L / 2^64)^2 ("raw"). A non-negative double orders like its bit
+// pattern read as an integer, so the cut-off test is an integer compare (off
+// the FP64 pipe).
 struct FixConst {
   double s2, ua, pref;
-  long long rc2_bits, lj2_bits;  // raw r_c^2 and raw LJ reach, as bits
+  long long lj2_bits;  // raw LJ reach, as bits
 };
 __device__ __forceinline__ FixConst fix_const(const DevParams& P) {
   FixConst F;
@@ -151,189 +141,205 @@ __device__ __forceinline__ FixConst fix_const(const DevParams& P) {
   F.s2 = s * s;
   F.ua = P.alpha * F.s2;
   F.pref = P.lB * P.sqrt_alpha;
-  F.rc2_bits = __double_as_longlong(P.real_cut * P.real_cut / F.s2);
   F.lj2_bits = P.use_pair ? __double_as_longlong(P.lj_max2 / F.s2) : 0;
   return F;
 }
 
-// One pair in the fixed-point form: adds its LJ energy at (k, r^2) to lj and
-// returns h(alpha r^2) inside the real-space cut-off (0 outside, and at
-// r = 0 as the reference's r > 0 test has it); the caller multiplies by the
-// charge product with lB sqrt(alpha) folded in.
-__device__ __forceinline__ double pair_fix(const DevParams& P, const FixConst& F,
-                                           unsigned long long ax, unsigned long long ay,
-                                           unsigned long long az, unsigned long long bx,
-                                           unsigned long long by, unsigned long long bz, int k,
-                                           double& lj) {
-  const double dx = __ll2double_rn((long long)(bx - ax));
-  const double dy = __ll2double_rn((long long)(by - ay));
-  const double dz = __ll2double_rn((long long)(bz - az));
-  const double raw = fma(dx, dx, fma(dy, dy, dz * dz));
-  const long long rb = __double_as_longlong(raw);
-  if (rb < F.lj2_bits) lj += lj64(P, k, raw * F.s2);
-  if (rb > 0 && rb <= F.rc2_bits) {
-    const long long bits = __double_as_longlong(raw * F.ua);
-    return bits >= kH64LoBits ? h64_tab(P.htab64, bits)
-                              : real_term64(P, raw * F.s2) / P.sqrt_alpha;
-  }
-  return 0.0;
+// ---------------------------------------------------------------- delta
+// One launch per move, two kinds of blocks side by side on every SM:
+//
+// k blocks (the first kgrid) own a run of k units each, so dS(k), the commit of
+// the last accepted change and the |S|^2 change need no other block: a warp's
+// lanes take 32 units, its eight warps share the moved beads, and the block
+// adds the eight sums. Their work is FP64.
+//
+// Pair blocks deal out the m x N (moved, other) pairs. In the integer form
+// (fix_pair.h) a thread takes one other bead against a run of kFixRun moved
+// beads: the sums stay integers over beads of one charge and meet the FP64 pipe
+// once per run, so the k blocks keep that pipe and the pair blocks the integer
+// one. Pairs with both beads moved are taken once (j > i), at trial positions
+// for both.
+//
+// A move of the 20,000-bead system (7,812 k-vectors), the serial step included:
+// 71 us, 130 us with FP64 pairs and k tiles x bead groups joined by tickets; of
+// the 1,000-bead system with r_c = 0.7 L (image cells): 41 us, 94 us before.
+constexpr int kFixStage = 256;  // moved beads staged at a time
+constexpr int kFixRun = 4;      // moved beads per thread and other bead
+constexpr int kUnits = 32;      // k units of a k block at a time
+constexpr int kDeltaWarps = kPairThreads / 32;
+
+// Moved beads per phase-table chunk of a k block: 32 where their z tables and xy
+// parts fit the table budget.
+__host__ __device__ inline int k_beads(const DevParams& P) {
+  const int fit = kKTableBytes / (2 * (P.kmax[2] + 1 + kUnits) * (int)sizeof(double2));
+  return fit < 1 ? 1 : (fit > 32 ? 32 : fit);
 }
 
-// ---------------------------------------------------------------- delta
-// Pair sweep: the m x N (moved, other) pairs are numbered p = i*N + j and dealt
-// to every thread of the grid in turn, so even a one-bead move spreads over
-// all SMs (FP64 issue rate per SM is low on GB300; parallel width is what
-// counts). Pairs with both beads moved are taken once (j > i), at trial
-// positions for both.
-// k-space: items (k tile of kKTile vectors) x (group of kchunk_delta moved
-// beads); each item stores its dS(k) part, and the last item of a k tile to
-// finish (atomic ticket) adds the groups in order -- deterministic -- and
-// writes dS(k) and the tile's energy change.
-constexpr int kKTile = 128;
-constexpr int kFixStage = 128;  // moved beads the fixed-point pair form stages
-constexpr size_t kFixBytes = kFixStage * (6 * sizeof(unsigned long long) + sizeof(double) +
-                                          sizeof(int));
+struct FixStage {
+  ulonglong2 a, b, c;  // trial (x, y, z), current (x, y, z)
+  double q;            // charge x lB sqrt(alpha) x table unit
+  int k, pad;          // row of the LJ table
+};
 
-__global__ void __launch_bounds__(kPairThreads)
-    k_delta64(const DevParams P, const DevBuffers B) {
-  extern __shared__ __align__(32) unsigned char smem[];
-  __shared__ double red[kPairThreads / 32];
-  __shared__ int s_last;
-  const DevState* st = B.state;
-  const int b_lo = st->b_lo, b_hi = st->b_hi;
-  const int m = st->pending ? b_hi - b_lo : 0;
-  const int sk_pend = st->sk_pending, sk_buf = st->sk_buf, cur_buf = st->cur_buf;
-  __shared__ int s_final;
+// A pair near enough for LJ or below the table, in FP64: dx, dy, dz the full
+// (unhalved) differences. Adds LJ to lj; returns h where the table has none.
+__device__ __forceinline__ double fix_near(const DevParams& P, const FixConst& F, uint64_t dx,
+                                           uint64_t dy, uint64_t dz, bool below, int k,
+                                           double& lj) {
+  const double x = __ll2double_rn((long long)dx), y = __ll2double_rn((long long)dy),
+               z = __ll2double_rn((long long)dz);
+  const double raw = fma(x, x, fma(y, y, z * z));
+  const long long rb = __double_as_longlong(raw);
+  if (rb < F.lj2_bits) lj += lj64(P, k, raw * F.s2);
+  if (!below || rb <= 0) return 0.0;
+  const long long bits = __double_as_longlong(raw * F.ua);
+  return bits >= kH64LoBits ? h64_tab(P.htab64, bits)
+                            : real_term64(P, raw * F.s2) / P.sqrt_alpha;
+}
+
+// The integer pair sweep of pair block `blk` of `nblk`.
+template <int kMode>
+__device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& B, FixStage* st,
+                                          int blk, int nblk, int b_lo, int m, double& acc_lj,
+                                          double& acc_re) {
+  const FixTab T = P.fx;
+  const FixConst F = fix_const(P);
+  const double qs = F.pref * T.unit, hs = 1.0 / T.unit;
+  const auto tab = [&](uint64_t s) { return fix_h(T.c01, T.c23, T.c45, T.base, s); };
   const int N = P.n_bead;
-
-  double acc_lj = 0.0, acc_re = 0.0;
-  if (m > 0 && m <= kFixStage && B.fpos64 && fix_pairs(P)) {
-    // Fixed-point pair form: the moved beads (trial and current) are staged
-    // once per block as 64-bit fixed-point fractions of the box, the other
-    // beads come from the context's 64-bit mirror; pairs are dealt over the
-    // grid by the same flat index as below. A moved other bead j pairs once
-    // with each moved bead i < j, both at trial or both at current positions.
-    unsigned long long* fx = reinterpret_cast<unsigned long long*>(smem);  // [6][kFixStage]
-    double* fq = reinterpret_cast<double*>(fx + 6 * kFixStage);
-    int* fk = reinterpret_cast<int*>(fq + kFixStage);
-    const FixConst F = fix_const(P);
-    for (int t = threadIdx.x; t < m; t += blockDim.x) {
-      const ulonglong4_32a a = fix64x4(P, B.trial[b_lo + t]), c = fix64x4(P, B.pos[b_lo + t]);
-      fx[t] = a.x;
-      fx[kFixStage + t] = a.y;
-      fx[2 * kFixStage + t] = a.z;
-      fx[3 * kFixStage + t] = c.x;
-      fx[4 * kFixStage + t] = c.y;
-      fx[5 * kFixStage + t] = c.z;
-      fq[t] = __longlong_as_double((long long)c.w) * F.pref;
-      fk[t] = B.type[b_lo + t] * P.n_type;
+  double lj1 = 0.0, lj0 = 0.0;
+  for (int g0 = 0; g0 < m; g0 += kFixStage) {
+    const int gn = min(kFixStage, m - g0);
+    __syncthreads();  // the previous group is consumed
+    for (int t = threadIdx.x; t < gn; t += blockDim.x) {
+      const int i = b_lo + g0 + t;
+      const ulonglong4_32a a = fix64x4(P, B.trial[i]), c = B.fpos64[i];
+      st[t].a = make_ulonglong2(a.x, a.y);
+      st[t].b = make_ulonglong2(a.z, c.x);
+      st[t].c = make_ulonglong2(c.y, c.z);
+      st[t].q = __longlong_as_double((long long)c.w) * qs;
+      st[t].k = B.type[i] * P.n_type;
     }
     __syncthreads();
-    const long long total = (long long)m * N;
-    const long long G = (long long)gridDim.x * blockDim.x;
-    const long long p0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int gq = (int)(G / N), gr = (int)(G % N);
-    int ii = (int)(p0 / N), j = (int)(p0 % N);
-    double lj0 = 0.0;  // LJ at current positions, subtracted at the end
-    for (long long p = p0; p < total; p += G, ii += gq, j += gr) {
+    const int runs = (gn + kFixRun - 1) / kFixRun;
+    // job run * N + j, dealt with stride G; (run, j) advanced without a division
+    const int G = nblk * (int)blockDim.x, p0 = blk * (int)blockDim.x + (int)threadIdx.x;
+    const int gq = G / N, gr = G % N;
+    for (int run = p0 / N, j = p0 % N; run < runs; run += gq, j += gr) {
       if (j >= N) {
         j -= N;
-        ii++;
+        if (++run >= runs) break;
       }
-      const bool jm = j >= b_lo && j < b_hi;
-      if (jm && j <= b_lo + ii) continue;
-      const ulonglong4_32a o = B.fpos64[j];
-      const int k = fk[ii] + B.type[j];
-      const double qq = fq[ii] * __longlong_as_double((long long)o.w);
-      const int l = jm ? j - b_lo : 0;
-      const double h1 =
-          pair_fix(P, F, fx[ii], fx[kFixStage + ii], fx[2 * kFixStage + ii],
-                   jm ? fx[l] : o.x, jm ? fx[kFixStage + l] : o.y,
-                   jm ? fx[2 * kFixStage + l] : o.z, k, acc_lj);
-      const double h0 = pair_fix(P, F, fx[3 * kFixStage + ii], fx[4 * kFixStage + ii],
-                                 fx[5 * kFixStage + ii], o.x, o.y, o.z, k, lj0);
-      acc_re = fma(qq, h1 - h0, acc_re);
-    }
-    acc_lj -= lj0;
-  } else if (P.use_pair || P.use_ewald) {
-    // pair p = ii * N + j, dealt with stride G; (ii, j) advanced without a
-    // division per pair
-    const long long total = (long long)m * N;
-    const long long G = (long long)gridDim.x * blockDim.x;
-    const long long p0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int gq = (int)(G / N), gr = (int)(G % N);
-    int ii = (int)(p0 / N), j = (int)(p0 % N);
-    for (long long p = p0; p < total; p += G, ii += gq, j += gr) {
-      if (j >= N) {
-        j -= N;
-        ii++;
-      }
-      const int i = b_lo + ii;
-      const bool jm = j >= b_lo && j < b_hi;
-      if (jm && j <= i) continue;
-      const double4_32a ti = B.trial[i], ci = B.pos[i];
-      const int tyi = B.type[i], tyj = B.type[j];
-      const double4_32a cj = B.pos[j];
-      const double4_32a tj = jm ? B.trial[j] : cj;
-      double l1 = 0, r1 = 0, l0 = 0, r0 = 0;
-      pair64(P, ti, tyi, tj, tyj, l1, r1);
-      pair64(P, ci, tyi, cj, tyj, l0, r0);
-      if (!hs_bonded(P, B.mol_start, i, j)) acc_lj += l1 - l0;
-      acc_re += r1 - r0;
-    }
-  }
-  double t0 = block_sum<kPairThreads>(acc_lj, red);
-  double t1 = block_sum<kPairThreads>(acc_re, red);
-  if (threadIdx.x == 0) {
-    B.partial[4 * blockIdx.x + 0] = t0;
-    B.partial[4 * blockIdx.x + 1] = t1;
-  }
-
-  const bool kwork = P.use_ewald && m > 0;
-  const int chunk = P.kchunk_delta;
-  const int n_groups = kwork ? (m + chunk - 1) / chunk : 0;
-  const int n_tiles = (P.n_k + kKTile - 1) / kKTile;
-  const int n_items = n_tiles * n_groups;
-  double2* tabs = reinterpret_cast<double2*>(smem);  // [chunk][2][kper]
-  const int per = P.kper;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int tile = item % n_tiles, grp = item / n_tiles;
-    const int c0 = b_lo + grp * chunk;
-    const int cnt = min(chunk, b_hi - c0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < cnt * 6; t += blockDim.x) {
-      int bead = t / 6, which = (t / 3) & 1, axis = t % 3;
-      double4_32a p = which ? B.pos[c0 + bead] : B.trial[c0 + bead];
-      build_axis_table(P, p, axis, tabs + (bead * 2 + which) * per);
-    }
-    __syncthreads();
-    const int k = tile * kKTile + threadIdx.x;
-    const bool mine = threadIdx.x < kKTile && k < P.n_k;
-    if (mine) {
-      const short4 kv = B.kn[k];
-      double2 ds = make_double2(0.0, 0.0);
-      for (int b = 0; b < cnt; b++) {
-        double2 e1 = phase_from(P, tabs + (b * 2 + 0) * per, kv);
-        double2 e0 = phase_from(P, tabs + (b * 2 + 1) * per, kv);
-        ds.x += e1.x - e0.x;
-        ds.y += e1.y - e0.y;
-      }
-      B.dsk_part[(size_t)grp * P.n_k + k] = ds;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&B.ktile_count[tile], 1) == n_groups - 1;
-    __syncthreads();
-    if (s_last) {
-      __threadfence();
-      double e = 0.0;
-      if (mine) {
-        double2 ds = make_double2(0.0, 0.0);
-        for (int g = 0; g < n_groups; g++) {
-          double2 v = __ldcg(&B.dsk_part[(size_t)g * P.n_k + k]);
-          ds.x += v.x;
-          ds.y += v.y;
+      const ulonglong4_32a o0 = B.fpos64[j];
+      const int tj = B.type[j];
+      const double qj = __longlong_as_double((long long)o0.w);
+      // a moved other bead: its trial position, and only moved beads before it
+      const int l = j - b_lo - g0;
+      const bool jm = j >= b_lo && j < b_lo + m;
+      const ulonglong4_32a o1 = jm ? fix64x4(P, B.trial[j]) : o0;
+      const int u0 = run * kFixRun, u1 = min(gn, u0 + kFixRun);
+      double acc = 0.0, q = st[u0].q;
+      int64_t sum = 0;
+      for (int u = u0; u < u1; u++) {
+        const ulonglong2 a = st[u].a, b = st[u].b, c = st[u].c;
+        if (jm && u >= l) break;
+        if (st[u].q != q) {
+          acc = fma(q, (double)sum, acc);
+          q = st[u].q;
+          sum = 0;
         }
+        uint64_t s1, s0;
+        sum += fix_term<kMode>(T, tab, o1.x - a.x, o1.y - a.y, o1.z - b.x, s1);
+        sum -= fix_term<kMode>(T, tab, o0.x - b.y, o0.y - c.x, o0.z - c.y, s0);
+        if (min(s1, s0) < T.s_near) {
+          const int k = st[u].k + tj;
+          double h = 0.0;
+          if (s1 < T.s_near)
+            h = fix_near(P, F, o1.x - a.x, o1.y - a.y, o1.z - b.x, s1 < T.s_lo, k, lj1);
+          if (s0 < T.s_near)
+            h -= fix_near(P, F, o0.x - b.y, o0.y - c.x, o0.z - c.y, s0 < T.s_lo, k, lj0);
+          acc = fma(q * hs, h, acc);
+        }
+      }
+      acc = fma(q, (double)sum, acc);
+      acc_re = fma(acc, qj, acc_re);
+    }
+  }
+  acc_lj += lj1 - lj0;
+}
+
+// dS(k), the S(k) commit and the |S|^2 change of units [u0, u1) (k block).
+// smem, kb = k_beads: [kb][2][zn] e^{i n theta_z}, then [kb][2][kUnits] xy parts.
+__device__ __forceinline__ double k_block(const DevParams& P, const DevBuffers& B,
+                                          unsigned char* smem, int u0, int u1, int b_lo, int b_hi,
+                                          int sk_pend, int sk_buf, int cur_buf) {
+  const int zn = P.kmax[2] + 1, kb = k_beads(P);
+  double2* s_z = reinterpret_cast<double2*>(smem);
+  double2* s_xy = s_z + (size_t)kb * 2 * zn;
+  __shared__ short2 s_col[kUnits];
+  __shared__ int s_ncol;
+  __shared__ double s_sum[kDeltaWarps][4][kUnits];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double e = 0.0;
+  for (int c0 = u0; c0 < u1; c0 += kUnits) {
+    const int un = min(kUnits, u1 - c0);
+    const KUnit ku = lane < un ? B.ku[c0 + lane] : KUnit{0, 0, 0, 0, -1, -1};
+    // the units' (nx, ny) columns, numbered in order
+    const int px = __shfl_up_sync(0xffffffffu, ku.nx, 1), py = __shfl_up_sync(0xffffffffu, ku.ny, 1);
+    const bool head = lane < un && (lane == 0 || px != ku.nx || py != ku.ny);
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const int col = __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
+    int zmax = lane < un ? ku.nz : 0;
+    for (int o = 16; o > 0; o >>= 1) zmax = max(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
+    __syncthreads();  // the previous units are done with the tables
+    if (warp == 0 && head) s_col[col] = make_short2(ku.nx, ku.ny);
+    if (threadIdx.x == 0) s_ncol = __popc(heads);
+    double2 A = make_double2(0.0, 0.0), Bs = A;
+    for (int g0 = b_lo; g0 < b_hi; g0 += kb) {
+      const int cnt = min(kb, b_hi - g0);
+      __syncthreads();
+      const int ncol = s_ncol, nt = cnt * 2;
+      // nt z recursions, then nt x ncol xy phases, one per thread
+      for (int t = threadIdx.x; t < nt * (1 + ncol); t += blockDim.x) {
+        const int it = t % nt, c = t / nt - 1;
+        const double4_32a p = (it & 1) ? B.pos[g0 + (it >> 1)] : B.trial[g0 + (it >> 1)];
+        if (c < 0) {
+          const double2 e1 = turn_exp(turn64(P, p.z, 2));
+          double2 v = make_double2(1.0, 0.0);
+          double2* z = s_z + (size_t)it * zn;
+          z[0] = v;
+          for (int n = 1; n <= zmax; n++) {
+            v = cmul(v, e1);
+            z[n] = v;
+          }
+        } else {
+          const short2 kc = s_col[c];
+          const double2 v = turn_exp(turn64(P, p.x, 0) * (uint64_t)(int64_t)kc.x +
+                                     turn64(P, p.y, 1) * (uint64_t)(int64_t)kc.y);
+          const double q = (it & 1) ? -p.w : p.w;  // trial minus current
+          s_xy[it * kUnits + c] = make_double2(q * v.x, q * v.y);
+        }
+      }
+      __syncthreads();
+      if (lane < un)
+        for (int it = warp; it < nt; it += kDeltaWarps)
+          unit_add(s_xy[it * kUnits + col], s_z[(size_t)it * zn + ku.nz], A, Bs);
+    }
+    s_sum[warp][0][lane] = A.x;
+    s_sum[warp][1][lane] = A.y;
+    s_sum[warp][2][lane] = Bs.x;
+    s_sum[warp][3][lane] = Bs.y;
+    __syncthreads();
+    if (warp < 2 && lane < un) {  // warp 0: +nz, warp 1: -nz
+      double v[4];
+      for (int q = 0; q < 4; q++) {
+        v[q] = 0.0;
+        for (int w = 0; w < kDeltaWarps; w++) v[q] += s_sum[w][q][lane];
+      }
+      const int k = warp == 0 ? ku.kp : ku.km;
+      if (k >= 0) {
+        const double2 SA = make_double2(v[0], v[1]), SB = make_double2(v[2], v[3]);
+        const double2 ds = warp == 0 ? unit_plus(SA, SB) : unit_minus(SA, SB);
         double2 s = B.sk[k];
         if (sk_pend) {
           const double2 p = B.dsk[(size_t)sk_buf * P.n_k + k];
@@ -341,17 +347,75 @@ __global__ void __launch_bounds__(kPairThreads)
           B.sk[k] = s;
         }
         B.dsk[(size_t)cur_buf * P.n_k + k] = ds;
-        e = B.kw[k] * (2.0 * (s.x * ds.x + s.y * ds.y) + (ds.x * ds.x + ds.y * ds.y));
-      }
-      e = block_sum<kPairThreads>(e, red);
-      if (threadIdx.x == 0) {
-        B.kpartial[tile] = e;
-        B.ktile_count[tile] = 0;
+        e += B.kw[k] * (2.0 * (s.x * ds.x + s.y * ds.y) + (ds.x * ds.x + ds.y * ds.y));
       }
     }
   }
-  // Last block to finish adds every block's and every k tile's sums in a
-  // fixed order (deterministic) for the serial kernel.
+  return e;
+}
+
+template <int kMode>
+__global__ void __launch_bounds__(kPairThreads, 2)
+    k_delta64(const DevParams P, const DevBuffers B, int kgrid) {
+  extern __shared__ __align__(32) unsigned char smem[];
+  __shared__ double red[kPairThreads / 32];
+  __shared__ int s_final;
+  const DevState* st = B.state;
+  const int b_lo = st->b_lo, b_hi = st->b_hi;
+  const int m = st->pending ? b_hi - b_lo : 0;
+  const int N = P.n_bead;
+  if ((int)blockIdx.x < kgrid) {
+    double e = 0.0;
+    if (P.use_ewald && m > 0) {
+      const int u0 = (int)((long long)P.n_ku * blockIdx.x / kgrid);
+      const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / kgrid);
+      e = k_block(P, B, smem, u0, u1, b_lo, b_hi, st->sk_pending, st->sk_buf, st->cur_buf);
+    }
+    e = block_sum<kPairThreads>(e, red);
+    if (threadIdx.x == 0) B.partial[4 * blockIdx.x] = e;
+  } else {
+    const int blk = blockIdx.x - kgrid, nblk = gridDim.x - kgrid;
+    double acc_lj = 0.0, acc_re = 0.0;
+    if (kMode) {
+      if (m > 0)
+        fix_sweep<kMode>(P, B, reinterpret_cast<FixStage*>(smem), blk, nblk, b_lo, m, acc_lj,
+                         acc_re);
+    } else if (P.use_pair || P.use_ewald) {
+      // pair p = ii * N + j, dealt with stride G; (ii, j) advanced without a
+      // division per pair
+      const long long total = (long long)m * N;
+      const long long G = (long long)nblk * blockDim.x;
+      const long long p0 = (long long)blk * blockDim.x + threadIdx.x;
+      const int gq = (int)(G / N), gr = (int)(G % N);
+      int ii = (int)(p0 / N), j = (int)(p0 % N);
+      for (long long p = p0; p < total; p += G, ii += gq, j += gr) {
+        if (j >= N) {
+          j -= N;
+          ii++;
+        }
+        const int i = b_lo + ii;
+        const bool jm = j >= b_lo && j < b_hi;
+        if (jm && j <= i) continue;
+        const double4_32a ti = B.trial[i], ci = B.pos[i];
+        const int tyi = B.type[i], tyj = B.type[j];
+        const double4_32a cj = B.pos[j];
+        const double4_32a tj = jm ? B.trial[j] : cj;
+        double l1 = 0, r1 = 0, l0 = 0, r0 = 0;
+        pair64(P, ti, tyi, tj, tyj, l1, r1);
+        pair64(P, ci, tyi, cj, tyj, l0, r0);
+        if (!hs_bonded(P, B.mol_start, i, j)) acc_lj += l1 - l0;
+        acc_re += r1 - r0;
+      }
+    }
+    const double t0 = block_sum<kPairThreads>(acc_lj, red);
+    const double t1 = block_sum<kPairThreads>(acc_re, red);
+    if (threadIdx.x == 0) {
+      B.partial[4 * blockIdx.x + 0] = t0;
+      B.partial[4 * blockIdx.x + 1] = t1;
+    }
+  }
+  // Last block to finish adds every block's sums in a fixed order
+  // (deterministic) for the serial kernel.
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_final = atomicAdd(B.done_count, 1) == (int)gridDim.x - 1;
@@ -360,11 +424,14 @@ __global__ void __launch_bounds__(kPairThreads)
     __threadfence();
     double a = 0.0, b = 0.0, c = 0.0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-      a += __ldcg(&B.partial[4 * i]);
-      b += __ldcg(&B.partial[4 * i + 1]);
+      const double x = __ldcg(&B.partial[4 * i]);
+      if (i < kgrid) {
+        c += x;
+      } else {
+        a += x;
+        b += __ldcg(&B.partial[4 * i + 1]);
+      }
     }
-    if (kwork)
-      for (int i = threadIdx.x; i < n_tiles; i += blockDim.x) c += __ldcg(&B.kpartial[i]);
     a = block_sum<kPairThreads>(a, red);
     b = block_sum<kPairThreads>(b, red);
     c = block_sum<kPairThreads>(c, red);
@@ -378,8 +445,6 @@ __global__ void __launch_bounds__(kPairThreads)
   }
 }
 
-int ktile_count(const DevParams& P) { return (P.n_k + kKTile - 1) / kKTile; }
-
 static int g_pair_grid = 0;
 
 int pair_grid() {
@@ -392,19 +457,33 @@ int pair_grid() {
   return g_pair_grid;
 }
 
+// Shared memory of a k block's phase tables, and of the staged moved beads.
 static size_t delta_smem(const DevParams& P) {
-  const size_t k = P.use_ewald ? (size_t)P.kchunk_delta * 2 * P.kper * sizeof(double2) : 0;
-  return fix_pairs(P) ? std::max(k, kFixBytes) : k;
+  const size_t k = P.use_ewald && P.n_ku > 0
+                       ? (size_t)k_beads(P) * 2 * (P.kmax[2] + 1 + kUnits) * sizeof(double2) : 0;
+  return std::max(k, P.fx.mode ? kFixStage * sizeof(FixStage) : 0);
+}
+
+template <int kMode>
+static void launch_delta64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_delta64<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kKTableBytes + 4096);
+    attr = true;
+  }
+  const int sms = pair_grid() / 2;
+  const int kgrid = P.use_ewald ? std::min(sms, P.n_ku) : 0;
+  k_delta64<kMode><<<kgrid + 2 * sms, kPairThreads, delta_smem(P), s>>>(P, B, kgrid);
 }
 
 void launch_delta_pairs64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_delta64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         std::max((size_t)kKTableBytes + 4096, kFixBytes));
-    attr = true;
-  }
-  k_delta64<<<pair_grid(), kPairThreads, delta_smem(P), s>>>(P, B);
+  if (P.fx.mode == 1)
+    launch_delta64<1>(P, B, s);
+  else if (P.fx.mode == 2)
+    launch_delta64<2>(P, B, s);
+  else
+    launch_delta64<0>(P, B, s);
 }
 
 // ---------------------------------------------------------------- totals
@@ -456,50 +535,89 @@ __global__ void __launch_bounds__(kTotTile)
   }
 }
 
-// k_total64 for LJ + Ewald in a cubic box periodic on every axis, one image
-// (r_c <= L/2) and one box for both terms: positions as 64-bit fixed-point
-// fractions of the box, staged per tile, so one integer subtraction is the
-// minimum-image difference (each fraction carries the rounding of x / L, about
-// one ulp of the coordinate, as its FP64 value does; the subtraction is exact
-// and the conversion to FP64 rounds once). r^2 in FP64, in units of
-// (L / 2^64)^2; the cut-off tests as integer compares of the FP64 bit
-// patterns; the real-space term sqrt(alpha) h(alpha r^2) from the FP64 table,
-// with lB sqrt(alpha) q_i folded into the thread's charge.
-__global__ void __launch_bounds__(kTotTile)
-    k_total64_fix(const DevParams P, const DevBuffers B, double* out) {
-  __shared__ unsigned long long sx[kTotTile], sy[kTotTile], sz[kTotTile];
-  __shared__ double sq[kTotTile];
-  __shared__ int st[kTotTile];
-  __shared__ double red[2 * (kTotTile / 32)];
-  const int nt = (P.n_bead + kTotTile - 1) / kTotTile;
+// The same sum in the integer form (fix_pair.h): 256 x 256 tiles of the i < j
+// triangle, a thread per i against the staged j's (their sums stay integers
+// over up to 16 beads of one charge). The table is staged too, as the lanes'
+// gathers from it run at a bank's pace there and a line's pace from L1; a small
+// system's tiles are cut into `parts` of the j's instead, so that they fill the
+// SMs, and read it in place. 20,000 beads: 1.35 ms (6.2 ms in FP64).
+constexpr int kFixTile = 256;
+constexpr int kFixFlush = 16;
+struct FixOther {
+  ulonglong2 a;  // x, y
+  unsigned long long z;
+  double q;
+};
+
+template <int kMode, bool kStaged>
+__global__ void __launch_bounds__(kFixTile)
+    k_total64_fix(const DevParams P, const DevBuffers B, double* out, int parts) {
+  extern __shared__ __align__(32) unsigned char smem[];
+  __shared__ FixOther so[kFixTile];
+  __shared__ int st[kFixTile];
+  __shared__ double red[kFixTile / 32];
+  const int nt = (P.n_bead + kFixTile - 1) / kFixTile;
   int ta, tb;
-  tri_unrank(blockIdx.x, nt, ta, tb);
-  const int j0 = tb * kTotTile;
-  const int jn = min(kTotTile, P.n_bead - j0);
-  const double inv = P.inv_ebox[0];
-  if (threadIdx.x < jn) {
-    const double4_32a p = B.pos[j0 + threadIdx.x];
-    sx[threadIdx.x] = fix64(p.x, inv);
-    sy[threadIdx.x] = fix64(p.y, inv);
-    sz[threadIdx.x] = fix64(p.z, inv);
-    sq[threadIdx.x] = p.w;
+  tri_unrank(blockIdx.x / parts, nt, ta, tb);
+  const int per = kFixTile / parts;
+  const int j0 = tb * kFixTile + (int)(blockIdx.x % parts) * per;
+  const int jn = min(per, P.n_bead - j0);
+  const FixTab T = P.fx;
+  const FixPair64* c01 = T.c01;
+  const FixPair64* c23 = T.c23;
+  const FixPair32* c45 = T.c45;
+  if (kStaged) {
+    FixPair64* s01 = reinterpret_cast<FixPair64*>(smem);
+    FixPair64* s23 = s01 + T.n_bin;
+    FixPair32* s45 = reinterpret_cast<FixPair32*>(s23 + T.n_bin);
+    for (int i = threadIdx.x; i < T.n_bin; i += kFixTile) {
+      s01[i] = T.c01[i];
+      s23[i] = T.c23[i];
+      s45[i] = T.c45[i];
+    }
+    c01 = s01, c23 = s23, c45 = s45;
+  }
+  if ((int)threadIdx.x < jn) {
+    const ulonglong4_32a p = fix64x4(P, B.pos[j0 + threadIdx.x]);
+    so[threadIdx.x].a = make_ulonglong2(p.x, p.y);
+    so[threadIdx.x].z = p.z;
+    so[threadIdx.x].q = __longlong_as_double((long long)p.w);
     st[threadIdx.x] = B.type[j0 + threadIdx.x];
   }
   __syncthreads();
   const FixConst F = fix_const(P);
+  const auto tab = [&](uint64_t s) { return fix_h(c01, c23, c45, T.base, s); };
   double lj = 0.0, re = 0.0;
-  const int i = ta * kTotTile + threadIdx.x;
-  if (i < P.n_bead) {
-    const double4_32a pi = B.pos[i];
-    const unsigned long long ux = fix64(pi.x, inv), uy = fix64(pi.y, inv), uz = fix64(pi.z, inv);
-    const double qi = pi.w * F.pref;
+  const int i = ta * kFixTile + threadIdx.x;
+  if (i < P.n_bead && jn > 0) {
+    const ulonglong4_32a pi = fix64x4(P, B.pos[i]);
+    const double hs = 1.0 / T.unit;
     const int kt = B.type[i] * P.n_type;
-    for (int jj = ta == tb ? (int)threadIdx.x + 1 : 0; jj < jn; jj++)
-      re = fma(qi * sq[jj], pair_fix(P, F, ux, uy, uz, sx[jj], sy[jj], sz[jj], kt + st[jj], lj),
-               re);
+    double q = so[0].q;
+    int64_t sum = 0;
+    int held = 0;
+    for (int jj = 0; jj < jn; jj++) {
+      const ulonglong2 a = so[jj].a;
+      const unsigned long long z = so[jj].z;
+      if (so[jj].q != q || held == kFixFlush) {
+        re = fma(q, (double)sum, re);
+        q = so[jj].q;
+        sum = 0;
+        held = 0;
+      }
+      held++;
+      if (j0 + jj <= i) continue;
+      uint64_t s;
+      sum += fix_term<kMode>(T, tab, a.x - pi.x, a.y - pi.y, z - pi.z, s);
+      if (s < T.s_near)
+        re = fma(q * hs, fix_near(P, F, a.x - pi.x, a.y - pi.y, z - pi.z, s < T.s_lo, kt + st[jj],
+                                  lj), re);
+    }
+    re = fma(q, (double)sum, re);
+    re *= __longlong_as_double((long long)pi.w) * F.pref * T.unit;
   }
-  const double a = block_sum<kTotTile>(lj, red);
-  const double b = block_sum<kTotTile>(re, red + kTotTile / 32);
+  const double a = block_sum<kFixTile>(lj, red);
+  const double b = block_sum<kFixTile>(re, red);
   if (threadIdx.x == 0) {
     out[2 * blockIdx.x] = a;
     out[2 * blockIdx.x + 1] = b;
@@ -516,38 +634,65 @@ void launch_fix64_all(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
   if (B.fpos64 && P.n_bead > 0) k_fix64_all<<<(P.n_bead + 255) / 256, 256, 0, s>>>(P, B);
 }
 
+// Parts of a 256 x 256 tile: enough for two blocks per SM, at most 16.
+static int fix_parts(const DevParams& P) {
+  const long long nt = (P.n_bead + kFixTile - 1) / kFixTile, tiles = nt * (nt + 1) / 2;
+  int parts = 1;
+  while (parts < 16 && tiles * parts < pair_grid()) parts *= 2;
+  return parts;
+}
+
 int total_partials_count(const DevParams& P) {
-  long long nt = (P.n_bead + kTotTile - 1) / kTotTile;
-  return (int)(nt * (nt + 1) / 2);
+  const int tile = P.fx.mode ? kFixTile : kTotTile;
+  const long long nt = (P.n_bead + tile - 1) / tile;
+  return (int)(nt * (nt + 1) / 2) * (P.fx.mode ? fix_parts(P) : 1);
+}
+
+template <int kMode>
+static void launch_total_fix(const DevParams& P, const DevBuffers& B, double* out, int n_part,
+                             cudaStream_t s) {
+  const int parts = fix_parts(P);
+  const size_t smem = (size_t)P.fx.n_bin * (2 * sizeof(FixPair64) + sizeof(FixPair32));
+  if (parts == 1) {
+    static bool attr = false;
+    if (!attr) {
+      cudaFuncSetAttribute(k_total64_fix<kMode, true>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, kFixMaxBins * 40);
+      attr = true;
+    }
+    k_total64_fix<kMode, true><<<n_part, kFixTile, smem, s>>>(P, B, out, parts);
+  } else {
+    k_total64_fix<kMode, false><<<n_part, kFixTile, 0, s>>>(P, B, out, parts);
+  }
 }
 
 void launch_total64(const DevParams& P, const DevBuffers& B, double* out, int n_part,
                     cudaStream_t s) {
-  if (fix_pairs(P))
-    k_total64_fix<<<n_part, kTotTile, 0, s>>>(P, B, out);
+  if (P.fx.mode == 1)
+    launch_total_fix<1>(P, B, out, n_part, s);
+  else if (P.fx.mode == 2)
+    launch_total_fix<2>(P, B, out, n_part, s);
   else
     k_total64<<<n_part, kTotTile, 0, s>>>(P, B, out);
 }
 
-// S(k) from scratch: block (k tile, bead group) writes a partial; a second
-// pass adds the groups in order.
-// Each thread takes kSkPer consecutive k-vectors (a tile of kSkTile per
-// block); vectors of one (n_x, n_y) column (n_z runs fastest in the k list)
-// share the product e^{i(k_x x + k_y y)} per bead, and each phase is the same
-// cmul(cmul(ex, ey), ez) as phase_from's. Bead groups split the beads so that
-// the grid is one wave of two blocks per SM; a second pass adds the groups in
-// order.
+// S(k) from scratch: block (unit tile, bead group) writes a partial, a second
+// pass adds the groups in order. A thread takes kSkPer consecutive units (+-nz
+// pairs, see KUnit), which mostly share their column's xy product: five FP64
+// operations per unit and bead, 2.5 per vector (6.5 with a complex product per
+// vector). The grid is one wave of two blocks per SM.
 constexpr int kSkPer = 4;
 constexpr int kSkTile = kSkPer * kPairThreads;
 constexpr int kSkGroupsMax = 512;
 
 int sk_full_groups(const DevParams& P) {
-  const int tiles = std::max(1, (P.n_k + kSkTile - 1) / kSkTile);
-  const int want = (pair_grid() + tiles - 1) / tiles;  // two blocks per SM, one wave
-  return std::max(1, std::min(kSkGroupsMax, want));  // groups past the beads add zero
+  const int tiles = std::max(1, (P.n_ku + kSkTile - 1) / kSkTile);
+  const int want = std::max(1, pair_grid() / tiles);
+  // a group of fewer than 8 beads would spend more on its tables than its sums
+  return std::max(1, std::min(std::min(kSkGroupsMax, want), (P.n_bead + 7) / 8));
 }
 
-__global__ void __launch_bounds__(kPairThreads)
+__global__ void __launch_bounds__(kPairThreads, 2)
     k_sk64(const DevParams P, const DevBuffers B, double2* part, int groups) {
   extern __shared__ __align__(32) unsigned char smem[];
   double2* tabs = reinterpret_cast<double2*>(smem);
@@ -556,27 +701,24 @@ __global__ void __launch_bounds__(kPairThreads)
   const int g = blockIdx.y;
   const int per_g = (P.n_bead + groups - 1) / groups;
   const int b0 = g * per_g, b1 = min(P.n_bead, b0 + per_g);
-  int kk[kSkPer], ox[kSkPer], oy[kSkPer], oz[kSkPer];
-  bool mine[kSkPer], col[kSkPer], ny[kSkPer], nz[kSkPer];
-  double2 s[kSkPer];
+  KUnit un[kSkPer];
+  bool mine[kSkPer], col[kSkPer];
+  double2 A[kSkPer], Bs[kSkPer];
 #pragma unroll
   for (int q = 0; q < kSkPer; q++) {
-    kk[q] = blockIdx.x * kSkTile + threadIdx.x * kSkPer + q;
-    mine[q] = kk[q] < P.n_k;
-    const short4 kv = mine[q] ? B.kn[kk[q]] : make_short4(0, 0, 0, 0);
-    ox[q] = P.koff[0] + kv.x;
-    oy[q] = P.koff[1] + (kv.y >= 0 ? kv.y : -kv.y);
-    oz[q] = P.koff[2] + (kv.z >= 0 ? kv.z : -kv.z);
-    ny[q] = kv.y < 0;
-    nz[q] = kv.z < 0;
-    col[q] = q == 0 || ox[q] != ox[q - 1] || oy[q] != oy[q - 1] || ny[q] != ny[q - 1];
-    s[q] = make_double2(0.0, 0.0);
+    const int u = blockIdx.x * kSkTile + threadIdx.x * kSkPer + q;
+    mine[q] = u < P.n_ku;
+    un[q] = mine[q] ? B.ku[u] : KUnit{0, 0, 0, 0, -1, -1};
+    // a new (nx, ny) column: recompute the xy product
+    col[q] = q == 0 || un[q].nx != un[q - 1].nx || un[q].ny != un[q - 1].ny;
+    A[q] = Bs[q] = make_double2(0.0, 0.0);
   }
   for (int c0 = b0; c0 < b1; c0 += chunk) {
     const int cnt = min(chunk, b1 - c0);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * 3; t += blockDim.x)
-      build_axis_table(P, B.pos[c0 + t / 3], t % 3, tabs + (t / 3) * per);
+    // axis by axis, so that a warp's lanes share the length of their recursion
+    for (int t = threadIdx.x; t < 3 * 32; t += kPairThreads)
+      if ((t & 31) < cnt) build_axis_table(P, B.pos[c0 + (t & 31)], t >> 5, tabs + (t & 31) * per);
     __syncthreads();
     if (mine[0])
       for (int b = 0; b < cnt; b++) {
@@ -585,34 +727,40 @@ __global__ void __launch_bounds__(kPairThreads)
 #pragma unroll
         for (int q = 0; q < kSkPer; q++)
           if (mine[q]) {
-            if (col[q]) {
-              double2 ey = tb[oy[q]];
-              if (ny[q]) ey.y = -ey.y;
-              xy = cmul(tb[ox[q]], ey);
-            }
-            double2 ez = tb[oz[q]];
-            if (nz[q]) ez.y = -ez.y;
-            const double2 e = cmul(xy, ez);
-            s[q].x += e.x;
-            s[q].y += e.y;
+            if (col[q]) xy = unit_xy(P, tb, un[q].nx, un[q].ny);
+            unit_add(xy, tb[P.koff[2] + un[q].nz], A[q], Bs[q]);
           }
       }
   }
 #pragma unroll
   for (int q = 0; q < kSkPer; q++)
-    if (mine[q]) part[(size_t)g * P.n_k + kk[q]] = s[q];
+    if (mine[q]) {
+      if (un[q].kp >= 0) part[(size_t)g * P.n_k + un[q].kp] = unit_plus(A[q], Bs[q]);
+      if (un[q].km >= 0) part[(size_t)g * P.n_k + un[q].km] = unit_minus(A[q], Bs[q]);
+    }
 }
 
-__global__ void k_sk_sum(int n_k, int groups, const double2* part, double2* sk) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n_k) return;
+// Eight threads per k-vector add every eighth group, then their sums in order.
+__global__ void __launch_bounds__(256) k_sk_sum(int n_k, int groups, const double2* part,
+                                                double2* sk) {
+  __shared__ double2 sh[8][32];
+  const int l = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x * 32 + l;
   double2 s = make_double2(0.0, 0.0);
-  for (int g = 0; g < groups; g++) {
-    double2 p = part[(size_t)g * n_k + k];
-    s.x += p.x;
-    s.y += p.y;
+  if (k < n_k)
+    for (int g = w; g < groups; g += 8) {
+      const double2 p = part[(size_t)g * n_k + k];
+      s.x += p.x;
+      s.y += p.y;
+    }
+  sh[w][l] = s;
+  __syncthreads();
+  if (w == 0 && k < n_k) {
+    for (int q = 1; q < 8; q++) {
+      s.x += sh[q][l].x;
+      s.y += sh[q][l].y;
+    }
+    sk[k] = s;
   }
-  sk[k] = s;
 }
 
 void launch_sk_full64(const DevParams& P, const DevBuffers& B, double2* part, cudaStream_t s) {
@@ -624,57 +772,58 @@ void launch_sk_full64(const DevParams& P, const DevBuffers& B, double2* part, cu
   }
   size_t smem = (size_t)P.kchunk_sk * P.kper * sizeof(double2);
   const int groups = sk_full_groups(P);
-  dim3 grid((P.n_k + kSkTile - 1) / kSkTile, groups);
+  dim3 grid((P.n_ku + kSkTile - 1) / kSkTile, groups);
   k_sk64<<<grid, kPairThreads, smem, s>>>(P, B, part, groups);
-  k_sk_sum<<<(P.n_k + 255) / 256, 256, 0, s>>>(P.n_k, groups, part, B.sk);
+  k_sk_sum<<<(P.n_k + 31) / 32, 256, 0, s>>>(P.n_k, groups, part, B.sk);
 }
 
-// Bond energy of molecule m on coordinates p (potential_spring.cc:22-48),
-// summed in bond order.
-__device__ double bond_mol64(const DevParams& P, const double4_32a* p, int b0, int b1) {
-  double e = 0.0;
-  for (int i = b0; i < b1 - 1; i++) {
-    double dx = p[i].x - p[i + 1].x, dy = p[i].y - p[i + 1].y, dz = p[i].z - p[i + 1].z;
-    double r = sqrt(dx * dx + dy * dy + dz * dz);
-    e += 0.5 * P.k_bond * (r - P.r0) * (r - P.r0);
-  }
-  return e;
-}
-
-// Misc totals: out6 = {bond, ext, self, self_images, mz, unused}.
-// Also fills bond_mol[]. One block, fixed-order reduction.
+// Misc totals: block b writes its {bond, ext, self, self_images, mz} to out +
+// 5 b (k_assemble_total adds the blocks in order) and bond_mol[]. A warp per
+// molecule sums its bonds (potential_spring.cc:22-48); the beads are dealt over
+// the grid. (One block with a thread per molecule took 470 us on 20,000 beads.)
 __global__ void __launch_bounds__(256) k_misc64(const DevParams P, const DevBuffers B,
-                                                double* out6) {
+                                                double* out) {
   __shared__ double red[8];
-  double eb = 0, ee = 0, es = 0, ei = 0, mz = 0;
-  double img = 0.0;
-  if (P.use_ewald) img = real_images64(P, 0.0, 0.0, 0.0);
-  for (int m = threadIdx.x; m < P.n_mol; m += blockDim.x) {
+  __shared__ double s_img;
+  double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  if (threadIdx.x == 0) s_img = P.use_ewald ? real_images64(P, 0.0, 0.0, 0.0) : 0.0;
+  __syncthreads();
+  const double img = s_img;
+  const int lane = threadIdx.x & 31;
+  for (int m = blockIdx.x * 8 + (threadIdx.x >> 5); m < P.n_mol; m += gridDim.x * 8) {
     double e = 0.0;
-    if (P.use_bond) e = bond_mol64(P, B.pos, B.mol_start[m], B.mol_start[m + 1]);
-    B.bond_mol[m] = e;
-    eb += e;
-  }
-  for (int i = threadIdx.x; i < P.n_bead; i += blockDim.x) {
-    double4_32a p = B.pos[i];
-    if (P.use_ext) ee += wall64(P, p.z, B.type[i]);
-    if (P.use_ewald) {
-      es += P.self_coef * p.w * p.w;
-      ei += 0.5 * P.lB * p.w * p.w * img;
-      mz += p.w * p.z;
+    if (P.use_bond) {
+      const int b0 = B.mol_start[m], b1 = B.mol_start[m + 1];
+      for (int i = b0 + lane; i < b1 - 1; i += 32) {
+        const double4_32a p = B.pos[i], q = B.pos[i + 1];
+        const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        e += 0.5 * P.k_bond * (r - P.r0) * (r - P.r0);
+      }
+      for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    }
+    if (lane == 0) {
+      B.bond_mol[m] = e;
+      v[0] += e;
     }
   }
-  double v[5] = {eb, ee, es, ei, mz};
-  for (int q = 0; q < 5; q++) {
-    double t = block_sum<256>(v[q], red);
-    if (threadIdx.x == 0) out6[q] = t;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < P.n_bead; i += gridDim.x * 256) {
+    const double4_32a p = B.pos[i];
+    if (P.use_ext) v[1] += wall64(P, p.z, B.type[i]);
+    if (P.use_ewald) {
+      v[2] += P.self_coef * p.w * p.w;
+      v[3] += 0.5 * P.lB * p.w * p.w * img;
+      v[4] += p.w * p.z;
+    }
   }
-  if (threadIdx.x == 0) out6[5] = 0.0;
+  for (int q = 0; q < 5; q++) {
+    const double t = block_sum<256>(v[q], red);
+    if (threadIdx.x == 0) out[5 * blockIdx.x + q] = t;
+  }
 }
 
-void launch_misc_total64(const DevParams& P, const DevBuffers& B, double* out6,
-                         cudaStream_t s) {
-  k_misc64<<<1, 256, 0, s>>>(P, B, out6);
+void launch_misc_total64(const DevParams& P, const DevBuffers& B, double* out, cudaStream_t s) {
+  k_misc64<<<kMiscBlocks, 256, 0, s>>>(P, B, out);
 }
 
 // Rg^2, axis components and end-to-end^2 (simulation.cc:406-500); one block
@@ -754,64 +903,6 @@ void launch_rhoz(const DevParams& P, const DevBuffers& B, double res, int n_bins
   cudaMemsetAsync(cnt, 0, sizeof(unsigned) * 3 * (size_t)n_bins, s);
   const int m = P.n_mol - P.phantom;
   if (m > 0) k_rhoz<<<std::min(m, 4 * 152), 128, 0, s>>>(P, B, res, n_bins, cnt);
-}
-
-
-// An FP64 table over u: per bin the degree-8 Chebyshev interpolant of f at the
-// 9 Chebyshev nodes of y in [-1/2, 1/2] (u = lo + (y + 1/2) w), in long double,
-// then rewritten in powers of y.
-template <class F>
-static std::vector<double> build_table64(F f_of) {
-  constexpr int n = 9;
-  const long double pi = 3.141592653589793238462643383279503L;
-  long double T[n][n] = {};  // T_j(t) coefficients in powers of t
-  T[0][0] = 1.0L;
-  T[1][1] = 1.0L;
-  for (int j = 2; j < n; j++)
-    for (int q = 0; q < n; q++)
-      T[j][q] = (q ? 2.0L * T[j - 1][q - 1] : 0.0L) - T[j - 2][q];
-  long double tk[n], cs[n][n];  // nodes t = 2 y in [-1, 1], cos(j arccos t)
-  for (int k = 0; k < n; k++) {
-    tk[k] = std::cos(pi * (k + 0.5L) / n);
-    for (int j = 0; j < n; j++) cs[j][k] = std::cos(pi * j * (k + 0.5L) / n);
-  }
-  std::vector<double> out((size_t)kH64Bins * kH64Stride, 0.0);
-  int b = 0;
-  for (int e = kH64ELo; e < kH64EHi; e++)
-    for (int j = 0; j < kH64Per; j++, b++) {
-      const long double lo = std::ldexp(1.0L + (long double)j / kH64Per, e);
-      const long double w = std::ldexp(1.0L / kH64Per, e);
-      long double f[n];
-      for (int k = 0; k < n; k++) f[k] = f_of(lo + (0.5L * tk[k] + 0.5L) * w);
-      long double mono[n] = {};  // powers of y
-      for (int jj = 0; jj < n; jj++) {
-        long double a = 0.0L;
-        for (int k = 0; k < n; k++) a += f[k] * cs[jj][k];
-        a *= (jj ? 2.0L : 1.0L) / n;
-        for (int q = 0; q < n; q++) mono[q] += a * T[jj][q] * std::ldexp(1.0L, q);
-      }
-      for (int q = 0; q < n; q++) out[(size_t)b * kH64Stride + q] = (double)mono[q];
-    }
-  return out;
-}
-
-// The tables hold constants, so a process makes each once (5,000 long-double
-// erfcs; on aarch64, where long double is done in software, tens of
-// milliseconds that every context used to spend).
-const std::vector<double>& h64_table() {
-  static const std::vector<double> t = build_table64([](long double u) {
-    const long double r = std::sqrt(u);
-    return std::erfc(r) / r;
-  });
-  return t;
-}
-
-const std::vector<double>& g64_table() {
-  static const std::vector<double> t = build_table64([](long double u) {
-    const long double r = std::sqrt(u);
-    return (std::erfc(r) / r + 2.0L / std::sqrt(3.14159265359L) * std::exp(-u)) / u;
-  });
-  return t;
 }
 
 }  // namespace plum

@@ -29,6 +29,8 @@ namespace plum {
 
 constexpr int kKTile32 = 128;
 
+int ktile_count(const DevParams& P) { return (P.n_k + kKTile32 - 1) / kKTile32; }
+
 template <int NT>
 __device__ __forceinline__ float block_sum32(float v, float* sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -5,27 +5,63 @@
 
 namespace plum {
 
-// e^{i n theta} tables for one bead: tab[koff[axis] + n], n = 0..kmax[axis];
-// q folded into the x table.
-__device__ __forceinline__ void build_axis_table(const DevParams& P, double4_32a p,
-                                                 int axis, double2* tab) {
-  double w = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
-  if (axis < P.npbc) w -= P.ebox[axis] * floor(w * P.inv_ebox[axis]);
-  double s, c;
-  sincos(P.kunit[axis] * w, &s, &c);
-  double2 e = axis == 0 ? make_double2(p.w, 0.0) : make_double2(1.0, 0.0);
-  double2* t = tab + P.koff[axis];
-  t[0] = e;
-  for (int n = 1; n <= P.kmax[axis]; n++) {
-    double re = e.x * c - e.y * s;
-    double im = e.x * s + e.y * c;
-    e = make_double2(re, im);
-    t[n] = e;
-  }
+// A coordinate as a 64-bit fraction of a turn: frac(w / L) 2^64, times kPi / pi
+// (the reference's phases are 2 kPi n w / L with its 12-digit kPi), so that n
+// times it, mod 2^64, is the phase of n exactly.
+__device__ __forceinline__ uint64_t turn64(const DevParams& P, double w, int axis) {
+  double f = w * P.inv_ebox[axis];
+  double g = f - floor(f);
+  if (axis < P.npbc) f = g;  // wrapped into the primary cell
+  if (g >= 1.0) g = 0.0;     // a tiny negative w / L rounds up to 1
+  return __double2ull_rn(g * 0x1p64) + (uint64_t)__double2ll_rn(f * P.turn_eps);
+}
+
+// e^{2 pi i phi / 2^64}: the nearest quarter turn taken off in integers, then the
+// Taylor series of sine and cosine on |theta| <= pi / 4 (through theta^15 and
+// theta^16: the next terms are under 5e-17). About 20 FP64 operations, with no
+// range reduction (sincos of a general argument: five times that).
+__device__ __forceinline__ double2 turn_exp(uint64_t phi) {
+  const int q = (int)((phi + (1ull << 61)) >> 62);
+  const double t = (double)(int64_t)(phi - ((uint64_t)q << 62)) *
+                   (6.283185307179586476925286766559 * 0x1p-64);
+  const double x = t * t;
+  double s = -1.0 / 1307674368000.0;
+  s = fma(s, x, 1.0 / 6227020800.0);
+  s = fma(s, x, -1.0 / 39916800.0);
+  s = fma(s, x, 1.0 / 362880.0);
+  s = fma(s, x, -1.0 / 5040.0);
+  s = fma(s, x, 1.0 / 120.0);
+  s = fma(s, x, -1.0 / 6.0);
+  s = fma(s * x, t, t);
+  double c = 1.0 / 20922789888000.0;
+  c = fma(c, x, -1.0 / 87178291200.0);
+  c = fma(c, x, 1.0 / 479001600.0);
+  c = fma(c, x, -1.0 / 3628800.0);
+  c = fma(c, x, 1.0 / 40320.0);
+  c = fma(c, x, -1.0 / 720.0);
+  c = fma(c, x, 1.0 / 24.0);
+  c = fma(c, x, -0.5);
+  c = fma(c, x, 1.0);
+  const double a = q & 1 ? s : c, b = q & 1 ? c : s;  // |cos|, |sin| of the turn
+  return make_double2(q == 1 || q == 2 ? -a : a, q & 2 ? -b : b);
 }
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// e^{i n theta} tables for one bead: tab[koff[axis] + n], n = 0..kmax[axis];
+// q folded into the x table.
+__device__ __forceinline__ void build_axis_table(const DevParams& P, double4_32a p,
+                                                 int axis, double2* tab) {
+  const double2 e1 = turn_exp(turn64(P, axis == 0 ? p.x : (axis == 1 ? p.y : p.z), axis));
+  double2 e = axis == 0 ? make_double2(p.w, 0.0) : make_double2(1.0, 0.0);
+  double2* t = tab + P.koff[axis];
+  t[0] = e;
+  for (int n = 1; n <= P.kmax[axis]; n++) {
+    e = cmul(e, e1);
+    t[n] = e;
+  }
 }
 
 // The xy part c = q e^{i(kx x + ky y)} of a unit's column from a bead's tables
