@@ -687,9 +687,7 @@ constexpr int kSkGroupsMax = 512;
 
 int sk_full_groups(const DevParams& P) {
   const int tiles = std::max(1, (P.n_ku + kSkTile - 1) / kSkTile);
-  const int want = std::max(1, pair_grid() / tiles);
-  // a group of fewer than 8 beads would spend more on its tables than its sums
-  return std::max(1, std::min(std::min(kSkGroupsMax, want), (P.n_bead + 7) / 8));
+  return std::max(1, std::min(kSkGroupsMax, pair_grid() / tiles));
 }
 
 __global__ void __launch_bounds__(kPairThreads, 2)
@@ -771,7 +769,8 @@ void launch_sk_full64(const DevParams& P, const DevBuffers& B, double2* part, cu
     attr = true;
   }
   size_t smem = (size_t)P.kchunk_sk * P.kper * sizeof(double2);
-  const int groups = sk_full_groups(P);
+  // a group of fewer than 8 beads would spend more on its tables than its sums
+  const int groups = std::max(1, std::min(sk_full_groups(P), (P.n_bead + 7) / 8));
   dim3 grid((P.n_ku + kSkTile - 1) / kSkTile, groups);
   k_sk64<<<grid, kPairThreads, smem, s>>>(P, B, part, groups);
   k_sk_sum<<<(P.n_k + 31) / 32, 256, 0, s>>>(P.n_k, groups, part, B.sk);
