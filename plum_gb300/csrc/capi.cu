@@ -91,6 +91,9 @@ struct plum_ctx {
   bool host_pending = false;
   int max_len = 1;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // the next move's generation runs beside the energy change
+  cudaStream_t s_gen = nullptr;
+  cudaEvent_t gen_go = nullptr, gen_done = nullptr;
   double last_ms = 0.0;
   long last_kernels = 0;
   long recompute_every = 0;    // full FP64 recompute cadence of plum_run (0: never)
@@ -366,27 +369,34 @@ void enqueue_loop(plum_ctx* c, int n_moves, const DevBuffers& B) {
   // with a training log, each generated chain move's descriptor is taken
   // before its energy change
   const bool desc = B.log_desc != nullptr;
+  launch_gen64(c->P, B, true, c->s);
   launch_serial64(c->P, B, kModeGen, c->s);
-  if (desc) launch_desc_batch(c->d_rp1, c->d_rb1, 1, B.desc_acc, c->P.form, 0, c->s);
   for (int i = 0; i < n_moves; i++) {
+    const bool more = i + 1 < n_moves;
+    if (more) {
+      cudaEventRecord(c->gen_go, c->s);
+      cudaStreamWaitEvent(c->s_gen, c->gen_go, 0);
+      launch_gen64(c->P, B, false, c->s_gen);
+      cudaEventRecord(c->gen_done, c->s_gen);
+    }
+    if (desc) launch_desc_batch(c->d_rp1, c->d_rb1, 1, B.desc_acc, c->P.form, 0, c->s);
     if (c->kt_on) kt_mark(c, 0);
     launch_delta(c, B);
     if (c->kt_on) kt_mark(c, 1);
-    int mode = kModeFinish | kModeDecide | (i + 1 < n_moves ? kModeGen : 0);
-    launch_serial64(c->P, B, mode, c->s);
+    if (more) cudaStreamWaitEvent(c->s, c->gen_done, 0);
+    launch_serial64(c->P, B, kModeFinish | kModeDecide | (more ? kModeGen : 0), c->s);
     if (c->kt_on) kt_mark(c, 2);
-    if (desc && i + 1 < n_moves)
-      launch_desc_batch(c->d_rp1, c->d_rb1, 1, B.desc_acc, c->P.form, 0, c->s);
   }
 }
 
-// The device MC loop: gen, then (pairs, finish+decide+gen) per step. Batches
+// The device MC loop: gen, then (energy change beside the next move's gen, finish
+// + decide + adopt) per step. Batches
 // of a repeated size run as one CUDA graph, captured on the second use (the
 // first runs as plain launches so lazy kernel set-up happens outside a
 // capture); the kernels read the pending move from device state, so one
 // capture replays for every batch.
 int device_loop(plum_ctx* c, int n_moves, DevBuffers B) {
-  const long k = 1 + 2L * n_moves + (B.log_desc ? n_moves : 0);
+  const long k = 1 + 3L * n_moves + (B.log_desc ? n_moves : 0);
   if (B.log_desc) CK(cudaMemcpyAsync(c->d_rb1, &B, sizeof(B), cudaMemcpyHostToDevice, c->s));
   if (c->kt_on) {
     enqueue_loop(c, n_moves, B);
@@ -640,6 +650,9 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     return fail(PLUM_ERR_CUDA, "cannot select CUDA device " + std::to_string(device));
   }
   if (cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->s_gen, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->gen_go, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->gen_done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
     plum_ctx_destroy(c);
     return fail(PLUM_ERR_CUDA, "cannot create the context's stream and events");
@@ -663,6 +676,10 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   rc |= dalloc(&B.fpos, nb);
   rc |= dalloc(&B.fq, nb);
   rc |= dalloc(&B.ftrial, c->max_len);
+  P.max_len = c->max_len;
+  rc |= dalloc(&B.plan, 1);
+  rc |= dalloc(&B.ctrial, kCands * (size_t)c->max_len);
+  rc |= dalloc(&B.cftrial, kCands * (size_t)c->max_len);
   {
     int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
     rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
@@ -755,6 +772,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   cudaMemset(B.state, 0, sizeof(DevState));
   cudaMemset(B.ktile_count, 0, sizeof(int) * std::max(1, ktile_count(P)));
   cudaMemset(B.done_count, 0, sizeof(int));
+  cudaMemset(B.plan, 0, sizeof(StepPlan));
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     plum_ctx_destroy(c);
@@ -784,14 +802,17 @@ int plum_ctx_destroy(plum_ctx* c) {
                   c->d_stream,   c->d_mt,      c->d_log_type, c->d_log_acc, c->d_log_e,
                   c->d_press,    c->d_sk_part, c->d_log_de, c->d_htab, c->d_htab64,
                   c->B.fpos64,   c->B.ku,      c->d_gtab64,
-                  c->d_fx};
+                  c->d_fx,       c->B.plan,    c->B.ctrial, c->B.cftrial};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->gen_go) cudaEventDestroy(c->gen_go);
+  if (c->gen_done) cudaEventDestroy(c->gen_done);
   for (cudaEvent_t e : c->kt_ev) cudaEventDestroy(e);
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
+  if (c->s_gen) cudaStreamDestroy(c->s_gen);
   if (c->s) cudaStreamDestroy(c->s);
   delete c;
   return PLUM_OK;
@@ -916,7 +937,7 @@ int rebuild_system(plum_ctx* c) {
   P.n_ion_total = (int)ions.size();
   const bool mirror64 = B.fpos64 != nullptr;
   void* old[] = {B.pos,      B.trial,      B.type,     B.mol_start, B.chain_ids, B.ion_ids,
-                 B.fpos,     B.fq,         B.ftrial,   B.dsk_part32, B.bond_mol,
+                 B.fpos,     B.fq,         B.ftrial,   B.dsk_part32, B.bond_mol, B.ctrial, B.cftrial,
                  c->d_tot_part, c->d_obs_per, c->cb_b, c->cb_c,    c->cb_part,  c->cb_u,
                  B.fpos64};
   for (void* q : old)
@@ -924,7 +945,9 @@ int rebuild_system(plum_ctx* c) {
   B.pos = B.trial = nullptr;
   B.fpos64 = nullptr;
   B.type = B.mol_start = B.chain_ids = B.ion_ids = nullptr;
-  B.fpos = B.ftrial = nullptr;
+  B.fpos = B.ftrial = B.cftrial = nullptr;
+  B.ctrial = nullptr;
+  P.max_len = c->max_len;
   B.fq = nullptr;
   B.dsk_part32 = nullptr;
   B.bond_mol = nullptr;
@@ -935,7 +958,9 @@ int rebuild_system(plum_ctx* c) {
   int rc = dalloc(&B.pos, nb) | dalloc(&B.trial, nb) | dalloc(&B.type, nb) |
            dalloc(&B.mol_start, in.n_mol + 1) | dalloc(&B.chain_ids, chains.size()) |
            dalloc(&B.ion_ids, ions.size()) | dalloc(&B.fpos, nb) | dalloc(&B.fq, nb) |
-           dalloc(&B.ftrial, c->max_len) | dalloc(&B.bond_mol, in.n_mol);
+           dalloc(&B.ftrial, c->max_len) | dalloc(&B.bond_mol, in.n_mol) |
+           dalloc(&B.ctrial, kCands * (size_t)c->max_len) |
+           dalloc(&B.cftrial, kCands * (size_t)c->max_len);
   if (mirror64) rc |= dalloc(&B.fpos64, nb);
   const int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
   rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
@@ -1922,6 +1947,9 @@ struct plum_batch {
   int groups = 1;
   cudaStream_t s2 = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+  // per chain: the next moves' generation beside the pending ones' energy change
+  cudaStream_t s_gen[2] = {nullptr, nullptr};
+  cudaEvent_t gen_go[2] = {nullptr, nullptr}, gen_done[2] = {nullptr, nullptr};
   int cell_moved = 0;     // longest molecule among them (0: none)
   bool cells_on = true;
   bool cells_built = false;  // a batch of steps with the surrogate has rebuilt them
@@ -2008,7 +2036,7 @@ long batch_kernels(const plum_batch* b, int steps) {
   // descriptor (cell kernel, or the all-pairs kernel), smearing, inference
   const long stage = b->sg ? 3 : 0;
   const long chains = (b->groups > 1 && b->reps.size() > 1) ? 2 : 1;
-  return (cells ? (b->cells_on ? 4 : 1) : 0) + chains * (1 + 2L * steps + steps * stage);
+  return (cells ? (b->cells_on ? 4 : 1) : 0) + chains * (1 + 3L * steps + steps * stage);
 }
 
 // After a batch of steps: when a replica's list of beads that changed cell
@@ -2033,7 +2061,7 @@ int cells_check(plum_batch* b) {
 
 // The step chain of replicas [r0, r0 + n) on stream st with its own slots
 // and work queue.
-void chain_enqueue(plum_batch* b, int steps, int r0, int n, double* slots, int* queue,
+void chain_enqueue(plum_batch* b, int steps, int chain, int r0, int n, double* slots, int* queue,
                    cudaStream_t st) {
   const DevParams* rp = b->d_rp + r0;
   const DevBuffers* rb = b->d_rb + r0;
@@ -2045,14 +2073,22 @@ void chain_enqueue(plum_batch* b, int steps, int r0, int n, double* slots, int* 
     launch_mlp_infer_i(b->sg->net, b->d_desc + (size_t)mlp::kIn * r0, n, nullptr,
                        DaArgs{b->d_sts + r0, b->d_rp + r0}, b->d_err, st);
   };
+  launch_batch_gen(rp, rb, n, true, st);
   launch_batch_serial(rp, rb, item_off, slots, n, kModeGen, st);
-  stage_one();
   for (int i = 0; i < steps; i++) {
+    const bool more = i + 1 < steps;
+    if (more) {
+      cudaEventRecord(b->gen_go[chain], st);
+      cudaStreamWaitEvent(b->s_gen[chain], b->gen_go[chain], 0);
+      launch_batch_gen(rp, rb, n, false, b->s_gen[chain]);
+      cudaEventRecord(b->gen_done[chain], b->s_gen[chain]);
+    }
+    stage_one();
     launch_batch_delta32(rp, rb, n, item_off, slots, b->kt_smem, b->tune, queue, b->d_htab,
                          b->cut_scale, st);
-    int mode = kModeFinish | kModeDecide | (i + 1 < steps ? kModeGen : 0);
-    launch_batch_serial(rp, rb, item_off, slots, n, mode, st);
-    if (i + 1 < steps) stage_one();
+    if (more) cudaStreamWaitEvent(st, b->gen_done[chain], 0);
+    launch_batch_serial(rp, rb, item_off, slots, n,
+                        kModeFinish | kModeDecide | (more ? kModeGen : 0), st);
   }
 }
 
@@ -2064,14 +2100,14 @@ void batch_enqueue(plum_batch* b, int steps) {
   const int R = (int)b->reps.size();
   cells_enqueue(b);
   if (b->groups < 2 || R < 2) {
-    chain_enqueue(b, steps, 0, R, b->d_slots, b->d_queue, b->s);
+    chain_enqueue(b, steps, 0, 0, R, b->d_slots, b->d_queue, b->s);
     return;
   }
   const int h = R / 2;
   cudaEventRecord(b->fork_ev, b->s);
   cudaStreamWaitEvent(b->s2, b->fork_ev, 0);
-  chain_enqueue(b, steps, 0, h, b->d_slots, b->d_queue, b->s);
-  chain_enqueue(b, steps, h, R - h, b->d_slots2, b->d_queue + 2, b->s2);
+  chain_enqueue(b, steps, 0, 0, h, b->d_slots, b->d_queue, b->s);
+  chain_enqueue(b, steps, 1, h, R - h, b->d_slots2, b->d_queue + 2, b->s2);
   cudaEventRecord(b->join_ev, b->s2);
   cudaStreamWaitEvent(b->s, b->join_ev, 0);
 }
@@ -2187,6 +2223,11 @@ int plum_batch_destroy(plum_batch* b) {
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->fork_ev) cudaEventDestroy(b->fork_ev);
   if (b->join_ev) cudaEventDestroy(b->join_ev);
+  for (int q = 0; q < 2; q++) {
+    if (b->gen_go[q]) cudaEventDestroy(b->gen_go[q]);
+    if (b->gen_done[q]) cudaEventDestroy(b->gen_done[q]);
+    if (b->s_gen[q]) cudaStreamDestroy(b->s_gen[q]);
+  }
   if (b->s2) cudaStreamDestroy(b->s2);
   if (b->s) cudaStreamDestroy(b->s);
   delete b;
@@ -2221,7 +2262,13 @@ int plum_batch_create(int n, const char* const* dirs, const char* const* runins,
       cudaStreamCreateWithFlags(&b->s2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->join_ev, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess) {
+      cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&b->s_gen[0], cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&b->s_gen[1], cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->gen_go[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->gen_go[1], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->gen_done[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->gen_done[1], cudaEventDisableTiming) != cudaSuccess) {
     plum_batch_destroy(b);
     return fail(PLUM_ERR_CUDA, "cannot create the batch's streams and events");
   }
@@ -2541,6 +2588,7 @@ int plum_batch_time_kernels(plum_batch* b, int n_steps, double* out4) {
                          b->s);
     });
   };
+  launch_batch_gen(b->d_rp, b->d_rb, R, true, b->s);
   int rc = timed(1, [&] {
     launch_batch_serial(b->d_rp, b->d_rb, b->d_item_off, b->d_slots, R, kModeGen, b->s);
   });
@@ -2551,6 +2599,8 @@ int plum_batch_time_kernels(plum_batch* b, int n_steps, double* out4) {
                          b->d_queue, b->d_htab, b->cut_scale, b->s);
     });
     const int mode = kModeFinish | kModeDecide | (i + 1 < n_steps ? kModeGen : 0);
+    // (here in the same stream, so that each kernel is timed alone)
+    if (!rc && i + 1 < n_steps) launch_batch_gen(b->d_rp, b->d_rb, R, false, b->s);
     if (!rc)
       rc = timed(1, [&] {
         launch_batch_serial(b->d_rp, b->d_rb, b->d_item_off, b->d_slots, R, mode, b->s);

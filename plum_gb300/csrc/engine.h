@@ -51,6 +51,7 @@ constexpr int PLUM_ERR_STREAM_DEV = 6;
 struct DevParams {
   int n_bead, n_mol, n_type, npbc;
   int phantom, grafted, n_chain_total, n_ion_total;  // chain/ion pick lists
+  int max_len;  // beads of the longest molecule
   double box[3], inv_box[3];
   double ebox[3], inv_ebox[3];
   int use_pair, use_ewald, use_bond, use_rigid, use_ext, dipole;
@@ -163,6 +164,29 @@ struct alignas(16) KUnit {
   int kp, km;
 };
 
+// The next step's move, generated while the pending one's energy change is still
+// being computed. Its draws depend on the stream position only (the acceptance
+// test takes one draw, or none), its positions on the outcome too, so there are
+// three candidates: kCandAccept (one draw, the pending trial committed),
+// kCandReject (one draw, not committed), kCandSkip (no draw, not committed: an
+// overlap, a stage-one rejection, or no pending move). The serial step adopts
+// the one that came true.
+constexpr int kCandAccept = 0, kCandReject = 1, kCandSkip = 2, kCands = 3;
+struct MoveCand {
+  int type;     // move type, -1 none
+  int mol, b_lo, b_hi;
+  int overrun;  // the stream ran out while generating it
+  int ext_bad;  // a trial bead overlaps a wall
+  long long pos;  // stream position after its draws
+  double u1;      // delayed acceptance's stage-one draw
+  // walls, sum q dz and the molecule's bonds at the trial positions
+  double ext, dmz, bond;
+};
+struct StepPlan {
+  MoveCand cand[kCands];
+  MoveCand now;  // the pending move's (its sums, for the finish)
+};
+
 struct DevBuffers {  // all pointers: copied word-wise into shared memory by the batch kernels
   double4_32a* pos;
   double4_32a* trial;
@@ -183,6 +207,9 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   int4* fpos;        // [n_bead] current (X, Y, Z, type)
   float* fq;         // [n_bead] charges
   int4* ftrial;      // [max molecule length] trial of the pending move's beads
+  StepPlan* plan;
+  double4_32a* ctrial;  // [kCands][max_len] trial positions of the candidates
+  int4* cftrial;     // [kCands][max_len] their fixed-point mirror (precision form)
   float2* dsk_part32;  // [groups][n_k]
   int* ktile_count;  // [k tiles] arrival tickets (reset by the last arrival)
   int* done_count;   // [1] block arrival ticket of the delta kernel
@@ -240,7 +267,8 @@ void launch_total64(const DevParams& P, const DevBuffers& B, double* out_partial
                     int n_part, cudaStream_t s);
 int total_partials_count(const DevParams& P);
 // S(k) from scratch; part: sk_full_groups() * n_k double2 of scratch owned by
-// the caller (one per context, so contexts on different streams never share it)
+// the caller (one per context, so contexts on different streams never share it;
+// the number does not depend on the beads, which exchanges add to)
 int sk_full_groups(const DevParams& P);
 void launch_sk_full64(const DevParams& P, const DevBuffers& B, double2* part, cudaStream_t s);
 constexpr int kMiscBlocks = 64;  // five sums each
@@ -249,9 +277,11 @@ void launch_misc_total64(const DevParams& P, const DevBuffers& B, double* out, c
 // Serial step: mode bits
 constexpr int kModeFinish = 1;   // reduce partials, compose dE
 constexpr int kModeDecide = 2;   // Metropolis draw from the stream + commit
-constexpr int kModeGen = 4;      // generate the next move from the stream
+constexpr int kModeGen = 4;      // adopt the next move's candidate (launch_gen64 before)
 constexpr int kModeCommit = 8;   // commit/reject by state->last_accept (host decided)
 void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStream_t s);
+// The next move's candidates; first: no move is pending (kCandSkip only).
+void launch_gen64(const DevParams& P, const DevBuffers& B, bool first, cudaStream_t s);
 void launch_set_move(const DevBuffers& B, int mol, int b_lo, int b_hi, cudaStream_t s);
 void launch_observables64(const DevParams& P, const DevBuffers& B, double* per_mol,
                           double* out5, cudaStream_t s);
@@ -353,6 +383,8 @@ void launch_batch_delta32(const DevParams* rp, const DevBuffers* rb, int n_rep, 
                           const float4* htab, float cut_scale, cudaStream_t s);
 void launch_batch_serial(const DevParams* rp, const DevBuffers* rb, const int* item_off,
                          const double* slots, int n_rep, int mode, cudaStream_t s);
+void launch_batch_gen(const DevParams* rp, const DevBuffers* rb, int n_rep, bool first,
+                      cudaStream_t s);
 // per replica r: if need[r], shift the unread words [pos[r], len[r]) of out[r]
 // to the front and fill the rest up to cap[r] from state[r] (625 words)
 void launch_mt_fill_batch(uint32_t* const* states, uint32_t* const* outs, const long long* pos,

@@ -1,19 +1,28 @@
-// Serial part of a Monte Carlo step (one CTA):
+// Serial part of a Monte Carlo step. Two kernels:
 //
-//   finish  adds the per-block partials of k_delta64 in a fixed order, adds
-//           the wall (potential_external.cc:100-117) and bond
-//           (potential_spring.cc:63-80) terms, and composes dE exactly as
+// k_serial64 / k_batch_serial, one block per system, on the step's critical path:
+//   finish  takes the pending move's pair and k sums (the delta kernel's) and its
+//           wall, bond and q dz sums (the generator's) and composes dE exactly as
 //           ForceField::EnergyDifference does (force_field.cc:407-434): pair,
 //           early return at >= 1e8, external, early return, Ewald (real +
 //           reciprocal + the dipole term from the *current* z, which is what
 //           the reference evaluates at potential_ewald.cc:527-531), bond.
 //   decide  one draw u; accept if dE < 1e8 and u < exp(-beta dE); no draw at
 //           dE >= 1e8 (simulation.cc:324-332)
-//   commit  trial -> current, S(k) += dS(k), running totals
-//           (force_field.cc:436-451, simulation.cc:336-351)
-//   gen     the next step's draws in the reference's order: one draw for the
-//           GC check (simulation.cc:221), chain and ion picks, move type
-//           (simulation.cc:247-276), then the move itself (molecule.cc:103-312)
+//   commit  trial -> current, running totals (force_field.cc:436-451,
+//           simulation.cc:336-351); S(k) += dS(k) is left to the next delta kernel
+//   adopt   the next move: the candidate that came true
+//
+// k_gen / k_batch_gen, one block per candidate, beside the energy change:
+//   the next step's draws in the reference's order: one draw for the GC check
+//   (simulation.cc:221), chain and ion picks, move type (simulation.cc:247-276),
+//   then the move itself (molecule.cc:103-312), its walls
+//   (potential_external.cc:100-117), bonds (potential_spring.cc:63-80) and q dz.
+//
+// Generating a move is a chain of dependent draws, scans and FP64 arithmetic on
+// one block; as part of the serial step it stood on the critical path of every
+// move (1,000 beads: 40 us per move with it there, 30 us beside the energy
+// change; 32 replicas of 20,000 beads: the serial step 36 to 24 us).
 //
 // Build note: this file is compiled with -fmad=false. The draw-consuming
 // tests (randSphere's r1^2 + r2^2 > 1, the move-type and pick thresholds)
@@ -254,18 +263,28 @@ __device__ __forceinline__ void pivot_draws(const DevParams& P, int wlen, GenPla
   __syncthreads();
 }
 
+// The positions a candidate starts from: the current ones, with the pending
+// move's trial beads [lo, hi) in their place where it is taken as accepted.
+struct PosView {
+  const double4_32a* pos;
+  const double4_32a* trial;
+  int lo, hi;
+  __device__ __forceinline__ double4_32a at(int i) const {
+    return i >= lo && i < hi ? trial[i] : pos[i];
+  }
+};
+
 // Thread 0, after the move's own draws: delayed acceptance's stage-one draw,
 // the stream check and the stream position.
-__device__ __forceinline__ void gen_tail(DevState* st, const DevBuffers& B, Draws& d,
-                                         GenPlan& plan) {
+__device__ __forceinline__ void gen_tail(const DevState* st, const DevBuffers& B, Draws& d,
+                                         GenPlan& plan, MoveCand& C) {
   // Delayed acceptance: a chain move (pivot, crankshaft, reptation) takes
   // its stage-one draw right after its own draws.
-  if (plan.type >= 2 && st->da_on && B.desc_acc && B.desc_fine) st->da_u1 = d.u();
-  if (d.overrun) {
-    st->error = PLUM_ERR_STREAM_DEV;
-    plan.type = -1;
-  }
-  st->stream_pos = d.pos;
+  C.u1 = 0.0;
+  if (plan.type >= 2 && st->da_on && B.desc_acc && B.desc_fine) C.u1 = d.u();
+  C.overrun = d.overrun;
+  if (d.overrun) plan.type = -1;
+  C.pos = d.pos;
 }
 
 // Thread 0's sequential pivot scan for chains up to kPivotMax beads: records
@@ -287,28 +306,69 @@ __device__ __forceinline__ void pivot_draws_seq(const DevParams& P, Draws& d, lo
   }
 }
 
+// Where a candidate's trial positions go ([max_len], from its b_lo on).
+struct TrialOut {
+  double4_32a* t;
+  int4* f;
+};
+
 // The trial position of bead i, and its fixed-point mirror for the precision
 // form's pair sweep.
-__device__ __forceinline__ void put_trial(const DevParams& P, const DevBuffers& B, int b_lo, int i,
-                                          double4_32a t) {
-  B.trial[i] = t;
-  if (P.form) B.ftrial[i - b_lo] = fix_point(P, t, B.type[i]);
+__device__ __forceinline__ void put_trial(const DevParams& P, const DevBuffers& B, TrialOut O,
+                                          int b_lo, int i, double4_32a t) {
+  O.t[i - b_lo] = t;
+  if (P.form) O.f[i - b_lo] = fix_point(P, t, B.type[i]);
 }
 
-// Generates the next step's trial move into `trial` (and the fixed-point
-// mirror for the precision form); thread 0 consumes the draws, the block
-// applies the geometry.
-__device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B, DevState& S,
-                                      Draws& d, long long wbase, GenPlan& plan, int* s_off,
-                                      int* s_boff, double (*s_w)[kPivotMax],
+// Walls and sum q dz of the moved beads, and the moved molecule's bonds at the
+// trial positions, into C.
+template <class Trial>
+__device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& B, bool on, int mol,
+                                          int b_lo, int b_hi, const PosView& V, const Trial& T,
+                                          MoveCand& C, double* red) {
+  if (threadIdx.x == 0) C.ext_bad = 0;
+  __syncthreads();
+  double ext = 0.0, dmz = 0.0, bt = 0.0;
+  if (on) {
+    for (int i = b_lo + threadIdx.x; i < b_hi; i += blockDim.x) {
+      double4_32a t = T(i), p = V.at(i);
+      if (P.use_ext) {
+        int ty = B.type[i];
+        double en = wall64(P, t.z, ty);
+        if (en >= kVeryLarge) C.ext_bad = 1;  // every writer stores the same value
+        ext += en - wall64(P, p.z, ty);
+      }
+      dmz += t.w * (t.z - p.z);
+    }
+    const int m0 = B.mol_start[mol], m1 = B.mol_start[mol + 1];
+    if (P.use_bond && m1 - m0 > 1)
+      for (int i = m0 + threadIdx.x; i < m1 - 1; i += blockDim.x) {
+        double4_32a p = T(i), q = T(i + 1);
+        double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+        double r = sqrt(dx * dx + dy * dy + dz * dz);
+        bt += 0.5 * P.k_bond * (r - P.r0) * (r - P.r0);
+      }
+  }
+  bsum3<kSerialThreads>(ext, dmz, bt, red);
+  if (threadIdx.x == 0) {
+    C.ext = ext;
+    C.dmz = dmz;
+    C.bond = bt;
+  }
+}
+
+// Generates candidate C from stream position d.pos and positions V; thread 0
+// consumes the draws, the block applies the geometry.
+__device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B,
+                                      const DevState* st, const PosView& V, TrialOut O,
+                                      MoveCand& C, Draws& d, long long wbase, GenPlan& plan,
+                                      int* s_off, int* s_boff, double (*s_w)[kPivotMax],
                                       short (*jump)[kDrawWindow + 1],
-                                      const unsigned* accbits) {
-  DevState* const st = &S;
+                                      const unsigned* accbits, double* red) {
   // ----------------------------------------------------- generate next move
   if (threadIdx.x == 0) {
     plan.type = -1;
     plan.scan = 0;
-    st->step_open = 1;
     (void)d.next();  // simulation.cc:221 (the GC draw)
     const int n_ch = P.n_chain_total, n_io = P.n_ion_total;
     if (P.n_mol - P.phantom > 0) {
@@ -376,15 +436,16 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
           } else {
             plan.pivot = -1;
             const double eq = P.bond_len;
+            O.t[pivot] = V.at(b0 + pivot);
             for (int dirn = 0; dirn < 2; dirn++) {
               double T[3] = {0.0, 0.0, 0.0};
-              double4_32a pv = B.pos[b0 + pivot];
+              double4_32a pv = V.at(b0 + pivot);
               double prev[3] = {pv.x, pv.y, pv.z};
               int i = dirn == 0 ? pivot + 1 : pivot - 1;
               for (; dirn == 0 ? i < len : i >= 0; i += dirn == 0 ? 1 : -1) {
                 double v[3];
                 rand_sphere(d, v, accbits);
-                double4_32a o = B.pos[b0 + i];
+                double4_32a o = V.at(b0 + i);
                 double p[3] = {o.x + T[0], o.y + T[1], o.z + T[2]};
                 double dx = (p[0] + s * v[0]) - prev[0];
                 double dy = (p[1] + s * v[1]) - prev[1];
@@ -397,7 +458,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
                   T[a] += c[a] - p[a];
                   prev[a] = c[a];
                 }
-                B.trial[b0 + i] = make_double4_32a(c[0], c[1], c[2], o.w);
+                O.t[i] = make_double4_32a(c[0], c[1], c[2], o.w);
                 if (d.overrun) break;
               }
             }
@@ -408,7 +469,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
           int first = (int)floor((len - 2) * (double)d.next() / kMtMax);
           int last = (int)floor((len - first) * (double)d.next() / kMtMax) + first;
           if (last > len - 1) last = len - 1;  // the reference reads past the chain here
-          double4_32a pf = B.pos[b0 + first], pl = B.pos[b0 + last];
+          double4_32a pf = V.at(b0 + first), pl = V.at(b0 + last);
           double ax[3] = {pl.x - pf.x, pl.y - pf.y, pl.z - pf.z};
           double z2 = ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2];
           if (z2 > 0) {
@@ -452,7 +513,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
         }
       }
     }
-    if (!plan.scan) gen_tail(st, B, d, plan);
+    if (!plan.scan) gen_tail(st, B, d, plan, C);
   }
   __syncthreads();
   if (plan.scan) {
@@ -464,7 +525,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
         d.pos = wbase + plan.scan_rel;
         pivot_draws_seq(P, d, wbase, plan.b1 - plan.b0, plan.pivot, s_off, s_boff, accbits);
       }
-      gen_tail(st, B, d, plan);
+      gen_tail(st, B, d, plan, C);
     }
     __syncthreads();
   }
@@ -473,19 +534,19 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
   const GenPlan g = plan;
   if (g.type == 0 || g.type == 1) {
     for (int i = g.b_lo + threadIdx.x; i < g.b_hi; i += blockDim.x) {
-      double4_32a o = B.pos[i];
-      put_trial(P, B, g.b_lo, i,
+      double4_32a o = V.at(i);
+      put_trial(P, B, O, g.b_lo, i,
                 make_double4_32a(o.x + g.vec[0], o.y + g.vec[1], o.z + g.vec[2], o.w));
     }
   } else if (g.type == 3) {
-    const double4_32a pf = B.pos[g.b0 + g.first];
+    const double4_32a pf = V.at(g.b0 + g.first);
     for (int i = g.b_lo + threadIdx.x; i < g.b_hi; i += blockDim.x) {
-      double4_32a o = B.pos[i];
+      double4_32a o = V.at(i);
       double v[3] = {o.x - pf.x, o.y - pf.y, o.z - pf.z};
       double r[3];
       for (int a = 0; a < 3; a++)
         r[a] = ((g.R[3 * a] * v[0] + g.R[3 * a + 1] * v[1]) + g.R[3 * a + 2] * v[2]);
-      put_trial(P, B, g.b_lo, i, make_double4_32a(r[0] + pf.x, r[1] + pf.y, r[2] + pf.z, o.w));
+      put_trial(P, B, O, g.b_lo, i, make_double4_32a(r[0] + pf.x, r[1] + pf.y, r[2] + pf.z, o.w));
     }
   } else if (g.type == 2 && g.pivot >= 0) {
     const int len = g.b1 - g.b0, pv = g.pivot;
@@ -497,7 +558,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
       sphere_vec(d.at(wbase + s_off[i]), d.at(wbase + s_off[i] + 1), v);
       double bl = eq;
       if (P.vary_bond) bl += (eq / 5.0) * (unit_draw(d.at(wbase + s_boff[i])) - 0.5);
-      const double4_32a oi = B.pos[g.b0 + i], oj = B.pos[g.b0 + j];
+      const double4_32a oi = V.at(g.b0 + i), oj = V.at(g.b0 + j);
       double dx = (oi.x - oj.x) + g.s * v[0];
       double dy = (oi.y - oj.y) + g.s * v[1];
       double dz = (oi.z - oj.z) + g.s * v[2];
@@ -526,67 +587,94 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
       }
     }
     __syncthreads();
-    const double4_32a pp = B.pos[g.b0 + pv];
+    const double4_32a pp = V.at(g.b0 + pv);
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       const int i = k < nf ? pv + 1 + k : pv - 1 - (k - nf);
-      const double q = B.pos[g.b0 + i].w;
-      put_trial(P, B, g.b_lo, g.b0 + i,
+      const double q = V.at(g.b0 + i).w;
+      put_trial(P, B, O, g.b_lo, g.b0 + i,
                 make_double4_32a(pp.x + s_w[0][k], pp.y + s_w[1][k], pp.z + s_w[2][k], q));
     }
-    // the pivot bead stays where it is (its trial entry equals its position)
-    if (P.form && threadIdx.x == 0)
-      B.ftrial[g.b0 + pv - g.b_lo] = fix_point(P, B.trial[g.b0 + pv], B.type[g.b0 + pv]);
+    // the pivot bead stays where it is
+    if (threadIdx.x == 0) put_trial(P, B, O, g.b_lo, g.b0 + pv, pp);
   } else if (g.type == 4) {
     const int len = g.b1 - g.b0;
     for (int i = threadIdx.x; i < len; i += blockDim.x) {
       double4_32a nw;
       if (i == g.end) {
-        double4_32a o = B.pos[g.b0 + i];
+        double4_32a o = V.at(g.b0 + i);
         nw = make_double4_32a(o.x + g.vec[0], o.y + g.vec[1], o.z + g.vec[2], o.w);
       } else {
-        double4_32a o = B.pos[g.b0 + i + g.dir];
-        nw = make_double4_32a(o.x, o.y, o.z, B.pos[g.b0 + i].w);
+        double4_32a o = V.at(g.b0 + i + g.dir);
+        nw = make_double4_32a(o.x, o.y, o.z, V.at(g.b0 + i).w);
       }
-      put_trial(P, B, g.b_lo, g.b0 + i, nw);
+      put_trial(P, B, O, g.b_lo, g.b0 + i, nw);
     }
   }
-  if (P.form && g.type == 2 && g.pivot < 0) {
+  __syncthreads();
+  if (P.form && g.type == 2 && g.pivot < 0)
     // fixed-point trial coordinates of the sequential pivot
-    __syncthreads();
     for (int i = g.b_lo + threadIdx.x; i < g.b_hi; i += blockDim.x)
-      B.ftrial[i - g.b_lo] = fix_point(P, B.trial[i], B.type[i]);
-  }
-  // surrogate move: its descriptor is accumulated from zero by the next launch
-  const bool surr = g.type >= 2 && B.desc_acc && B.desc_fine && (st->da_on || B.log_desc);
-  if (surr)
-    for (int k = threadIdx.x; k < mlp::kFineAll; k += blockDim.x) B.desc_fine[k] = 0u;
+      O.f[i - g.b_lo] = fix_point(P, O.t[i - g.b_lo], B.type[i]);
+  move_sums(P, B, g.type >= 0, g.mol, g.b_lo, g.b_hi, V,
+            [&](int i) { return i >= g.b_lo && i < g.b_hi ? O.t[i - g.b_lo] : V.at(i); }, C, red);
   if (threadIdx.x == 0) {
-    st->da_active = surr ? 1 : 0;
-    st->da_skip = 0;
+    C.type = g.type;
     if (g.type >= 0) {
-      st->pending = 1;
-      st->mol = g.mol;
-      st->b_lo = g.b_lo;
-      st->b_hi = g.b_hi;
-      st->move_type = g.type;
-    } else {
-      st->pending = 0;
+      C.mol = g.mol;
+      C.b_lo = g.b_lo;
+      C.b_hi = g.b_hi;
     }
   }
 }
 
-// Shared memory of one serial step.
-struct SerialSmem {
+// Shared memory of one candidate's generation.
+struct GenSmem {
   uint32_t win[kDrawWindow];
   unsigned accbits[kDrawWindow / 32];  // randSphere acceptance per position
   double red[3 * (kSerialThreads / 32)];
   GenPlan plan;
-  int s_accept, s_ext_bad;
   int s_off[kPivotMax], s_boff[kPivotMax];  // draw offsets per bead
   union {
     short jump[kJumpLevels][kDrawWindow + 1];  // pivot draws: 2^l beads on
     double s_w[3][kPivotMax];                  // pivot bond steps (used after)
   };
+  MoveCand C;
+};
+
+// Candidate c of the step after the pending move.
+__device__ __forceinline__ void gen_body(const DevParams& P, const DevBuffers& B, int c,
+                                         GenSmem& sm) {
+  const DevState* st = B.state;
+  const int pending = st->pending;
+  if (st->error || (!pending && c != kCandSkip)) return;
+  const long long base = st->stream_pos + (c == kCandSkip ? 0 : 1), len = st->stream_len;
+  const long long avail = len - base;
+  const int wlen = (int)(avail < kDrawWindow ? (avail > 0 ? avail : 0) : kDrawWindow);
+  for (int i = threadIdx.x; i < wlen; i += blockDim.x) sm.win[i] = B.stream[base + i];
+  __syncthreads();
+  // every window position's randSphere test, one position per thread; a
+  // warp's ballot makes the word of its 32 positions
+  for (int p0 = threadIdx.x & ~31; p0 < kDrawWindow; p0 += blockDim.x) {
+    const int p = p0 + (threadIdx.x & 31);
+    const bool ok = p + 1 < wlen && !sphere_reject(sm.win[p], sm.win[p + 1]);
+    const unsigned bits = __ballot_sync(0xFFFFFFFFu, ok);
+    if ((threadIdx.x & 31) == 0) sm.accbits[p0 >> 5] = bits;
+  }
+  __syncthreads();
+  Draws d{B.stream, sm.win, base, len, base, wlen, 0};
+  const bool took = c == kCandAccept;
+  const PosView V{B.pos, B.trial, took ? st->b_lo : 0, took ? st->b_hi : 0};
+  const TrialOut O{B.ctrial + (size_t)c * P.max_len, B.cftrial + (size_t)c * P.max_len};
+  gen_move(P, B, st, V, O, sm.C, d, base, sm.plan, sm.s_off, sm.s_boff, sm.s_w, sm.jump, sm.accbits,
+           sm.red);
+  if (threadIdx.x == 0) B.plan->cand[c] = sm.C;
+}
+
+// Shared memory of one serial step.
+struct SerialSmem {
+  double red[3 * (kSerialThreads / 32)];
+  int s_accept, s_cand;
+  StepPlan plan;
   // The state lives in shared memory for the step: thread 0's chain of
   // decisions then never waits on global memory for it.
   DevState S;
@@ -601,22 +689,18 @@ struct SlotSums {
 
 __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers& B, int mode,
                                             SerialSmem& sm, const SlotSums* slots) {
-  uint32_t* const win = sm.win;
-  unsigned* const accbits = sm.accbits;
   double* const red = sm.red;
-  GenPlan& plan = sm.plan;
   int& s_accept = sm.s_accept;
-  int& s_ext_bad = sm.s_ext_bad;
-  int* const s_off = sm.s_off;
-  int* const s_boff = sm.s_boff;
-  double(*const s_w)[kPivotMax] = sm.s_w;
-  short(*const jump)[kDrawWindow + 1] = sm.jump;
   DevState& S = sm.S;
   {
     const int nw = (int)(sizeof(DevState) / sizeof(int));
     const int* src = reinterpret_cast<const int*>(B.state);
     int* dst = reinterpret_cast<int*>(&S);
     for (int i = threadIdx.x; i < nw; i += blockDim.x) dst[i] = src[i];
+    const int np = (int)(sizeof(StepPlan) / sizeof(int));
+    src = reinterpret_cast<const int*>(B.plan);
+    dst = reinterpret_cast<int*>(&sm.plan);
+    for (int i = threadIdx.x; i < np; i += blockDim.x) dst[i] = src[i];
   }
   __syncthreads();
   if (S.error) return;
@@ -637,27 +721,11 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
     __syncthreads();
   }
 
-  // Stage the next stream words.
-  const long long wbase = S.stream_pos;
-  int wlen = 0;
-  if (mode & (kModeDecide | kModeGen)) {
-    long long avail = S.stream_len - wbase;
-    wlen = (int)(avail < kDrawWindow ? (avail > 0 ? avail : 0) : kDrawWindow);
-    for (int i = threadIdx.x; i < wlen; i += blockDim.x) win[i] = B.stream[wbase + i];
-  }
-  __syncthreads();
-  if (mode & kModeGen) {
-    // every window position's randSphere test, one position per thread; a
-    // warp's ballot makes the word of its 32 positions
-    for (int p0 = threadIdx.x & ~31; p0 < kDrawWindow; p0 += blockDim.x) {
-      const int p = p0 + (threadIdx.x & 31);
-      const bool ok = p + 1 < wlen && !sphere_reject(win[p], win[p + 1]);
-      const unsigned bits = __ballot_sync(0xFFFFFFFFu, ok);
-      if ((threadIdx.x & 31) == 0) accbits[p0 >> 5] = bits;
-    }
-    __syncthreads();
-  }
-  Draws d{B.stream, win, wbase, S.stream_len, wbase, wlen, 0};
+  // the acceptance test's draw, loaded while dE is composed
+  uint32_t word = 0;
+  const int have = (mode & kModeDecide) && S.stream_pos < S.stream_len ? 1 : 0;
+  if (have && threadIdx.x == 0) word = B.stream[S.stream_pos];
+  Draws d{B.stream, &word, S.stream_pos, S.stream_len, S.stream_pos, have, 0};
 
   const int pending = S.pending;
   const int b_lo = S.b_lo, b_hi = S.b_hi, mol = S.mol;
@@ -682,31 +750,14 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
     }
     __syncthreads();
   } else if ((mode & kModeFinish) && pending) {
-    // walls of the moved beads, sum q dz
-    if (threadIdx.x == 0) s_ext_bad = 0;
-    __syncthreads();
-    double ext = 0.0, dmz = 0.0;
-    for (int i = b_lo + threadIdx.x; i < b_hi; i += blockDim.x) {
-      double4_32a t = B.trial[i], p = B.pos[i];
-      if (P.use_ext) {
-        int ty = B.type[i];
-        double en = wall64(P, t.z, ty);
-        if (en >= kVeryLarge) s_ext_bad = 1;
-        ext += en - wall64(P, p.z, ty);
-      }
-      dmz += t.w * (t.z - p.z);
-    }
-    // bonds of the moved molecule at trial positions
+    // a move set by the host has no candidate's sums
+    MoveCand& now = sm.plan.now;
+    if (S.move_type < 0)
+      move_sums(P, B, true, mol, b_lo, b_hi, PosView{B.pos, B.trial, 0, 0},
+                [&](int i) { return B.trial[i]; }, now, red);
+    const double ext = now.ext, dmz = now.dmz, bt = now.bond;
+    const int ext_bad = now.ext_bad;
     const int m0 = B.mol_start[mol], m1 = B.mol_start[mol + 1];
-    double bt = 0.0;
-    if (P.use_bond && m1 - m0 > 1)
-      for (int i = m0 + threadIdx.x; i < m1 - 1; i += blockDim.x) {
-        double4_32a p = B.trial[i], q = B.trial[i + 1];
-        double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        double r = sqrt(dx * dx + dy * dy + dz * dz);
-        bt += 0.5 * P.k_bond * (r - P.r0) * (r - P.r0);
-      }
-    bsum3<kSerialThreads>(ext, dmz, bt, red);
     if (threadIdx.x == 0) {
       // the delta kernel applied any pending S(k) commit if it ran k tiles
       if (P.use_ewald && b_hi > b_lo) S.sk_pending = 0;
@@ -720,7 +771,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
         done = de >= kVeryLarge;
       }
       if (!done && P.use_ext) {
-        dx = s_ext_bad ? kVeryLarge : ext;
+        dx = ext_bad ? kVeryLarge : ext;
         de += dx;
         done = de >= kVeryLarge;
       }
@@ -764,6 +815,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
   if ((mode & (kModeDecide | kModeCommit)) && pending) {
     if (threadIdx.x == 0) {
       int acc = 0;
+      const long long at = d.pos;
       if (mode & kModeDecide) {
         if (S.da_active && S.da_on) {
           // Delayed acceptance, stage two: with the stage-one probability
@@ -783,6 +835,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
         acc = S.last_accept;
       }
       s_accept = acc;
+      sm.s_cand = acc ? kCandAccept : (d.pos != at ? kCandReject : kCandSkip);
     }
     __syncthreads();
     const int acc = s_accept;
@@ -854,11 +907,42 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
   }
   __syncthreads();
 
-  if ((mode & kModeGen) && !S.error)
-    gen_move(P, B, S, d, wbase, plan, s_off, s_boff, s_w, jump, accbits);
+  if ((mode & kModeGen) && !S.error) {
+    const int c = pending ? sm.s_cand : kCandSkip;
+    const MoveCand& C = sm.plan.cand[c];
+    const double4_32a* t = B.ctrial + (size_t)c * P.max_len;
+    const int4* f = B.cftrial + (size_t)c * P.max_len;
+    if (C.type >= 0)
+      for (int i = threadIdx.x; i < C.b_hi - C.b_lo; i += blockDim.x) {
+        B.trial[C.b_lo + i] = t[i];
+        if (P.form) B.ftrial[i] = f[i];
+      }
+    // surrogate move: its descriptor is accumulated from zero by the next launch
+    const bool surr = C.type >= 2 && B.desc_acc && B.desc_fine && (S.da_on || B.log_desc);
+    if (surr)
+      for (int k = threadIdx.x; k < mlp::kFineAll; k += blockDim.x) B.desc_fine[k] = 0u;
+    if (threadIdx.x == 0) {
+      S.step_open = 1;
+      S.stream_pos = C.pos;
+      if (C.overrun) S.error = PLUM_ERR_STREAM_DEV;
+      S.da_active = surr ? 1 : 0;
+      S.da_skip = 0;
+      if (surr && S.da_on) S.da_u1 = C.u1;
+      if (C.type >= 0) {
+        S.pending = 1;
+        S.mol = C.mol;
+        S.b_lo = C.b_lo;
+        S.b_hi = C.b_hi;
+        S.move_type = C.type;
+        B.plan->now = C;
+      } else {
+        S.pending = 0;
+      }
+    }
+  }
 
   // write the state back
-  if (threadIdx.x == 0) S.stream_pos = S.stream_pos > d.pos ? S.stream_pos : d.pos;
+  if (threadIdx.x == 0 && S.stream_pos < d.pos) S.stream_pos = d.pos;
   __syncthreads();
   {
     const int nw = (int)(sizeof(DevState) / sizeof(int));
@@ -874,6 +958,20 @@ __global__ void __launch_bounds__(kSerialThreads)
   serial_body(P, B, mode, sm, nullptr);
 }
 
+// A replica's parameters and buffers into shared memory.
+__device__ __forceinline__ void stage_system(const DevParams* rp, const DevBuffers* rb,
+                                             DevParams& P, DevBuffers& B) {
+  const int* src = reinterpret_cast<const int*>(rp);
+  int* dst = reinterpret_cast<int*>(&P);
+  for (int i = threadIdx.x; i < (int)(sizeof(DevParams) / sizeof(int)); i += blockDim.x)
+    dst[i] = src[i];
+  const long long* bs = reinterpret_cast<const long long*>(rb);
+  long long* bd = reinterpret_cast<long long*>(&B);
+  for (int i = threadIdx.x; i < (int)(sizeof(DevBuffers) / sizeof(long long)); i += blockDim.x)
+    bd[i] = bs[i];
+  __syncthreads();
+}
+
 // One block per replica: the replica's parameters and buffers are staged in
 // shared memory, then the same serial step runs on them.
 __global__ void __launch_bounds__(kSerialThreads)
@@ -883,20 +981,35 @@ __global__ void __launch_bounds__(kSerialThreads)
   __shared__ DevParams P;
   __shared__ DevBuffers B;
   const int r = blockIdx.x;
-  {
-    const int* src = reinterpret_cast<const int*>(rp + r);
-    int* dst = reinterpret_cast<int*>(&P);
-    for (int i = threadIdx.x; i < (int)(sizeof(DevParams) / sizeof(int)); i += blockDim.x)
-      dst[i] = src[i];
-    const long long* bs = reinterpret_cast<const long long*>(rb + r);
-    long long* bd = reinterpret_cast<long long*>(&B);
-    for (int i = threadIdx.x; i < (int)(sizeof(DevBuffers) / sizeof(long long)); i += blockDim.x)
-      bd[i] = bs[i];
-  }
-  __syncthreads();
+  stage_system(rp + r, rb + r, P, B);
   SlotSums ss{slots, item_off[4 * r], item_off[4 * r + 1], item_off[4 * r + 2],
               item_off[4 * r + 3]};
   serial_body(P, B, mode, sm, &ss);
+}
+
+__global__ void __launch_bounds__(kSerialThreads)
+    k_gen(const DevParams P, const DevBuffers B, int c0) {
+  __shared__ GenSmem sm;
+  gen_body(P, B, c0 + (int)blockIdx.x, sm);
+}
+
+__global__ void __launch_bounds__(kSerialThreads)
+    k_batch_gen(const DevParams* __restrict__ rp, const DevBuffers* __restrict__ rb, int c0) {
+  __shared__ GenSmem sm;
+  __shared__ DevParams P;
+  __shared__ DevBuffers B;
+  stage_system(rp + blockIdx.x, rb + blockIdx.x, P, B);
+  gen_body(P, B, c0 + (int)blockIdx.y, sm);
+}
+
+void launch_gen64(const DevParams& P, const DevBuffers& B, bool first, cudaStream_t s) {
+  k_gen<<<first ? 1 : kCands, kSerialThreads, 0, s>>>(P, B, first ? kCandSkip : 0);
+}
+
+void launch_batch_gen(const DevParams* rp, const DevBuffers* rb, int n_rep, bool first,
+                      cudaStream_t s) {
+  k_batch_gen<<<dim3(n_rep, first ? 1 : kCands), kSerialThreads, 0, s>>>(rp, rb,
+                                                                        first ? kCandSkip : 0);
 }
 
 void launch_batch_serial(const DevParams* rp, const DevBuffers* rb, const int* item_off,
