@@ -261,6 +261,7 @@ void launch_slit_pressure(const SlitPressParams& S, const DevParams& P, const De
 
 // Launch helpers (kern_energy.cu / kern_moves.cu). All enqueue on `s`.
 int pair_grid();
+int delta_blocks64();  // blocks of the FP64 energy change, four partial sums each
 int ktile_count(const DevParams& P);
 void launch_delta_pairs64(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 void launch_total64(const DevParams& P, const DevBuffers& B, double* out_partials,

@@ -146,33 +146,36 @@ __device__ __forceinline__ FixConst fix_const(const DevParams& P) {
 }
 
 // ---------------------------------------------------------------- delta
-// One launch per move, two kinds of blocks side by side on every SM:
+// One launch per move, one block per SM. Four of its warps (k role) own a run of
+// k units, so dS(k), the commit of the last accepted change and the |S|^2 change
+// need no other block; their work is FP64. The other twelve (pair role) deal out
+// the m x N (moved, other) pairs; in the integer form (fix_pair.h) a thread takes
+// one other bead against a run of moved beads, its sums staying integers over
+// beads of one charge, so the two roles load different pipes. Each block leaves
+// three sums to the serial step, which adds the blocks in order: a ticket and a
+// last block doing so cost 3 us per move, and three blocks per SM a second wave.
+// Pairs with both beads moved are taken once (j > i), at trial positions for both.
 //
-// k blocks (the first kgrid) own a run of k units each, so dS(k), the commit of
-// the last accepted change and the |S|^2 change need no other block: a warp's
-// lanes take 32 units, its eight warps share the moved beads, and the block
-// adds the eight sums. Their work is FP64.
-//
-// Pair blocks deal out the m x N (moved, other) pairs. In the integer form
-// (fix_pair.h) a thread takes one other bead against a run of kFixRun moved
-// beads: the sums stay integers over beads of one charge and meet the FP64 pipe
-// once per run, so the k blocks keep that pipe and the pair blocks the integer
-// one. Pairs with both beads moved are taken once (j > i), at trial positions
-// for both.
-//
-// A move of the 20,000-bead system (7,812 k-vectors), the serial step included:
-// 71 us, 130 us with FP64 pairs and k tiles x bead groups joined by tickets; of
-// the 1,000-bead system with r_c = 0.7 L (image cells): 41 us, 94 us before.
+// A move with its serial step (kern_moves.cu): 23 us for 1,000 beads and 1,687
+// k-vectors, 24 us with image cells, 46 us for 20,000 beads and 7,812 k-vectors
+// (50, 94 and 130 us with FP64 pairs, k tiles x bead groups and a move generated
+// in the serial step).
+constexpr int kDeltaThreads = 512;
+constexpr int kKThreads = 128;  // k role
 constexpr int kFixStage = 256;  // moved beads staged at a time
-constexpr int kFixRun = 4;      // moved beads per thread and other bead
-constexpr int kUnits = 32;      // k units of a k block at a time
-constexpr int kDeltaWarps = kPairThreads / 32;
+constexpr int kFixRun = 4;      // most moved beads per thread and other bead
+constexpr int kUnits = 32;      // k units of a block at a time
 
-// Moved beads per phase-table chunk of a k block: 32 where their z tables and xy
+// Moved beads per phase-table chunk of the k role: 32 where their z tables and xy
 // parts fit the table budget.
 __host__ __device__ inline int k_beads(const DevParams& P) {
   const int fit = kKTableBytes / (2 * (P.kmax[2] + 1 + kUnits) * (int)sizeof(double2));
   return fit < 1 ? 1 : (fit > 32 ? 32 : fit);
+}
+
+// Barrier of one role's threads.
+__device__ __forceinline__ void role_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 struct FixStage {
@@ -197,21 +200,46 @@ __device__ __forceinline__ double fix_near(const DevParams& P, const FixConst& F
                             : real_term64(P, raw * F.s2) / P.sqrt_alpha;
 }
 
-// The integer pair sweep of pair block `blk` of `nblk`.
+// The integer pair sweep of pair thread t of nt in every block. The table is
+// read in place for a few pairs per thread; for more it is copied to shared
+// memory first, where a warp's gather goes at a bank's pace (10 cycles a load)
+// and not a line's (32): from 4 pairs a thread on, the copy (51 KB a block, about
+// 1 us) pays.
+constexpr int kFixStagePairs = 4;
+
 template <int kMode>
 __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& B, FixStage* st,
-                                          int blk, int nblk, int b_lo, int m, double& acc_lj,
-                                          double& acc_re) {
+                                          unsigned char* tabs, int t0, int nt, int b_lo, int m,
+                                          double& acc_lj, double& acc_re) {
   const FixTab T = P.fx;
   const FixConst F = fix_const(P);
   const double qs = F.pref * T.unit, hs = 1.0 / T.unit;
-  const auto tab = [&](uint64_t s) { return fix_h(T.c01, T.c23, T.c45, T.base, s); };
   const int N = P.n_bead;
+  const int G = (int)gridDim.x * nt, p0 = (int)blockIdx.x * nt + t0;
+  const long long pairs = (long long)m * N;
+  const FixPair64* c01 = T.c01;
+  const FixPair64* c23 = T.c23;
+  const FixPair32* c45 = T.c45;
+  if (pairs >= (long long)kFixStagePairs * G) {
+    FixPair64* s01 = reinterpret_cast<FixPair64*>(tabs);
+    FixPair64* s23 = s01 + T.n_bin;
+    FixPair32* s45 = reinterpret_cast<FixPair32*>(s23 + T.n_bin);
+#pragma unroll 4
+    for (int i = t0; i < T.n_bin; i += nt) {
+      s01[i] = c01[i];
+      s23[i] = c23[i];
+      s45[i] = c45[i];
+    }
+    c01 = s01, c23 = s23, c45 = s45;
+  }
+  const auto tab = [&](uint64_t s) { return fix_h(c01, c23, c45, T.base, s); };
+  // a run of moved beads per job, shorter while there are fewer jobs than threads
+  const int run_len = pairs >= 2LL * kFixRun * G ? kFixRun : (pairs >= 4LL * G ? 2 : 1);
   double lj1 = 0.0, lj0 = 0.0;
   for (int g0 = 0; g0 < m; g0 += kFixStage) {
     const int gn = min(kFixStage, m - g0);
-    __syncthreads();  // the previous group is consumed
-    for (int t = threadIdx.x; t < gn; t += blockDim.x) {
+    if (g0) role_sync(2, nt);  // the previous group is consumed
+    for (int t = t0; t < gn; t += nt) {
       const int i = b_lo + g0 + t;
       const ulonglong4_32a a = fix64x4(P, B.trial[i]), c = B.fpos64[i];
       st[t].a = make_ulonglong2(a.x, a.y);
@@ -220,10 +248,9 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
       st[t].q = __longlong_as_double((long long)c.w) * qs;
       st[t].k = B.type[i] * P.n_type;
     }
-    __syncthreads();
-    const int runs = (gn + kFixRun - 1) / kFixRun;
+    role_sync(2, nt);
+    const int runs = (gn + run_len - 1) / run_len;
     // job run * N + j, dealt with stride G; (run, j) advanced without a division
-    const int G = nblk * (int)blockDim.x, p0 = blk * (int)blockDim.x + (int)threadIdx.x;
     const int gq = G / N, gr = G % N;
     for (int run = p0 / N, j = p0 % N; run < runs; run += gq, j += gr) {
       if (j >= N) {
@@ -237,7 +264,7 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
       const int l = j - b_lo - g0;
       const bool jm = j >= b_lo && j < b_lo + m;
       const ulonglong4_32a o1 = jm ? fix64x4(P, B.trial[j]) : o0;
-      const int u0 = run * kFixRun, u1 = min(gn, u0 + kFixRun);
+      const int u0 = run * run_len, u1 = min(gn, u0 + run_len);
       double acc = 0.0, q = st[u0].q;
       int64_t sum = 0;
       for (int u = u0; u < u1; u++) {
@@ -268,40 +295,43 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
   acc_lj += lj1 - lj0;
 }
 
-// dS(k), the S(k) commit and the |S|^2 change of units [u0, u1) (k block).
+// dS(k), the S(k) commit and the |S|^2 change of units [u0, u1) by the k role's
+// threads. A thread takes one of up to 32 units and every slices-th moved bead (a
+// block of a small k-set has few units: their beads then spread over the lanes).
 // smem, kb = k_beads: [kb][2][zn] e^{i n theta_z}, then [kb][2][kUnits] xy parts.
-__device__ __forceinline__ double k_block(const DevParams& P, const DevBuffers& B,
-                                          unsigned char* smem, int u0, int u1, int b_lo, int b_hi,
-                                          int sk_pend, int sk_buf, int cur_buf) {
+__device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B,
+                                         unsigned char* smem, int u0, int u1, int b_lo, int b_hi,
+                                         int sk_pend, int sk_buf, int cur_buf) {
   const int zn = P.kmax[2] + 1, kb = k_beads(P);
   double2* s_z = reinterpret_cast<double2*>(smem);
   double2* s_xy = s_z + (size_t)kb * 2 * zn;
   __shared__ short2 s_col[kUnits];
-  __shared__ int s_ncol;
-  __shared__ double s_sum[kDeltaWarps][4][kUnits];
+  __shared__ double s_sum[4][kKThreads];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double e = 0.0;
   for (int c0 = u0; c0 < u1; c0 += kUnits) {
     const int un = min(kUnits, u1 - c0);
-    const KUnit ku = lane < un ? B.ku[c0 + lane] : KUnit{0, 0, 0, 0, -1, -1};
-    // the units' (nx, ny) columns, numbered in order
-    const int px = __shfl_up_sync(0xffffffffu, ku.nx, 1), py = __shfl_up_sync(0xffffffffu, ku.ny, 1);
-    const bool head = lane < un && (lane == 0 || px != ku.nx || py != ku.ny);
+    // the units' (nx, ny) columns, numbered in order (the same in every warp)
+    const KUnit lu = lane < un ? B.ku[c0 + lane] : KUnit{0, 0, 0, 0, -1, -1};
+    const int px = __shfl_up_sync(0xffffffffu, lu.nx, 1), py = __shfl_up_sync(0xffffffffu, lu.ny, 1);
+    const bool head = lane < un && (lane == 0 || px != lu.nx || py != lu.ny);
     const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const int col = __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
-    int zmax = lane < un ? ku.nz : 0;
+    const int ncol = __popc(heads);
+    int zmax = lane < un ? lu.nz : 0;
     for (int o = 16; o > 0; o >>= 1) zmax = max(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
-    __syncthreads();  // the previous units are done with the tables
-    if (warp == 0 && head) s_col[col] = make_short2(ku.nx, ku.ny);
-    if (threadIdx.x == 0) s_ncol = __popc(heads);
+    const int slices = kKThreads / un;
+    const int u = (int)threadIdx.x % un, sl = (int)threadIdx.x / un;
+    const int col = __popc(heads & (0xffffffffu >> (31 - u))) - 1;
+    const int nz = __shfl_sync(0xffffffffu, (int)lu.nz, u);
+    if (warp == 0 && head)
+      s_col[__popc(heads & (0xffffffffu >> (31 - lane))) - 1] = make_short2(lu.nx, lu.ny);
     double2 A = make_double2(0.0, 0.0), Bs = A;
     for (int g0 = b_lo; g0 < b_hi; g0 += kb) {
-      const int cnt = min(kb, b_hi - g0);
-      __syncthreads();
-      const int ncol = s_ncol, nt = cnt * 2;
+      const int nt = 2 * min(kb, b_hi - g0);
+      role_sync(1, kKThreads);  // the tables (and s_sum) are free, s_col is written
       // nt z recursions, then nt x ncol xy phases, one per thread
-      for (int t = threadIdx.x; t < nt * (1 + ncol); t += blockDim.x) {
-        const int it = t % nt, c = t / nt - 1;
+      for (int t = threadIdx.x; t < nt * (1 + ncol); t += kKThreads) {
+        const int c = t / nt - 1, it = t - (c + 1) * nt;
         const double4_32a p = (it & 1) ? B.pos[g0 + (it >> 1)] : B.trial[g0 + (it >> 1)];
         if (c < 0) {
           const double2 e1 = turn_exp(turn64(P, p.z, 2));
@@ -320,25 +350,29 @@ __device__ __forceinline__ double k_block(const DevParams& P, const DevBuffers& 
           s_xy[it * kUnits + c] = make_double2(q * v.x, q * v.y);
         }
       }
-      __syncthreads();
-      if (lane < un)
-        for (int it = warp; it < nt; it += kDeltaWarps)
-          unit_add(s_xy[it * kUnits + col], s_z[(size_t)it * zn + ku.nz], A, Bs);
+      role_sync(1, kKThreads);
+      if (sl < slices)
+        for (int it = sl; it < nt; it += slices)
+          unit_add(s_xy[it * kUnits + col], s_z[(size_t)it * zn + nz], A, Bs);
     }
-    s_sum[warp][0][lane] = A.x;
-    s_sum[warp][1][lane] = A.y;
-    s_sum[warp][2][lane] = Bs.x;
-    s_sum[warp][3][lane] = Bs.y;
-    __syncthreads();
+    s_sum[0][threadIdx.x] = A.x;
+    s_sum[1][threadIdx.x] = A.y;
+    s_sum[2][threadIdx.x] = Bs.x;
+    s_sum[3][threadIdx.x] = Bs.y;
+    role_sync(1, kKThreads);
+    // the slices of each (unit, sum), added in order by a thread each
+    if ((int)threadIdx.x < 4 * un) {
+      const int q = (int)threadIdx.x / un, v = (int)threadIdx.x % un;
+      double t = 0.0;
+      for (int w = 0; w < slices; w++) t += s_sum[q][w * un + v];
+      s_sum[q][v] = t;  // slice 0's place: read by this thread only
+    }
+    role_sync(1, kKThreads);
     if (warp < 2 && lane < un) {  // warp 0: +nz, warp 1: -nz
-      double v[4];
-      for (int q = 0; q < 4; q++) {
-        v[q] = 0.0;
-        for (int w = 0; w < kDeltaWarps; w++) v[q] += s_sum[w][q][lane];
-      }
-      const int k = warp == 0 ? ku.kp : ku.km;
+      const int k = warp == 0 ? lu.kp : lu.km;
       if (k >= 0) {
-        const double2 SA = make_double2(v[0], v[1]), SB = make_double2(v[2], v[3]);
+        const double2 SA = make_double2(s_sum[0][lane], s_sum[1][lane]);
+        const double2 SB = make_double2(s_sum[2][lane], s_sum[3][lane]);
         const double2 ds = warp == 0 ? unit_plus(SA, SB) : unit_minus(SA, SB);
         double2 s = B.sk[k];
         if (sk_pend) {
@@ -354,38 +388,41 @@ __device__ __forceinline__ double k_block(const DevParams& P, const DevBuffers& 
   return e;
 }
 
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 template <int kMode>
-__global__ void __launch_bounds__(kPairThreads, 2)
-    k_delta64(const DevParams P, const DevBuffers B, int kgrid) {
+__global__ void __launch_bounds__(kDeltaThreads, 1)
+    k_delta64(const DevParams P, const DevBuffers B, int tab_bytes) {
   extern __shared__ __align__(32) unsigned char smem[];
-  __shared__ double red[kPairThreads / 32];
-  __shared__ int s_final;
+  __shared__ double s_part[kDeltaThreads / 32][2];
   const DevState* st = B.state;
   const int b_lo = st->b_lo, b_hi = st->b_hi;
   const int m = st->pending ? b_hi - b_lo : 0;
-  const int N = P.n_bead;
-  if ((int)blockIdx.x < kgrid) {
-    double e = 0.0;
-    if (P.use_ewald && m > 0) {
-      const int u0 = (int)((long long)P.n_ku * blockIdx.x / kgrid);
-      const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / kgrid);
-      e = k_block(P, B, smem, u0, u1, b_lo, b_hi, st->sk_pending, st->sk_buf, st->cur_buf);
-    }
-    e = block_sum<kPairThreads>(e, red);
-    if (threadIdx.x == 0) B.partial[4 * blockIdx.x] = e;
+  const int kthreads = P.use_ewald && P.n_ku > 0 ? kKThreads : 0;
+  const int warp = threadIdx.x >> 5;
+  double a = 0.0, b = 0.0;  // k role: k energy; pair role: LJ and real space
+  if ((int)threadIdx.x < kthreads) {
+    const int u0 = (int)((long long)P.n_ku * blockIdx.x / gridDim.x);
+    const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / gridDim.x);
+    if (m > 0)
+      a = k_role(P, B, smem + tab_bytes, u0, u1, b_lo, b_hi, st->sk_pending, st->sk_buf,
+                 st->cur_buf);
   } else {
-    const int blk = blockIdx.x - kgrid, nblk = gridDim.x - kgrid;
-    double acc_lj = 0.0, acc_re = 0.0;
+    const int t0 = (int)threadIdx.x - kthreads, nt = kDeltaThreads - kthreads;
+    const int N = P.n_bead;
     if (kMode) {
       if (m > 0)
-        fix_sweep<kMode>(P, B, reinterpret_cast<FixStage*>(smem), blk, nblk, b_lo, m, acc_lj,
-                         acc_re);
+        fix_sweep<kMode>(P, B, reinterpret_cast<FixStage*>(smem),
+                         smem + kFixStage * sizeof(FixStage), t0, nt, b_lo, m, a, b);
     } else if (P.use_pair || P.use_ewald) {
       // pair p = ii * N + j, dealt with stride G; (ii, j) advanced without a
       // division per pair
       const long long total = (long long)m * N;
-      const long long G = (long long)nblk * blockDim.x;
-      const long long p0 = (long long)blk * blockDim.x + threadIdx.x;
+      const long long G = (long long)gridDim.x * nt;
+      const long long p0 = (long long)blockIdx.x * nt + t0;
       const int gq = (int)(G / N), gr = (int)(G % N);
       int ii = (int)(p0 / N), j = (int)(p0 % N);
       for (long long p = p0; p < total; p += G, ii += gq, j += gr) {
@@ -403,45 +440,27 @@ __global__ void __launch_bounds__(kPairThreads, 2)
         double l1 = 0, r1 = 0, l0 = 0, r0 = 0;
         pair64(P, ti, tyi, tj, tyj, l1, r1);
         pair64(P, ci, tyi, cj, tyj, l0, r0);
-        if (!hs_bonded(P, B.mol_start, i, j)) acc_lj += l1 - l0;
-        acc_re += r1 - r0;
+        if (!hs_bonded(P, B.mol_start, i, j)) a += l1 - l0;
+        b += r1 - r0;
       }
-    }
-    const double t0 = block_sum<kPairThreads>(acc_lj, red);
-    const double t1 = block_sum<kPairThreads>(acc_re, red);
-    if (threadIdx.x == 0) {
-      B.partial[4 * blockIdx.x + 0] = t0;
-      B.partial[4 * blockIdx.x + 1] = t1;
     }
   }
-  // Last block to finish adds every block's sums in a fixed order
-  // (deterministic) for the serial kernel.
-  __threadfence();
+  // (LJ is zero in most warps)
+  __syncwarp();
+  if (__any_sync(0xffffffffu, a != 0.0)) a = warp_sum(a);
+  if ((int)threadIdx.x >= kthreads) b = warp_sum(b);
+  if ((threadIdx.x & 31) == 0) {
+    s_part[warp][0] = a;
+    s_part[warp][1] = b;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) s_final = atomicAdd(B.done_count, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (s_final) {
-    __threadfence();
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-      const double x = __ldcg(&B.partial[4 * i]);
-      if (i < kgrid) {
-        c += x;
-      } else {
-        a += x;
-        b += __ldcg(&B.partial[4 * i + 1]);
-      }
-    }
-    a = block_sum<kPairThreads>(a, red);
-    b = block_sum<kPairThreads>(b, red);
-    c = block_sum<kPairThreads>(c, red);
-    if (threadIdx.x == 0) {
-      DevState* ws = B.state;
-      ws->red_lj = a;
-      ws->red_re = b;
-      ws->red_k = c;
-      *B.done_count = 0;
-    }
+  if (threadIdx.x < 3) {
+    // sums 0 LJ, 1 real space over the pair warps, 2 over the k warps
+    const int kw = kthreads / 32, w0 = threadIdx.x == 2 ? 0 : kw;
+    const int w1 = threadIdx.x == 2 ? kw : kDeltaThreads / 32;
+    double t = 0.0;
+    for (int w = w0; w < w1; w++) t += s_part[w][threadIdx.x == 1];
+    B.partial[4 * blockIdx.x + threadIdx.x] = t;
   }
 }
 
@@ -457,24 +476,25 @@ int pair_grid() {
   return g_pair_grid;
 }
 
-// Shared memory of a k block's phase tables, and of the staged moved beads.
-static size_t delta_smem(const DevParams& P) {
-  const size_t k = P.use_ewald && P.n_ku > 0
-                       ? (size_t)k_beads(P) * 2 * (P.kmax[2] + 1 + kUnits) * sizeof(double2) : 0;
-  return std::max(k, P.fx.mode ? kFixStage * sizeof(FixStage) : 0);
-}
+// One block per SM (a block takes nearly all of an SM's registers), but for the
+// SMs that the next move's candidates run on meanwhile: with a block on every SM
+// those waited for the energy change, or it for them.
+int delta_blocks64() { return std::max(1, pair_grid() / 2 - kCands); }
 
 template <int kMode>
 static void launch_delta64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
+  constexpr size_t stage = kFixStage * sizeof(FixStage) + kFixMaxBins * 40;
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_delta64<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kKTableBytes + 4096);
+                         stage + kKTableBytes);
     attr = true;
   }
-  const int sms = pair_grid() / 2;
-  const int kgrid = P.use_ewald ? std::min(sms, P.n_ku) : 0;
-  k_delta64<kMode><<<kgrid + 2 * sms, kPairThreads, delta_smem(P), s>>>(P, B, kgrid);
+  // the staged moved beads and the table, then the k role's phase tables
+  const size_t tab = kMode ? kFixStage * sizeof(FixStage) + (size_t)P.fx.n_bin * 40 : 0;
+  const size_t k = P.use_ewald && P.n_ku > 0
+                       ? (size_t)k_beads(P) * 2 * (P.kmax[2] + 1 + kUnits) * sizeof(double2) : 0;
+  k_delta64<kMode><<<delta_blocks64(), kDeltaThreads, tab + k, s>>>(P, B, (int)tab);
 }
 
 void launch_delta_pairs64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {

@@ -234,11 +234,16 @@ __device__ __forceinline__ void pivot_draws(const DevParams& P, int wlen, GenPla
   const int n = len - 1, nf = len - 1 - pv;
   int nl = 0;
   while ((1 << nl) < n) nl++;  // ranks 0 .. n-1 need nl bits
-  for (int x = threadIdx.x; x <= kDrawWindow; x += blockDim.x)
-    jump[0][x] = (short)(x < kDrawWindow ? next_accept(accbits, wlen, x + step) : kDrawWindow);
+  // offsets past lim count as outside the window: a bead takes 3.5 words on
+  // average, so n beads stay below it (else the sequential scan)
+  const int lim = min(kDrawWindow, plan.scan_rel + 6 * n + 64);
+  const auto inside = [&](int p) { return p < lim ? p : kDrawWindow; };
+  for (int x = plan.scan_rel + (int)threadIdx.x; x < lim; x += blockDim.x)
+    jump[0][x] = (short)inside(next_accept(accbits, wlen, x + step));
+  if ((int)threadIdx.x < nl) jump[threadIdx.x][kDrawWindow] = kDrawWindow;
   for (int l = 1; l < nl; l++) {
     __syncthreads();
-    for (int x = threadIdx.x; x <= kDrawWindow; x += blockDim.x)
+    for (int x = plan.scan_rel + (int)threadIdx.x; x < lim; x += blockDim.x)
       jump[l][x] = jump[l - 1][jump[l - 1][x]];
   }
   if (threadIdx.x == 0) {
@@ -246,7 +251,7 @@ __device__ __forceinline__ void pivot_draws(const DevParams& P, int wlen, GenPla
     plan.scan_end = plan.scan_rel;
   }
   __syncthreads();
-  const int p0 = next_accept(accbits, wlen, plan.scan_rel);
+  const int p0 = inside(next_accept(accbits, wlen, plan.scan_rel));
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     int p = p0;
     for (int l = 0; l < nl; l++)
@@ -357,44 +362,82 @@ __device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& 
   }
 }
 
-// Generates candidate C from stream position d.pos and positions V; thread 0
-// consumes the draws, the block applies the geometry.
+// Worked out from the draws' places alone (see gen_picks).
+struct GenPre {
+  double crank_s, crank_c;  // of the angle drawn by the seventh word
+  double pivot_s;           // from the sixth
+};
+
+// floor(n x / M) of a draw x, M = 2^32 - 1, 0 <= n < 2^20: the reference's FP64
+// product is exact and its quotient, at least 1 / M away from the next integer
+// unless it is one, cannot round up to it; so the integer quotient, and no
+// division (n x = a 2^32 + b = a M + (a + b)).
+__device__ __forceinline__ int draw_floor(int n, uint32_t x) {
+  const unsigned long long v = (unsigned long long)n * x;
+  const unsigned long long a = v >> 32, r = a + (v & 0xFFFFFFFFull);
+  return (int)(a + (r >= 0xFFFFFFFFull ? 1 : 0));
+}
+
+// What warp 0 finds before the acceptance bits are there: the picks (two loads
+// deep), and what the other warps work out beside it from the draws' fixed
+// places: the crankshaft's sine and cosine and the pivot's displacement.
+struct GenPicks {
+  int mt, mol, b0, b1;  // mol -1: nothing is moved
+  bool any;             // molecules to pick from: the picks' draws are taken
+};
+
+__device__ __forceinline__ GenPicks gen_picks(const DevParams& P, const DevBuffers& B, Draws& d) {
+  GenPicks g{0, -1, 0, 0, P.n_mol - P.phantom > 0};
+  (void)d.next();  // simulation.cc:221 (the GC draw)
+  if (!g.any) return g;
+  const int n_ch = P.n_chain_total, n_io = P.n_ion_total;
+  int wc = (int)floor(unit_draw(d.next()) * n_ch);
+  int wi = (int)floor(unit_draw(d.next()) * n_io);
+  if (wc == n_ch) wc--;
+  if (wi == n_io) wi--;
+  const int chain_id = (wc >= 0 && wc < n_ch) ? B.chain_ids[wc] : -1;
+  const int ion_id = (wi >= 0 && wi < n_io) ? B.ion_ids[wi] : -1;
+  double u = unit_draw(d.next());
+  double cur = P.move_prob[0];
+  while (cur < u && g.mt < 4) {
+    g.mt++;
+    cur += P.move_prob[g.mt];
+  }
+  if (cur < u) g.mt++;
+  if (g.mt > 4) g.mt = 4;
+  if (g.mt == 0 && n_io > 0)
+    g.mol = ion_id;
+  else if (n_ch > 0)
+    g.mol = chain_id;
+  if (!((g.mt == 0 && n_io > 0) || (g.mt > 0 && n_ch > 0))) g.mol = -1;
+  if (g.mol >= 0) {
+    g.b0 = B.mol_start[g.mol];
+    g.b1 = B.mol_start[g.mol + 1];
+  }
+  return g;
+}
+
+// Generates candidate C from stream position d.pos and positions V. Warp 0
+// consumes the draws, every lane the same way but for the three components of a
+// vector, which take a lane each (one division's latency instead of three); the
+// block applies the geometry.
 __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B,
                                       const DevState* st, const PosView& V, TrialOut O,
                                       MoveCand& C, Draws& d, long long wbase, GenPlan& plan,
                                       int* s_off, int* s_boff, double (*s_w)[kPivotMax],
                                       short (*jump)[kDrawWindow + 1],
-                                      const unsigned* accbits, double* red) {
+                                      const unsigned* accbits, double* red, const GenPicks& gp,
+                                      const GenPre& pre) {
   // ----------------------------------------------------- generate next move
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const auto part = [&](const double* v) { return lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]); };
     plan.type = -1;
     plan.scan = 0;
-    (void)d.next();  // simulation.cc:221 (the GC draw)
-    const int n_ch = P.n_chain_total, n_io = P.n_ion_total;
-    if (P.n_mol - P.phantom > 0) {
-      int wc = (int)floor(unit_draw(d.next()) * n_ch);
-      int wi = (int)floor(unit_draw(d.next()) * n_io);
-      if (wc == n_ch) wc--;
-      if (wi == n_io) wi--;
-      int chain_id = (wc >= 0 && wc < n_ch) ? B.chain_ids[wc] : -1;
-      int ion_id = (wi >= 0 && wi < n_io) ? B.ion_ids[wi] : -1;
-      int mt = 0;
-      double u = unit_draw(d.next());
-      double cur = P.move_prob[0];
-      while (cur < u && mt < 4) {
-        mt++;
-        cur += P.move_prob[mt];
-      }
-      if (cur < u) mt++;
-      if (mt > 4) mt = 4;
-      int molid = -1;
-      if (mt == 0 && n_io > 0)
-        molid = ion_id;
-      else if (n_ch > 0)
-        molid = chain_id;
-      const bool attempted = (mt == 0 && n_io > 0) || (mt > 0 && n_ch > 0);
-      if (attempted && molid >= 0) {
-        const int b0 = B.mol_start[molid], b1 = B.mol_start[molid + 1];
+    if (gp.any) {
+      const int mt = gp.mt, molid = gp.mol;
+      if (molid >= 0) {
+        const int b0 = gp.b0, b1 = gp.b1;
         const int len = b1 - b0;
         plan.mol = molid;
         plan.b0 = b0;
@@ -408,25 +451,30 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
           rand_sphere(d, v, accbits);
           double vl = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
           if (vl > 0) vl = 3 * P.move_size / vl;
-          for (int a = 0; a < 3; a++) plan.vec[a] = vl * v[a];
+          if (lane < 3) plan.vec[lane] = vl * part(v);
           plan.b_hi = b0 + 1;
         } else if (mt == 1) {
           // Molecule::COMTranslate (molecule.cc:135-151). Here, and in the
-          // pivot and crankshaft picks, the reference multiplies the word
-          // before dividing, so these keep the division (unit_draw is the
-          // quotient of the word alone).
-          for (int a = 0; a < 3; a++) plan.vec[a] = 0.5 * P.move_size * (double)d.next() / kMtMax;
-          for (int a = 0; a < 3; a++)
-            if (d.next() % 2u == 0u) plan.vec[a] = -plan.vec[a];
+          // pivot's displacement, the reference multiplies the word before
+          // dividing, so these keep the division (unit_draw is the quotient of
+          // the word alone).
+          uint32_t w[3], sg[3];
+          for (int a = 0; a < 3; a++) w[a] = d.next();
+          for (int a = 0; a < 3; a++) sg[a] = d.next();
+          const double wl = lane == 0 ? (double)w[0] : (lane == 1 ? (double)w[1] : (double)w[2]);
+          const uint32_t sl = lane == 0 ? sg[0] : (lane == 1 ? sg[1] : sg[2]);
+          const double x = 0.5 * P.move_size * wl / kMtMax;
+          if (lane < 3) plan.vec[lane] = sl % 2u == 0u ? -x : x;
         } else if (mt == 2) {
           // Molecule::Pivot (molecule.cc:153-237). Bead i's new position is
           // the previous one plus bl_i * unit(old_i - old_prev + s v_i): the
           // reference's running translation of the chain tail cancels out of
           // the bond direction. Thread 0 only locates each bead's draws; the
           // geometry and the running sum are done by the block below.
-          int pivot = (int)floor(len * (double)d.next() / kMtMax);
+          int pivot = draw_floor(len, d.next());
           if (pivot == len) pivot--;
-          double s = P.move_size * (double)d.next() / kMtMax;
+          (void)d.next();
+          const double s = pre.pivot_s;
           plan.s = s;
           plan.pivot = pivot;
           if (len <= kPivotMax) {
@@ -466,20 +514,19 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
         } else if (mt == 3) {
           // Molecule::Crankshaft (molecule.cc:239-265); Rodrigues rotation in
           // the per-entry grouping of Eigen's AngleAxis::toRotationMatrix.
-          int first = (int)floor((len - 2) * (double)d.next() / kMtMax);
-          int last = (int)floor((len - first) * (double)d.next() / kMtMax) + first;
+          int first = draw_floor(len - 2, d.next());
+          int last = draw_floor(len - first, d.next()) + first;
+          (void)d.next();  // the angle
           if (last > len - 1) last = len - 1;  // the reference reads past the chain here
           double4_32a pf = V.at(b0 + first), pl = V.at(b0 + last);
           double ax[3] = {pl.x - pf.x, pl.y - pf.y, pl.z - pf.z};
           double z2 = ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2];
           if (z2 > 0) {
             double n = sqrt(z2);
-            for (int a = 0; a < 3; a++) ax[a] /= n;
+            const double al = part(ax) / n;
+            for (int a = 0; a < 3; a++) ax[a] = __shfl_sync(0xffffffffu, al, a);
           }
-          const double pi_libm = 3.14159265358979323846;
-          double ang = P.move_size * (unit_draw(d.next()) * 2 * pi_libm - pi_libm);
-          double sn, cs;
-          sincos(ang, &sn, &cs);
+          const double sn = pre.crank_s, cs = pre.crank_c;
           double sa[3] = {sn * ax[0], sn * ax[1], sn * ax[2]};
           double ca[3] = {(1.0 - cs) * ax[0], (1.0 - cs) * ax[1], (1.0 - cs) * ax[2]};
           double t = ca[0] * ax[1];
@@ -507,7 +554,8 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
           double v[3];
           rand_sphere(d, v, accbits);
           double vl = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-          for (int a = 0; a < 3; a++) plan.vec[a] = bl * v[a] / vl;
+          const double x = bl * part(v) / vl;
+          if (lane < 3) plan.vec[lane] = x;
           plan.dir = dir;
           plan.end = end;
         }
@@ -639,6 +687,7 @@ struct GenSmem {
     double s_w[3][kPivotMax];                  // pivot bond steps (used after)
   };
   MoveCand C;
+  GenPre pre;
 };
 
 // Candidate c of the step after the pending move.
@@ -652,6 +701,17 @@ __device__ __forceinline__ void gen_body(const DevParams& P, const DevBuffers& B
   const int wlen = (int)(avail < kDrawWindow ? (avail > 0 ? avail : 0) : kDrawWindow);
   for (int i = threadIdx.x; i < wlen; i += blockDim.x) sm.win[i] = B.stream[base + i];
   __syncthreads();
+  Draws d{B.stream, sm.win, base, len, base, wlen, 0};
+  GenPicks gp{0, -1, 0, 0, false};
+  const int warp = threadIdx.x >> 5;
+  if (warp == 0) gp = gen_picks(P, B, d);
+  if (warp == 1 && base + 6 < len) {
+    const double pi_libm = 3.14159265358979323846;
+    const double ang = P.move_size * (unit_draw(d.at(base + 6)) * 2 * pi_libm - pi_libm);
+    sincos(ang, &sm.pre.crank_s, &sm.pre.crank_c);
+  }
+  if (warp == 2 && base + 5 < len)
+    sm.pre.pivot_s = P.move_size * (double)d.at(base + 5) / kMtMax;
   // every window position's randSphere test, one position per thread; a
   // warp's ballot makes the word of its 32 positions
   for (int p0 = threadIdx.x & ~31; p0 < kDrawWindow; p0 += blockDim.x) {
@@ -661,12 +721,11 @@ __device__ __forceinline__ void gen_body(const DevParams& P, const DevBuffers& B
     if ((threadIdx.x & 31) == 0) sm.accbits[p0 >> 5] = bits;
   }
   __syncthreads();
-  Draws d{B.stream, sm.win, base, len, base, wlen, 0};
   const bool took = c == kCandAccept;
   const PosView V{B.pos, B.trial, took ? st->b_lo : 0, took ? st->b_hi : 0};
   const TrialOut O{B.ctrial + (size_t)c * P.max_len, B.cftrial + (size_t)c * P.max_len};
   gen_move(P, B, st, V, O, sm.C, d, base, sm.plan, sm.s_off, sm.s_boff, sm.s_w, sm.jump, sm.accbits,
-           sm.red);
+           sm.red, gp, sm.pre);
   if (threadIdx.x == 0) B.plan->cand[c] = sm.C;
 }
 
@@ -687,8 +746,30 @@ struct SlotSums {
   int pair_off, n_pair, k_off, n_k;
 };
 
+// The FP64 energy change's block sums {LJ, real space, k, unused}, added in order
+// by one warp.
+__device__ __forceinline__ void block_sums(const double* part, int blocks, DevState& S) {
+  double a = 0.0, b = 0.0, c = 0.0;
+  for (int i = threadIdx.x; i < blocks; i += 32) {
+    a += part[4 * i];
+    b += part[4 * i + 1];
+    c += part[4 * i + 2];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  }
+  if (threadIdx.x == 0) {
+    S.red_lj = a;
+    S.red_re = b;
+    S.red_k = c;
+  }
+}
+
 __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers& B, int mode,
-                                            SerialSmem& sm, const SlotSums* slots) {
+                                            SerialSmem& sm, const SlotSums* slots,
+                                            int part_blocks) {
   double* const red = sm.red;
   int& s_accept = sm.s_accept;
   DevState& S = sm.S;
@@ -720,6 +801,9 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
     }
     __syncthreads();
   }
+
+  if (part_blocks && (mode & kModeFinish) && S.pending && threadIdx.x < 32)
+    block_sums(B.partial, part_blocks, S);
 
   // the acceptance test's draw, loaded while dE is composed
   uint32_t word = 0;
@@ -953,9 +1037,9 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
 }
 
 __global__ void __launch_bounds__(kSerialThreads)
-    k_serial64(const DevParams P, const DevBuffers B, int mode) {
+    k_serial64(const DevParams P, const DevBuffers B, int mode, int part_blocks) {
   __shared__ SerialSmem sm;
-  serial_body(P, B, mode, sm, nullptr);
+  serial_body(P, B, mode, sm, nullptr, part_blocks);
 }
 
 // A replica's parameters and buffers into shared memory.
@@ -984,7 +1068,7 @@ __global__ void __launch_bounds__(kSerialThreads)
   stage_system(rp + r, rb + r, P, B);
   SlotSums ss{slots, item_off[4 * r], item_off[4 * r + 1], item_off[4 * r + 2],
               item_off[4 * r + 3]};
-  serial_body(P, B, mode, sm, &ss);
+  serial_body(P, B, mode, sm, &ss, 0);
 }
 
 __global__ void __launch_bounds__(kSerialThreads)
@@ -1018,7 +1102,8 @@ void launch_batch_serial(const DevParams* rp, const DevBuffers* rb, const int* i
 }
 
 void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStream_t s) {
-  k_serial64<<<1, kSerialThreads, 0, s>>>(P, B, mode);
+  // (the precision form's energy change adds its blocks itself)
+  k_serial64<<<1, kSerialThreads, 0, s>>>(P, B, mode, P.form ? 0 : delta_blocks64());
 }
 
 __global__ void k_set_move(DevState* st, int mol, int b_lo, int b_hi) {
