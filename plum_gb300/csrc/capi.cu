@@ -99,11 +99,12 @@ struct plum_ctx {
   long recompute_every = 0;    // full FP64 recompute cadence of plum_run (0: never)
   long since_recompute = 0;
   // configurational-bias scratch
-  double4_32a* cb_b = nullptr;   // [2 * cap] trial beads and counterions
-  double4_32a* cb_c = nullptr;   // [2 * cap] grown chain and counterions
+  double4_32a* cb_in = nullptr;  // [4 * cap] trial beads, grown chain, counterions
+  double4_32a* h_cb = nullptr;   // the same, pinned
+  double* cb_slots = nullptr;    // block sums of the one-launch FP64 kernel
   double2* cb_so = nullptr;
   double* cb_part = nullptr;
-  double* cb_u = nullptr;
+  double* cb_u = nullptr;        // [cap] results (pinned, written by the kernels)
   int cb_cap = 0;
   double* cb_part32 = nullptr;   // slots of the precision form's trial kernel
   long long cb_part32_cap = 0;
@@ -796,8 +797,8 @@ int plum_ctx_destroy(plum_ctx* c) {
                   c->B.ion_ids,  c->B.kn,      c->B.kw,    c->B.sk,        c->B.dsk,
                   c->B.partial,  c->B.bond_mol, c->B.state, c->d_tot_part,  c->d_out,
                   c->B.ktile_count, c->B.kpartial, c->B.fpos, c->B.done_count,
-                  c->B.fq,       c->B.ftrial,  c->B.dsk_part32, c->cb_b, c->cb_c, c->cb_so,
-                  c->cb_part,    c->cb_u,      c->d_obs_per, c->d_rhoz, c->desc_acc,
+                  c->B.fq,       c->B.ftrial,  c->B.dsk_part32, c->cb_in, c->cb_slots, c->cb_so,
+                  c->cb_part,    c->d_obs_per, c->d_rhoz, c->desc_acc,
                   c->d_rp1,      c->d_rb1,     c->desc_fine, c->cb_part32, c->cb_ticket,
                   c->d_stream,   c->d_mt,      c->d_log_type, c->d_log_acc, c->d_log_e,
                   c->d_press,    c->d_sk_part, c->d_log_de, c->d_htab, c->d_htab64,
@@ -806,6 +807,8 @@ int plum_ctx_destroy(plum_ctx* c) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
+  if (c->h_cb) cudaFreeHost(c->h_cb);
+  if (c->cb_u) cudaFreeHost(c->cb_u);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->gen_go) cudaEventDestroy(c->gen_go);
@@ -938,8 +941,7 @@ int rebuild_system(plum_ctx* c) {
   const bool mirror64 = B.fpos64 != nullptr;
   void* old[] = {B.pos,      B.trial,      B.type,     B.mol_start, B.chain_ids, B.ion_ids,
                  B.fpos,     B.fq,         B.ftrial,   B.dsk_part32, B.bond_mol, B.ctrial, B.cftrial,
-                 c->d_tot_part, c->d_obs_per, c->cb_b, c->cb_c,    c->cb_part,  c->cb_u,
-                 B.fpos64};
+                 c->d_tot_part, c->d_obs_per, B.fpos64};
   for (void* q : old)
     if (q) cudaFree(q);
   B.pos = B.trial = nullptr;
@@ -952,9 +954,6 @@ int rebuild_system(plum_ctx* c) {
   B.dsk_part32 = nullptr;
   B.bond_mol = nullptr;
   c->d_tot_part = c->d_obs_per = nullptr;
-  c->cb_b = c->cb_c = nullptr;
-  c->cb_part = c->cb_u = nullptr;
-  c->cb_cap = 0;
   int rc = dalloc(&B.pos, nb) | dalloc(&B.trial, nb) | dalloc(&B.type, nb) |
            dalloc(&B.mol_start, in.n_mol + 1) | dalloc(&B.chain_ids, chains.size()) |
            dalloc(&B.ion_ids, ions.size()) | dalloc(&B.fpos, nb) | dalloc(&B.fq, nb) |
@@ -1643,44 +1642,50 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
                                   "trial kernel");
   }
   const int cap = std::max(n_trials, std::max(chain_len, in.gc_chain_len));
-  const int groups = cbmc_groups(c->P);
   if (cap > c->cb_cap) {
-    cudaFree(c->cb_b);
-    cudaFree(c->cb_c);
+    cudaFree(c->cb_in);
     cudaFree(c->cb_part);
-    cudaFree(c->cb_u);
-    int rc = dalloc(&c->cb_b, 2 * (size_t)cap) | dalloc(&c->cb_c, 2 * (size_t)cap) |
-             dalloc(&c->cb_part, 2 * (size_t)cap * groups) | dalloc(&c->cb_u, cap);
+    cudaFree(c->cb_slots);
+    if (c->h_cb) cudaFreeHost(c->h_cb);
+    if (c->cb_u) cudaFreeHost(c->cb_u);
+    c->cb_in = nullptr;
+    c->cb_part = c->cb_slots = c->cb_u = nullptr;
+    c->h_cb = nullptr;
+    c->cb_cap = 0;
+    int rc = dalloc(&c->cb_in, 4 * (size_t)cap) | dalloc(&c->cb_part, 2 * (size_t)cap * kCbmcGroups) |
+             dalloc(&c->cb_slots, 3 * (size_t)cap * cbmc_blocks());
     if (rc) return PLUM_ERR_CUDA;
+    // pinned: the sites go up in one asynchronous copy, and the kernels write
+    // the energies here themselves
+    CK(cudaMallocHost(&c->h_cb, sizeof(double4_32a) * 4 * (size_t)cap));
+    CK(cudaMallocHost(&c->cb_u, sizeof(double) * (size_t)cap));
     c->cb_cap = cap;
   }
   if (!c->cb_so && dalloc(&c->cb_so, std::max(1, c->P.n_k))) return PLUM_ERR_CUDA;
-  if (fp32) {
-    if (G.slots > c->cb_part32_cap) {
-      cudaFree(c->cb_part32);
-      c->cb_part32 = nullptr;
-      if (dalloc(&c->cb_part32, (size_t)G.slots)) return PLUM_ERR_CUDA;
-      c->cb_part32_cap = G.slots;
-    }
-    if (!c->cb_ticket) {
-      if (dalloc(&c->cb_ticket, 1)) return PLUM_ERR_CUDA;
-      CK(cudaMemsetAsync(c->cb_ticket, 0, sizeof(int), c->s));
-    }
+  if (fp32 && G.slots > c->cb_part32_cap) {
+    cudaFree(c->cb_part32);
+    c->cb_part32 = nullptr;
+    c->cb_part32_cap = 0;
+    if (dalloc(&c->cb_part32, (size_t)G.slots)) return PLUM_ERR_CUDA;
+    c->cb_part32_cap = G.slots;
+  }
+  if (!c->cb_ticket) {
+    if (dalloc(&c->cb_ticket, 1)) return PLUM_ERR_CUDA;
+    CK(cudaMemsetAsync(c->cb_ticket, 0, sizeof(int), c->s));
   }
   int type = (int)(std::find(in.type_names.begin(), in.type_names.end(), in.gc_symbol) -
                    in.type_names.begin());
   const double q1 = in.gc_bead_charge, q2 = -in.gc_bead_charge;
-  std::vector<double4_32a> hb(2 * n_trials), hc(2 * std::max(chain_len, 1));
-  for (int t = 0; t < n_trials; t++) {
-    hb[t] = make_double4_32a(b1[3 * t], b1[3 * t + 1], b1[3 * t + 2], q1);
-    hb[n_trials + t] = charged ? make_double4_32a(b2[3 * t], b2[3 * t + 1], b2[3 * t + 2], q2)
-                               : hb[t];
-  }
-  for (int i = 0; i < chain_len; i++) {
-    hc[i] = make_double4_32a(chain[3 * i], chain[3 * i + 1], chain[3 * i + 2], q1);
-    hc[chain_len + i] = charged ? make_double4_32a(chain_ci[3 * i], chain_ci[3 * i + 1],
-                                                   chain_ci[3 * i + 2], q2)
-                                : hc[i];
+  // trial beads, grown chain, then (charged species) their counterions
+  double4_32a* h = c->h_cb;
+  const auto put = [&h](const double* x, int n, double q) {
+    for (int t = 0; t < n; t++) *h++ = make_double4_32a(x[3 * t], x[3 * t + 1], x[3 * t + 2], q);
+  };
+  put(b1, n_trials, q1);
+  put(chain, chain_len, q1);
+  if (charged) {
+    put(b2, n_trials, q2);
+    put(chain_ci, chain_len, q2);
   }
   CbmcJob J;
   J.n_trials = n_trials;
@@ -1694,31 +1699,31 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
     J.ex_lo = in.mol_start[delete_mol];
     J.ex_hi = in.mol_start[last + 1];
   }
-  // copies from pageable memory: the host vectors may go once these return
-  CK(cudaMemcpyAsync(c->cb_b, hb.data(), sizeof(double4_32a) * 2 * n_trials,
+  CK(cudaMemcpyAsync(c->cb_in, c->h_cb, sizeof(double4_32a) * (h - c->h_cb),
                      cudaMemcpyHostToDevice, c->s));
-  if (chain_len > 0)
-    CK(cudaMemcpyAsync(c->cb_c, hc.data(), sizeof(double4_32a) * 2 * chain_len,
-                       cudaMemcpyHostToDevice, c->s));
-  J.b1 = c->cb_b;
-  J.b2 = c->cb_b + n_trials;
-  J.chain = c->cb_c;
-  J.chain_ci = c->cb_c + chain_len;
+  J.b1 = c->cb_in;
+  J.chain = J.b1 + n_trials;
+  J.b2 = charged ? J.chain + chain_len : J.b1;
+  J.chain_ci = charged ? J.b2 + n_trials : J.chain;
   J.s_o = c->cb_so;
   J.part = fp32 ? c->cb_part32 : c->cb_part;
   J.u = c->cb_u;
+  J.slots = c->cb_slots;
+  J.ticket = c->cb_ticket;
   *Jp = J;
   *Gp = G;
   return PLUM_OK;
 }
 
 // One growth step's trial energies on the context's stream: one launch in the
-// precision form, the FP64 kernels (S_o, system sweep, per-trial sums) in the
-// plain form.
+// precision form and where the integer pair form applies, else the FP64 kernels
+// (S_o, system sweep, per-trial sums).
 static int cbmc_launch(plum_ctx* c, const CbmcJob& J, const Cbmc32Layout& G) {
   if (c->form == PLUM_FORM_FP32) {
     if (launch_cbmc32(c->P, c->B, J, G, c->cb_ticket, c->s))
       return fail(PLUM_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+  } else if (c->B.fpos64) {
+    launch_cbmc64(c->P, c->B, J, c->s);
   } else {
     launch_cbmc(c->P, c->B, J, c->s);
   }
@@ -1736,8 +1741,8 @@ int plum_cbmc_trials(plum_ctx* c, int n_trials, const double* b1, const double* 
   if (rc) return rc;
   rc = cbmc_launch(c, J, G);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(u_out, c->cb_u, sizeof(double) * n_trials, cudaMemcpyDeviceToHost, c->s));
   CK(cudaStreamSynchronize(c->s));
+  std::memcpy(u_out, c->cb_u, sizeof(double) * n_trials);
   return PLUM_OK;
 }
 
@@ -1760,7 +1765,8 @@ int plum_cbmc_time(plum_ctx* c, int n_trials, const double* b1, const double* b2
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   *ms_out = (double)ms / reps;
   if (launches_out)
-    *launches_out = c->form == PLUM_FORM_FP32 ? 1 : ((c->P.use_ewald && c->P.n_k > 0) ? 3 : 2);
+    *launches_out = c->form == PLUM_FORM_FP32 || c->B.fpos64
+                        ? 1 : ((c->P.use_ewald && c->P.n_k > 0) ? 3 : 2);
   return PLUM_OK;
 }
 

@@ -307,9 +307,15 @@ struct CbmcJob {
   double2* s_o;                     // [n_k] scratch: S(k) of the other charges
   double* part;                     // [n_trials][groups][2] scratch
   double* u;                        // [n_trials] result
+  double* slots;                    // [cbmc_blocks()][n_trials][3] block sums
+  int* ticket;                      // zero before the first launch, left zero
 };
+constexpr int kCbmcGroups = 64;  // most that cbmc_groups returns
 int cbmc_groups(const DevParams& P);
+int cbmc_blocks();
 void launch_cbmc(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s);
+// One launch, for contexts with B.fpos64 (so P.fx applies).
+void launch_cbmc64(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s);
 // The precision form's one-launch trial kernel (kern_cbmc32.cu): J.part holds
 // `slots` doubles laid out by cbmc32_layout; J.s_o is unused. ticket is one
 // int, zero before the first launch (each launch leaves it zero).

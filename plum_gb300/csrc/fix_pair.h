@@ -122,6 +122,14 @@ PLUM_FIX_HD uint64_t fix_h(const FixPair64* c01, const FixPair64* c23, const Fix
   return fix_mul(v1, p, r, k01.a);
 }
 
+// S of the nearest image alone.
+template <int kMode>
+PLUM_FIX_HD uint64_t fix_near_r2(uint64_t dx, uint64_t dy, uint64_t dz) {
+  if (kMode == 1) return fix_r2(dx, dy, dz);
+  return fix_r2((uint64_t)((int64_t)dx >> 1), (uint64_t)((int64_t)dy >> 1),
+                (uint64_t)((int64_t)dz >> 1));
+}
+
 // The table sum (in table units) of one pair at difference d, image
 // cells included; S of the nearest image in s0.
 template <int kMode, class Tab>

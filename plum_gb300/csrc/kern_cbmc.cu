@@ -19,6 +19,8 @@
 
 #include "device_common.cuh"
 #include "engine.h"
+#include "fix_device.cuh"
+#include "kspace64.cuh"
 
 namespace plum {
 
@@ -225,9 +227,234 @@ __global__ void __launch_bounds__(kCbThreads)
   }
 }
 
+// The same energies in one launch where the integer pair form applies (and the
+// context keeps the 64-bit position mirror).
+//   pair role  a warp's lanes take 32 trials, so a system bead (and, as the
+//              list's tail, a grown bead) is one broadcast load and no sum
+//              crosses lanes; opposite charges of a trial and its counterion
+//              leave one integer per bead
+//   k role     (charged species) a block's own k units: S_o(k) from the
+//              committed S(k), the deleted and the grown beads, then every
+//              trial's kw (2 S_o.e + |e|^2)
+// The last block to finish adds the blocks' sums in order and the trial's own
+// terms. No split depends on the number of trials, so neither does a result. One growth step of 32 trials on 6,400 beads, r_c = 0.7 L: XXX us, 430 us
+// in three FP64 launches (27 image cells per pair, a sincos per trial and k).
+constexpr int kCb64Threads = 512, kCb64K = 128;
+
+int cbmc_blocks() { return pair_grid() / 2; }
+
+template <int kMode>
+__global__ void __launch_bounds__(kCb64Threads, 1)
+    k_cbmc64(const DevParams P, const DevBuffers B, CbmcJob J) {
+  extern __shared__ __align__(32) unsigned char smem[];
+  __shared__ double s_red[3][kCb64Threads];
+  __shared__ double s_w[2][kCb64K / 32][4];
+  __shared__ int s_last;
+  const int kth = J.charged && P.use_ewald && P.n_ku > 0 ? kCb64K : 0;
+  const int tid = threadIdx.x, T = J.n_trials, N = P.n_bead;
+  const int grown = J.cl * (J.charged ? 2 : 1);
+  const auto grown_bead = [&](int i) { return i < J.cl ? J.chain[i] : J.chain_ci[i - J.cl]; };
+  double* const slots = J.slots + (size_t)blockIdx.x * T * 3;
+  if (tid < kth) {
+    for (int c0 = 0; c0 < T; c0 += kCb64K) {
+      const int tl = min(kCb64K, T - c0);
+      uint64_t x[2] = {0, 0}, y[2] = {0, 0}, z[2] = {0, 0};
+      double q[2] = {0.0, 0.0};
+      if (tid < tl)
+        for (int b = 0; b < 2; b++) {
+          const double4_32a v = b ? J.b2[c0 + tid] : J.b1[c0 + tid];
+          x[b] = turn64(P, v.x, 0);
+          y[b] = turn64(P, v.y, 1);
+          z[b] = turn64(P, v.z, 2);
+          q[b] = v.w;
+        }
+      const int u0 = (int)((long long)P.n_ku * blockIdx.x / gridDim.x);
+      const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / gridDim.x);
+      const int gone = J.ex_hi - J.ex_lo;
+      const int pend = B.state->sk_pending, buf = B.state->sk_buf;
+      double acc = 0.0;
+      for (int u = u0; u < u1; u++) {
+        const KUnit ku = B.ku[u];
+        const uint64_t nx = (uint64_t)ku.nx, ny = (uint64_t)(int64_t)ku.ny, nz = (uint64_t)ku.nz;
+        double o[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int i = tid; i < gone + grown; i += kCb64K) {
+          double4_32a v = i < gone ? B.pos[J.ex_lo + i] : grown_bead(i - gone);
+          if (i < gone) v.w = -v.w;
+          const uint64_t xy = nx * turn64(P, v.x, 0) + ny * turn64(P, v.y, 1);
+          const uint64_t zz = nz * turn64(P, v.z, 2);
+          const double2 ep = turn_exp(xy + zz), em = turn_exp(xy - zz);
+          o[0] = fma(v.w, ep.x, o[0]);
+          o[1] = fma(v.w, ep.y, o[1]);
+          o[2] = fma(v.w, em.x, o[2]);
+          o[3] = fma(v.w, em.y, o[3]);
+        }
+        for (int c = 0; c < 4; c++) {
+          o[c] = warp_sum(o[c]);
+          if ((tid & 31) == 0) s_w[u & 1][tid >> 5][c] = o[c];
+        }
+        role_sync(1, kCb64K);  // (the other buffer is read before the next one)
+        if (tid < tl) {
+          double2 e[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+          for (int b = 0; b < 2; b++) {
+            const uint64_t xy = nx * x[b] + ny * y[b], zz = nz * z[b];
+            const double2 ep = turn_exp(xy + zz), em = turn_exp(xy - zz);
+            e[0].x = fma(q[b], ep.x, e[0].x);
+            e[0].y = fma(q[b], ep.y, e[0].y);
+            e[1].x = fma(q[b], em.x, e[1].x);
+            e[1].y = fma(q[b], em.y, e[1].y);
+          }
+          for (int h = 0; h < 2; h++) {
+            const int k = h ? ku.km : ku.kp;
+            if (k < 0) continue;
+            double2 so = B.sk[k];
+            if (pend) {
+              const double2 d = B.dsk[(size_t)buf * P.n_k + k];
+              so.x += d.x;
+              so.y += d.y;
+            }
+            for (int w = 0; w < kCb64K / 32; w++) {
+              so.x += s_w[u & 1][w][2 * h];
+              so.y += s_w[u & 1][w][2 * h + 1];
+            }
+            acc += B.kw[k] * (2.0 * (so.x * e[h].x + so.y * e[h].y) +
+                              (e[h].x * e[h].x + e[h].y * e[h].y));
+          }
+        }
+      }
+      if (tid < tl) slots[3 * (c0 + tid) + 2] = acc;
+      role_sync(1, kCb64K);  // s_w is read
+    }
+  } else {
+    const int id = tid - kth, nt = kCb64Threads - kth;
+    const int lane = id & 31, sl = id >> 5, slices = nt >> 5;
+    FixTab Tb = P.fx;
+    if (J.charged) fix_stage(Tb, smem, id, nt);
+    const auto tab = [&](uint64_t s) { return fix_h(Tb.c01, Tb.c23, Tb.c45, Tb.base, s); };
+    const double unit = fix_scale(P), hs = 1.0 / Tb.unit;
+    const int nb = J.charged ? 2 : 1;
+    role_sync(2, nt);
+    for (int c0 = 0; c0 < T; c0 += 32) {
+      // (the lanes past the last trial repeat it)
+      const int t = min(c0 + lane, T - 1);
+      const double4_32a p1 = J.b1[t];
+      const double4_32a p2 = J.charged ? J.b2[t] : p1;
+      const ulonglong4_32a f1 = fix64x4(P, p1), f2 = fix64x4(P, p2);
+      double lj = 0.0, re = 0.0;
+      for (int j = (int)blockIdx.x * slices + sl; j < N + grown; j += (int)gridDim.x * slices) {
+        if (j >= J.ex_lo && j < J.ex_hi) continue;
+        const bool own = j >= N;
+        const ulonglong4_32a o = own ? fix64x4(P, grown_bead(j - N)) : B.fpos64[j];
+        const int k = J.type * P.n_type + (own ? J.type : B.type[j]);
+        int64_t v = 0;  // the trial's table sum minus its counterion's
+        double h = 0.0, none = 0.0;
+        for (int b = 0; b < nb; b++) {
+          const uint64_t dx = o.x - (b ? f2.x : f1.x), dy = o.y - (b ? f2.y : f1.y),
+                         dz = o.z - (b ? f2.z : f1.z);
+          uint64_t s0;
+          if (J.charged) {
+            const int64_t w = fix_term<kMode>(Tb, tab, dx, dy, dz, s0);
+            v += b ? -w : w;
+          } else {
+            s0 = fix_near_r2<kMode>(dx, dy, dz);
+          }
+          if (s0 < Tb.s_near) {
+            // no LJ with the preceding grown bead (cbmc.cc:57-58)
+            const bool bonded = own && b == 0 && j - N == J.cl - 1;
+            const double w = fix_near(P, b ? p2 : p1, own ? grown_bead(j - N) : B.pos[j],
+                                      J.charged && s0 < Tb.s_lo, k, bonded ? none : lj);
+            h += b ? -w : w;
+          }
+        }
+        if (J.charged)
+          re = fma(p1.w * __longlong_as_double((long long)o.w) * unit, (double)v + h * hs, re);
+      }
+      s_red[0][id] = lj;
+      s_red[1][id] = re;
+      role_sync(2, nt);
+      if (sl < 2 && c0 + lane < T) {  // the slices of each sum, in order
+        double x = 0.0;
+        for (int w = 0; w < slices; w++) x += s_red[sl][w * 32 + lane];
+        slots[3 * t + sl] = x;
+        if (!kth && sl == 0) slots[3 * t + 2] = 0.0;
+      }
+      role_sync(2, nt);
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(J.ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int lane = tid & 31, part = tid >> 5;
+  constexpr int parts = kCb64Threads / 32;
+  for (int c0 = 0; c0 < T; c0 += 32) {
+    const int t = min(c0 + lane, T - 1);
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int b = part; b < (int)gridDim.x; b += parts) {
+      const double* s = J.slots + ((size_t)b * T + t) * 3;
+      for (int c = 0; c < 3; c++) v[c] += __ldcg(s + c);
+    }
+    for (int c = 0; c < 3; c++) s_red[c][tid] = v[c];
+    __syncthreads();
+    if (part == 0 && c0 + lane < T) {
+      for (int c = 0; c < 3; c++) {
+        v[c] = 0.0;
+        for (int w = 0; w < parts; w++) v[c] += s_red[c][w * 32 + lane];
+      }
+      const double4_32a b1 = J.b1[t], b2 = J.charged ? J.b2[t] : b1;
+      double pair_e = v[0], ew = 0.0;
+      if (J.charged) {
+        const ulonglong4_32a f1 = fix64x4(P, b1), f2 = fix64x4(P, b2);
+        const uint64_t dx = f2.x - f1.x, dy = f2.y - f1.y, dz = f2.z - f1.z;
+        uint64_t s0;
+        const auto tab = [&](uint64_t s) {
+          return fix_h(P.fx.c01, P.fx.c23, P.fx.c45, P.fx.base, s);
+        };
+        double re = (double)fix_term<kMode>(P.fx, tab, dx, dy, dz, s0) * P.fx.unit;
+        if (s0 < P.fx.s_near)
+          re += fix_near(P, b1, b2, s0 < P.fx.s_lo, J.type * P.n_type + J.type, pair_e);
+        if (P.use_ewald && pair_e < kVeryLarge) {
+          ew = v[1] + P.kpref * v[2] + P.lB * P.sqrt_alpha * b1.w * b2.w * re;
+          ew += P.self_coef * (b1.w * b1.w + b2.w * b2.w);
+          if (P.real_cut >= P.ebox[0])  // a bead's own images
+            ew += 0.5 * (cb_real(P, b1, b1) + cb_real(P, b2, b2));
+        }
+      }
+      if (P.use_ext) {
+        pair_e += wall64(P, b1.z, J.type);
+        if (J.charged) pair_e += wall64(P, b2.z, J.type);
+      }
+      J.u[t] = pair_e >= kVeryLarge ? kVeryLarge : pair_e + ew;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) *J.ticket = 0;
+}
+
+template <int kMode>
+static void launch_one64(const DevParams& P, const DevBuffers& B, const CbmcJob& J,
+                         cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_cbmc64<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kFixMaxBins * 40);
+    attr = true;
+  }
+  k_cbmc64<kMode><<<cbmc_blocks(), kCb64Threads, J.charged ? (size_t)P.fx.n_bin * 40 : 0, s>>>(
+      P, B, J);
+}
+
+void launch_cbmc64(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s) {
+  if (P.fx.mode == 1)
+    launch_one64<1>(P, B, J, s);
+  else
+    launch_one64<2>(P, B, J, s);
+}
+
 int cbmc_groups(const DevParams& P) {
   int g = (P.n_bead + kCbThreads * 4 - 1) / (kCbThreads * 4);
-  return g < 1 ? 1 : (g > 64 ? 64 : g);
+  return g < 1 ? 1 : (g > kCbmcGroups ? kCbmcGroups : g);
 }
 
 void launch_cbmc(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s) {
@@ -255,7 +482,7 @@ void launch_cbmc(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cuda
 // trial) before reading it. All calls on a device share the array, so calls
 // that overlap on the GPU race.
 namespace na {
-constexpr int kMaxTrials = 256, kMaxChain = 1024, kMaxK = 32768, kMaxGroups = 64;
+constexpr int kMaxTrials = 256, kMaxChain = 1024, kMaxK = 32768, kMaxGroups = kCbmcGroups;
 constexpr size_t kBeadsOff = 0;
 constexpr size_t kChainOff = kBeadsOff + sizeof(double4_32a) * 2 * kMaxTrials;
 constexpr size_t kSoOff = kChainOff + sizeof(double4_32a) * 2 * kMaxChain;
@@ -309,7 +536,6 @@ int cbmc_trials_noalloc(const DevParams& P, const DevBuffers& B, cudaStream_t s,
     say("plum_cbmc_trials_noalloc: more than 32768 half-space k-vectors");
     return 1;
   }
-  static_assert(na::kMaxGroups >= 64, "cbmc_groups() is at most 64");
   if (device < 0 || device >= 64) {
     say("plum_cbmc_trials_noalloc: device index out of range");
     return 1;

@@ -26,26 +26,10 @@
 
 #include "engine.h"
 #include "device_common.cuh"
+#include "fix_device.cuh"
 #include "kspace64.cuh"
 
 namespace plum {
-
-__device__ __forceinline__ double wrap_d(double d, double L, double invL) {
-  return d - L * rint(d * invL);
-}
-
-// LJ of one pair at squared distance r2 (the reference's r <= 0 overlap gives
-// the 1e8 sentinel).
-__device__ __forceinline__ double lj64(const DevParams& P, int k, double r2) {
-  if (P.pair_kind == 1) return sqrt(r2) <= P.hs_sum[k] ? kVeryLarge : 0.0;  // hard spheres
-  if (r2 <= 0.0) return kVeryLarge;
-  if (r2 < P.lj_rc2[k]) {
-    double s2 = P.lj_sig2[k] / r2;
-    double s6 = s2 * s2 * s2;
-    return P.lj_eps4[k] * (s6 * s6 - s6) - P.lj_eref[k];
-  }
-  return 0.0;
-}
 
 // sum over periodic images with 0 < |d + n L| <= r_c of erfc(sqrt(a) r)/r.
 // An image whose single component already exceeds r_c cannot be inside the
@@ -127,24 +111,6 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return t;  // valid in thread 0
 }
 
-// Constants of the integer pair form's FP64 path (near pairs): squared distances
-// in units of (L / 2^64)^2 ("raw"). A non-negative double orders like its bit
-// pattern read as an integer, so the cut-off test is an integer compare (off
-// the FP64 pipe).
-struct FixConst {
-  double s2, ua, pref;
-  long long lj2_bits;  // raw LJ reach, as bits
-};
-__device__ __forceinline__ FixConst fix_const(const DevParams& P) {
-  FixConst F;
-  const double s = P.ebox[0] * 0x1p-64;  // L / 2^64
-  F.s2 = s * s;
-  F.ua = P.alpha * F.s2;
-  F.pref = P.lB * P.sqrt_alpha;
-  F.lj2_bits = P.use_pair ? __double_as_longlong(P.lj_max2 / F.s2) : 0;
-  return F;
-}
-
 // ---------------------------------------------------------------- delta
 // One launch per move, one block per SM. Four of its warps (k role) own a run of
 // k units, so dS(k), the commit of the last accepted change and the |S|^2 change
@@ -173,66 +139,29 @@ __host__ __device__ inline int k_beads(const DevParams& P) {
   return fit < 1 ? 1 : (fit > 32 ? 32 : fit);
 }
 
-// Barrier of one role's threads.
-__device__ __forceinline__ void role_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 struct FixStage {
   ulonglong2 a, b, c;  // trial (x, y, z), current (x, y, z)
   double q;            // charge x lB sqrt(alpha) x table unit
   int k, pad;          // row of the LJ table
 };
 
-// A pair near enough for LJ or below the table, in FP64: dx, dy, dz the full
-// (unhalved) differences. Adds LJ to lj; returns h where the table has none.
-__device__ __forceinline__ double fix_near(const DevParams& P, const FixConst& F, uint64_t dx,
-                                           uint64_t dy, uint64_t dz, bool below, int k,
-                                           double& lj) {
-  const double x = __ll2double_rn((long long)dx), y = __ll2double_rn((long long)dy),
-               z = __ll2double_rn((long long)dz);
-  const double raw = fma(x, x, fma(y, y, z * z));
-  const long long rb = __double_as_longlong(raw);
-  if (rb < F.lj2_bits) lj += lj64(P, k, raw * F.s2);
-  if (!below || rb <= 0) return 0.0;
-  const long long bits = __double_as_longlong(raw * F.ua);
-  return bits >= kH64LoBits ? h64_tab(P.htab64, bits)
-                            : real_term64(P, raw * F.s2) / P.sqrt_alpha;
-}
-
 // The integer pair sweep of pair thread t of nt in every block. The table is
-// read in place for a few pairs per thread; for more it is copied to shared
-// memory first, where a warp's gather goes at a bank's pace (10 cycles a load)
-// and not a line's (32): from 4 pairs a thread on, the copy (51 KB a block, about
-// 1 us) pays.
+// read in place for a few pairs per thread; from 4 on, copying it to shared
+// memory first (51 KB a block, about 1 us) pays: a gather then takes 10 cycles
+// and not 32.
 constexpr int kFixStagePairs = 4;
 
 template <int kMode>
 __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& B, FixStage* st,
                                           unsigned char* tabs, int t0, int nt, int b_lo, int m,
                                           double& acc_lj, double& acc_re) {
-  const FixTab T = P.fx;
-  const FixConst F = fix_const(P);
-  const double qs = F.pref * T.unit, hs = 1.0 / T.unit;
+  FixTab T = P.fx;
+  const double qs = fix_scale(P), hs = 1.0 / T.unit;
   const int N = P.n_bead;
   const int G = (int)gridDim.x * nt, p0 = (int)blockIdx.x * nt + t0;
   const long long pairs = (long long)m * N;
-  const FixPair64* c01 = T.c01;
-  const FixPair64* c23 = T.c23;
-  const FixPair32* c45 = T.c45;
-  if (pairs >= (long long)kFixStagePairs * G) {
-    FixPair64* s01 = reinterpret_cast<FixPair64*>(tabs);
-    FixPair64* s23 = s01 + T.n_bin;
-    FixPair32* s45 = reinterpret_cast<FixPair32*>(s23 + T.n_bin);
-#pragma unroll 4
-    for (int i = t0; i < T.n_bin; i += nt) {
-      s01[i] = c01[i];
-      s23[i] = c23[i];
-      s45[i] = c45[i];
-    }
-    c01 = s01, c23 = s23, c45 = s45;
-  }
-  const auto tab = [&](uint64_t s) { return fix_h(c01, c23, c45, T.base, s); };
+  if (pairs >= (long long)kFixStagePairs * G) fix_stage(T, tabs, t0, nt);
+  const auto tab = [&](uint64_t s) { return fix_h(T.c01, T.c23, T.c45, T.base, s); };
   // a run of moved beads per job, shorter while there are fewer jobs than threads
   const int run_len = pairs >= 2LL * kFixRun * G ? kFixRun : (pairs >= 4LL * G ? 2 : 1);
   double lj1 = 0.0, lj0 = 0.0;
@@ -281,10 +210,10 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
         if (min(s1, s0) < T.s_near) {
           const int k = st[u].k + tj;
           double h = 0.0;
+          const int i = b_lo + g0 + u;
           if (s1 < T.s_near)
-            h = fix_near(P, F, o1.x - a.x, o1.y - a.y, o1.z - b.x, s1 < T.s_lo, k, lj1);
-          if (s0 < T.s_near)
-            h -= fix_near(P, F, o0.x - b.y, o0.y - c.x, o0.z - c.y, s0 < T.s_lo, k, lj0);
+            h = fix_near(P, B.trial[i], jm ? B.trial[j] : B.pos[j], s1 < T.s_lo, k, lj1);
+          if (s0 < T.s_near) h -= fix_near(P, B.pos[i], B.pos[j], s0 < T.s_lo, k, lj0);
           acc = fma(q * hs, h, acc);
         }
       }
@@ -386,11 +315,6 @@ __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B
     }
   }
   return e;
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
 template <int kMode>
@@ -582,21 +506,8 @@ __global__ void __launch_bounds__(kFixTile)
   const int per = kFixTile / parts;
   const int j0 = tb * kFixTile + (int)(blockIdx.x % parts) * per;
   const int jn = min(per, P.n_bead - j0);
-  const FixTab T = P.fx;
-  const FixPair64* c01 = T.c01;
-  const FixPair64* c23 = T.c23;
-  const FixPair32* c45 = T.c45;
-  if (kStaged) {
-    FixPair64* s01 = reinterpret_cast<FixPair64*>(smem);
-    FixPair64* s23 = s01 + T.n_bin;
-    FixPair32* s45 = reinterpret_cast<FixPair32*>(s23 + T.n_bin);
-    for (int i = threadIdx.x; i < T.n_bin; i += kFixTile) {
-      s01[i] = T.c01[i];
-      s23[i] = T.c23[i];
-      s45[i] = T.c45[i];
-    }
-    c01 = s01, c23 = s23, c45 = s45;
-  }
+  FixTab T = P.fx;
+  if (kStaged) fix_stage(T, smem, threadIdx.x, kFixTile);
   if ((int)threadIdx.x < jn) {
     const ulonglong4_32a p = fix64x4(P, B.pos[j0 + threadIdx.x]);
     so[threadIdx.x].a = make_ulonglong2(p.x, p.y);
@@ -605,8 +516,7 @@ __global__ void __launch_bounds__(kFixTile)
     st[threadIdx.x] = B.type[j0 + threadIdx.x];
   }
   __syncthreads();
-  const FixConst F = fix_const(P);
-  const auto tab = [&](uint64_t s) { return fix_h(c01, c23, c45, T.base, s); };
+  const auto tab = [&](uint64_t s) { return fix_h(T.c01, T.c23, T.c45, T.base, s); };
   double lj = 0.0, re = 0.0;
   const int i = ta * kFixTile + threadIdx.x;
   if (i < P.n_bead && jn > 0) {
@@ -630,11 +540,10 @@ __global__ void __launch_bounds__(kFixTile)
       uint64_t s;
       sum += fix_term<kMode>(T, tab, a.x - pi.x, a.y - pi.y, z - pi.z, s);
       if (s < T.s_near)
-        re = fma(q * hs, fix_near(P, F, a.x - pi.x, a.y - pi.y, z - pi.z, s < T.s_lo, kt + st[jj],
-                                  lj), re);
+        re = fma(q * hs, fix_near(P, B.pos[i], B.pos[j0 + jj], s < T.s_lo, kt + st[jj], lj), re);
     }
     re = fma(q, (double)sum, re);
-    re *= __longlong_as_double((long long)pi.w) * F.pref * T.unit;
+    re *= __longlong_as_double((long long)pi.w) * fix_scale(P);
   }
   const double a = block_sum<kFixTile>(lj, red);
   const double b = block_sum<kFixTile>(re, red);
