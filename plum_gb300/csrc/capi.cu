@@ -89,7 +89,8 @@ struct plum_ctx {
   double* d_log_de = nullptr;
   int log_cap = 0;
   bool host_pending = false;
-  int max_len = 1;
+  int max_len = 1;   // beads of the longest molecule that moves by itself
+  int most_len = 1;  // and of any (the host may move every one)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // the next move's generation runs beside the energy change
   cudaStream_t s_gen = nullptr;
@@ -161,6 +162,7 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
   P.alpha = in.alpha;
   P.kpref = in.lB / (kPiRef * vol) * (4 * kPiRef * kPiRef);
   P.turn_eps = (double)((kPiRef / 3.141592653589793238462643383279503L - 1.0L) * 0x1p64L);
+  P.turn_eps32 = (uint32_t)std::llround(P.turn_eps);
   P.self_coef = -in.lB * std::sqrt(in.alpha / kPiRef);
   P.dip_coef = in.lB * 2 * kPiRef / (vol / 1.0);
   P.dipole = in.dipole;
@@ -604,6 +606,8 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     (sz > 1 ? chains : ions).push_back(m);
     c->max_len = std::max(c->max_len, sz);
   }
+  for (int m = 0; m < in.n_mol; m++)
+    c->most_len = std::max(c->most_len, in.mol_start[m + 1] - in.mol_start[m]);
   P.n_chain_total = (int)chains.size();
   P.n_ion_total = (int)ions.size();
   std::vector<short4> kn;
@@ -676,7 +680,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   rc |= dalloc(&B.partial, 4 * (size_t)std::max(pair_grid(), pair_grid32()));
   rc |= dalloc(&B.fpos, nb);
   rc |= dalloc(&B.fq, nb);
-  rc |= dalloc(&B.ftrial, c->max_len);
+  rc |= dalloc(&B.ftrial, c->most_len);
   P.max_len = c->max_len;
   rc |= dalloc(&B.plan, 1);
   rc |= dalloc(&B.ctrial, kCands * (size_t)c->max_len);
@@ -728,7 +732,9 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     }
   }
   // the plain form's 64-bit position mirror for its integer pair loop
-  if (form == PLUM_FORM_FP64 && P.fx.mode) rc |= dalloc(&c->B.fpos64, nb);
+  if (form == PLUM_FORM_FP64 && P.fx.mode)
+    rc |= dalloc(&B.fpos64, nb) | dalloc(&B.ftrial64, c->most_len) |
+          dalloc(&B.ctrial64, kCands * (size_t)c->max_len);
   c->n_tot_part = total_partials_count(P);
   rc |= dalloc(&c->d_tot_part, 2 * (size_t)c->n_tot_part);
   // the precision form's real-space term from the h(u) table where the
@@ -803,7 +809,8 @@ int plum_ctx_destroy(plum_ctx* c) {
                   c->d_stream,   c->d_mt,      c->d_log_type, c->d_log_acc, c->d_log_e,
                   c->d_press,    c->d_sk_part, c->d_log_de, c->d_htab, c->d_htab64,
                   c->B.fpos64,   c->B.ku,      c->d_gtab64,
-                  c->d_fx,       c->B.plan,    c->B.ctrial, c->B.cftrial};
+                  c->d_fx,       c->B.plan,    c->B.ctrial, c->B.cftrial,
+                  c->B.ftrial64, c->B.ctrial64};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
@@ -891,7 +898,7 @@ int plum_delta_energy(plum_ctx* c, int mol, const double* trial, const int* move
   if (hi > lo)
     CK(cudaMemcpyAsync(c->B.trial + lo, span.data(), sizeof(double4_32a) * (hi - lo),
                        cudaMemcpyHostToDevice, c->s));
-  launch_set_move(c->B, mol, lo, hi, c->s);
+  launch_set_move(c->P, c->B, mol, lo, hi, c->s);
   if (c->form == PLUM_FORM_FP32) launch_fix_trial(c->P, c->B, c->s);
   launch_delta(c, c->B);
   launch_serial64(c->P, c->B, kModeFinish, c->s);
@@ -934,6 +941,9 @@ int rebuild_system(plum_ctx* c) {
     (sz > 1 ? chains : ions).push_back(m);
     c->max_len = std::max(c->max_len, sz);
   }
+  c->most_len = 1;
+  for (int m = 0; m < in.n_mol; m++)
+    c->most_len = std::max(c->most_len, in.mol_start[m + 1] - in.mol_start[m]);
   P.n_bead = nb;
   P.n_mol = in.n_mol;
   P.n_chain_total = (int)chains.size();
@@ -941,11 +951,11 @@ int rebuild_system(plum_ctx* c) {
   const bool mirror64 = B.fpos64 != nullptr;
   void* old[] = {B.pos,      B.trial,      B.type,     B.mol_start, B.chain_ids, B.ion_ids,
                  B.fpos,     B.fq,         B.ftrial,   B.dsk_part32, B.bond_mol, B.ctrial, B.cftrial,
-                 c->d_tot_part, c->d_obs_per, B.fpos64};
+                 c->d_tot_part, c->d_obs_per, B.fpos64, B.ftrial64, B.ctrial64};
   for (void* q : old)
     if (q) cudaFree(q);
   B.pos = B.trial = nullptr;
-  B.fpos64 = nullptr;
+  B.fpos64 = B.ftrial64 = B.ctrial64 = nullptr;
   B.type = B.mol_start = B.chain_ids = B.ion_ids = nullptr;
   B.fpos = B.ftrial = B.cftrial = nullptr;
   B.ctrial = nullptr;
@@ -957,10 +967,12 @@ int rebuild_system(plum_ctx* c) {
   int rc = dalloc(&B.pos, nb) | dalloc(&B.trial, nb) | dalloc(&B.type, nb) |
            dalloc(&B.mol_start, in.n_mol + 1) | dalloc(&B.chain_ids, chains.size()) |
            dalloc(&B.ion_ids, ions.size()) | dalloc(&B.fpos, nb) | dalloc(&B.fq, nb) |
-           dalloc(&B.ftrial, c->max_len) | dalloc(&B.bond_mol, in.n_mol) |
+           dalloc(&B.ftrial, c->most_len) | dalloc(&B.bond_mol, in.n_mol) |
            dalloc(&B.ctrial, kCands * (size_t)c->max_len) |
            dalloc(&B.cftrial, kCands * (size_t)c->max_len);
-  if (mirror64) rc |= dalloc(&B.fpos64, nb);
+  if (mirror64)
+    rc |= dalloc(&B.fpos64, nb) | dalloc(&B.ftrial64, c->most_len) |
+          dalloc(&B.ctrial64, kCands * (size_t)c->max_len);
   const int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
   rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
   c->n_tot_part = total_partials_count(P);
@@ -1669,7 +1681,7 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
     if (dalloc(&c->cb_part32, (size_t)G.slots)) return PLUM_ERR_CUDA;
     c->cb_part32_cap = G.slots;
   }
-  if (!c->cb_ticket) {
+  if (fp32 && !c->cb_ticket) {
     if (dalloc(&c->cb_ticket, 1)) return PLUM_ERR_CUDA;
     CK(cudaMemsetAsync(c->cb_ticket, 0, sizeof(int), c->s));
   }
@@ -1709,14 +1721,13 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
   J.part = fp32 ? c->cb_part32 : c->cb_part;
   J.u = c->cb_u;
   J.slots = c->cb_slots;
-  J.ticket = c->cb_ticket;
   *Jp = J;
   *Gp = G;
   return PLUM_OK;
 }
 
 // One growth step's trial energies on the context's stream: one launch in the
-// precision form and where the integer pair form applies, else the FP64 kernels
+// precision form, two where the integer pair form applies, else the FP64 kernels
 // (S_o, system sweep, per-trial sums).
 static int cbmc_launch(plum_ctx* c, const CbmcJob& J, const Cbmc32Layout& G) {
   if (c->form == PLUM_FORM_FP32) {
@@ -1765,8 +1776,8 @@ int plum_cbmc_time(plum_ctx* c, int n_trials, const double* b1, const double* b2
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   *ms_out = (double)ms / reps;
   if (launches_out)
-    *launches_out = c->form == PLUM_FORM_FP32 || c->B.fpos64
-                        ? 1 : ((c->P.use_ewald && c->P.n_k > 0) ? 3 : 2);
+    *launches_out = c->form == PLUM_FORM_FP32
+                        ? 1 : ((c->P.use_ewald && c->P.n_k > 0 && !c->B.fpos64) ? 3 : 2);
   return PLUM_OK;
 }
 

@@ -113,6 +113,7 @@ struct DevParams {
   // every axis, r_c <= L, one box for both terms; mode 0 where it does not apply
   FixTab fx;
   double turn_eps;  // (kPi / pi - 1) 2^64: phases count turns of the reference's 2 kPi
+  uint32_t turn_eps32, pad32;  // the same as an integer
 };
 
 // The pending move: beads [b_lo, b_hi) of molecule `mol` hold trial
@@ -203,6 +204,8 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   // plain form mirror (where P.fx applies; null otherwise): 64-bit
   // fixed-point fractions of the box (X, Y, Z) and the charge's bits
   ulonglong4_32a* fpos64;  // [n_bead] current positions
+  ulonglong4_32a* ftrial64;  // [longest molecule] trial of the pending move's beads, from b_lo on
+  ulonglong4_32a* ctrial64;  // [kCands][max_len] the candidates'
   // precision form mirrors: 32-bit fixed-point fractions of the Ewald box
   int4* fpos;        // [n_bead] current (X, Y, Z, type)
   float* fq;         // [n_bead] charges
@@ -283,7 +286,8 @@ constexpr int kModeCommit = 8;   // commit/reject by state->last_accept (host de
 void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStream_t s);
 // The next move's candidates; first: no move is pending (kCandSkip only).
 void launch_gen64(const DevParams& P, const DevBuffers& B, bool first, cudaStream_t s);
-void launch_set_move(const DevBuffers& B, int mol, int b_lo, int b_hi, cudaStream_t s);
+void launch_set_move(const DevParams& P, const DevBuffers& B, int mol, int b_lo, int b_hi,
+                     cudaStream_t s);
 void launch_observables64(const DevParams& P, const DevBuffers& B, double* per_mol,
                           double* out5, cudaStream_t s);
 void launch_rhoz(const DevParams& P, const DevBuffers& B, double res, int n_bins, unsigned* cnt,
@@ -308,13 +312,12 @@ struct CbmcJob {
   double* part;                     // [n_trials][groups][2] scratch
   double* u;                        // [n_trials] result
   double* slots;                    // [cbmc_blocks()][n_trials][3] block sums
-  int* ticket;                      // zero before the first launch, left zero
 };
 constexpr int kCbmcGroups = 64;  // most that cbmc_groups returns
 int cbmc_groups(const DevParams& P);
 int cbmc_blocks();
 void launch_cbmc(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s);
-// One launch, for contexts with B.fpos64 (so P.fx applies).
+// Two launches, for contexts with B.fpos64 (so P.fx applies).
 void launch_cbmc64(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s);
 // The precision form's one-launch trial kernel (kern_cbmc32.cu): J.part holds
 // `slots` doubles laid out by cbmc32_layout; J.s_o is unused. ticket is one

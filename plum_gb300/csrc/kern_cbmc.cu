@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(kCbThreads)
   }
 }
 
-// The same energies in one launch where the integer pair form applies (and the
-// context keeps the 64-bit position mirror).
+// The same energies where the integer pair form applies (and the context keeps
+// the 64-bit position mirror), in a sweep and a sum per trial.
 //   pair role  a warp's lanes take 32 trials, so a system bead (and, as the
 //              list's tail, a grown bead) is one broadcast load and no sum
 //              crosses lanes; opposite charges of a trial and its counterion
@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(kCbThreads)
 //   k role     (charged species) a block's own k units: S_o(k) from the
 //              committed S(k), the deleted and the grown beads, then every
 //              trial's kw (2 S_o.e + |e|^2)
-// The last block to finish adds the blocks' sums in order and the trial's own
-// terms. No split depends on the number of trials, so neither does a result. One growth step of 32 trials on 6,400 beads, r_c = 0.7 L: XXX us, 430 us
+// k_cbmc64_sum adds the blocks' sums of a trial in order and its own terms, a block
+// per trial (the last block of the sweep doing it for all took longer than the
+// launch). No split depends on the number of trials, so neither does a result. One growth step of 32 trials on 6,400 beads, r_c = 0.7 L: XXX us, 430 us
 // in three FP64 launches (27 image cells per pair, a sincos per trial and k).
 constexpr int kCb64Threads = 512, kCb64K = 128;
 
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
   extern __shared__ __align__(32) unsigned char smem[];
   __shared__ double s_red[3][kCb64Threads];
   __shared__ double s_w[2][kCb64K / 32][4];
-  __shared__ int s_last;
+  __shared__ ulonglong4_32a s_site[2][32];
   const int kth = J.charged && P.use_ewald && P.n_ku > 0 ? kCb64K : 0;
   const int tid = threadIdx.x, T = J.n_trials, N = P.n_bead;
   const int grown = J.cl * (J.charged ? 2 : 1);
@@ -262,11 +263,11 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
       double q[2] = {0.0, 0.0};
       if (tid < tl)
         for (int b = 0; b < 2; b++) {
-          const double4_32a v = b ? J.b2[c0 + tid] : J.b1[c0 + tid];
-          x[b] = turn64(P, v.x, 0);
-          y[b] = turn64(P, v.y, 1);
-          z[b] = turn64(P, v.z, 2);
-          q[b] = v.w;
+          const ulonglong4_32a v = fix64x4(P, b ? J.b2[c0 + tid] : J.b1[c0 + tid]);
+          x[b] = turn_fix(P, v.x);
+          y[b] = turn_fix(P, v.y);
+          z[b] = turn_fix(P, v.z);
+          q[b] = __longlong_as_double((long long)v.w);
         }
       const int u0 = (int)((long long)P.n_ku * blockIdx.x / gridDim.x);
       const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / gridDim.x);
@@ -278,15 +279,16 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
         const uint64_t nx = (uint64_t)ku.nx, ny = (uint64_t)(int64_t)ku.ny, nz = (uint64_t)ku.nz;
         double o[4] = {0.0, 0.0, 0.0, 0.0};
         for (int i = tid; i < gone + grown; i += kCb64K) {
-          double4_32a v = i < gone ? B.pos[J.ex_lo + i] : grown_bead(i - gone);
-          if (i < gone) v.w = -v.w;
-          const uint64_t xy = nx * turn64(P, v.x, 0) + ny * turn64(P, v.y, 1);
-          const uint64_t zz = nz * turn64(P, v.z, 2);
+          const ulonglong4_32a v =
+              i < gone ? B.fpos64[J.ex_lo + i] : fix64x4(P, grown_bead(i - gone));
+          const double w0 = __longlong_as_double((long long)v.w), w = i < gone ? -w0 : w0;
+          const uint64_t xy = nx * turn_fix(P, v.x) + ny * turn_fix(P, v.y);
+          const uint64_t zz = nz * turn_fix(P, v.z);
           const double2 ep = turn_exp(xy + zz), em = turn_exp(xy - zz);
-          o[0] = fma(v.w, ep.x, o[0]);
-          o[1] = fma(v.w, ep.y, o[1]);
-          o[2] = fma(v.w, em.x, o[2]);
-          o[3] = fma(v.w, em.y, o[3]);
+          o[0] = fma(w, ep.x, o[0]);
+          o[1] = fma(w, ep.y, o[1]);
+          o[2] = fma(w, em.x, o[2]);
+          o[3] = fma(w, em.y, o[3]);
         }
         for (int c = 0; c < 4; c++) {
           o[c] = warp_sum(o[c]);
@@ -338,7 +340,9 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
       const int t = min(c0 + lane, T - 1);
       const double4_32a p1 = J.b1[t];
       const double4_32a p2 = J.charged ? J.b2[t] : p1;
-      const ulonglong4_32a f1 = fix64x4(P, p1), f2 = fix64x4(P, p2);
+      if (sl < nb) s_site[sl][lane] = fix64x4(P, sl ? p2 : p1);
+      role_sync(2, nt);
+      const ulonglong4_32a f1 = s_site[0][lane], f2 = nb > 1 ? s_site[1][lane] : f1;
       double lj = 0.0, re = 0.0;
       for (int j = (int)blockIdx.x * slices + sl; j < N + grown; j += (int)gridDim.x * slices) {
         if (j >= J.ex_lo && j < J.ex_hi) continue;
@@ -380,56 +384,52 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
       role_sync(2, nt);
     }
   }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = atomicAdd(J.ticket, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const int lane = tid & 31, part = tid >> 5;
-  constexpr int parts = kCb64Threads / 32;
-  for (int c0 = 0; c0 < T; c0 += 32) {
-    const int t = min(c0 + lane, T - 1);
-    double v[3] = {0.0, 0.0, 0.0};
-    for (int b = part; b < (int)gridDim.x; b += parts) {
-      const double* s = J.slots + ((size_t)b * T + t) * 3;
-      for (int c = 0; c < 3; c++) v[c] += __ldcg(s + c);
-    }
-    for (int c = 0; c < 3; c++) s_red[c][tid] = v[c];
-    __syncthreads();
-    if (part == 0 && c0 + lane < T) {
-      for (int c = 0; c < 3; c++) {
-        v[c] = 0.0;
-        for (int w = 0; w < parts; w++) v[c] += s_red[c][w * 32 + lane];
-      }
-      const double4_32a b1 = J.b1[t], b2 = J.charged ? J.b2[t] : b1;
-      double pair_e = v[0], ew = 0.0;
-      if (J.charged) {
-        const ulonglong4_32a f1 = fix64x4(P, b1), f2 = fix64x4(P, b2);
-        const uint64_t dx = f2.x - f1.x, dy = f2.y - f1.y, dz = f2.z - f1.z;
-        uint64_t s0;
-        const auto tab = [&](uint64_t s) {
-          return fix_h(P.fx.c01, P.fx.c23, P.fx.c45, P.fx.base, s);
-        };
-        double re = (double)fix_term<kMode>(P.fx, tab, dx, dy, dz, s0) * P.fx.unit;
-        if (s0 < P.fx.s_near)
-          re += fix_near(P, b1, b2, s0 < P.fx.s_lo, J.type * P.n_type + J.type, pair_e);
-        if (P.use_ewald && pair_e < kVeryLarge) {
-          ew = v[1] + P.kpref * v[2] + P.lB * P.sqrt_alpha * b1.w * b2.w * re;
-          ew += P.self_coef * (b1.w * b1.w + b2.w * b2.w);
-          if (P.real_cut >= P.ebox[0])  // a bead's own images
-            ew += 0.5 * (cb_real(P, b1, b1) + cb_real(P, b2, b2));
-        }
-      }
-      if (P.use_ext) {
-        pair_e += wall64(P, b1.z, J.type);
-        if (J.charged) pair_e += wall64(P, b2.z, J.type);
-      }
-      J.u[t] = pair_e >= kVeryLarge ? kVeryLarge : pair_e + ew;
-    }
-    __syncthreads();
+}
+
+constexpr int kCb64Sum = 128;
+
+template <int kMode>
+__global__ void __launch_bounds__(kCb64Sum)
+    k_cbmc64_sum(const DevParams P, const DevBuffers B, CbmcJob J, int blocks) {
+  __shared__ double s_w[kCb64Sum / 32][3];
+  const int t = blockIdx.x, tid = threadIdx.x;
+  double v[3] = {0.0, 0.0, 0.0};
+  for (int b = tid; b < blocks; b += kCb64Sum)
+    for (int c = 0; c < 3; c++) v[c] += J.slots[((size_t)b * J.n_trials + t) * 3 + c];
+  for (int c = 0; c < 3; c++) {
+    v[c] = warp_sum(v[c]);
+    if ((tid & 31) == 0) s_w[tid >> 5][c] = v[c];
   }
-  if (tid == 0) *J.ticket = 0;
+  __syncthreads();
+  if (tid) return;
+  for (int c = 0; c < 3; c++) {
+    v[c] = 0.0;
+    for (int w = 0; w < kCb64Sum / 32; w++) v[c] += s_w[w][c];
+  }
+  const double4_32a b1 = J.b1[t], b2 = J.charged ? J.b2[t] : b1;
+  double pair_e = v[0], ew = 0.0;
+  if (J.charged) {
+    const ulonglong4_32a f1 = fix64x4(P, b1), f2 = fix64x4(P, b2);
+    uint64_t s0;
+    const auto tab = [&](uint64_t s) {
+      return fix_h(P.fx.c01, P.fx.c23, P.fx.c45, P.fx.base, s);
+    };
+    double re = (double)fix_term<kMode>(P.fx, tab, f2.x - f1.x, f2.y - f1.y, f2.z - f1.z, s0) *
+                P.fx.unit;
+    if (s0 < P.fx.s_near)
+      re += fix_near(P, b1, b2, s0 < P.fx.s_lo, J.type * P.n_type + J.type, pair_e);
+    if (P.use_ewald && pair_e < kVeryLarge) {
+      ew = v[1] + P.kpref * v[2] + P.lB * P.sqrt_alpha * b1.w * b2.w * re;
+      ew += P.self_coef * (b1.w * b1.w + b2.w * b2.w);
+      if (P.real_cut >= P.ebox[0])  // a bead's own images
+        ew += 0.5 * (cb_real(P, b1, b1) + cb_real(P, b2, b2));
+    }
+  }
+  if (P.use_ext) {
+    pair_e += wall64(P, b1.z, J.type);
+    if (J.charged) pair_e += wall64(P, b2.z, J.type);
+  }
+  J.u[t] = pair_e >= kVeryLarge ? kVeryLarge : pair_e + ew;
 }
 
 template <int kMode>
@@ -443,6 +443,7 @@ static void launch_one64(const DevParams& P, const DevBuffers& B, const CbmcJob&
   }
   k_cbmc64<kMode><<<cbmc_blocks(), kCb64Threads, J.charged ? (size_t)P.fx.n_bin * 40 : 0, s>>>(
       P, B, J);
+  k_cbmc64_sum<kMode><<<J.n_trials, kCb64Sum, 0, s>>>(P, B, J, cbmc_blocks());
 }
 
 void launch_cbmc64(const DevParams& P, const DevBuffers& B, const CbmcJob& J, cudaStream_t s) {

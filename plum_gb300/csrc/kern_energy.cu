@@ -170,7 +170,7 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
     if (g0) role_sync(2, nt);  // the previous group is consumed
     for (int t = t0; t < gn; t += nt) {
       const int i = b_lo + g0 + t;
-      const ulonglong4_32a a = fix64x4(P, B.trial[i]), c = B.fpos64[i];
+      const ulonglong4_32a a = B.ftrial64[g0 + t], c = B.fpos64[i];
       st[t].a = make_ulonglong2(a.x, a.y);
       st[t].b = make_ulonglong2(a.z, c.x);
       st[t].c = make_ulonglong2(c.y, c.z);
@@ -192,7 +192,7 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
       // a moved other bead: its trial position, and only moved beads before it
       const int l = j - b_lo - g0;
       const bool jm = j >= b_lo && j < b_lo + m;
-      const ulonglong4_32a o1 = jm ? fix64x4(P, B.trial[j]) : o0;
+      const ulonglong4_32a o1 = jm ? B.ftrial64[j - b_lo] : o0;
       const int u0 = run * run_len, u1 = min(gn, u0 + run_len);
       double acc = 0.0, q = st[u0].q;
       int64_t sum = 0;
@@ -228,6 +228,7 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
 // threads. A thread takes one of up to 32 units and every slices-th moved bead (a
 // block of a small k-set has few units: their beads then spread over the lanes).
 // smem, kb = k_beads: [kb][2][zn] e^{i n theta_z}, then [kb][2][kUnits] xy parts.
+template <int kMode>
 __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B,
                                          unsigned char* smem, int u0, int u1, int b_lo, int b_hi,
                                          int sk_pend, int sk_buf, int cur_buf) {
@@ -261,9 +262,24 @@ __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B
       // nt z recursions, then nt x ncol xy phases, one per thread
       for (int t = threadIdx.x; t < nt * (1 + ncol); t += kKThreads) {
         const int c = t / nt - 1, it = t - (c + 1) * nt;
-        const double4_32a p = (it & 1) ? B.pos[g0 + (it >> 1)] : B.trial[g0 + (it >> 1)];
+        const int bead = g0 + (it >> 1);
+        uint64_t tx, ty, tz;
+        double q;
+        if (kMode) {  // in integers from the mirrors
+          const ulonglong4_32a p = (it & 1) ? B.fpos64[bead] : B.ftrial64[bead - b_lo];
+          tx = turn_fix(P, p.x);
+          ty = turn_fix(P, p.y);
+          tz = turn_fix(P, p.z);
+          q = __longlong_as_double((long long)p.w);
+        } else {
+          const double4_32a p = (it & 1) ? B.pos[bead] : B.trial[bead];
+          tx = c < 0 ? 0 : turn64(P, p.x, 0);
+          ty = c < 0 ? 0 : turn64(P, p.y, 1);
+          tz = c < 0 ? turn64(P, p.z, 2) : 0;
+          q = p.w;
+        }
         if (c < 0) {
-          const double2 e1 = turn_exp(turn64(P, p.z, 2));
+          const double2 e1 = turn_exp(tz);
           double2 v = make_double2(1.0, 0.0);
           double2* z = s_z + (size_t)it * zn;
           z[0] = v;
@@ -273,9 +289,8 @@ __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B
           }
         } else {
           const short2 kc = s_col[c];
-          const double2 v = turn_exp(turn64(P, p.x, 0) * (uint64_t)(int64_t)kc.x +
-                                     turn64(P, p.y, 1) * (uint64_t)(int64_t)kc.y);
-          const double q = (it & 1) ? -p.w : p.w;  // trial minus current
+          const double2 v = turn_exp(tx * (uint64_t)(int64_t)kc.x + ty * (uint64_t)(int64_t)kc.y);
+          if (it & 1) q = -q;  // trial minus current
           s_xy[it * kUnits + c] = make_double2(q * v.x, q * v.y);
         }
       }
@@ -332,7 +347,7 @@ __global__ void __launch_bounds__(kDeltaThreads, 1)
     const int u0 = (int)((long long)P.n_ku * blockIdx.x / gridDim.x);
     const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / gridDim.x);
     if (m > 0)
-      a = k_role(P, B, smem + tab_bytes, u0, u1, b_lo, b_hi, st->sk_pending, st->sk_buf,
+      a = k_role<kMode>(P, B, smem + tab_bytes, u0, u1, b_lo, b_hi, st->sk_pending, st->sk_buf,
                  st->cur_buf);
   } else {
     const int t0 = (int)threadIdx.x - kthreads, nt = kDeltaThreads - kthreads;

@@ -315,6 +315,7 @@ __device__ __forceinline__ void pivot_draws_seq(const DevParams& P, Draws& d, lo
 struct TrialOut {
   double4_32a* t;
   int4* f;
+  ulonglong4_32a* u;
 };
 
 // The trial position of bead i, and its fixed-point mirror for the precision
@@ -323,6 +324,7 @@ __device__ __forceinline__ void put_trial(const DevParams& P, const DevBuffers& 
                                           int b_lo, int i, double4_32a t) {
   O.t[i - b_lo] = t;
   if (P.form) O.f[i - b_lo] = fix_point(P, t, B.type[i]);
+  if (B.fpos64) O.u[i - b_lo] = fix64x4(P, t);
 }
 
 // Walls and sum q dz of the moved beads, and the moved molecule's bonds at the
@@ -659,10 +661,10 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
     }
   }
   __syncthreads();
-  if (P.form && g.type == 2 && g.pivot < 0)
+  if (g.type == 2 && g.pivot < 0)
     // fixed-point trial coordinates of the sequential pivot
     for (int i = g.b_lo + threadIdx.x; i < g.b_hi; i += blockDim.x)
-      O.f[i - g.b_lo] = fix_point(P, O.t[i - g.b_lo], B.type[i]);
+      put_trial(P, B, O, g.b_lo, i, O.t[i - g.b_lo]);
   move_sums(P, B, g.type >= 0, g.mol, g.b_lo, g.b_hi, V,
             [&](int i) { return i >= g.b_lo && i < g.b_hi ? O.t[i - g.b_lo] : V.at(i); }, C, red);
   if (threadIdx.x == 0) {
@@ -723,7 +725,8 @@ __device__ __forceinline__ void gen_body(const DevParams& P, const DevBuffers& B
   __syncthreads();
   const bool took = c == kCandAccept;
   const PosView V{B.pos, B.trial, took ? st->b_lo : 0, took ? st->b_hi : 0};
-  const TrialOut O{B.ctrial + (size_t)c * P.max_len, B.cftrial + (size_t)c * P.max_len};
+  const size_t at = (size_t)c * P.max_len;
+  const TrialOut O{B.ctrial + at, B.cftrial + at, B.ctrial64 + at};
   gen_move(P, B, st, V, O, sm.C, d, base, sm.plan, sm.s_off, sm.s_boff, sm.s_w, sm.jump, sm.accbits,
            sm.red, gp, sm.pre);
   if (threadIdx.x == 0) B.plan->cand[c] = sm.C;
@@ -927,7 +930,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
       for (int i = b_lo + threadIdx.x; i < b_hi; i += blockDim.x) {
         const int4 old_f = P.form ? B.fpos[i] : make_int4(0, 0, 0, 0);
         B.pos[i] = B.trial[i];
-        if (B.fpos64) B.fpos64[i] = fix64x4(P, B.trial[i]);
+        if (B.fpos64) B.fpos64[i] = B.ftrial64[i - b_lo];
         if (P.form) B.fpos[i] = B.ftrial[i - b_lo];
         if (P.cell_cap && B.cell_key) {
           // the bead's entry follows it: rewritten in place while it stays in
@@ -1000,6 +1003,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
       for (int i = threadIdx.x; i < C.b_hi - C.b_lo; i += blockDim.x) {
         B.trial[C.b_lo + i] = t[i];
         if (P.form) B.ftrial[i] = f[i];
+        if (B.fpos64) B.ftrial64[i] = B.ctrial64[(size_t)c * P.max_len + i];
       }
     // surrogate move: its descriptor is accumulated from zero by the next launch
     const bool surr = C.type >= 2 && B.desc_acc && B.desc_fine && (S.da_on || B.log_desc);
@@ -1106,16 +1110,23 @@ void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStre
   k_serial64<<<1, kSerialThreads, 0, s>>>(P, B, mode, P.form ? 0 : delta_blocks64());
 }
 
-__global__ void k_set_move(DevState* st, int mol, int b_lo, int b_hi) {
-  st->pending = 1;
-  st->mol = mol;
-  st->b_lo = b_lo;
-  st->b_hi = b_hi;
-  st->move_type = -1;
+__global__ void k_set_move(const DevParams P, const DevBuffers B, int mol, int b_lo, int b_hi) {
+  if (threadIdx.x == 0) {
+    DevState* st = B.state;
+    st->pending = 1;
+    st->mol = mol;
+    st->b_lo = b_lo;
+    st->b_hi = b_hi;
+    st->move_type = -1;
+  }
+  if (B.fpos64)
+    for (int i = b_lo + threadIdx.x; i < b_hi; i += blockDim.x)
+      B.ftrial64[i - b_lo] = fix64x4(P, B.trial[i]);
 }
 
-void launch_set_move(const DevBuffers& B, int mol, int b_lo, int b_hi, cudaStream_t s) {
-  k_set_move<<<1, 1, 0, s>>>(B.state, mol, b_lo, b_hi);
+void launch_set_move(const DevParams& P, const DevBuffers& B, int mol, int b_lo, int b_hi,
+                     cudaStream_t s) {
+  k_set_move<<<1, 128, 0, s>>>(P, B, mol, b_lo, b_hi);
 }
 
 // ------------------------------------------------------------ mt19937 fill

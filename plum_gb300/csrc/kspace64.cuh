@@ -16,6 +16,12 @@ __device__ __forceinline__ uint64_t turn64(const DevParams& P, double w, int axi
   return __double2ull_rn(g * 0x1p64) + (uint64_t)__double2ll_rn(f * P.turn_eps);
 }
 
+// The same of a coordinate's box fraction X (fix64; a cubic periodic box): X kPi /
+// pi, in integers.
+__device__ __forceinline__ uint64_t turn_fix(const DevParams& P, uint64_t X) {
+  return X + __umulhi((uint32_t)(X >> 32), P.turn_eps32);
+}
+
 // e^{2 pi i phi / 2^64}: the nearest quarter turn taken off in integers, then the
 // Taylor series of sine and cosine on |theta| <= pi / 4 (through theta^15 and
 // theta^16: the next terms are under 5e-17). About 20 FP64 operations, with no
