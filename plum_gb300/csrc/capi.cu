@@ -539,6 +539,8 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   P.beta = in.beta;
   P.move_size = in.move_size;
   for (int i = 0; i < 5; i++) P.move_prob[i] = in.move_prob[i];
+  double cum = P.move_prob[0];
+  for (int i = 0; i < 4; cum += P.move_prob[++i]) std::memcpy(&P.move_cum[i], &cum, sizeof(cum));
   // simulation.cc:286-296
   P.bond_len = 0;
   P.vary_bond = 0;
@@ -600,10 +602,10 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     auto ir = in.wall_radius.find(in.type_names[i]);
     P.wall_rad[i] = ir != in.wall_radius.end() ? ir->second : 0.0;
   }
-  std::vector<int> chains, ions;
+  std::vector<int4> chains, ions;
   for (int m = in.phantom; m < in.n_mol; m++) {
     int sz = in.mol_start[m + 1] - in.mol_start[m];
-    (sz > 1 ? chains : ions).push_back(m);
+    (sz > 1 ? chains : ions).push_back(make_int4(m, in.mol_start[m], in.mol_start[m + 1], 0));
     c->max_len = std::max(c->max_len, sz);
   }
   for (int m = 0; m < in.n_mol; m++)
@@ -768,9 +770,9 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   cudaMemcpy(B.mol_start, in.mol_start.data(), sizeof(int) * (in.n_mol + 1),
              cudaMemcpyHostToDevice);
   if (!chains.empty())
-    cudaMemcpy(B.chain_ids, chains.data(), sizeof(int) * chains.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(B.chain_ids, chains.data(), sizeof(int4) * chains.size(), cudaMemcpyHostToDevice);
   if (!ions.empty())
-    cudaMemcpy(B.ion_ids, ions.data(), sizeof(int) * ions.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(B.ion_ids, ions.data(), sizeof(int4) * ions.size(), cudaMemcpyHostToDevice);
   if (!kn.empty()) {
     cudaMemcpy(B.kn, kn.data(), sizeof(short4) * kn.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(B.kw, kw.data(), sizeof(double) * kw.size(), cudaMemcpyHostToDevice);
@@ -934,11 +936,11 @@ int rebuild_system(plum_ctx* c) {
   DevBuffers& B = c->B;
   const int nb = (int)in.q.size();
   CK(cudaStreamSynchronize(c->s));
-  std::vector<int> chains, ions;
+  std::vector<int4> chains, ions;
   c->max_len = 1;
   for (int m = in.phantom; m < in.n_mol; m++) {
     const int sz = in.mol_start[m + 1] - in.mol_start[m];
-    (sz > 1 ? chains : ions).push_back(m);
+    (sz > 1 ? chains : ions).push_back(make_int4(m, in.mol_start[m], in.mol_start[m + 1], 0));
     c->max_len = std::max(c->max_len, sz);
   }
   c->most_len = 1;
@@ -956,7 +958,8 @@ int rebuild_system(plum_ctx* c) {
     if (q) cudaFree(q);
   B.pos = B.trial = nullptr;
   B.fpos64 = B.ftrial64 = B.ctrial64 = nullptr;
-  B.type = B.mol_start = B.chain_ids = B.ion_ids = nullptr;
+  B.type = B.mol_start = nullptr;
+  B.chain_ids = B.ion_ids = nullptr;
   B.fpos = B.ftrial = B.cftrial = nullptr;
   B.ctrial = nullptr;
   P.max_len = c->max_len;
@@ -987,10 +990,10 @@ int rebuild_system(plum_ctx* c) {
   CK(cudaMemcpyAsync(B.mol_start, in.mol_start.data(), sizeof(int) * (in.n_mol + 1),
                      cudaMemcpyHostToDevice, c->s));
   if (!chains.empty())
-    CK(cudaMemcpyAsync(B.chain_ids, chains.data(), sizeof(int) * chains.size(),
+    CK(cudaMemcpyAsync(B.chain_ids, chains.data(), sizeof(int4) * chains.size(),
                        cudaMemcpyHostToDevice, c->s));
   if (!ions.empty())
-    CK(cudaMemcpyAsync(B.ion_ids, ions.data(), sizeof(int) * ions.size(), cudaMemcpyHostToDevice,
+    CK(cudaMemcpyAsync(B.ion_ids, ions.data(), sizeof(int4) * ions.size(), cudaMemcpyHostToDevice,
                        c->s));
   if (c->d_rp1) CK(cudaMemcpyAsync(c->d_rp1, &P, sizeof(P), cudaMemcpyHostToDevice, c->s));
   DevState st;

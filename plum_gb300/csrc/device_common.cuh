@@ -75,15 +75,20 @@ __device__ __forceinline__ double wall64(const DevParams& P, double z, int ty) {
   return energy;
 }
 
-__device__ __forceinline__ int fix_axis(double x, double L, double inv_fix, bool periodic) {
-  double w = periodic ? x - L * floor(x / L) : x;
+__device__ __forceinline__ int fix_axis(double x, double L, double inv, double inv_fix,
+                                        bool periodic) {
+  double w = periodic ? x - L * floor(x * inv) : x;
   long long v = llrint(w * inv_fix);
   return (int)(unsigned int)(unsigned long long)v;
 }
 
-// 64-bit fixed-point fraction of the box: frac(x / L) 2^64.
+// 64-bit fixed-point fraction of the box: frac(x / L) 2^64. Within 16 boxes of the
+// origin one conversion of x / L in units of 2^-58 boxes does (x / L itself is
+// rounded at 2^-54 or coarser from 1/2 on), and the shift drops the whole boxes.
 __device__ __forceinline__ unsigned long long fix64(double x, double inv) {
   double f = x * inv;
+  if ((__double2hiint(f) & 0x7FF00000) < ((1023 + 4) << 20))
+    return (unsigned long long)__double2ll_rn(f * 0x1p58) << 6;
   f -= floor(f);
   if (f >= 1.0) f = 0.0;  // a tiny negative x / L rounds up to 1
   return __double2ull_rn(f * 0x1p64);
@@ -97,9 +102,9 @@ __device__ __forceinline__ ulonglong4_32a fix64x4(const DevParams& P, double4_32
 }
 
 __device__ __forceinline__ int4 fix_point(const DevParams& P, double4_32a p, int type) {
-  return make_int4(fix_axis(p.x, P.ebox[0], P.inv_fix[0], true),
-                   fix_axis(p.y, P.ebox[1], P.inv_fix[1], true),
-                   fix_axis(p.z, P.ebox[2], P.inv_fix[2], P.npbc > 2), type);
+  return make_int4(fix_axis(p.x, P.ebox[0], P.inv_ebox[0], P.inv_fix[0], true),
+                   fix_axis(p.y, P.ebox[1], P.inv_ebox[1], P.inv_fix[1], true),
+                   fix_axis(p.z, P.ebox[2], P.inv_ebox[2], P.inv_fix[2], P.npbc > 2), type);
 }
 
 // Hard spheres leave out the pair energy of a chain's bonded neighbours

@@ -56,6 +56,7 @@ struct DevParams {
   double ebox[3], inv_ebox[3];
   int use_pair, use_ewald, use_bond, use_rigid, use_ext, dipole;
   double beta, move_size, move_prob[5];
+  long long move_cum[4];  // running sums of move_prob, as bits
   double bond_len;   // r0 (bond potential) or the rigid length
   int vary_bond;     // bond potential on: +-10% bond length draws
   // LJ per ordered type pair k = ti*n_type+tj (potential_truncated_lj.cc:49-85)
@@ -182,6 +183,8 @@ struct MoveCand {
   double u1;      // delayed acceptance's stage-one draw
   // walls, sum q dz and the molecule's bonds at the trial positions
   double ext, dmz, bond;
+  double bond_old;  // the molecule's bond energy before it
+  int bonded, pad;  // the molecule has bonds
 };
 struct StepPlan {
   MoveCand cand[kCands];
@@ -193,8 +196,8 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   double4_32a* trial;
   int* type;
   int* mol_start;
-  int* chain_ids;
-  int* ion_ids;
+  int4* chain_ids;   // molecules to pick from: (molecule, first bead, one past it, 0)
+  int4* ion_ids;
   short4* kn;
   KUnit* ku;         // [n_ku] the k list as +-nz pairs
   double* kw;

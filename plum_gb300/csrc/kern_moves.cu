@@ -81,7 +81,7 @@ __device__ __forceinline__ bool sphere_reject(uint32_t u1, uint32_t u2) {
 }
 
 // Consumes randSphere's draws; returns the stream index of the accepted pair.
-__device__ long long sphere_scan(Draws& d) {
+__device__ __forceinline__ long long sphere_scan(Draws& d) {
   for (int guard = 0; guard < (1 << 20); guard++) {
     long long o = d.pos;
     uint32_t u1 = d.next(), u2 = d.next();
@@ -96,7 +96,7 @@ __device__ long long sphere_scan(Draws& d) {
 // position p: bit p set when the pair (p, p+1) is accepted. A pair starting at
 // `pos` is followed by the pair at pos+2, so thread 0 looks for the next set
 // bit of pos's parity; past the window it falls back to sphere_scan.
-__device__ long long sphere_scan_bits(Draws& d, const unsigned* accbits) {
+__device__ __forceinline__ long long sphere_scan_bits(Draws& d, const unsigned* accbits) {
   const long long rel0 = d.pos - d.wbase;
   if (rel0 < 0) return sphere_scan(d);
   long long rel = rel0;
@@ -118,7 +118,7 @@ __device__ long long sphere_scan_bits(Draws& d, const unsigned* accbits) {
 }
 
 // The unit vector randSphere returns for an accepted pair.
-__device__ void sphere_vec(uint32_t u1, uint32_t u2, double* v) {
+__device__ __forceinline__ void sphere_vec(uint32_t u1, uint32_t u2, double* v) {
   double r1 = 1.0 - 2.0 * unit_draw(u1);
   double r2 = 1.0 - 2.0 * unit_draw(u2);
   double rs = r1 * r1 + r2 * r2;
@@ -128,7 +128,7 @@ __device__ void sphere_vec(uint32_t u1, uint32_t u2, double* v) {
   v[2] = (1.0 - 2.0 * rs);
 }
 
-__device__ void rand_sphere(Draws& d, double* v, const unsigned* accbits) {
+__device__ __forceinline__ void rand_sphere(Draws& d, double* v, const unsigned* accbits) {
   long long o = sphere_scan_bits(d, accbits);
   if (o < 0) {
     v[0] = v[1] = 0.0;
@@ -138,48 +138,35 @@ __device__ void rand_sphere(Draws& d, double* v, const unsigned* accbits) {
   sphere_vec(d.at(o), d.at(o + 1), v);
 }
 
+// Three block sums of values that only the first n threads hold (the others zero):
+// value q ends in thread q, q < 3. Lanes are added pairwise, then the warps in
+// order, by one thread per value: on this chip's FP64 pipe (16 cycles an
+// instruction, 64 until its result) eight warps adding all three for every thread
+// took 5,000 cycles. sh: 3 NT / 32 doubles.
 template <int NT>
-__device__ __forceinline__ double bsum(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int i = 0; i < NT / 32; i++) t += sh[i];
-  __syncthreads();
-  return t;  // valid in every thread
-}
-
-// Three block sums at once (two barriers for all three, plus one before sh
-// is reused); each value is added in bsum's order, so the results are the
-// same bits as three bsum calls. sh: 3 NT / 32 doubles.
-template <int NT>
-__device__ __forceinline__ void bsum3(double& a, double& b, double& c, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-  }
+__device__ __forceinline__ double bsum3(double a, double b, double c, int n, double* sh) {
   constexpr int W = NT / 32;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) {
-    sh[w] = a;
-    sh[W + w] = b;
-    sh[2 * W + w] = c;
+  double v[3] = {a, b, c};
+  if (32 * w < n) {
+    const int left = n - 32 * w;  // lanes with a value, when under a warp
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const bool any = __any_sync(0xffffffffu, __double_as_longlong(v[q]) << 1 != 0);
+      if (any)
+        for (int o = 16; o > 0; o >>= 1)
+          if (o < left) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    }
   }
   __syncthreads();
-  double ta = 0.0, tb = 0.0, tc = 0.0;
-  for (int i = 0; i < W; i++) {
-    ta += sh[i];
-    tb += sh[W + i];
-    tc += sh[2 * W + i];
-  }
+  if (l == 0)
+#pragma unroll
+    for (int q = 0; q < 3; q++) sh[q * W + w] = v[q];
   __syncthreads();
-  a = ta;
-  b = tb;
-  c = tc;
+  double t = 0.0;
+  if (threadIdx.x < 3)
+    for (int i = 0; i < W && 32 * i < n; i++) t += sh[threadIdx.x * W + i];
+  return t;
 }
 
 struct GenPlan {
@@ -210,7 +197,7 @@ __device__ __forceinline__ int next_accept(const unsigned* accbits, int wlen, in
   int w = x >> 5;
   unsigned m = accbits[w] & par & (0xFFFFFFFFu << (x & 31));
   while (!m) {
-    if (++w >= kDrawWindow / 32) return kDrawWindow;
+    if (++w >= (wlen + 31) / 32) return kDrawWindow;
     m = accbits[w] & par;
   }
   return (w << 5) + (__ffs(m) - 1);
@@ -327,12 +314,12 @@ __device__ __forceinline__ void put_trial(const DevParams& P, const DevBuffers& 
   if (B.fpos64) O.u[i - b_lo] = fix64x4(P, t);
 }
 
-// Walls and sum q dz of the moved beads, and the moved molecule's bonds at the
-// trial positions, into C.
+// Walls and sum q dz of the moved beads [b_lo, b_hi), and the bonds of their
+// molecule [m0, m1) at the trial positions, into C.
 template <class Trial>
-__device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& B, bool on, int mol,
-                                          int b_lo, int b_hi, const PosView& V, const Trial& T,
-                                          MoveCand& C, double* red) {
+__device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& B, bool on, int m0,
+                                          int m1, int b_lo, int b_hi, const PosView& V,
+                                          const Trial& T, MoveCand& C, double* red) {
   if (threadIdx.x == 0) C.ext_bad = 0;
   __syncthreads();
   double ext = 0.0, dmz = 0.0, bt = 0.0;
@@ -347,7 +334,6 @@ __device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& 
       }
       dmz += t.w * (t.z - p.z);
     }
-    const int m0 = B.mol_start[mol], m1 = B.mol_start[mol + 1];
     if (P.use_bond && m1 - m0 > 1)
       for (int i = m0 + threadIdx.x; i < m1 - 1; i += blockDim.x) {
         double4_32a p = T(i), q = T(i + 1);
@@ -356,19 +342,34 @@ __device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& 
         bt += 0.5 * P.k_bond * (r - P.r0) * (r - P.r0);
       }
   }
-  bsum3<kSerialThreads>(ext, dmz, bt, red);
-  if (threadIdx.x == 0) {
-    C.ext = ext;
-    C.dmz = dmz;
-    C.bond = bt;
-  }
+  const double v = bsum3<kSerialThreads>(ext, dmz, bt, on ? max(b_hi - b_lo, m1 - m0) : 0, red);
+  if (threadIdx.x == 0) C.ext = v;
+  if (threadIdx.x == 1) C.dmz = v;
+  if (threadIdx.x == 2) C.bond = v;
+  __syncwarp();
 }
 
-// Worked out from the draws' places alone (see gen_picks).
+// Worked out beside the picks by the other warps, from the draws' fixed places: a
+// move's own draws start at the fifth word. *_end: window offset after the draws
+// (0: they ran past the window, and warp 0 makes them one by one).
 struct GenPre {
   double crank_s, crank_c;  // of the angle drawn by the seventh word
   double pivot_s;           // from the sixth
+  double ion[3], com[3], rep[3];
+  int ion_end, rep_end;
 };
+
+// The vector of the first pair randSphere accepts from window offset k on, a lane
+// per pair: offset after the pair, or 0 where none of 32 lies in the window.
+__device__ __forceinline__ int pre_sphere(const uint32_t* win, int wlen, int k, double* v) {
+  const int p = k + 2 * (int)(threadIdx.x & 31);
+  const unsigned ok =
+      __ballot_sync(0xffffffffu, p + 1 < wlen && !sphere_reject(win[p], win[p + 1]));
+  if (!ok) return 0;
+  const int o = k + 2 * (__ffs(ok) - 1);
+  sphere_vec(win[o], win[o + 1], v);
+  return o + 2;
+}
 
 // floor(n x / M) of a draw x, M = 2^32 - 1, 0 <= n < 2^20: the reference's FP64
 // product is exact and its quotient, at least 1 / M away from the next integer
@@ -380,43 +381,65 @@ __device__ __forceinline__ int draw_floor(int n, uint32_t x) {
   return (int)(a + (r >= 0xFFFFFFFFull ? 1 : 0));
 }
 
-// What warp 0 finds before the acceptance bits are there: the picks (two loads
-// deep), and what the other warps work out beside it from the draws' fixed
-// places: the crankshaft's sine and cosine and the pivot's displacement.
+// floor(fl(fl(x / M) n)): the picks' product. Both roundings together move it by
+// less than n 2^-52, under 1 / M for n < 2^20, so unless n x / M is a whole number
+// the floor is the integer quotient's.
+__device__ __forceinline__ int draw_pick(int n, uint32_t x) {
+  const unsigned long long v = (unsigned long long)n * x;
+  const unsigned long long a = v >> 32, r = a + (v & 0xFFFFFFFFull);
+  if (n < 0 || n >= (1 << 20) || r == 0 || r == 0xFFFFFFFFull || r == 0x1FFFFFFFEull)
+    return (int)floor(unit_draw(x) * n);
+  return (int)(a + (r >= 0xFFFFFFFFull ? 1 : 0));
+}
+
+// What warp 0 finds before the acceptance bits are there.
 struct GenPicks {
   int mt, mol, b0, b1;  // mol -1: nothing is moved
+  double bond_old;      // the molecule's bond energy
   bool any;             // molecules to pick from: the picks' draws are taken
 };
 
 __device__ __forceinline__ GenPicks gen_picks(const DevParams& P, const DevBuffers& B, Draws& d) {
-  GenPicks g{0, -1, 0, 0, P.n_mol - P.phantom > 0};
+  GenPicks g{0, -1, 0, 0, 0.0, P.n_mol - P.phantom > 0};
   (void)d.next();  // simulation.cc:221 (the GC draw)
   if (!g.any) return g;
   const int n_ch = P.n_chain_total, n_io = P.n_ion_total;
-  int wc = (int)floor(unit_draw(d.next()) * n_ch);
-  int wi = (int)floor(unit_draw(d.next()) * n_io);
+  int wc = draw_pick(n_ch, d.next());
+  int wi = draw_pick(n_io, d.next());
   if (wc == n_ch) wc--;
   if (wi == n_io) wi--;
-  const int chain_id = (wc >= 0 && wc < n_ch) ? B.chain_ids[wc] : -1;
-  const int ion_id = (wi >= 0 && wi < n_io) ? B.ion_ids[wi] : -1;
-  double u = unit_draw(d.next());
-  double cur = P.move_prob[0];
-  while (cur < u && g.mt < 4) {
-    g.mt++;
-    cur += P.move_prob[g.mt];
-  }
-  if (cur < u) g.mt++;
-  if (g.mt > 4) g.mt = 4;
+  const int4 none = make_int4(-1, 0, 0, 0);
+  const int4 chain = (wc >= 0 && wc < n_ch) ? B.chain_ids[wc] : none;
+  const int4 ion = (wi >= 0 && wi < n_io) ? B.ion_ids[wi] : none;
+  // the reference's running sum of the probabilities (move_cum) against the draw,
+  // as bits: non-negative doubles order as integers
+  const long long u = __double_as_longlong(unit_draw(d.next()));
+  while (g.mt < 4 && P.move_cum[g.mt] < u) g.mt++;
+  int4 m = none;
   if (g.mt == 0 && n_io > 0)
-    g.mol = ion_id;
-  else if (n_ch > 0)
-    g.mol = chain_id;
-  if (!((g.mt == 0 && n_io > 0) || (g.mt > 0 && n_ch > 0))) g.mol = -1;
-  if (g.mol >= 0) {
-    g.b0 = B.mol_start[g.mol];
-    g.b1 = B.mol_start[g.mol + 1];
-  }
+    m = ion;
+  else if (g.mt > 0 && n_ch > 0)
+    m = chain;
+  g.mol = m.x;
+  g.b0 = m.y;
+  g.b1 = m.z;
   return g;
+}
+
+// Component `lane` (0, 1, else 2) of v.
+__device__ __forceinline__ double pick3(const double* v, int lane) {
+  return lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]);
+}
+// That component of the ion's displacement and of the reptation's end bond along
+// randSphere's v.
+__device__ __forceinline__ double ion_part(const DevParams& P, const double* v, int lane) {
+  double vl = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  if (vl > 0) vl = 3 * P.move_size / vl;
+  return vl * pick3(v, lane);
+}
+__device__ __forceinline__ double rep_part(double bl, const double* v, int lane) {
+  const double vl = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  return bl * pick3(v, lane) / vl;
 }
 
 // Generates candidate C from stream position d.pos and positions V. Warp 0
@@ -433,7 +456,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
   // ----------------------------------------------------- generate next move
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
-    const auto part = [&](const double* v) { return lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]); };
+    const auto part = [&](const double* v) { return pick3(v, lane); };
     plan.type = -1;
     plan.scan = 0;
     if (gp.any) {
@@ -449,24 +472,24 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
         plan.type = mt;
         if (mt == 0) {
           // Molecule::BeadTranslate (molecule.cc:103-133)
-          double v[3];
-          rand_sphere(d, v, accbits);
-          double vl = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-          if (vl > 0) vl = 3 * P.move_size / vl;
-          if (lane < 3) plan.vec[lane] = vl * part(v);
+          double x;
+          if (pre.ion_end) {
+            x = part(pre.ion);
+            d.pos = wbase + pre.ion_end;
+          } else {
+            double v[3];
+            rand_sphere(d, v, accbits);
+            x = ion_part(P, v, lane);
+          }
+          if (lane < 3) plan.vec[lane] = x;
           plan.b_hi = b0 + 1;
         } else if (mt == 1) {
           // Molecule::COMTranslate (molecule.cc:135-151). Here, and in the
           // pivot's displacement, the reference multiplies the word before
           // dividing, so these keep the division (unit_draw is the quotient of
           // the word alone).
-          uint32_t w[3], sg[3];
-          for (int a = 0; a < 3; a++) w[a] = d.next();
-          for (int a = 0; a < 3; a++) sg[a] = d.next();
-          const double wl = lane == 0 ? (double)w[0] : (lane == 1 ? (double)w[1] : (double)w[2]);
-          const uint32_t sl = lane == 0 ? sg[0] : (lane == 1 ? sg[1] : sg[2]);
-          const double x = 0.5 * P.move_size * wl / kMtMax;
-          if (lane < 3) plan.vec[lane] = sl % 2u == 0u ? -x : x;
+          for (int a = 0; a < 6; a++) (void)d.next();
+          if (lane < 3) plan.vec[lane] = pre.com[lane];
         } else if (mt == 2) {
           // Molecule::Pivot (molecule.cc:153-237). Bead i's new position is
           // the previous one plus bl_i * unit(old_i - old_prev + s v_i): the
@@ -553,10 +576,15 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
             dir = -1;
             end = 0;
           }
-          double v[3];
-          rand_sphere(d, v, accbits);
-          double vl = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-          const double x = bl * part(v) / vl;
+          double x;
+          if (pre.rep_end) {
+            x = part(pre.rep);
+            d.pos = wbase + pre.rep_end;
+          } else {
+            double v[3];
+            rand_sphere(d, v, accbits);
+            x = rep_part(bl, v, lane);
+          }
           if (lane < 3) plan.vec[lane] = x;
           plan.dir = dir;
           plan.end = end;
@@ -665,7 +693,7 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
     // fixed-point trial coordinates of the sequential pivot
     for (int i = g.b_lo + threadIdx.x; i < g.b_hi; i += blockDim.x)
       put_trial(P, B, O, g.b_lo, i, O.t[i - g.b_lo]);
-  move_sums(P, B, g.type >= 0, g.mol, g.b_lo, g.b_hi, V,
+  move_sums(P, B, g.type >= 0, g.b0, g.b1, g.b_lo, g.b_hi, V,
             [&](int i) { return i >= g.b_lo && i < g.b_hi ? O.t[i - g.b_lo] : V.at(i); }, C, red);
   if (threadIdx.x == 0) {
     C.type = g.type;
@@ -673,6 +701,8 @@ __device__ __forceinline__ void gen_move(const DevParams& P, const DevBuffers& B
       C.mol = g.mol;
       C.b_lo = g.b_lo;
       C.b_hi = g.b_hi;
+      C.bonded = g.b1 - g.b0 > 1;
+      C.bond_old = gp.bond_old;
     }
   }
 }
@@ -700,23 +730,52 @@ __device__ __forceinline__ void gen_body(const DevParams& P, const DevBuffers& B
   if (st->error || (!pending && c != kCandSkip)) return;
   const long long base = st->stream_pos + (c == kCandSkip ? 0 : 1), len = st->stream_len;
   const long long avail = len - base;
-  const int wlen = (int)(avail < kDrawWindow ? (avail > 0 ? avail : 0) : kDrawWindow);
+  // the words a move of the longest molecule takes (see pivot_draws), within the
+  // window; moves that take more make their draws one by one
+  const int most = min(kDrawWindow, (6 * P.max_len + 80 + 63) & ~31);
+  const int wlen = (int)(avail < most ? (avail > 0 ? avail : 0) : most);
   for (int i = threadIdx.x; i < wlen; i += blockDim.x) sm.win[i] = B.stream[base + i];
   __syncthreads();
   Draws d{B.stream, sm.win, base, len, base, wlen, 0};
-  GenPicks gp{0, -1, 0, 0, false};
+  GenPicks gp{0, -1, 0, 0, 0.0, false};
   const int warp = threadIdx.x >> 5;
-  if (warp == 0) gp = gen_picks(P, B, d);
+  if (warp == 0) {
+    gp = gen_picks(P, B, d);
+    if (gp.mol >= 0 && P.use_bond)
+      gp.bond_old =
+          c == kCandAccept && gp.mol == st->mol ? B.plan->now.bond : B.bond_mol[gp.mol];
+  }
   if (warp == 1 && base + 6 < len) {
     const double pi_libm = 3.14159265358979323846;
     const double ang = P.move_size * (unit_draw(d.at(base + 6)) * 2 * pi_libm - pi_libm);
     sincos(ang, &sm.pre.crank_s, &sm.pre.crank_c);
   }
+  const int lane = threadIdx.x & 31;
   if (warp == 2 && base + 5 < len)
     sm.pre.pivot_s = P.move_size * (double)d.at(base + 5) / kMtMax;
+  if (warp == 3) {
+    double v[3] = {0.0, 0.0, 1.0};
+    const int end = pre_sphere(sm.win, wlen, 4, v);
+    const double x = ion_part(P, v, lane);
+    if (lane < 3) sm.pre.ion[lane] = x;
+    if (lane == 0) sm.pre.ion_end = end;
+  }
+  if (warp == 4) {
+    const int k = P.vary_bond ? 5 : 4;  // the direction's word
+    double v[3] = {0.0, 0.0, 1.0}, bl = P.bond_len;
+    if (P.vary_bond && wlen > 4) bl += (P.bond_len / 5.0) * (unit_draw(sm.win[4]) - 0.5);
+    const int end = pre_sphere(sm.win, wlen, k + 1, v);
+    const double x = rep_part(bl, v, lane);
+    if (lane < 3) sm.pre.rep[lane] = x;
+    if (lane == 0) sm.pre.rep_end = end;
+  }
+  if (warp == 5 && lane < 3 && base + 9 < len) {
+    const double x = 0.5 * P.move_size * (double)d.at(base + 4 + lane) / kMtMax;
+    sm.pre.com[lane] = d.at(base + 7 + lane) % 2u == 0u ? -x : x;
+  }
   // every window position's randSphere test, one position per thread; a
   // warp's ballot makes the word of its 32 positions
-  for (int p0 = threadIdx.x & ~31; p0 < kDrawWindow; p0 += blockDim.x) {
+  for (int p0 = threadIdx.x & ~31; p0 < most; p0 += blockDim.x) {
     const int p = p0 + (threadIdx.x & 31);
     const bool ok = p + 1 < wlen && !sphere_reject(sm.win[p], sm.win[p + 1]);
     const unsigned bits = __ballot_sync(0xFFFFFFFFu, ok);
@@ -734,7 +793,7 @@ __device__ __forceinline__ void gen_body(const DevParams& P, const DevBuffers& B
 
 // Shared memory of one serial step.
 struct SerialSmem {
-  double red[3 * (kSerialThreads / 32)];
+  double red[3 + 3 * (kSerialThreads / 32)];  // block sums, then bsum3's
   int s_accept, s_cand;
   StepPlan plan;
   // The state lives in shared memory for the step: thread 0's chain of
@@ -749,24 +808,40 @@ struct SlotSums {
   int pair_off, n_pair, k_off, n_k;
 };
 
-// The FP64 energy change's block sums {LJ, real space, k, unused}, added in order
-// by one warp.
-__device__ __forceinline__ void block_sums(const double* part, int blocks, DevState& S) {
+// The FP64 energy change's block sums {LJ, real space, k, unused} by one warp,
+// lane l taking blocks l, l + 32, ...; a lane's loads are all in flight at once
+// (a loop of load and add took 2.4 us for 149 blocks).
+__device__ __forceinline__ void block_sums(const double* part, int blocks, double* sum) {
+  const int lane = threadIdx.x & 31;
+  const double4_32a* p = reinterpret_cast<const double4_32a*>(part);
   double a = 0.0, b = 0.0, c = 0.0;
-  for (int i = threadIdx.x; i < blocks; i += 32) {
-    a += part[4 * i];
-    b += part[4 * i + 1];
-    c += part[4 * i + 2];
+  for (int i0 = 0; i0 < blocks; i0 += 256) {
+    double4_32a v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = i0 + lane + 32 * u;
+      v[u] = i < blocks ? p[i] : make_double4_32a(0.0, 0.0, 0.0, 0.0);
+    }
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+      for (int u = 0; u < h; u++) {
+        v[u].x += v[u + h].x;
+        v[u].y += v[u + h].y;
+        v[u].z += v[u + h].z;
+      }
+    a += v[0].x;
+    b += v[0].y;
+    c += v[0].z;
   }
   for (int o = 16; o > 0; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
     c += __shfl_xor_sync(0xffffffffu, c, o);
   }
-  if (threadIdx.x == 0) {
-    S.red_lj = a;
-    S.red_re = b;
-    S.red_k = c;
+  if (lane == 0) {
+    sum[0] = a;
+    sum[1] = b;
+    sum[2] = c;
   }
 }
 
@@ -776,6 +851,9 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
   double* const red = sm.red;
   int& s_accept = sm.s_accept;
   DevState& S = sm.S;
+  // (beside the state's load; with no pending move nobody reads them)
+  if (part_blocks && (mode & kModeFinish) && (threadIdx.x >> 5) == 7)
+    block_sums(B.partial, part_blocks, red);
   {
     const int nw = (int)(sizeof(DevState) / sizeof(int));
     const int* src = reinterpret_cast<const int*>(B.state);
@@ -796,17 +874,18 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
     }
     for (int i = threadIdx.x; i < slots->n_k; i += blockDim.x)
       c += slots->slots[2 * (slots->k_off + i)];
-    bsum3<kSerialThreads>(a, b, c, red);
-    if (threadIdx.x == 0) {
-      S.red_lj = a;
-      S.red_re = b;
-      S.red_k = c;
-    }
+    const double v = bsum3<kSerialThreads>(a, b, c, max(slots->n_pair, slots->n_k), red + 3);
+    if (threadIdx.x == 0) S.red_lj = v;
+    if (threadIdx.x == 1) S.red_re = v;
+    if (threadIdx.x == 2) S.red_k = v;
     __syncthreads();
   }
 
-  if (part_blocks && (mode & kModeFinish) && S.pending && threadIdx.x < 32)
-    block_sums(B.partial, part_blocks, S);
+  if (part_blocks && (mode & kModeFinish) && threadIdx.x == 0) {
+    S.red_lj = red[0];
+    S.red_re = red[1];
+    S.red_k = red[2];
+  }
 
   // the acceptance test's draw, loaded while dE is composed
   uint32_t word = 0;
@@ -818,34 +897,26 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
   const int b_lo = S.b_lo, b_hi = S.b_hi, mol = S.mol;
 
   if ((mode & kModeFinish) && pending && S.da_skip) {
-    // Stage one rejected the move: no exact change was computed, and no
-    // delta kernel applied the S(k) change of the last accepted move.
-    if (P.use_ewald && S.sk_pending) {
-      const double2* add = B.dsk + (size_t)S.sk_buf * P.n_k;
-      for (int k = threadIdx.x; k < P.n_k; k += blockDim.x) {
-        const double2 a = add[k];
-        double2 v = B.sk[k];
-        v.x += a.x;
-        v.y += a.y;
-        B.sk[k] = v;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      S.sk_pending = 0;
-      S.de = 0.0;
-    }
+    // Stage one rejected the move: no exact change was computed. The S(k) change
+    // of the last accepted move, if still pending, stays so until the next energy
+    // change applies it (7,812 vectors added by this one block took 10 us).
+    if (threadIdx.x == 0) S.de = 0.0;
     __syncthreads();
   } else if ((mode & kModeFinish) && pending) {
     // a move set by the host has no candidate's sums
     MoveCand& now = sm.plan.now;
-    if (S.move_type < 0)
-      move_sums(P, B, true, mol, b_lo, b_hi, PosView{B.pos, B.trial, 0, 0},
-                [&](int i) { return B.trial[i]; }, now, red);
-    const double ext = now.ext, dmz = now.dmz, bt = now.bond;
-    const int ext_bad = now.ext_bad;
-    const int m0 = B.mol_start[mol], m1 = B.mol_start[mol + 1];
+    if (S.move_type < 0) {
+      const int m0 = B.mol_start[mol], m1 = B.mol_start[mol + 1];
+      move_sums(P, B, true, m0, m1, b_lo, b_hi, PosView{B.pos, B.trial, 0, 0},
+                [&](int i) { return B.trial[i]; }, now, red + 3);
+      if (threadIdx.x == 0) {
+        now.bonded = m1 - m0 > 1;
+        now.bond_old = B.bond_mol[mol];
+      }
+    }
     if (threadIdx.x == 0) {
+      const double ext = now.ext, dmz = now.dmz, bt = now.bond;
+      const int ext_bad = now.ext_bad;
       // the delta kernel applied any pending S(k) commit if it ran k tiles
       if (P.use_ewald && b_hi > b_lo) S.sk_pending = 0;
       const double de_lj = S.red_lj, de_re = S.red_re, de_k = b_hi > b_lo ? S.red_k : 0.0;
@@ -870,8 +941,8 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
         }
         de += dw;
       }
-      if (!done && P.use_bond && m1 - m0 > 1) {
-        db = bt - B.bond_mol[mol];
+      if (!done && P.use_bond && now.bonded) {
+        db = bt - now.bond_old;
         de += db;
       }
       if (!isfinite(de)) S.n_nonfinite++;  // flagged, rejected as the reference does
