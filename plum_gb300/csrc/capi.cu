@@ -678,8 +678,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   rc |= dalloc(&B.ku, ku.size());
   rc |= dalloc(&B.sk, kn.size());
   rc |= dalloc(&B.dsk, 2 * kn.size());
-  rc |= dalloc(&B.done_count, 1);
-  rc |= dalloc(&B.partial, 4 * (size_t)std::max(pair_grid(), pair_grid32()));
+  rc |= dalloc(&B.partial, 4 * (size_t)delta_blocks());
   rc |= dalloc(&B.fpos, nb);
   rc |= dalloc(&B.fq, nb);
   rc |= dalloc(&B.ftrial, c->most_len);
@@ -687,12 +686,6 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   rc |= dalloc(&B.plan, 1);
   rc |= dalloc(&B.ctrial, kCands * (size_t)c->max_len);
   rc |= dalloc(&B.cftrial, kCands * (size_t)c->max_len);
-  {
-    int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
-    rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
-    rc |= dalloc(&B.ktile_count, ktile_count(P));
-    rc |= dalloc(&B.kpartial, ktile_count(P));
-  }
   rc |= dalloc(&B.bond_mol, in.n_mol);
   rc |= dalloc(&B.state, 1);
   rc |= dalloc(&c->d_sk_part, (size_t)sk_full_groups(P) * std::max(1, P.n_k));
@@ -779,8 +772,6 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     cudaMemcpy(B.ku, ku.data(), sizeof(KUnit) * ku.size(), cudaMemcpyHostToDevice);
   }
   cudaMemset(B.state, 0, sizeof(DevState));
-  cudaMemset(B.ktile_count, 0, sizeof(int) * std::max(1, ktile_count(P)));
-  cudaMemset(B.done_count, 0, sizeof(int));
   cudaMemset(B.plan, 0, sizeof(StepPlan));
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
@@ -804,8 +795,7 @@ int plum_ctx_destroy(plum_ctx* c) {
   void* ptrs[] = {c->B.pos,      c->B.trial,   c->B.type,  c->B.mol_start, c->B.chain_ids,
                   c->B.ion_ids,  c->B.kn,      c->B.kw,    c->B.sk,        c->B.dsk,
                   c->B.partial,  c->B.bond_mol, c->B.state, c->d_tot_part,  c->d_out,
-                  c->B.ktile_count, c->B.kpartial, c->B.fpos, c->B.done_count,
-                  c->B.fq,       c->B.ftrial,  c->B.dsk_part32, c->cb_in, c->cb_slots, c->cb_so,
+                  c->B.fpos,     c->B.fq,      c->B.ftrial, c->cb_in,  c->cb_slots, c->cb_so,
                   c->cb_part,    c->d_obs_per, c->d_rhoz, c->desc_acc,
                   c->d_rp1,      c->d_rb1,     c->desc_fine, c->cb_part32, c->cb_ticket,
                   c->d_stream,   c->d_mt,      c->d_log_type, c->d_log_acc, c->d_log_e,
@@ -952,7 +942,7 @@ int rebuild_system(plum_ctx* c) {
   P.n_ion_total = (int)ions.size();
   const bool mirror64 = B.fpos64 != nullptr;
   void* old[] = {B.pos,      B.trial,      B.type,     B.mol_start, B.chain_ids, B.ion_ids,
-                 B.fpos,     B.fq,         B.ftrial,   B.dsk_part32, B.bond_mol, B.ctrial, B.cftrial,
+                 B.fpos,     B.fq,         B.ftrial,   B.bond_mol, B.ctrial, B.cftrial,
                  c->d_tot_part, c->d_obs_per, B.fpos64, B.ftrial64, B.ctrial64};
   for (void* q : old)
     if (q) cudaFree(q);
@@ -964,7 +954,6 @@ int rebuild_system(plum_ctx* c) {
   B.ctrial = nullptr;
   P.max_len = c->max_len;
   B.fq = nullptr;
-  B.dsk_part32 = nullptr;
   B.bond_mol = nullptr;
   c->d_tot_part = c->d_obs_per = nullptr;
   int rc = dalloc(&B.pos, nb) | dalloc(&B.trial, nb) | dalloc(&B.type, nb) |
@@ -976,8 +965,6 @@ int rebuild_system(plum_ctx* c) {
   if (mirror64)
     rc |= dalloc(&B.fpos64, nb) | dalloc(&B.ftrial64, c->most_len) |
           dalloc(&B.ctrial64, kCands * (size_t)c->max_len);
-  const int groups = (c->max_len + std::max(1, P.kchunk_delta) - 1) / std::max(1, P.kchunk_delta);
-  rc |= dalloc(&B.dsk_part32, (size_t)groups * std::max(1, P.n_k));
   c->n_tot_part = total_partials_count(P);
   rc |= dalloc(&c->d_tot_part, 2 * (size_t)c->n_tot_part);
   rc |= dalloc(&c->d_obs_per, 5 * (size_t)std::max(1, in.n_mol));

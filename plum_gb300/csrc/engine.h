@@ -13,8 +13,6 @@
 //                           an accepted change is added to sk by the next
 //                           delta kernel)
 //   partial double[grid*4]  per-block partial sums of the pending move
-//   dsk_part32 float2[groups*n_k], kpartial double[k tiles]: the precision
-//                           form's k-space parts
 //   state  DevState         running energies, the pending move, stream cursor
 // Everything here is a few MB even at 20,000 beads and 15,624 k-vectors, so
 // it stays L2-resident across moves; the pair sweeps are FP64/FP32-pipe
@@ -216,10 +214,6 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   StepPlan* plan;
   double4_32a* ctrial;  // [kCands][max_len] trial positions of the candidates
   int4* cftrial;     // [kCands][max_len] their fixed-point mirror (precision form)
-  float2* dsk_part32;  // [groups][n_k]
-  int* ktile_count;  // [k tiles] arrival tickets (reset by the last arrival)
-  int* done_count;   // [1] block arrival ticket of the delta kernel
-  double* kpartial;  // [k tiles] energy change per k tile
   double* bond_mol;  // [n_mol]
   DevState* state;
   const uint32_t* stream;
@@ -267,8 +261,7 @@ void launch_slit_pressure(const SlitPressParams& S, const DevParams& P, const De
 
 // Launch helpers (kern_energy.cu / kern_moves.cu). All enqueue on `s`.
 int pair_grid();
-int delta_blocks64();  // blocks of the FP64 energy change, four partial sums each
-int ktile_count(const DevParams& P);
+int delta_blocks();  // blocks of the energy change, four partial sums each
 void launch_delta_pairs64(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 void launch_total64(const DevParams& P, const DevBuffers& B, double* out_partials,
                     int n_part, cudaStream_t s);

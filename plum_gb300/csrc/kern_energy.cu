@@ -418,7 +418,7 @@ int pair_grid() {
 // One block per SM (a block takes nearly all of an SM's registers), but for the
 // SMs that the next move's candidates run on meanwhile: with a block on every SM
 // those waited for the energy change, or it for them.
-int delta_blocks64() { return std::max(1, pair_grid() / 2 - kCands); }
+int delta_blocks() { return std::max(1, pair_grid() / 2 - kCands); }
 
 template <int kMode>
 static void launch_delta64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
@@ -433,7 +433,7 @@ static void launch_delta64(const DevParams& P, const DevBuffers& B, cudaStream_t
   const size_t tab = kMode ? kFixStage * sizeof(FixStage) + (size_t)P.fx.n_bin * 40 : 0;
   const size_t k = P.use_ewald && P.n_ku > 0
                        ? (size_t)k_beads(P) * 2 * (P.kmax[2] + 1 + kUnits) * sizeof(double2) : 0;
-  k_delta64<kMode><<<delta_blocks64(), kDeltaThreads, tab + k, s>>>(P, B, (int)tab);
+  k_delta64<kMode><<<delta_blocks(), kDeltaThreads, tab + k, s>>>(P, B, (int)tab);
 }
 
 void launch_delta_pairs64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {

@@ -14,8 +14,6 @@
 // In the slab geometry z is not wrapped (|dz| < H < L_z,Ewald / 2), so the same
 // subtraction gives the raw dz the reference uses (GetDistVector, npbc = 2).
 //
-// Work decomposition is the FP64 kernel's: every (moved, other) pair dealt
-// across the grid, k tiles x moved-bead groups with a last-arrival reduction.
 // Per-thread and per-block sums are FP32; blocks are added in FP64 by the
 // serial kernel.
 #include <algorithm>
@@ -23,13 +21,10 @@
 
 #include "engine.h"
 #include "device_common.cuh"
+#include "fix_device.cuh"
 #include "fp32_pair.cuh"
 
 namespace plum {
-
-constexpr int kKTile32 = 128;
-
-int ktile_count(const DevParams& P) { return (P.n_k + kKTile32 - 1) / kKTile32; }
 
 template <int NT>
 __device__ __forceinline__ float block_sum32(float v, float* sh) {
@@ -69,18 +64,6 @@ __device__ __forceinline__ float2 block_sum32x2(float a, float b, float* sh) {
   return t;
 }
 
-__device__ __forceinline__ double block_sum_d(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)blockDim.x / 32; i++) t += sh[i];
-  return t;
-}
-
 // Exact per-entry table: e^{i 2 pi n X / 2^32}, n = 0..kmax, q folded into x.
 __device__ __forceinline__ void table32(const DevParams& P, int4 f, float q, int axis,
                                         float2* tab) {
@@ -99,108 +82,190 @@ __device__ __forceinline__ float2 cmul32(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-__device__ __forceinline__ float2 phase32(const DevParams& P, const float2* tab, short4 k) {
-  float2 ex = tab[P.koff[0] + k.x];
-  float2 ey = tab[P.koff[1] + (k.y >= 0 ? k.y : -k.y)];
-  if (k.y < 0) ey.y = -ey.y;
-  float2 ez = tab[P.koff[2] + (k.z >= 0 ? k.z : -k.z)];
-  if (k.z < 0) ez.y = -ez.y;
-  return cmul32(cmul32(ex, ey), ez);
+// ---------------------------------------------------------------- one system
+// As the FP64 form's k_delta64: one block per SM but for the SMs that the next
+// move's candidates run on, k warps that own a run of k units and pair warps that
+// deal out the (moved, other) pairs; each block leaves three sums to the serial
+// step. What bounds it for a short move is latency, so a thread takes one other bead
+// against a run of staged moved beads and the h(u) table is copied to shared memory
+// (10 KB); for a long one the FP32 pipe (some 25 instructions per evaluation).
+// With 20,000 beads and 7,812 k-vectors: 13.4 us, and 21.5 us a move (32.6 and 34.3 us
+// with every pair's four loads, k tiles x bead groups and a ticket for the last block).
+// Hard spheres, image cells and a cut-off beyond the table take the general pair
+// loop below.
+constexpr int kD32Threads = 768;
+constexpr int kD32K = 256;      // k role
+constexpr int kD32Stage = 256;  // moved beads staged at a time
+constexpr int kD32Run = 4;      // most moved beads per thread and other bead
+constexpr int kD32Units = 32;   // k units of a block at a time
+
+struct Stage32 {
+  int4 t, c;  // trial (w: charge as float bits), current (w: row of the LJ table)
+};
+
+__host__ __device__ inline int k_beads32(const DevParams& P) {
+  const int fit = kKTableBytes / (2 * (P.kmax[2] + 1 + kD32Units) * (int)sizeof(float2));
+  return fit < 1 ? 1 : (fit > 64 ? 64 : fit);
 }
 
-__global__ void __launch_bounds__(kPairThreads)
-    k_delta32(const DevParams P, const DevBuffers B) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ float red[kPairThreads / 32];
-  __shared__ double redd[kPairThreads / 32];
-  __shared__ int s_last;
-  const DevState* st = B.state;
-  const int b_lo = st->b_lo, b_hi = st->b_hi;
-  const int m = st->pending ? b_hi - b_lo : 0;
-  const int sk_pend = st->sk_pending, sk_buf = st->sk_buf, cur_buf = st->cur_buf;
-  __shared__ int s_final;
-  const int N = P.n_bead;
+__device__ __forceinline__ float2 turn32(unsigned phi) {
+  float s, c;
+  sincospif((float)(int)phi * 4.6566128730773926e-10f, &s, &c);  // * 2^-31
+  return make_float2(c, s);
+}
 
-  float acc_lj = 0.0f, acc_re = 0.0f;
-  if (P.use_pair || P.use_ewald) {
-    // pair p = ii * N + j, dealt with stride G; (ii, j) advanced without a
-    // division per pair
-    const long long total = (long long)m * N;
-    const long long G = (long long)gridDim.x * blockDim.x;
-    const long long p0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int gq = (int)(G / N), gr = (int)(G % N);
-    int ii = (int)(p0 / N), j = (int)(p0 % N);
-    for (long long p = p0; p < total; p += G, ii += gq, j += gr) {
+// The pairs of pair thread t0 of nt: one image, LJ + Ewald, the h(u) table.
+__device__ __forceinline__ void sweep32(const DevParams& P, const DevBuffers& B, Stage32* st,
+                                        float4* s_h, int t0, int nt, int b_lo, int m,
+                                        float& acc_lj, float& acc_re) {
+  const int N = P.n_bead, n_type = P.n_type;
+  const int G = (int)gridDim.x * nt, p0 = (int)blockIdx.x * nt + t0;
+  const long long pairs = (long long)m * N;
+  const int run_len = pairs >= 2LL * kD32Run * G ? kD32Run : (pairs >= 4LL * G ? 2 : 1);
+  const float rc2 = P.f_real_cut * P.f_real_cut;
+  const float ua = P.f_sqrt_alpha * P.f_sqrt_alpha, pref = P.f_lB * P.f_sqrt_alpha;
+  float ljm = P.use_pair ? 1e-30f : 0.0f;  // r2 = 0 (coincident beads) must reach lj32
+  if (P.use_pair)
+    for (int k = 0; k < n_type * n_type; k++) ljm = fmaxf(ljm, P.f_lj_rc2[k]);
+  const float2 sx = make_float2(P.f_scale[0], P.f_scale[0]);
+  const float2 sy = make_float2(P.f_scale[1], P.f_scale[1]);
+  const float2 sz = make_float2(P.f_scale[2], P.f_scale[2]);
+  const float2 ua2 = make_float2(ua, ua);
+  for (int i = t0; i < kH32Bins; i += nt) s_h[i] = P.htab[i];
+  for (int g0 = 0; g0 < m; g0 += kD32Stage) {
+    const int gn = min(kD32Stage, m - g0);
+    if (g0) role_sync(2, nt);  // the previous group is consumed
+    for (int t = t0; t < gn; t += nt) {
+      const int i = b_lo + g0 + t;
+      int4 a = B.ftrial[g0 + t], c = B.fpos[i];
+      a.w = __float_as_int(B.fq[i]);
+      c.w *= n_type;
+      st[t] = Stage32{a, c};
+    }
+    role_sync(2, nt);
+    const int runs = (gn + run_len - 1) / run_len;
+    // job run * N + j, dealt with stride G; (run, j) advanced without a division
+    const int gq = G / N, gr = G % N;
+    for (int run = p0 / N, j = p0 % N; run < runs; run += gq, j += gr) {
       if (j >= N) {
         j -= N;
-        ii++;
+        if (++run >= runs) break;
       }
-      const int i = b_lo + ii;
-      const bool jm = j >= b_lo && j < b_hi;
-      if (jm && j <= i) continue;
-      const int4 ti = B.ftrial[ii], ci = B.fpos[i];
-      const float qi = B.fq[i], qj = B.fq[j];
-      const int4 cj = B.fpos[j];
-      const int4 tj = jm ? B.ftrial[j - b_lo] : cj;
-      float l1 = 0, r1 = 0, l0 = 0, r0 = 0;
-      pair32(P, ti, qi, tj, qj, l1, r1);
-      pair32(P, ci, qi, cj, qj, l0, r0);
-      if (!hs_bonded(P, B.mol_start, i, j)) acc_lj += l1 - l0;
-      acc_re += r1 - r0;
-    }
-  }
-  float t0 = block_sum32<kPairThreads>(acc_lj, red);
-  float t1 = block_sum32<kPairThreads>(acc_re, red);
-  if (threadIdx.x == 0) {
-    B.partial[4 * blockIdx.x + 0] = (double)t0;
-    B.partial[4 * blockIdx.x + 1] = (double)t1;
-  }
-
-  const bool kwork = P.use_ewald && m > 0;
-  const int chunk = P.kchunk_delta;
-  const int n_groups = kwork ? (m + chunk - 1) / chunk : 0;
-  const int n_tiles = (P.n_k + kKTile32 - 1) / kKTile32;
-  const int n_items = n_tiles * n_groups;
-  float2* tabs = reinterpret_cast<float2*>(smem);  // [chunk][2][kper]
-  const int per = P.kper;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int tile = item % n_tiles, grp = item / n_tiles;
-    const int c0 = b_lo + grp * chunk;
-    const int cnt = min(chunk, b_hi - c0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < cnt * 6; t += blockDim.x) {
-      int bead = t / 6, which = (t / 3) & 1, axis = t % 3;
-      int4 f = which ? B.fpos[c0 + bead] : B.ftrial[c0 - b_lo + bead];
-      table32(P, f, B.fq[c0 + bead], axis, tabs + (bead * 2 + which) * per);
-    }
-    __syncthreads();
-    const int k = tile * kKTile32 + threadIdx.x;
-    const bool mine = threadIdx.x < kKTile32 && k < P.n_k;
-    if (mine) {
-      const short4 kv = B.kn[k];
-      float2 ds = make_float2(0.0f, 0.0f);
-      for (int b = 0; b < cnt; b++) {
-        float2 e1 = phase32(P, tabs + (b * 2 + 0) * per, kv);
-        float2 e0 = phase32(P, tabs + (b * 2 + 1) * per, kv);
-        ds.x += e1.x - e0.x;
-        ds.y += e1.y - e0.y;
-      }
-      B.dsk_part32[(size_t)grp * P.n_k + k] = ds;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&B.ktile_count[tile], 1) == n_groups - 1;
-    __syncthreads();
-    if (s_last) {
-      __threadfence();
-      float e = 0.0f;
-      if (mine) {
-        float2 ds = make_float2(0.0f, 0.0f);
-        for (int g = 0; g < n_groups; g++) {
-          float2 v = __ldcg(&B.dsk_part32[(size_t)g * P.n_k + k]);
-          ds.x += v.x;
-          ds.y += v.y;
+      // a moved other bead: its trial position, and only moved beads before it
+      const int4 o0 = B.fpos[j];
+      const float qj = B.fq[j] * pref;
+      const int l = j - b_lo - g0;
+      const bool jm = j >= b_lo && j < b_lo + m;
+      const int4 o1 = jm ? B.ftrial[j - b_lo] : o0;
+      const int u0 = run * run_len, u1 = min(gn, jm ? min(l, u0 + run_len) : u0 + run_len);
+      float acc = 0.0f;
+      for (int u = u0; u < u1; u++) {
+        const int4 t = st[u].t, c = st[u].c;
+        const float2 dx = __fmul2_rn(make_float2((float)(int)((unsigned)o1.x - (unsigned)t.x),
+                                                 (float)(int)((unsigned)o0.x - (unsigned)c.x)), sx);
+        const float2 dy = __fmul2_rn(make_float2((float)(int)((unsigned)o1.y - (unsigned)t.y),
+                                                 (float)(int)((unsigned)o0.y - (unsigned)c.y)), sy);
+        const float2 dz = __fmul2_rn(make_float2((float)(int)((unsigned)o1.z - (unsigned)t.z),
+                                                 (float)(int)((unsigned)o0.z - (unsigned)c.z)), sz);
+        const float2 r = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        if (fminf(r.x, r.y) < ljm) {
+          const int k = c.w + o0.w;
+          acc_lj += lj32(P, k, r.x) - lj32(P, k, r.y);
         }
+        const float2 v = __fmul2_rn(r, ua2);
+        const int b1 = __float_as_int(v.x), b0 = __float_as_int(v.y);
+        float h1 = h32_tab(s_h, b1), h0 = h32_tab(s_h, b0);
+        if (min(b1, b0) < kH32LoBits) {
+          if (b1 < kH32LoBits) h1 = h32_small(v.x);
+          if (b0 < kH32LoBits) h0 = h32_small(v.y);
+        }
+        h1 = r.x <= rc2 ? h1 : 0.0f;
+        h0 = r.y <= rc2 ? h0 : 0.0f;
+        acc = fmaf(__int_as_float(t.w), h1 - h0, acc);
+      }
+      acc_re = fmaf(qj, acc, acc_re);
+    }
+  }
+}
+
+// dS(k), the S(k) commit and the |S|^2 change of units [u0, u1). smem, kb =
+// k_beads32: [kb][2][zn] e^{i nz theta_z}, then [kb][2][kD32Units] xy parts, every
+// entry from its exact integer phase.
+__device__ __forceinline__ float k_role32(const DevParams& P, const DevBuffers& B,
+                                          unsigned char* smem, int u0, int u1, int b_lo, int b_hi,
+                                          int sk_pend, int sk_buf, int cur_buf) {
+  const int zn = P.kmax[2] + 1, kb = k_beads32(P);
+  float2* s_z = reinterpret_cast<float2*>(smem);
+  float2* s_xy = s_z + (size_t)kb * 2 * zn;
+  __shared__ short2 s_col[kD32Units];
+  __shared__ float s_sum[4][kD32K];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float e = 0.0f;
+  for (int c0 = u0; c0 < u1; c0 += kD32Units) {
+    const int un = min(kD32Units, u1 - c0);
+    // the units' (nx, ny) columns, numbered in order (the same in every warp)
+    const KUnit lu = lane < un ? B.ku[c0 + lane] : KUnit{0, 0, 0, 0, -1, -1};
+    const int px = __shfl_up_sync(0xffffffffu, lu.nx, 1), py = __shfl_up_sync(0xffffffffu, lu.ny, 1);
+    const bool head = lane < un && (lane == 0 || px != lu.nx || py != lu.ny);
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const int ncol = __popc(heads);
+    int zmax = lane < un ? lu.nz : 0;
+    for (int o = 16; o > 0; o >>= 1) zmax = max(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
+    const int slices = kD32K / un;
+    const int u = (int)threadIdx.x % un, sl = (int)threadIdx.x / un;
+    const int col = __popc(heads & (0xffffffffu >> (31 - u))) - 1;
+    const int nz = __shfl_sync(0xffffffffu, (int)lu.nz, u);
+    if (warp == 0 && head)
+      s_col[__popc(heads & (0xffffffffu >> (31 - lane))) - 1] = make_short2(lu.nx, lu.ny);
+    float2 A = make_float2(0.0f, 0.0f), Bs = A;
+    for (int g0 = b_lo; g0 < b_hi; g0 += kb) {
+      const int nt = 2 * min(kb, b_hi - g0);
+      role_sync(1, kD32K);  // the tables (and s_sum) are free, s_col is written
+      // one entry per thread: nt x (zmax + 1) z phases, then nt x ncol xy phases
+      for (int t = threadIdx.x; t < nt * (zmax + 1 + ncol); t += kD32K) {
+        const int c = t / nt, it = t - c * nt;
+        const int bead = g0 + (it >> 1);
+        const int4 f = (it & 1) ? B.fpos[bead] : B.ftrial[bead - b_lo];
+        if (c <= zmax) {
+          s_z[(size_t)it * zn + c] = turn32((unsigned)f.z * (unsigned)c);
+        } else {
+          const short2 kc = s_col[c - zmax - 1];
+          const float2 v = turn32((unsigned)f.x * (unsigned)(int)kc.x +
+                                  (unsigned)f.y * (unsigned)(int)kc.y);
+          const float q = (it & 1) ? -B.fq[bead] : B.fq[bead];  // trial minus current
+          s_xy[it * kD32Units + c - zmax - 1] = make_float2(q * v.x, q * v.y);
+        }
+      }
+      role_sync(1, kD32K);
+      if (sl < slices)
+        for (int it = sl; it < nt; it += slices) {
+          const float2 xy = s_xy[it * kD32Units + col], ez = s_z[(size_t)it * zn + nz];
+          A.x = fmaf(xy.x, ez.x, A.x);
+          A.y = fmaf(xy.y, ez.x, A.y);
+          Bs.x = fmaf(xy.x, ez.y, Bs.x);
+          Bs.y = fmaf(xy.y, ez.y, Bs.y);
+        }
+    }
+    s_sum[0][threadIdx.x] = A.x;
+    s_sum[1][threadIdx.x] = A.y;
+    s_sum[2][threadIdx.x] = Bs.x;
+    s_sum[3][threadIdx.x] = Bs.y;
+    role_sync(1, kD32K);
+    // the slices of each (unit, sum), added in order by a thread each
+    if ((int)threadIdx.x < 4 * un) {
+      const int q = (int)threadIdx.x / un, v = (int)threadIdx.x % un;
+      float t = 0.0f;
+      for (int w = 0; w < slices; w++) t += s_sum[q][w * un + v];
+      s_sum[q][v] = t;  // slice 0's place: read by this thread only
+    }
+    role_sync(1, kD32K);
+    if (warp < 2 && lane < un) {  // warp 0: +nz, warp 1: -nz
+      const int k = warp == 0 ? lu.kp : lu.km;
+      if (k >= 0) {
+        const float2 SA = make_float2(s_sum[0][lane], s_sum[1][lane]);
+        const float2 SB = make_float2(s_sum[2][lane], s_sum[3][lane]);
+        const float2 ds = warp == 0 ? make_float2(SA.x - SB.y, SA.y + SB.x)
+                                    : make_float2(SA.x + SB.y, SA.y - SB.x);
         double2 s = B.sk[k];
         if (sk_pend) {
           const double2 p = B.dsk[(size_t)sk_buf * P.n_k + k];
@@ -208,41 +273,83 @@ __global__ void __launch_bounds__(kPairThreads)
           B.sk[k] = s;
         }
         B.dsk[(size_t)cur_buf * P.n_k + k] = make_double2((double)ds.x, (double)ds.y);
-        float sx = (float)s.x, sy = (float)s.y;
-        e = (float)B.kw[k] * (2.0f * (sx * ds.x + sy * ds.y) + (ds.x * ds.x + ds.y * ds.y));
-      }
-      e = block_sum32<kPairThreads>(e, red);
-      if (threadIdx.x == 0) {
-        B.kpartial[tile] = (double)e;
-        B.ktile_count[tile] = 0;
+        const float sx = (float)s.x, sy = (float)s.y;
+        e += (float)B.kw[k] * (2.0f * (sx * ds.x + sy * ds.y) + (ds.x * ds.x + ds.y * ds.y));
       }
     }
   }
-  // Last block to finish adds every block's and every k tile's sums in a
-  // fixed order (deterministic) for the serial kernel.
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_final = atomicAdd(B.done_count, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (s_final) {
-    __threadfence();
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-      a += __ldcg(&B.partial[4 * i]);
-      b += __ldcg(&B.partial[4 * i + 1]);
+  return e;
+}
+
+template <bool kTab>
+__global__ void __launch_bounds__(kD32Threads, 1)
+    k_delta32(const DevParams P, const DevBuffers B, int tab_bytes) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ float s_part[kD32Threads / 32][2];
+  const DevState* st = B.state;
+  const int b_lo = st->b_lo, b_hi = st->b_hi;
+  const int m = st->pending ? b_hi - b_lo : 0;
+  const int kthreads = P.use_ewald && P.n_ku > 0 ? kD32K : 0;
+  const int warp = threadIdx.x >> 5;
+  float a = 0.0f, b = 0.0f;  // k role: k energy; pair role: LJ and real space
+  if ((int)threadIdx.x < kthreads) {
+    const int u0 = (int)((long long)P.n_ku * blockIdx.x / gridDim.x);
+    const int u1 = (int)((long long)P.n_ku * (blockIdx.x + 1) / gridDim.x);
+    if (m > 0)
+      a = k_role32(P, B, smem + tab_bytes, u0, u1, b_lo, b_hi, st->sk_pending, st->sk_buf,
+                   st->cur_buf);
+  } else {
+    const int t0 = (int)threadIdx.x - kthreads, nt = kD32Threads - kthreads;
+    const int N = P.n_bead;
+    if (kTab) {
+      if (m > 0)
+        sweep32(P, B, reinterpret_cast<Stage32*>(smem),
+                reinterpret_cast<float4*>(smem + kD32Stage * sizeof(Stage32)), t0, nt, b_lo, m, a,
+                b);
+    } else if (P.use_pair || P.use_ewald) {
+      // pair p = ii * N + j, dealt with stride G; (ii, j) advanced without a
+      // division per pair
+      const long long total = (long long)m * N;
+      const long long G = (long long)gridDim.x * nt;
+      const long long p0 = (long long)blockIdx.x * nt + t0;
+      const int gq = (int)(G / N), gr = (int)(G % N);
+      int ii = (int)(p0 / N), j = (int)(p0 % N);
+      for (long long p = p0; p < total; p += G, ii += gq, j += gr) {
+        if (j >= N) {
+          j -= N;
+          ii++;
+        }
+        const int i = b_lo + ii;
+        const bool jm = j >= b_lo && j < b_hi;
+        if (jm && j <= i) continue;
+        const int4 ti = B.ftrial[ii], ci = B.fpos[i];
+        const float qi = B.fq[i], qj = B.fq[j];
+        const int4 cj = B.fpos[j];
+        const int4 tj = jm ? B.ftrial[j - b_lo] : cj;
+        float l1 = 0, r1 = 0, l0 = 0, r0 = 0;
+        pair32(P, ti, qi, tj, qj, l1, r1);
+        pair32(P, ci, qi, cj, qj, l0, r0);
+        if (!hs_bonded(P, B.mol_start, i, j)) a += l1 - l0;
+        b += r1 - r0;
+      }
     }
-    if (kwork)
-      for (int i = threadIdx.x; i < n_tiles; i += blockDim.x) c += __ldcg(&B.kpartial[i]);
-    a = block_sum_d(a, redd);
-    b = block_sum_d(b, redd);
-    c = block_sum_d(c, redd);
-    if (threadIdx.x == 0) {
-      DevState* ws = B.state;
-      ws->red_lj = a;
-      ws->red_re = b;
-      ws->red_k = c;
-      *B.done_count = 0;
-    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_part[warp][0] = a;
+    s_part[warp][1] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    // sums 0 LJ, 1 real space over the pair warps, 2 over the k warps
+    const int kw = kthreads / 32, w0 = threadIdx.x == 2 ? 0 : kw;
+    const int w1 = threadIdx.x == 2 ? kw : kD32Threads / 32;
+    float t = 0.0f;
+    for (int w = w0; w < w1; w++) t += s_part[w][threadIdx.x == 1];
+    B.partial[4 * blockIdx.x + threadIdx.x] = (double)t;
   }
 }
 
@@ -257,15 +364,26 @@ int pair_grid32() {
   return g_grid32;
 }
 
-void launch_delta_pairs32(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
+template <bool kTab>
+static void launch_delta32(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
+  const size_t tab = kTab ? kD32Stage * sizeof(Stage32) + kH32Bins * sizeof(float4) : 0;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_delta32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kKTableBytes + 4096);
+    cudaFuncSetAttribute(k_delta32<kTab>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kKTableBytes + 4096 + (int)tab);
     attr = true;
   }
-  size_t smem = P.use_ewald ? (size_t)P.kchunk_delta * 2 * P.kper * sizeof(float2) : 0;
-  k_delta32<<<pair_grid32(), kPairThreads, smem, s>>>(P, B);
+  const size_t k = P.use_ewald && P.n_ku > 0
+                       ? (size_t)k_beads32(P) * 2 * (P.kmax[2] + 1 + kD32Units) * sizeof(float2)
+                       : 0;
+  k_delta32<kTab><<<delta_blocks(), kD32Threads, tab + k, s>>>(P, B, (int)tab);
+}
+
+void launch_delta_pairs32(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
+  if (P.htab && P.single_image && P.pair_kind == 0 && P.use_ewald)
+    launch_delta32<true>(P, B, s);
+  else
+    launch_delta32<false>(P, B, s);
 }
 
 // Loop constants of a replica's pair sweep, in registers.
@@ -629,7 +747,7 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
       // moved beads' phase tables, built once per item, serve up to four
       // vectors per thread, and vectors of one (nx, ny) column (n_z runs
       // fastest in the k list) share the product e^{i(kx x + ky y)}: the
-      // phase of each is the same cmul(cmul(ex, ey), ez) as phase32's
+      // phase of each is cmul(cmul(ex, ey), ez)
       const int tile = local - s_np[r];
       const int sk_pend = st->sk_pending, sk_buf = st->sk_buf, cur_buf = st->cur_buf;
       const int nq = (kKTile32 + kPairThreads - 1) / kPairThreads;
