@@ -1190,8 +1190,8 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   // 2 + len (2 r + 1) with r rejected pairs per randSphere (mean 1.27).
   const int batch = 256;
   const long long per_move = 16 + 12LL * c->max_len;
-  const long long need = per_move * batch;
-  const long long cap = std::max<long long>(4 * need, 1 << 22);
+  const long long need = per_move * std::min(batch, n_moves);
+  const long long cap = std::max<long long>(4 * per_move * batch, 1 << 22);
   int rc = ensure_stream(c, cap);
   if (rc) return rc;
   DevState st;
@@ -1214,16 +1214,17 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   CK(cudaEventRecord(c->ev0, c->s));
   int done = 0;
   while (done < n_moves) {
-    // Keep at least `need` unread words: move the unread tail to the front
-    // and generate the rest on the device.
+    // Keep at least `need` unread words: move the unread tail to the front and
+    // generate twice that on the device (one block's work, in line with the moves:
+    // a buffer filled to the brim cost a new state's first call 5.5 ms).
     if (len - pos < need) {
       long long tail = len - pos;
       if (tail > 0)
         CK(cudaMemcpyAsync(c->d_stream, c->d_stream + pos, sizeof(uint32_t) * tail,
                            cudaMemcpyDeviceToDevice, c->s));
-      launch_mt_fill(c->d_mt, c->d_stream + tail, cap - tail, c->s);
+      len = std::min(cap, tail + 2 * need);
+      launch_mt_fill(c->d_mt, c->d_stream + tail, len - tail, c->s);
       c->last_kernels++;
-      len = cap;
       pos = 0;
       st.stream_pos = 0;
     }
