@@ -152,11 +152,18 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
     P.kper += E.kcell[a] + 1;
   }
   const int row = (int)(P.kper * sizeof(double2));
-  P.kchunk_delta = std::max(1, std::min(16, kKTableBytes / (2 * row)));
   P.kchunk_sk = std::max(1, std::min(32, kKTableBytes / row));
   const double rc = E.real_cut;
   P.real_cut = rc;
   P.single_image = rc <= 0.5 * E.ebox[0] && rc <= 0.5 * E.ebox[1] && rc <= 0.5 * E.ebox[2];
+  // the tabulated real-space term: one image, or at most two on each axis (r_c below
+  // every box length; the further one stays above the table's lower end)
+  bool two = true;
+  for (int a = 0; a < 3; a++) {
+    P.f_img[a] = rc > 0.5 * E.ebox[a] ? (float)E.ebox[a] : 2.0f * kNoImage;
+    two = two && rc < E.ebox[a] && in.alpha * 0.25 * E.ebox[a] * E.ebox[a] >= std::ldexp(1.0, kH32ELo);
+  }
+  P.images = P.single_image ? 1 : (two ? 2 : 0);
   P.lB = in.lB;
   P.sqrt_alpha = std::sqrt(in.alpha);
   P.alpha = in.alpha;
@@ -177,14 +184,16 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
   std::map<std::array<int, 3>, int> at;
   for (int k = 0; k < P.n_k; k++) at[{(*kn)[k].x, (*kn)[k].y, (*kn)[k].z}] = k;
   ku->clear();
+  unsigned short col = 0;
   for (int k = 0; k < P.n_k; k++) {
     const short4 v = (*kn)[k];
+    if (k > 0 && (v.x != (*kn)[k - 1].x || v.y != (*kn)[k - 1].y)) col++;
     const auto mate = at.find({v.x, v.y, -v.z});
     const int m = v.z == 0 || mate == at.end() ? -1 : mate->second;
     if (v.z >= 0)
-      ku->push_back(KUnit{v.x, v.y, v.z, 0, k, m});
+      ku->push_back(KUnit{v.x, v.y, v.z, col, k, m});
     else if (m < 0)
-      ku->push_back(KUnit{v.x, v.y, (short)-v.z, 0, -1, k});
+      ku->push_back(KUnit{v.x, v.y, (short)-v.z, col, -1, k});
   }
   P.n_ku = (int)ku->size();
   c->in.x_kcut2 = E.kc2;  // effective k^2 cut-off, reported by plum_ctx_info
@@ -2310,11 +2319,8 @@ int plum_batch_create(int n, const char* const* dirs, const char* const* runins,
     int most = 0;
     for (int m = 1; m <= c->max_len; m++)
       most = std::max(most, pair_item_count(m, P.n_bead, kMinItemPairs));
-    items += most + (P.n_k + kMinKTile - 1) / kMinKTile;
-    size_t sm = P.use_ewald ? (size_t)P.kchunk_delta * 2 * P.kper * sizeof(float2) : 0;
-    b->kt_smem = std::max(b->kt_smem, sm);
-    // staged moved beads of a pair item (trial and current int4, charge)
-    b->kt_smem = std::max(b->kt_smem, (size_t)kPairGroup * (2 * sizeof(int4) + sizeof(float)));
+    items += most + (P.n_ku + kMinKTile / 2 - 1) / (kMinKTile / 2);
+    b->kt_smem = std::max(b->kt_smem, (size_t)batch_delta_smem(P));
   }
   int rc = 0;
   rc |= dalloc(&b->d_rp, n);

@@ -46,6 +46,8 @@ constexpr int PLUM_ERR_TIMEOUT_DEV = 3;
 constexpr int PLUM_ERR_NONFINITE_DEV = 4;
 constexpr int PLUM_ERR_STREAM_DEV = 6;
 
+constexpr float kNoImage = 1e14f;
+
 struct DevParams {
   int n_bead, n_mol, n_type, npbc;
   int phantom, grafted, n_chain_total, n_ion_total;  // chain/ion pick lists
@@ -63,9 +65,10 @@ struct DevParams {
   double lB, sqrt_alpha, real_cut;
   int real_cell[3];
   int single_image;  // real_cut <= half of every Ewald box length
+  int images;        // 1 single_image, 2 real_cut below every box length, else 0
   int n_k, n_ku, kmax[3];
   int koff[3], kper;  // per-bead table: axis a at koff[a], n = 0..kmax[a]; kper entries
-  int kchunk_delta, kchunk_sk;  // beads per table chunk (fits kKTableBytes)
+  int kchunk_sk;  // beads per table chunk (fits kKTableBytes)
   double kunit[3];   // 2 kPi / ebox[a]
   double kpref;      // lB/(kPi V) * 4 kPi^2
   double self_coef;  // -lB sqrt(alpha/kPi)
@@ -90,6 +93,7 @@ struct DevParams {
   int form;              // 0 FP64, 1 FP32
   float f_scale[3];      // Ewald box length / 2^32: fixed-point unit per axis
   float f_box[3];        // Ewald box lengths
+  float f_img[3];        // f_box of the axes with two images in range, else past kNoImage
   float f_lj_sig2[kMaxT2], f_lj_eps4[kMaxT2], f_lj_rc2[kMaxT2], f_lj_eref[kMaxT2];
   float f_real_cut, f_sqrt_alpha, f_lB;
   double inv_fix[3];     // 2^32 / Ewald box length (FP64 -> fixed point)
@@ -160,7 +164,8 @@ struct DevState {
 // c sin(kz z): four multiply-adds per bead serve both vectors. Units of one
 // (nx, ny) column are consecutive.
 struct alignas(16) KUnit {
-  short nx, ny, nz, pad;
+  short nx, ny, nz;
+  unsigned short col;  // number of the (nx, ny) column, mod 2^16
   int kp, km;
 };
 
@@ -290,6 +295,8 @@ void launch_rhoz(const DevParams& P, const DevBuffers& B, double res, int n_bins
                  cudaStream_t s);
 // precision form (kern_fp32.cu)
 int pair_grid32();
+// Shared memory of a batch item's staged beads or phase tables.
+int batch_delta_smem(const DevParams& P);
 void launch_delta_pairs32(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 // the plain form's 64-bit position mirror (B.fpos64), where it has one
 void launch_fix64_all(const DevParams& P, const DevBuffers& B, cudaStream_t s);

@@ -64,22 +64,106 @@ __device__ __forceinline__ float2 block_sum32x2(float a, float b, float* sh) {
   return t;
 }
 
-// Exact per-entry table: e^{i 2 pi n X / 2^32}, n = 0..kmax, q folded into x.
-__device__ __forceinline__ void table32(const DevParams& P, int4 f, float q, int axis,
-                                        float2* tab) {
-  const unsigned X = (unsigned)(axis == 0 ? f.x : (axis == 1 ? f.y : f.z));
-  float2* t = tab + P.koff[axis];
-  const float w = axis == 0 ? q : 1.0f;
-  for (int n = 0; n <= P.kmax[axis]; n++) {
-    unsigned ph = X * (unsigned)n;
-    float s, c;
-    sincospif((float)(int)ph * 4.6566128730773926e-10f, &s, &c);  // * 2^-31
-    t[n] = make_float2(w * c, w * s);
-  }
+// ---------------------------------------------------------------- pair evaluation
+// Constants of the table-driven real-space term. Lengths are real ones, or fixed-point
+// units (cs: real r^2 per unit of r^2).
+struct TabPair {
+  float2 sx, sy, sz, ua;     // scales; table variable per r^2
+  float rc2, ljlim, cs, ius; // cut-off; largest LJ cut-off^2; u per table variable
+  float bx, by, bz;          // DevParams::f_img
+};
+
+// kCubic (equal fixed-point scales on the three axes): r^2 stays in fixed-point units
+// and the box scale is folded into the constants.
+template <bool kCubic, bool kCut>
+__device__ __forceinline__ TabPair tab_pair(const DevParams& P, float cut_scale) {
+  TabPair K;
+  const float s0 = P.f_scale[0], s1 = P.f_scale[1], s2 = P.f_scale[2];
+  K.sx = make_float2(s0, s0);
+  K.sy = make_float2(s1, s1);
+  K.sz = make_float2(s2, s2);
+  K.cs = kCubic ? s0 * s0 : 1.0f;
+  const float ics = 1.0f / K.cs;
+  K.rc2 = P.f_real_cut * P.f_real_cut * ics;
+  const float ua = P.f_sqrt_alpha * P.f_sqrt_alpha * K.cs * (kCut ? cut_scale : 1.0f);
+  K.ua = make_float2(ua, ua);
+  K.ius = kCut ? 1.0f / cut_scale : 1.0f;
+  float m = P.use_pair ? 1e-30f : 0.0f;  // r2 = 0 (coincident beads) must reach lj32
+  if (P.use_pair)
+    for (int k = 0; k < P.n_type * P.n_type; k++) m = fmaxf(m, P.f_lj_rc2[k]);
+  K.ljlim = m * ics;
+  K.bx = P.f_img[0];
+  K.by = P.f_img[1];
+  K.bz = P.f_img[2];
+  return K;
 }
 
-__device__ __forceinline__ float2 cmul32(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// h at the trial r^2 (r.x) less h at the current one (r.y). kCut: the table is zero
+// from the cut-off on; else a select at r_c. kNear: r may lie below the table.
+template <bool kCut, bool kNear>
+__device__ __forceinline__ float tab_diff(const TabPair& K, const float4* s_h, float2 r) {
+  const float2 u = __fmul2_rn(r, K.ua);
+  const int b1 = __float_as_int(u.x), b0 = __float_as_int(u.y);
+  float h1 = h32_tab(s_h, b1), h0 = h32_tab(s_h, b0);
+  if (kNear && min(b1, b0) < kH32LoBits) {
+    if (b1 < kH32LoBits) h1 = h32_small(u.x * K.ius);
+    if (b0 < kH32LoBits) h0 = h32_small(u.y * K.ius);
+  }
+  if (!kCut) {
+    h1 = r.x <= K.rc2 ? h1 : 0.0f;
+    h0 = r.y <= K.rc2 ? h0 : 0.0f;
+  }
+  return h1 - h0;
+}
+
+__device__ __forceinline__ float2 sq2(float2 a) { return __fmul2_rn(a, a); }
+__device__ __forceinline__ float2 add3(float2 a, float2 b, float2 c) {
+  return __fadd2_rn(__fadd2_rn(a, b), c);
+}
+// the image a box length to the other side: |d| -> L - |d|
+__device__ __forceinline__ float2 flip2(float b, float2 d) {
+  return make_float2(b - fabsf(d.x), b - fabsf(d.y));
+}
+
+// The real-space change (in units of lB sqrt(alpha) q q') of staged bead (t trial, c
+// current) with other bead (ot, oc), and the LJ change where lj is set. kImg (r_c below
+// every box length): an axis has at most one more image in range, the one on the other
+// side; with r_c under 0.7 L two axes at once never do, so those are behind a branch.
+template <bool kCubic, bool kCut, bool kImg>
+__device__ __forceinline__ float tab_eval(const DevParams& P, const TabPair& K, const float4* s_h,
+                                          const int4 t, const int4 c, const int4 ot, const int4 oc,
+                                          int k, bool lj, float& acc_lj) {
+  float2 dx = make_float2((float)(int)((unsigned)ot.x - (unsigned)t.x),
+                          (float)(int)((unsigned)oc.x - (unsigned)c.x));
+  float2 dy = make_float2((float)(int)((unsigned)ot.y - (unsigned)t.y),
+                          (float)(int)((unsigned)oc.y - (unsigned)c.y));
+  float2 dz = make_float2((float)(int)((unsigned)ot.z - (unsigned)t.z),
+                          (float)(int)((unsigned)oc.z - (unsigned)c.z));
+  if (!kCubic) {
+    dx = __fmul2_rn(dx, K.sx);
+    dy = __fmul2_rn(dy, K.sy);
+    dz = __fmul2_rn(dz, K.sz);
+  }
+  if (!kImg) {
+    const float2 r = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    if (lj && fminf(r.x, r.y) < K.ljlim)
+      acc_lj += lj32(P, k, r.x * K.cs) - lj32(P, k, r.y * K.cs);
+    return tab_diff<kCut, true>(K, s_h, r);
+  }
+  const float2 xx = sq2(dx), yy = sq2(dy), zz = sq2(dz);
+  const float2 r = add3(xx, yy, zz);
+  if (lj && fminf(r.x, r.y) < K.ljlim) acc_lj += lj32(P, k, r.x) - lj32(P, k, r.y);
+  float h = tab_diff<kCut, true>(K, s_h, r);
+  const float2 fx = sq2(flip2(K.bx, dx)), fy = sq2(flip2(K.by, dy)), fz = sq2(flip2(K.bz, dz));
+  if (K.bx < kNoImage) h += tab_diff<kCut, false>(K, s_h, add3(fx, yy, zz));
+  if (K.by < kNoImage) h += tab_diff<kCut, false>(K, s_h, add3(xx, fy, zz));
+  if (K.bz < kNoImage) h += tab_diff<kCut, false>(K, s_h, add3(xx, yy, fz));
+  const float2 xy = add3(fx, fy, zz), xz = add3(fx, yy, fz), yz = add3(xx, fy, fz);
+  if (fminf(fminf(fminf(xy.x, xy.y), fminf(xz.x, xz.y)), fminf(yz.x, yz.y)) <= K.rc2) {
+    h += tab_diff<kCut, false>(K, s_h, xy) + tab_diff<kCut, false>(K, s_h, xz);
+    h += tab_diff<kCut, false>(K, s_h, yz) + tab_diff<kCut, false>(K, s_h, add3(fx, fy, fz));
+  }
+  return h;
 }
 
 // ---------------------------------------------------------------- one system
@@ -91,8 +175,8 @@ __device__ __forceinline__ float2 cmul32(float2 a, float2 b) {
 // (10 KB); for a long one the FP32 pipe (some 25 instructions per evaluation).
 // With 20,000 beads and 7,812 k-vectors: 13.4 us, and 21.5 us a move (32.6 and 34.3 us
 // with every pair's four loads, k tiles x bead groups and a ticket for the last block).
-// Hard spheres, image cells and a cut-off beyond the table take the general pair
-// loop below.
+// Hard spheres and a cut-off beyond the table or the box take the general pair loop
+// below.
 constexpr int kD32Threads = 768;
 constexpr int kD32K = 256;      // k role
 constexpr int kD32Stage = 256;  // moved beads staged at a time
@@ -114,7 +198,8 @@ __device__ __forceinline__ float2 turn32(unsigned phi) {
   return make_float2(c, s);
 }
 
-// The pairs of pair thread t0 of nt: one image, LJ + Ewald, the h(u) table.
+// The pairs of pair thread t0 of nt: LJ + Ewald, the h(u) table.
+template <bool kImg>
 __device__ __forceinline__ void sweep32(const DevParams& P, const DevBuffers& B, Stage32* st,
                                         float4* s_h, int t0, int nt, int b_lo, int m,
                                         float& acc_lj, float& acc_re) {
@@ -122,15 +207,8 @@ __device__ __forceinline__ void sweep32(const DevParams& P, const DevBuffers& B,
   const int G = (int)gridDim.x * nt, p0 = (int)blockIdx.x * nt + t0;
   const long long pairs = (long long)m * N;
   const int run_len = pairs >= 2LL * kD32Run * G ? kD32Run : (pairs >= 4LL * G ? 2 : 1);
-  const float rc2 = P.f_real_cut * P.f_real_cut;
-  const float ua = P.f_sqrt_alpha * P.f_sqrt_alpha, pref = P.f_lB * P.f_sqrt_alpha;
-  float ljm = P.use_pair ? 1e-30f : 0.0f;  // r2 = 0 (coincident beads) must reach lj32
-  if (P.use_pair)
-    for (int k = 0; k < n_type * n_type; k++) ljm = fmaxf(ljm, P.f_lj_rc2[k]);
-  const float2 sx = make_float2(P.f_scale[0], P.f_scale[0]);
-  const float2 sy = make_float2(P.f_scale[1], P.f_scale[1]);
-  const float2 sz = make_float2(P.f_scale[2], P.f_scale[2]);
-  const float2 ua2 = make_float2(ua, ua);
+  const TabPair K = tab_pair<false, false>(P, 0.0f);
+  const float pref = P.f_lB * P.f_sqrt_alpha;
   for (int i = t0; i < kH32Bins; i += nt) s_h[i] = P.htab[i];
   for (int g0 = 0; g0 < m; g0 += kD32Stage) {
     const int gn = min(kD32Stage, m - g0);
@@ -161,27 +239,9 @@ __device__ __forceinline__ void sweep32(const DevParams& P, const DevBuffers& B,
       float acc = 0.0f;
       for (int u = u0; u < u1; u++) {
         const int4 t = st[u].t, c = st[u].c;
-        const float2 dx = __fmul2_rn(make_float2((float)(int)((unsigned)o1.x - (unsigned)t.x),
-                                                 (float)(int)((unsigned)o0.x - (unsigned)c.x)), sx);
-        const float2 dy = __fmul2_rn(make_float2((float)(int)((unsigned)o1.y - (unsigned)t.y),
-                                                 (float)(int)((unsigned)o0.y - (unsigned)c.y)), sy);
-        const float2 dz = __fmul2_rn(make_float2((float)(int)((unsigned)o1.z - (unsigned)t.z),
-                                                 (float)(int)((unsigned)o0.z - (unsigned)c.z)), sz);
-        const float2 r = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-        if (fminf(r.x, r.y) < ljm) {
-          const int k = c.w + o0.w;
-          acc_lj += lj32(P, k, r.x) - lj32(P, k, r.y);
-        }
-        const float2 v = __fmul2_rn(r, ua2);
-        const int b1 = __float_as_int(v.x), b0 = __float_as_int(v.y);
-        float h1 = h32_tab(s_h, b1), h0 = h32_tab(s_h, b0);
-        if (min(b1, b0) < kH32LoBits) {
-          if (b1 < kH32LoBits) h1 = h32_small(v.x);
-          if (b0 < kH32LoBits) h0 = h32_small(v.y);
-        }
-        h1 = r.x <= rc2 ? h1 : 0.0f;
-        h0 = r.y <= rc2 ? h0 : 0.0f;
-        acc = fmaf(__int_as_float(t.w), h1 - h0, acc);
+        acc = fmaf(__int_as_float(t.w),
+                   tab_eval<false, false, kImg>(P, K, s_h, t, c, o1, o0, c.w + o0.w, true, acc_lj),
+                   acc);
       }
       acc_re = fmaf(qj, acc, acc_re);
     }
@@ -281,7 +341,8 @@ __device__ __forceinline__ float k_role32(const DevParams& P, const DevBuffers& 
   return e;
 }
 
-template <bool kTab>
+// kMode: 0 the general pair loop, 1 one image, 2 image cells (DevParams::images)
+template <int kMode>
 __global__ void __launch_bounds__(kD32Threads, 1)
     k_delta32(const DevParams P, const DevBuffers B, int tab_bytes) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -301,11 +362,11 @@ __global__ void __launch_bounds__(kD32Threads, 1)
   } else {
     const int t0 = (int)threadIdx.x - kthreads, nt = kD32Threads - kthreads;
     const int N = P.n_bead;
-    if (kTab) {
+    if (kMode) {
       if (m > 0)
-        sweep32(P, B, reinterpret_cast<Stage32*>(smem),
-                reinterpret_cast<float4*>(smem + kD32Stage * sizeof(Stage32)), t0, nt, b_lo, m, a,
-                b);
+        sweep32<kMode == 2>(P, B, reinterpret_cast<Stage32*>(smem),
+                            reinterpret_cast<float4*>(smem + kD32Stage * sizeof(Stage32)), t0, nt,
+                            b_lo, m, a, b);
     } else if (P.use_pair || P.use_ewald) {
       // pair p = ii * N + j, dealt with stride G; (ii, j) advanced without a
       // division per pair
@@ -364,26 +425,29 @@ int pair_grid32() {
   return g_grid32;
 }
 
-template <bool kTab>
+template <int kMode>
 static void launch_delta32(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
-  const size_t tab = kTab ? kD32Stage * sizeof(Stage32) + kH32Bins * sizeof(float4) : 0;
+  const size_t tab = kMode ? kD32Stage * sizeof(Stage32) + kH32Bins * sizeof(float4) : 0;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_delta32<kTab>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_delta32<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kKTableBytes + 4096 + (int)tab);
     attr = true;
   }
   const size_t k = P.use_ewald && P.n_ku > 0
                        ? (size_t)k_beads32(P) * 2 * (P.kmax[2] + 1 + kD32Units) * sizeof(float2)
                        : 0;
-  k_delta32<kTab><<<delta_blocks(), kD32Threads, tab + k, s>>>(P, B, (int)tab);
+  k_delta32<kMode><<<delta_blocks(), kD32Threads, tab + k, s>>>(P, B, (int)tab);
 }
 
 void launch_delta_pairs32(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
-  if (P.htab && P.single_image && P.pair_kind == 0 && P.use_ewald)
-    launch_delta32<true>(P, B, s);
+  const int mode = P.htab && P.pair_kind == 0 && P.use_ewald ? P.images : 0;
+  if (mode == 1)
+    launch_delta32<1>(P, B, s);
+  else if (mode == 2)
+    launch_delta32<2>(P, B, s);
   else
-    launch_delta32<false>(P, B, s);
+    launch_delta32<0>(P, B, s);
 }
 
 // Loop constants of a replica's pair sweep, in registers.
@@ -438,11 +502,12 @@ __device__ __forceinline__ void pair32k(const DevParams& P, const PairConst& K, 
 // gn staged moved beads at their trial (s_mt[u]) and current
 // (s_mt[kPairGroup + u]) positions.
 template <bool kSingle>
-__device__ __forceinline__ void pair_sweep(const DevParams& P, const PairConst& K,
-                                           const DevBuffers& B, const int4* s_mt,
-                                           const float* s_mq, int gn, int g_lo, int c0, int c1,
-                                           int b_lo, int b_hi, float& acc_lj, float& acc_re) {
+__device__ __forceinline__ float2 pair_sweep(const DevParams& P, const DevBuffers& B,
+                                          const int4* s_mt, const float* s_mq, int gn, int g_lo,
+                                          int c0, int c1, int b_lo, int b_hi) {
+  const PairConst K = pair_const(P);
   const bool hs = P.pair_kind == 1;
+  float acc_lj = 0.0f, acc_re = 0.0f;
   for (int j = c0 + threadIdx.x; j < c1; j += kPairThreads) {
     if (j >= b_lo && j < b_hi) continue;  // moved pairs: the last item
     const int4 cj = B.fpos[j];
@@ -456,74 +521,29 @@ __device__ __forceinline__ void pair_sweep(const DevParams& P, const PairConst& 
       acc_re += r1 - r0;
     }
   }
+  return make_float2(acc_lj, acc_re);
 }
 
 // ------------------------------------------------ table-driven real space
-// pair_sweep for LJ + Ewald with r_c <= L/2 on every axis, the real-space term
-// from the h(u) table: per (moved u, other j) the trial and current distances
-// share the other bead's load, one LJ pre-test and the packed (two-lane FP32)
-// arithmetic of r^2 and u, so a warp runs no divergent erfc. Each thread takes
-// two other beads per staged bead, so one load of the staged trial and
-// current entries serves four evaluations; the other bead's charge multiplies
-// its sum once, after the staged beads. kCubic (equal fixed-point scales on
-// the three axes): r^2 stays in fixed-point units and the box scale is folded
-// into the constants. kCut: the table is the batch's cut table (variable
-// u' = cut_scale u, zero from the cut-off on), so the cut-off costs nothing;
-// else the universal table and a select at r_c. gn4 staged beads, a multiple
-// of 4; the trial entry's w holds the staged bead's charge (float bits) and
-// the current entry's w its type; the padding beads have q = 0 and equal
-// trial and current positions, so they add exactly zero.
-template <bool kCubic, bool kCut>
-__device__ __forceinline__ void pair_sweep_tab(const DevParams& P, const DevBuffers& B,
-                                               const int4* s_mt, const float4* s_h, int gn4,
-                                               int c0, int c1, int b_lo, int b_hi,
-                                               float cut_scale, float& acc_lj, float& acc_re) {
-  const float sx = P.f_scale[0], sy = P.f_scale[1], sz = P.f_scale[2];
-  const float cs = kCubic ? sx * sx : 1.0f;  // real r^2 per unit of r2 below
-  const float ics = 1.0f / cs;
-  const float rc2 = P.f_real_cut * P.f_real_cut * ics;
-  const float ua = P.f_sqrt_alpha * P.f_sqrt_alpha * cs * (kCut ? cut_scale : 1.0f);
-  const float ius = kCut ? 1.0f / cut_scale : 1.0f;  // table variable -> u
-  float ljm = 1e-30f;  // r2 = 0 (coincident beads) must reach lj32
-  for (int k = 0; k < P.n_type * P.n_type; k++) ljm = fmaxf(ljm, P.f_lj_rc2[k]);
-  const float ljlim = ljm * ics;
+// pair_sweep for LJ + Ewald from the h(u) table: per (moved u, other j) the trial and
+// current distances share the other bead's load, one LJ pre-test and the packed
+// (two-lane FP32) arithmetic of r^2 and u, so a warp runs no divergent erfc. Each
+// thread takes two other beads per staged bead, so one load of the staged trial and
+// current entries serves four evaluations; the other bead's charge multiplies its sum
+// once, after the staged beads. gn4 staged beads, a multiple of 4; the trial entry's w
+// holds the staged bead's charge (float bits) and the current entry's w its type; the
+// padding beads have q = 0 and equal trial and current positions, so they add exactly
+// zero. kCut: the table is the batch's cut table (variable u' = cut_scale u, zero from
+// the cut-off on), so the cut-off costs nothing.
+template <bool kCubic, bool kCut, bool kImg>
+__device__ __forceinline__ float2 pair_sweep_tab(const DevParams& P, const DevBuffers& B,
+                                              const int4* s_mt, const float4* s_h, int gn4,
+                                              int c0, int c1, int b_lo, int b_hi,
+                                              float cut_scale) {
+  float acc_lj = 0.0f, acc_re = 0.0f;
+  const TabPair K = tab_pair<kCubic, kCut>(P, cut_scale);
   const float pref = P.f_lB * P.f_sqrt_alpha;
   const int nt = P.n_type;
-  const bool use_pair = P.use_pair;
-  const float2 ua2 = make_float2(ua, ua);
-  const float2 s2x = make_float2(sx, sx), s2y = make_float2(sy, sy), s2z = make_float2(sz, sz);
-  // one evaluation pair (trial, current) of staged bead (t, c) with other
-  // bead o; ok: o is an other bead of this item (not moved, inside the chunk)
-  auto eval = [&](const int4 t, const int4 c, const int4 o, bool ok, float& acc) {
-    float2 dx = make_float2((float)(int)((unsigned)o.x - (unsigned)t.x),
-                            (float)(int)((unsigned)o.x - (unsigned)c.x));
-    float2 dy = make_float2((float)(int)((unsigned)o.y - (unsigned)t.y),
-                            (float)(int)((unsigned)o.y - (unsigned)c.y));
-    float2 dz = make_float2((float)(int)((unsigned)o.z - (unsigned)t.z),
-                            (float)(int)((unsigned)o.z - (unsigned)c.z));
-    if (!kCubic) {
-      dx = __fmul2_rn(dx, s2x);
-      dy = __fmul2_rn(dy, s2y);
-      dz = __fmul2_rn(dz, s2z);
-    }
-    const float2 r = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    if (use_pair && ok && fminf(r.x, r.y) < ljlim) {
-      const int k = c.w * nt + o.w;  // trial and current share the type
-      acc_lj += lj32(P, k, r.x * cs) - lj32(P, k, r.y * cs);
-    }
-    const float2 u = __fmul2_rn(r, ua2);
-    const int b1 = __float_as_int(u.x), b0 = __float_as_int(u.y);
-    float h1 = h32_tab(s_h, b1), h0 = h32_tab(s_h, b0);
-    if (min(b1, b0) < kH32LoBits) {
-      if (b1 < kH32LoBits) h1 = h32_small(u.x * ius);
-      if (b0 < kH32LoBits) h0 = h32_small(u.y * ius);
-    }
-    if (!kCut) {
-      h1 = r.x <= rc2 ? h1 : 0.0f;
-      h0 = r.y <= rc2 ? h0 : 0.0f;
-    }
-    acc = fmaf(__int_as_float(t.w), h1 - h0, acc);
-  };
   for (int j0 = c0 + threadIdx.x; j0 < c1; j0 += 2 * kPairThreads) {
     const int j1 = j0 + kPairThreads;
     const bool ok0 = !(j0 >= b_lo && j0 < b_hi);  // moved pairs: the last item
@@ -533,14 +553,44 @@ __device__ __forceinline__ void pair_sweep_tab(const DevParams& P, const DevBuff
     const float q0 = ok0 ? B.fq[j0] * pref : 0.0f;
     const float q1 = ok1 ? B.fq[j1] * pref : 0.0f;
     float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll 4
+#pragma unroll(kImg ? 2 : 4)
     for (int u = 0; u < gn4; u++) {
       const int4 t = s_mt[u], c = s_mt[kPairGroup + u];
-      eval(t, c, o0, ok0, a0);
-      eval(t, c, o1, ok1, a1);
+      const float q = __int_as_float(t.w);
+      const int k = c.w * nt;
+      a0 = fmaf(q, tab_eval<kCubic, kCut, kImg>(P, K, s_h, t, c, o0, o0, k + o0.w, ok0, acc_lj), a0);
+      a1 = fmaf(q, tab_eval<kCubic, kCut, kImg>(P, K, s_h, t, c, o1, o1, k + o1.w, ok1, acc_lj), a1);
     }
     acc_re = fmaf(q0, a0, fmaf(q1, a1, acc_re));
   }
+  return make_float2(acc_lj, acc_re);
+}
+
+// The pairs among the m moved beads, each once, from the table: rows a and m - 1 - a
+// together hold m - 1 pairs, dealt out by columns.
+template <bool kCut, bool kImg>
+__device__ __forceinline__ float2 moved_pairs_tab(const DevParams& P, const DevBuffers& B,
+                                               const float4* s_h, int b_lo, int m,
+                                               float cut_scale) {
+  float acc_lj = 0.0f, acc_re = 0.0f;
+  const TabPair K = tab_pair<false, kCut>(P, cut_scale);
+  const float pref = P.f_lB * P.f_sqrt_alpha;
+  const int n = ((m + 1) / 2) * (m - 1);
+  for (int p = threadIdx.x; p < n; p += kPairThreads) {
+    int a = p / (m - 1), b = p - a * (m - 1);
+    if (b < m - 1 - a) {
+      b += a + 1;
+    } else {
+      if (2 * a == m - 1) continue;  // the middle row stands alone
+      a = m - 1 - a;
+      b++;
+    }
+    const int4 c = B.fpos[b_lo + a], oc = B.fpos[b_lo + b];
+    const float h = tab_eval<false, kCut, kImg>(P, K, s_h, B.ftrial[a], c, B.ftrial[b], oc,
+                                                c.w * P.n_type + oc.w, true, acc_lj);
+    acc_re = fmaf(B.fq[b_lo + a] * B.fq[b_lo + b] * pref, h, acc_re);
+  }
+  return make_float2(acc_lj, acc_re);
 }
 
 // The table (kH32Bins float4): per bin the cubic in w = f / 32 (f the
@@ -587,17 +637,122 @@ void build_h32_table(float4* out, double scale, double cut) {
 }
 
 // ------------------------------------------------------------ replicas
-constexpr int kMaxKPerThread = 4;  // k vectors per thread of a k item (k_tile <= 1024)
-static_assert(kMaxKPerThread * kPairThreads >= 1024, "k items of up to 1024 vectors");
+constexpr int kKUnitsMost = 512;  // k units of a k item (k_tile <= 1024)
+constexpr int kKPer = kKUnitsMost / kPairThreads;
+
+// dS(k), the S(k) commit and the |S|^2 change of up to 512 units [u0, u0 + un). A thread
+// takes one unit and every slices-th moved bead, or two units and all of them. smem:
+// e^{i nz theta_z} of as many moved beads (trial and current) as fit, then their xy
+// parts per (nx, ny) column, every entry one thread's, from its exact integer phase.
+// (A vector's phase as a product of three table entries, the tables built by six
+// threads a bead: four times the instructions per vector.)
+__device__ __forceinline__ float k_item32(const DevParams& P, const DevBuffers& B,
+                                          unsigned char* smem, int smem_bytes, int u0, int un,
+                                          int b_lo, int b_hi, int sk_pend, int sk_buf,
+                                          int cur_buf) {
+  __shared__ short2 s_col[kKUnitsMost];
+  __shared__ float s_sum[4][kPairThreads];
+  __shared__ int s_zmax;
+  const int slices = un < kPairThreads ? kPairThreads / un : 1;
+  const int t0 = slices > 1 ? (int)threadIdx.x % un : (int)threadIdx.x;
+  const int sl = slices > 1 ? (int)threadIdx.x / un : 0;
+  KUnit ku[kKPer];
+  float2 A[kKPer], Bs[kKPer];
+  const int col0 = B.ku[u0].col;
+  const int ncol = ((B.ku[u0 + un - 1].col - col0) & 0xFFFF) + 1;
+  if (threadIdx.x == 0) s_zmax = 0;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kKPer; q++) {
+    const int u = t0 + q * kPairThreads;
+    ku[q] = u < un && sl < slices ? B.ku[u0 + u] : KUnit{0, 0, 0, B.ku[u0].col, -1, -1};
+    A[q] = Bs[q] = make_float2(0.0f, 0.0f);
+    const int zw = __reduce_max_sync(0xffffffffu, (int)ku[q].nz);
+    if ((threadIdx.x & 31) == 0 && zw > 0) atomicMax(&s_zmax, zw);
+    ku[q].col = (unsigned short)(ku[q].col - col0);
+    if (u < un && sl == 0) s_col[ku[q].col] = make_short2(ku[q].nx, ku[q].ny);
+  }
+  __syncthreads();
+  const int nz = s_zmax + 1, ne = nz + ncol;
+  const int kb = min(64, smem_bytes / (2 * ne * (int)sizeof(float2)));
+  float2* s_z = reinterpret_cast<float2*>(smem);
+  float2* s_xy = s_z + (size_t)kb * 2 * nz;
+  for (int g0 = b_lo; g0 < b_hi; g0 += kb) {
+    const int nt = 2 * min(kb, b_hi - g0);
+    if (g0 > b_lo) __syncthreads();  // the tables are free
+    for (int t = threadIdx.x; t < nt * ne; t += kPairThreads) {
+      const int c = t / nt, it = t - c * nt;
+      const int bead = g0 + (it >> 1);
+      const int4 f = (it & 1) ? B.fpos[bead] : B.ftrial[bead - b_lo];
+      if (c < nz) {
+        s_z[it * nz + c] = turn32((unsigned)f.z * (unsigned)c);
+      } else {
+        const short2 kc = s_col[c - nz];
+        const float2 v = turn32((unsigned)f.x * (unsigned)(int)kc.x +
+                                (unsigned)f.y * (unsigned)(int)kc.y);
+        const float w = (it & 1) ? -B.fq[bead] : B.fq[bead];  // trial minus current
+        s_xy[it * ncol + c - nz] = make_float2(w * v.x, w * v.y);
+      }
+    }
+    __syncthreads();
+    if (sl < slices)
+#pragma unroll
+      for (int q = 0; q < kKPer; q++)
+        if (t0 + q * kPairThreads < un)
+          for (int it = sl; it < nt; it += slices) {
+            const float2 xy = s_xy[it * ncol + ku[q].col], ez = s_z[it * nz + ku[q].nz];
+            A[q].x = fmaf(xy.x, ez.x, A[q].x);
+            A[q].y = fmaf(xy.y, ez.x, A[q].y);
+            Bs[q].x = fmaf(xy.x, ez.y, Bs[q].x);
+            Bs[q].y = fmaf(xy.y, ez.y, Bs[q].y);
+          }
+  }
+  if (slices > 1) {  // the slices of each (unit, sum), added in order
+    s_sum[0][threadIdx.x] = A[0].x;
+    s_sum[1][threadIdx.x] = A[0].y;
+    s_sum[2][threadIdx.x] = Bs[0].x;
+    s_sum[3][threadIdx.x] = Bs[0].y;
+    __syncthreads();
+    if (sl == 0)
+      for (int w = 1; w < slices; w++) {
+        A[0].x += s_sum[0][w * un + t0];
+        A[0].y += s_sum[1][w * un + t0];
+        Bs[0].x += s_sum[2][w * un + t0];
+        Bs[0].y += s_sum[3][w * un + t0];
+      }
+  }
+  float e = 0.0f;
+  if (sl == 0)
+#pragma unroll
+    for (int q = 0; q < kKPer; q++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {  // +nz, -nz (neither, past the last unit)
+        const int k = h ? ku[q].km : ku[q].kp;
+        if (k < 0) continue;
+        const float2 ds = h ? make_float2(A[q].x + Bs[q].y, A[q].y - Bs[q].x)
+                            : make_float2(A[q].x - Bs[q].y, A[q].y + Bs[q].x);
+        double2 s = B.sk[k];
+        if (sk_pend) {
+          const double2 p = B.dsk[(size_t)sk_buf * P.n_k + k];
+          s = make_double2(s.x + p.x, s.y + p.y);
+          B.sk[k] = s;
+        }
+        B.dsk[(size_t)cur_buf * P.n_k + k] = make_double2((double)ds.x, (double)ds.y);
+        const float sx = (float)s.x, sy = (float)s.y;
+        e += (float)B.kw[k] * (2.0f * (sx * ds.x + sy * ds.y) + (ds.x * ds.x + ds.y * ds.y));
+      }
+  return e;
+}
+
 // Batched replicas: every replica's pending move contributes pair items
 // (up to kPairGroup moved beads, staged in shared memory at their trial and
-// current positions, x a chunk of other beads, one per thread), one item for
-// the pairs among the moved beads, and k items (one k tile of kKTile32
-// vectors over all moved beads). Every block derives the same item list from
-// the replicas' states and takes items one at a time from a queue; each item
-// writes its own slot: pair items {lj, real}, k items {k-space energy
-// change}. The serial step of each replica adds its slots in item order, so
-// the result does not depend on which block took which item.
+// current positions, x a chunk of other beads), one item for the pairs among the
+// moved beads, and k items (k_tile / 2 units over all moved beads). Every block
+// derives the same item list from the replicas' states; its first item is its own
+// number, the next ones come from a queue, drawn while the one before is worked on.
+// Each item writes its own slot: pair items {lj, real}, k items {k-space energy
+// change}. The serial step of each replica adds its slots in item order, so the
+// result does not depend on which block took which item.
 // The item sizes, the grid and the register budget (kMinBlocks resident
 // blocks per SM) are run-time choices (BatchTune, picked by
 // plum_batch_autotune); defaults: 4096 pairs per item, 128-vector k tiles,
@@ -607,18 +762,18 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
     k_batch_delta32(const DevParams* __restrict__ rp, const DevBuffers* __restrict__ rb,
                     int n_rep, int* __restrict__ item_off, double* __restrict__ slots,
                     BatchTune tune, int* __restrict__ queue, const float4* __restrict__ htab,
-                    float cut_scale) {
-  const int kItemPairs = tune.item_pairs, kKTile32 = tune.k_tile;
+                    float cut_scale, int smem_bytes) {
+  const int kItemPairs = tune.item_pairs, kUnitsPer = tune.k_tile / 2;
   extern __shared__ __align__(16) unsigned char smem_all[];
-  // with the h(u) table: the table first, then the staging / k-table area
-  float4* s_h = reinterpret_cast<float4*>(smem_all);
-  unsigned char* smem = smem_all + (htab ? kH32Bins * sizeof(float4) : 0);
+  // the staging / k-table area, the h(u) table where there is one, the item counts
+  unsigned char* smem = smem_all;
+  float4* s_h = reinterpret_cast<float4*>(smem_all + smem_bytes);
+  int* s_pref = reinterpret_cast<int*>(s_h + (htab ? kH32Bins : 0));  // [n_rep + 1]
+  int* s_np = s_pref + n_rep + 1;                                     // [n_rep]
   if (htab)
     for (int i = threadIdx.x; i < kH32Bins; i += blockDim.x) s_h[i] = htab[i];
   __shared__ float red[2 * (kPairThreads / 32)];
-  __shared__ int s_pref[kMaxReplicas + 1];
-  __shared__ int s_np[kMaxReplicas];
-  __shared__ int s_total, s_item;
+  __shared__ int s_item;
   // 1. item counts per replica and their prefix (same in every block)
   for (int r = threadIdx.x; r < n_rep; r += blockDim.x) {
     const DevState* st = rb[r].state;
@@ -626,15 +781,27 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
     const int m = (st->pending && !st->da_skip) ? st->b_hi - st->b_lo : 0;
     const DevParams& pr = rp[r];
     const int np = (pr.use_pair || pr.use_ewald) ? pair_item_count(m, pr.n_bead, kItemPairs) : 0;
-    const int nk = (pr.use_ewald && m > 0) ? (pr.n_k + kKTile32 - 1) / kKTile32 : 0;
+    const int nk = (pr.use_ewald && m > 0) ? (pr.n_ku + kUnitsPer - 1) / kUnitsPer : 0;
     s_np[r] = np;
     s_pref[r + 1] = np + nk;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    s_pref[0] = 0;
-    for (int r = 0; r < n_rep; r++) s_pref[r + 1] += s_pref[r];
-    s_total = s_pref[n_rep];
+  if (threadIdx.x < 32) {  // a run of replicas per lane, then across the lanes
+    const int per = (n_rep + 31) / 32, r0 = min(n_rep, (int)threadIdx.x * per);
+    const int r1 = min(n_rep, r0 + per);
+    int sum = 0;
+    for (int r = r0; r < r1; r++) sum += s_pref[r + 1];
+    int off = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, off, o);
+      if ((int)threadIdx.x >= o) off += v;
+    }
+    off -= sum;
+    for (int r = r0; r < r1; r++) {
+      off += s_pref[r + 1];
+      s_pref[r + 1] = off;
+    }
+    if (threadIdx.x == 0) s_pref[0] = 0;
   }
   __syncthreads();
   if (blockIdx.x == 0)
@@ -644,17 +811,14 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
       item_off[4 * r + 2] = s_pref[r] + s_np[r];
       item_off[4 * r + 3] = s_pref[r + 1] - s_pref[r] - s_np[r];
     }
-  // 2. items are taken from a queue (queue[0]) one at a time: blocks that
-  // drew cheap items take more. Every item writes only its own slot, so
-  // the results do not depend on which block took it. The last block to
-  // run out resets the queue for the next launch.
-  const int T = s_total;
-  for (;;) {
-    __syncthreads();  // the previous item is done with s_item and the staging area
-    if (threadIdx.x == 0) s_item = atomicAdd(&queue[0], 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= T) break;
+  // 2. items are taken one at a time: blocks that drew cheap items take more.
+  // Every item writes only its own slot, so the results do not depend on which
+  // block took it. The last block to run out resets the queue for the next launch.
+  const int T = s_pref[n_rep];
+  int item = blockIdx.x;
+  while (item < T) {
+    int next = 0;
+    if (threadIdx.x == 0) next = (int)gridDim.x + atomicAdd(&queue[0], 1);
     // replica of this item (s_pref is ascending)
     int lo = 0, hi = n_rep - 1;
     while (lo < hi) {
@@ -668,20 +832,20 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
     const int b_lo = st->b_lo, b_hi = st->b_hi, m = b_hi - b_lo, N = P.n_bead;
     const int local = item - s_pref[r];
     if (local < s_np[r]) {
-      float acc_lj = 0.0f, acc_re = 0.0f;
+      float2 acc = make_float2(0.0f, 0.0f);  // LJ, real space
       const int chunk = pair_chunk(m, kItemPairs);
       const int n_chunk = (N + chunk - 1) / chunk;
       const int n_grid = ((m + kPairGroup - 1) / kPairGroup) * n_chunk;
+      const int tab = htab && P.pair_kind == 0 && P.use_ewald ? P.images : 0;
       if (local < n_grid) {
         const int g0 = (local / n_chunk) * kPairGroup, gn = min(kPairGroup, m - g0);
         const int c0 = (local % n_chunk) * chunk, c1 = min(N, c0 + chunk);
         int4* s_mt = reinterpret_cast<int4*>(smem);  // trial, then current
         float* s_mq = reinterpret_cast<float*>(s_mt + 2 * kPairGroup);
-        const bool tab = htab && P.single_image && P.pair_kind == 0 && P.use_ewald;
         // the table path pads the staged beads to a multiple of 4 with the
         // last bead's current position at both places and q = 0
         const int gn4 = tab ? (gn + 3) & ~3 : gn;
-        // (the barrier at the top of the item loop: every thread is done
+        // (the barriers at the end of the item loop: every thread is done
         // with the previous item's staging area)
         for (int u = threadIdx.x; u < gn4; u += kPairThreads) {
           if (u < gn) {
@@ -698,30 +862,30 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
           }
         }
         __syncthreads();
-        const PairConst K = pair_const(P);
-        if (tab) {
-          const bool cubic =
-              P.npbc == 3 && P.f_scale[0] == P.f_scale[1] && P.f_scale[1] == P.f_scale[2];
-          if (cut_scale > 0.0f) {
-            if (cubic)
-              pair_sweep_tab<true, true>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cut_scale,
-                                         acc_lj, acc_re);
-            else
-              pair_sweep_tab<false, true>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cut_scale,
-                                          acc_lj, acc_re);
-          } else if (cubic) {
-            pair_sweep_tab<true, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, 0.0f, acc_lj,
-                                        acc_re);
-          } else {
-            pair_sweep_tab<false, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, 0.0f, acc_lj,
-                                         acc_re);
-          }
-        } else if (P.single_image)
-          pair_sweep<true>(P, K, B, s_mt, s_mq, gn, b_lo + g0, c0, c1, b_lo, b_hi, acc_lj,
-                           acc_re);
-        else
-          pair_sweep<false>(P, K, B, s_mt, s_mq, gn, b_lo + g0, c0, c1, b_lo, b_hi, acc_lj,
-                            acc_re);
+        const bool cubic = tab == 1 && P.npbc == 3 && P.f_scale[0] == P.f_scale[1] &&
+                           P.f_scale[1] == P.f_scale[2];
+        const float cs = cut_scale;
+        if (!tab) {
+          acc = P.single_image
+                    ? pair_sweep<true>(P, B, s_mt, s_mq, gn, b_lo + g0, c0, c1, b_lo, b_hi)
+                    : pair_sweep<false>(P, B, s_mt, s_mq, gn, b_lo + g0, c0, c1, b_lo, b_hi);
+        } else if (cs > 0.0f) {
+          if (cubic)
+            acc = pair_sweep_tab<true, true, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+          else if (tab == 1)
+            acc = pair_sweep_tab<false, true, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+          else
+            acc = pair_sweep_tab<false, true, true>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+        } else if (cubic) {
+          acc = pair_sweep_tab<true, false, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+        } else if (tab == 1) {
+          acc = pair_sweep_tab<false, false, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+        } else {
+          acc = pair_sweep_tab<false, false, true>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+        }
+      } else if (tab) {
+        acc = cut_scale > 0.0f ? moved_pairs_tab<true, true>(P, B, s_h, b_lo, m, cut_scale)
+                               : moved_pairs_tab<false, true>(P, B, s_h, b_lo, m, cut_scale);
       } else {
         // pairs among the moved beads, each once (both trial / both current)
         const int lane = threadIdx.x & 31;
@@ -732,106 +896,29 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
           pair32(P, B.fpos[b_lo + a], B.fq[b_lo + a], B.fpos[b_lo + bb], B.fq[b_lo + bb], l0,
                  r0);
           // the moved beads are one molecule's: neighbours are bonded
-          if (!(P.pair_kind == 1 && bb == a + 1)) acc_lj += l1 - l0;
-          acc_re += r1 - r0;
+          if (!(P.pair_kind == 1 && bb == a + 1)) acc.x += l1 - l0;
+          acc.y += r1 - r0;
         }
       }
-      const float2 ab = block_sum32x2<kPairThreads>(acc_lj, acc_re, red);
+      const float2 ab = block_sum32x2<kPairThreads>(acc.x, acc.y, red);
       if (threadIdx.x == 0) {
         slots[2 * item] = (double)ab.x;
         slots[2 * item + 1] = (double)ab.y;
       }
     } else {
-      // a k item of up to kMaxKPerThread * kPairThreads vectors: thread t
-      // takes nq consecutive vectors k = tile * k_tile + t nq + q, so the
-      // moved beads' phase tables, built once per item, serve up to four
-      // vectors per thread, and vectors of one (nx, ny) column (n_z runs
-      // fastest in the k list) share the product e^{i(kx x + ky y)}: the
-      // phase of each is cmul(cmul(ex, ey), ez)
-      const int tile = local - s_np[r];
-      const int sk_pend = st->sk_pending, sk_buf = st->sk_buf, cur_buf = st->cur_buf;
-      const int nq = (kKTile32 + kPairThreads - 1) / kPairThreads;
-      int kk[kMaxKPerThread];
-      bool mine[kMaxKPerThread], col[kMaxKPerThread];
-      int ox[kMaxKPerThread], oy[kMaxKPerThread], oz[kMaxKPerThread];
-      bool ny[kMaxKPerThread], nz[kMaxKPerThread];
-      float2 ds[kMaxKPerThread];
-#pragma unroll
-      for (int q = 0; q < kMaxKPerThread; q++) {
-        const int t = threadIdx.x * nq + q;
-        kk[q] = tile * kKTile32 + t;
-        mine[q] = q < nq && t < kKTile32 && kk[q] < P.n_k;
-        const short4 kv = mine[q] ? B.kn[kk[q]] : make_short4(0, 0, 0, 0);
-        ox[q] = P.koff[0] + kv.x;
-        oy[q] = P.koff[1] + (kv.y >= 0 ? kv.y : -kv.y);
-        oz[q] = P.koff[2] + (kv.z >= 0 ? kv.z : -kv.z);
-        ny[q] = kv.y < 0;
-        nz[q] = kv.z < 0;
-        // a new (nx, ny) column: recompute the xy product
-        col[q] = q == 0 || ox[q] != ox[q - 1] || oy[q] != oy[q - 1] || ny[q] != ny[q - 1];
-        ds[q] = make_float2(0.0f, 0.0f);
-      }
-      float2* tabs = reinterpret_cast<float2*>(smem);
-      const int per = P.kper, chunk = P.kchunk_delta;
-      for (int c0 = b_lo; c0 < b_hi; c0 += chunk) {
-        const int cnt = min(chunk, b_hi - c0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < cnt * 6; t += blockDim.x) {
-          int bead = t / 6, which = (t / 3) & 1, axis = t % 3;
-          int4 f = which ? B.fpos[c0 + bead] : B.ftrial[c0 - b_lo + bead];
-          table32(P, f, B.fq[c0 + bead], axis, tabs + (bead * 2 + which) * per);
-        }
-        __syncthreads();
-        if (mine[0])
-          for (int bb = 0; bb < cnt; bb++) {
-            const float2* t1 = tabs + (bb * 2 + 0) * per;
-            const float2* t0 = t1 + per;
-            float2 xy1 = make_float2(0.0f, 0.0f), xy0 = xy1;
-#pragma unroll
-            for (int q = 0; q < kMaxKPerThread; q++)
-              if (mine[q]) {
-                if (col[q]) {
-                  float2 y1 = t1[oy[q]], y0 = t0[oy[q]];
-                  if (ny[q]) {
-                    y1.y = -y1.y;
-                    y0.y = -y0.y;
-                  }
-                  xy1 = cmul32(t1[ox[q]], y1);
-                  xy0 = cmul32(t0[ox[q]], y0);
-                }
-                float2 z1 = t1[oz[q]], z0 = t0[oz[q]];
-                if (nz[q]) {
-                  z1.y = -z1.y;
-                  z0.y = -z0.y;
-                }
-                const float2 e1 = cmul32(xy1, z1), e0 = cmul32(xy0, z0);
-                ds[q].x += e1.x - e0.x;
-                ds[q].y += e1.y - e0.y;
-              }
-          }
-      }
-      float e = 0.0f;
-#pragma unroll
-      for (int q = 0; q < kMaxKPerThread; q++)
-        if (mine[q]) {
-          const int k = kk[q];
-          double2 sv = B.sk[k];
-          if (sk_pend) {
-            const double2 pd = B.dsk[(size_t)sk_buf * P.n_k + k];
-            sv = make_double2(sv.x + pd.x, sv.y + pd.y);
-            B.sk[k] = sv;
-          }
-          const float2 d = ds[q];
-          B.dsk[(size_t)cur_buf * P.n_k + k] = make_double2((double)d.x, (double)d.y);
-          const float sx = (float)sv.x, sy = (float)sv.y;
-          e += (float)B.kw[k] * (2.0f * (sx * d.x + sy * d.y) + (d.x * d.x + d.y * d.y));
-        }
+      const int u0 = (local - s_np[r]) * kUnitsPer;
+      float e = k_item32(P, B, smem, smem_bytes, u0, min(kUnitsPer, P.n_ku - u0), b_lo, b_hi,
+                         st->sk_pending, st->sk_buf, st->cur_buf);
       e = block_sum32<kPairThreads>(e, red);
       if (threadIdx.x == 0) {
         slots[2 * item] = (double)e;
         slots[2 * item + 1] = 0.0;
       }
     }
+    __syncthreads();  // this item is done with the staging area and s_item
+    if (threadIdx.x == 0) s_item = next;
+    __syncthreads();
+    item = s_item;
   }
   // every block takes its last (empty) item before it counts itself out, so
   // the last one out knows that no block will read the queue again
@@ -841,12 +928,20 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
   }
 }
 
+constexpr int kKAreaBytes = 16 * 1024;
+
+int batch_delta_smem(const DevParams& P) {
+  const int k = P.use_ewald ? 2 * (P.kmax[2] + 1 + kKUnitsMost) * (int)sizeof(float2) : 0;
+  return std::max(kKAreaBytes, k);  // (the staged beads of a pair item take 2.2 KB)
+}
+
 void launch_batch_delta32(const DevParams* rp, const DevBuffers* rb, int n_rep, int* item_off,
                           double* slots, size_t smem, BatchTune tune, int* queue,
                           const float4* htab, float cut_scale, cudaStream_t s) {
   static bool attr = false;
   if (!attr) {
-    const int most = kKTableBytes + 4096 + kH32Bins * (int)sizeof(float4);
+    const int most = kKAreaBytes + 2 * (kMaxKmax + 1 + kKUnitsMost) * (int)sizeof(float2) +
+                     kH32Bins * (int)sizeof(float4) + (2 * kMaxReplicas + 1) * (int)sizeof(int);
     cudaFuncSetAttribute(k_batch_delta32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_batch_delta32<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_batch_delta32<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
@@ -855,16 +950,18 @@ void launch_batch_delta32(const DevParams* rp, const DevBuffers* rb, int n_rep, 
   const int grid = tune.grid > 0 ? tune.grid : pair_grid32();
   if (!tune.htab) htab = nullptr;
   if (!htab) cut_scale = 0.0f;
+  const int area = (int)smem;
   if (htab) smem += kH32Bins * sizeof(float4);
+  smem += (2 * (size_t)n_rep + 1) * sizeof(int);
   if (tune.min_blocks == 4)
     k_batch_delta32<4><<<grid, kPairThreads, smem, s>>>(rp, rb, n_rep, item_off, slots, tune,
-                                                        queue, htab, cut_scale);
+                                                        queue, htab, cut_scale, area);
   else if (tune.min_blocks == 3)
     k_batch_delta32<3><<<grid, kPairThreads, smem, s>>>(rp, rb, n_rep, item_off, slots, tune,
-                                                        queue, htab, cut_scale);
+                                                        queue, htab, cut_scale, area);
   else
     k_batch_delta32<2><<<grid, kPairThreads, smem, s>>>(rp, rb, n_rep, item_off, slots, tune,
-                                                        queue, htab, cut_scale);
+                                                        queue, htab, cut_scale, area);
 }
 
 __global__ void k_fix_all(const DevParams P, const DevBuffers B) {
