@@ -164,6 +164,12 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
     two = two && rc < E.ebox[a] && in.alpha * 0.25 * E.ebox[a] * E.ebox[a] >= std::ldexp(1.0, kH32ELo);
   }
   P.images = P.single_image ? 1 : (two ? 2 : 0);
+  P.two_axes = 0;
+  for (int a = 0; a < 3; a++) {
+    const double La = E.ebox[a], Lb = E.ebox[(a + 1) % 3];
+    if (rc > 0.5 * La && rc > 0.5 * Lb && rc * rc * 1.0001 >= 0.25 * (La * La + Lb * Lb))
+      P.two_axes = 1;
+  }
   P.lB = in.lB;
   P.sqrt_alpha = std::sqrt(in.alpha);
   P.alpha = in.alpha;
@@ -656,6 +662,10 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     P.f_lj_eref[k] = (float)P.lj_eref[k];
     P.f_hs_sum[k] = (float)P.hs_sum[k];
   }
+  P.f_lj_max2 = P.use_pair ? 1e-30f : 0.0f;
+  if (P.use_pair)
+    for (int k = 0; k < P.n_type * P.n_type; k++)
+      P.f_lj_max2 = std::max(P.f_lj_max2, P.f_lj_rc2[k]);
   P.f_real_cut = (float)P.real_cut;
   P.f_sqrt_alpha = (float)P.sqrt_alpha;
   P.f_lB = (float)P.lB;

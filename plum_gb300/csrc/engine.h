@@ -96,6 +96,8 @@ struct DevParams {
   float f_img[3];        // f_box of the axes with two images in range, else past kNoImage
   float f_lj_sig2[kMaxT2], f_lj_eps4[kMaxT2], f_lj_rc2[kMaxT2], f_lj_eref[kMaxT2];
   float f_real_cut, f_sqrt_alpha, f_lB;
+  float f_lj_max2;       // largest f_lj_rc2 (tiny, but not 0, where none is larger; 0: no pairs)
+  int two_axes;          // images of two axes at once can lie inside f_real_cut
   double inv_fix[3];     // 2^32 / Ewald box length (FP64 -> fixed point)
   // cell list of the surrogate descriptor (replica batches, precision form,
   // periodic on every axis): cell_nc cells per axis, each at least the
@@ -371,17 +373,16 @@ void build_h32_table(float4* out, double scale = 1.0, double cut = 0.0);  // kH3
 constexpr int kMinItemPairs = 1024;  // smallest item the slot buffers are sized for
 constexpr int kMinKTile = 64;
 // Pair items of the batched energy change: up to kPairGroup moved beads
-// (staged in shared memory) x a chunk of other beads (one per thread, a
-// multiple of the block size); one more item per move takes the pairs among
-// the moved beads.
+// (staged in shared memory) x a chunk of other beads; one more item per move takes
+// the pairs among the moved beads.
 constexpr int kPairGroup = 32;
-// Other beads per pair item: item_pairs over the staged group, the group
-// counted as the table loop stages it (padded to a multiple of 4), so that an
-// item of a one-bead move is no longer than a chain move's.
+// Other beads per pair item: item_pairs over the staged group, in steps of 64; a group
+// of a few beads counted as 4, so that an item of a one-bead move is no longer than a
+// chain move's.
 __host__ __device__ inline int pair_chunk(int m, int item_pairs) {
-  const int g = m < kPairGroup ? ((m > 0 ? m : 1) + 3) & ~3 : kPairGroup;
-  const int c = (item_pairs / g + kPairThreads - 1) / kPairThreads * kPairThreads;
-  return c > kPairThreads ? c : kPairThreads;
+  const int g = m < 4 ? 4 : (m < kPairGroup ? m : kPairGroup);
+  const int c = (item_pairs / g + 63) / 64 * 64;
+  return c > kPairThreads ? c / kPairThreads * kPairThreads : c;
 }
 __host__ __device__ inline int pair_item_count(int m, int n_bead, int item_pairs) {
   if (m <= 0) return 0;

@@ -39,12 +39,12 @@ constexpr int kH32LoBits = (127 + kH32ELo) << 23;  // float bits of 2^kH32ELo
 // float bits of u: the exponent and top five mantissa bits pick the bin, the
 // remaining 18 bits are the bin-local fraction f; placed under the exponent
 // of 1 they make the float 1 + f/32 exactly, and w = f/32 is exact too. The
-// bin's cubic is in w. Bins outside the table are clamped to the last one
-// (one unsigned minimum; a u below the table wraps to a huge index): the
-// caller replaces values below the table, and values above it are cut off.
-__device__ __forceinline__ float h32_tab(const float4* tab, int bits) {
-  const unsigned idx = min((unsigned)((bits >> 18) - ((127 + kH32ELo) << 5)),
-                           (unsigned)(kH32Bins - 1));
+// bin's cubic is in w. Bins past `last` are clamped to it (one unsigned
+// minimum; a u below the table wraps to a huge index): the caller replaces
+// values below the table, and values above it are cut off.
+__device__ __forceinline__ float h32_tab(const float4* tab, int bits,
+                                         unsigned last = kH32Bins - 1) {
+  const unsigned idx = min((unsigned)((bits >> 18) - ((127 + kH32ELo) << 5)), last);
   const float4 c = tab[idx];
   const float w = __int_as_float((bits & 0x3FFFF) | 0x3F800000) - 1.0f;
   return fmaf(fmaf(fmaf(c.w, w, c.z), w, c.y), w, c.x);

@@ -26,24 +26,11 @@
 
 namespace plum {
 
-template <int NT>
-__device__ __forceinline__ float block_sum32(float v, float* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  float t = 0.0f;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < NT / 32; i++) t += sh[i];
-  return t;
-}
-
-// Two sums at once (one pair of barriers); each value is added in
-// block_sum32's order, so the results are the same bits as two calls.
-// sh: 2 NT / 32 floats. Valid in thread 0.
+// Two sums of a block's values at once, one barrier pair; valid in thread 0. sh:
+// 2 NT / 32 floats.
 template <int NT>
 __device__ __forceinline__ float2 block_sum32x2(float a, float b, float* sh) {
+  static_assert(NT / 32 <= 16, "the warps' sums of both values in one warp");
   for (int o = 16; o > 0; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
@@ -55,13 +42,14 @@ __device__ __forceinline__ float2 block_sum32x2(float a, float b, float* sh) {
     sh[NT / 32 + w] = b;
   }
   __syncthreads();
-  float2 t = make_float2(0.0f, 0.0f);
-  if (threadIdx.x == 0)
-    for (int i = 0; i < NT / 32; i++) {
-      t.x += sh[i];
-      t.y += sh[NT / 32 + i];
-    }
-  return t;
+  float t = 0.0f;
+  if (w == 0) {
+    t = l < 2 * (NT / 32) ? sh[l] : 0.0f;
+    for (int o = NT / 64; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    a = t;
+    b = __shfl_sync(0xffffffffu, t, NT / 32);
+  }
+  return make_float2(a, b);
 }
 
 // ---------------------------------------------------------------- pair evaluation
@@ -70,7 +58,9 @@ __device__ __forceinline__ float2 block_sum32x2(float a, float b, float* sh) {
 struct TabPair {
   float2 sx, sy, sz, ua;     // scales; table variable per r^2
   float rc2, ljlim, cs, ius; // cut-off; largest LJ cut-off^2; u per table variable
+  unsigned last;             // the cut-off's bin: lanes beyond it share one address
   float bx, by, bz;          // DevParams::f_img
+  int two;                   // DevParams::two_axes
 };
 
 // kCubic (equal fixed-point scales on the three axes): r^2 stays in fixed-point units
@@ -88,13 +78,13 @@ __device__ __forceinline__ TabPair tab_pair(const DevParams& P, float cut_scale)
   const float ua = P.f_sqrt_alpha * P.f_sqrt_alpha * K.cs * (kCut ? cut_scale : 1.0f);
   K.ua = make_float2(ua, ua);
   K.ius = kCut ? 1.0f / cut_scale : 1.0f;
-  float m = P.use_pair ? 1e-30f : 0.0f;  // r2 = 0 (coincident beads) must reach lj32
-  if (P.use_pair)
-    for (int k = 0; k < P.n_type * P.n_type; k++) m = fmaxf(m, P.f_lj_rc2[k]);
-  K.ljlim = m * ics;
+  const int cut = __float_as_int(kCut ? (float)kH32Cut : K.rc2 * ua);
+  K.last = max(0, min(kH32Bins - 1, (cut >> 18) - ((127 + kH32ELo) << 5)));
+  K.ljlim = P.f_lj_max2 * ics;
   K.bx = P.f_img[0];
   K.by = P.f_img[1];
   K.bz = P.f_img[2];
+  K.two = P.two_axes;
   return K;
 }
 
@@ -104,7 +94,7 @@ template <bool kCut, bool kNear>
 __device__ __forceinline__ float tab_diff(const TabPair& K, const float4* s_h, float2 r) {
   const float2 u = __fmul2_rn(r, K.ua);
   const int b1 = __float_as_int(u.x), b0 = __float_as_int(u.y);
-  float h1 = h32_tab(s_h, b1), h0 = h32_tab(s_h, b0);
+  float h1 = h32_tab(s_h, b1, K.last), h0 = h32_tab(s_h, b0, K.last);
   if (kNear && min(b1, b0) < kH32LoBits) {
     if (b1 < kH32LoBits) h1 = h32_small(u.x * K.ius);
     if (b0 < kH32LoBits) h0 = h32_small(u.y * K.ius);
@@ -126,13 +116,15 @@ __device__ __forceinline__ float2 flip2(float b, float2 d) {
 }
 
 // The real-space change (in units of lB sqrt(alpha) q q') of staged bead (t trial, c
-// current) with other bead (ot, oc), and the LJ change where lj is set. kImg (r_c below
-// every box length): an axis has at most one more image in range, the one on the other
-// side; with r_c under 0.7 L two axes at once never do, so those are behind a branch.
+// current) with other bead (ot, oc), and the LJ change. kImg (r_c below every box
+// length): an axis has at most one more image in range, the one on the other side, and
+// two axes at once have one only where r_c reaches past half a face's diagonal. (Leaving
+// out the lookups of neutral staged beads, a branch per bead, gained nothing on brushes
+// with 13 to 77 % of their beads charged and cost 5 % on a fully charged system.)
 template <bool kCubic, bool kCut, bool kImg>
 __device__ __forceinline__ float tab_eval(const DevParams& P, const TabPair& K, const float4* s_h,
                                           const int4 t, const int4 c, const int4 ot, const int4 oc,
-                                          int k, bool lj, float& acc_lj) {
+                                          int k, float& acc_lj) {
   float2 dx = make_float2((float)(int)((unsigned)ot.x - (unsigned)t.x),
                           (float)(int)((unsigned)oc.x - (unsigned)c.x));
   float2 dy = make_float2((float)(int)((unsigned)ot.y - (unsigned)t.y),
@@ -146,22 +138,24 @@ __device__ __forceinline__ float tab_eval(const DevParams& P, const TabPair& K, 
   }
   if (!kImg) {
     const float2 r = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    if (lj && fminf(r.x, r.y) < K.ljlim)
+    if (fminf(r.x, r.y) < K.ljlim)
       acc_lj += lj32(P, k, r.x * K.cs) - lj32(P, k, r.y * K.cs);
     return tab_diff<kCut, true>(K, s_h, r);
   }
   const float2 xx = sq2(dx), yy = sq2(dy), zz = sq2(dz);
   const float2 r = add3(xx, yy, zz);
-  if (lj && fminf(r.x, r.y) < K.ljlim) acc_lj += lj32(P, k, r.x) - lj32(P, k, r.y);
+  if (fminf(r.x, r.y) < K.ljlim) acc_lj += lj32(P, k, r.x) - lj32(P, k, r.y);
   float h = tab_diff<kCut, true>(K, s_h, r);
   const float2 fx = sq2(flip2(K.bx, dx)), fy = sq2(flip2(K.by, dy)), fz = sq2(flip2(K.bz, dz));
   if (K.bx < kNoImage) h += tab_diff<kCut, false>(K, s_h, add3(fx, yy, zz));
   if (K.by < kNoImage) h += tab_diff<kCut, false>(K, s_h, add3(xx, fy, zz));
   if (K.bz < kNoImage) h += tab_diff<kCut, false>(K, s_h, add3(xx, yy, fz));
-  const float2 xy = add3(fx, fy, zz), xz = add3(fx, yy, fz), yz = add3(xx, fy, fz);
-  if (fminf(fminf(fminf(xy.x, xy.y), fminf(xz.x, xz.y)), fminf(yz.x, yz.y)) <= K.rc2) {
-    h += tab_diff<kCut, false>(K, s_h, xy) + tab_diff<kCut, false>(K, s_h, xz);
-    h += tab_diff<kCut, false>(K, s_h, yz) + tab_diff<kCut, false>(K, s_h, add3(fx, fy, fz));
+  if (K.two) {
+    const float2 xy = add3(fx, fy, zz), xz = add3(fx, yy, fz), yz = add3(xx, fy, fz);
+    if (fminf(fminf(fminf(xy.x, xy.y), fminf(xz.x, xz.y)), fminf(yz.x, yz.y)) <= K.rc2) {
+      h += tab_diff<kCut, false>(K, s_h, xy) + tab_diff<kCut, false>(K, s_h, xz);
+      h += tab_diff<kCut, false>(K, s_h, yz) + tab_diff<kCut, false>(K, s_h, add3(fx, fy, fz));
+    }
   }
   return h;
 }
@@ -240,7 +234,7 @@ __device__ __forceinline__ void sweep32(const DevParams& P, const DevBuffers& B,
       for (int u = u0; u < u1; u++) {
         const int4 t = st[u].t, c = st[u].c;
         acc = fmaf(__int_as_float(t.w),
-                   tab_eval<false, false, kImg>(P, K, s_h, t, c, o1, o0, c.w + o0.w, true, acc_lj),
+                   tab_eval<false, false, kImg>(P, K, s_h, t, c, o1, o0, c.w + o0.w, acc_lj),
                    acc);
       }
       acc_re = fmaf(qj, acc, acc_re);
@@ -467,10 +461,7 @@ __device__ __forceinline__ PairConst pair_const(const DevParams& P) {
   K.nt = P.n_type;
   K.use_pair = P.use_pair;
   K.use_ewald = P.use_ewald;
-  // r2 = 0 (coincident beads) must reach lj32, which returns the overlap value
-  float m2 = 1e-30f;
-  for (int k = 0; k < P.n_type * P.n_type; k++) m2 = fmaxf(m2, P.f_lj_rc2[k]);
-  K.ljmax2 = m2;
+  K.ljmax2 = P.f_lj_max2;
   return K;
 }
 
@@ -527,41 +518,37 @@ __device__ __forceinline__ float2 pair_sweep(const DevParams& P, const DevBuffer
 // ------------------------------------------------ table-driven real space
 // pair_sweep for LJ + Ewald from the h(u) table: per (moved u, other j) the trial and
 // current distances share the other bead's load, one LJ pre-test and the packed
-// (two-lane FP32) arithmetic of r^2 and u, so a warp runs no divergent erfc. Each
-// thread takes two other beads per staged bead, so one load of the staged trial and
-// current entries serves four evaluations; the other bead's charge multiplies its sum
-// once, after the staged beads. gn4 staged beads, a multiple of 4; the trial entry's w
-// holds the staged bead's charge (float bits) and the current entry's w its type; the
-// padding beads have q = 0 and equal trial and current positions, so they add exactly
-// zero. kCut: the table is the batch's cut table (variable u' = cut_scale u, zero from
-// the cut-off on), so the cut-off costs nothing.
+// (two-lane FP32) arithmetic of r^2 and u, so a warp runs no divergent erfc. A thread
+// takes one other bead; in an item of fewer others than threads, several threads share
+// the staged beads of each. The trial entry's w holds the staged bead's charge (float
+// bits) and the current entry's w its type; the other bead's charge multiplies its sum
+// once, after the staged beads. kCut: the table is the batch's cut table (variable
+// u' = cut_scale u, zero from the cut-off on), so the cut-off costs nothing.
 template <bool kCubic, bool kCut, bool kImg>
 __device__ __forceinline__ float2 pair_sweep_tab(const DevParams& P, const DevBuffers& B,
-                                              const int4* s_mt, const float4* s_h, int gn4,
-                                              int c0, int c1, int b_lo, int b_hi,
-                                              float cut_scale) {
+                                                 const int4* s_mt, const float4* s_h, int gn,
+                                                 int chunk, int c0, int c1, int b_lo, int b_hi,
+                                                 float cut_scale) {
   float acc_lj = 0.0f, acc_re = 0.0f;
   const TabPair K = tab_pair<kCubic, kCut>(P, cut_scale);
   const float pref = P.f_lB * P.f_sqrt_alpha;
   const int nt = P.n_type;
-  for (int j0 = c0 + threadIdx.x; j0 < c1; j0 += 2 * kPairThreads) {
-    const int j1 = j0 + kPairThreads;
-    const bool ok0 = !(j0 >= b_lo && j0 < b_hi);  // moved pairs: the last item
-    const bool ok1 = j1 < c1 && !(j1 >= b_lo && j1 < b_hi);
-    const int4 o0 = B.fpos[j0];
-    const int4 o1 = j1 < c1 ? B.fpos[j1] : o0;
-    const float q0 = ok0 ? B.fq[j0] * pref : 0.0f;
-    const float q1 = ok1 ? B.fq[j1] * pref : 0.0f;
-    float a0 = 0.0f, a1 = 0.0f;
+  const int per = min(chunk, kPairThreads), split = kPairThreads / per;
+  const int sub = (int)threadIdx.x / per;
+  const int u0 = gn * sub / split, u1 = sub < split ? gn * (sub + 1) / split : u0;
+  for (int j = c0 + (int)threadIdx.x - sub * per; j < c1; j += per) {
+    if (j >= b_lo && j < b_hi) continue;  // moved pairs: the last item
+    const int4 o = B.fpos[j];
+    const float q = B.fq[j] * pref;
+    float a = 0.0f;
 #pragma unroll(kImg ? 2 : 4)
-    for (int u = 0; u < gn4; u++) {
+    for (int u = u0; u < u1; u++) {
       const int4 t = s_mt[u], c = s_mt[kPairGroup + u];
-      const float q = __int_as_float(t.w);
-      const int k = c.w * nt;
-      a0 = fmaf(q, tab_eval<kCubic, kCut, kImg>(P, K, s_h, t, c, o0, o0, k + o0.w, ok0, acc_lj), a0);
-      a1 = fmaf(q, tab_eval<kCubic, kCut, kImg>(P, K, s_h, t, c, o1, o1, k + o1.w, ok1, acc_lj), a1);
+      a = fmaf(__int_as_float(t.w),
+               tab_eval<kCubic, kCut, kImg>(P, K, s_h, t, c, o, o, c.w * nt + o.w, acc_lj),
+               a);
     }
-    acc_re = fmaf(q0, a0, fmaf(q1, a1, acc_re));
+    acc_re = fmaf(q, a, acc_re);
   }
   return make_float2(acc_lj, acc_re);
 }
@@ -587,7 +574,7 @@ __device__ __forceinline__ float2 moved_pairs_tab(const DevParams& P, const DevB
     }
     const int4 c = B.fpos[b_lo + a], oc = B.fpos[b_lo + b];
     const float h = tab_eval<false, kCut, kImg>(P, K, s_h, B.ftrial[a], c, B.ftrial[b], oc,
-                                                c.w * P.n_type + oc.w, true, acc_lj);
+                                                c.w * P.n_type + oc.w, acc_lj);
     acc_re = fmaf(B.fq[b_lo + a] * B.fq[b_lo + b] * pref, h, acc_re);
   }
   return make_float2(acc_lj, acc_re);
@@ -637,11 +624,10 @@ void build_h32_table(float4* out, double scale, double cut) {
 }
 
 // ------------------------------------------------------------ replicas
-constexpr int kKUnitsMost = 512;  // k units of a k item (k_tile <= 1024)
-constexpr int kKPer = kKUnitsMost / kPairThreads;
+constexpr int kKUnitsMost = kPairThreads;  // most k units of a k item
 
-// dS(k), the S(k) commit and the |S|^2 change of up to 512 units [u0, u0 + un). A thread
-// takes one unit and every slices-th moved bead, or two units and all of them. smem:
+// dS(k), the S(k) commit and the |S|^2 change of units [u0, u0 + un), at most
+// kKUnitsMost. A thread takes one unit and every slices-th moved bead. smem:
 // e^{i nz theta_z} of as many moved beads (trial and current) as fit, then their xy
 // parts per (nx, ny) column, every entry one thread's, from its exact integer phase.
 // (A vector's phase as a product of three table entries, the tables built by six
@@ -653,25 +639,17 @@ __device__ __forceinline__ float k_item32(const DevParams& P, const DevBuffers& 
   __shared__ short2 s_col[kKUnitsMost];
   __shared__ float s_sum[4][kPairThreads];
   __shared__ int s_zmax;
-  const int slices = un < kPairThreads ? kPairThreads / un : 1;
-  const int t0 = slices > 1 ? (int)threadIdx.x % un : (int)threadIdx.x;
-  const int sl = slices > 1 ? (int)threadIdx.x / un : 0;
-  KUnit ku[kKPer];
-  float2 A[kKPer], Bs[kKPer];
+  const int slices = kPairThreads / un;
+  const int u = (int)threadIdx.x % un, sl = (int)threadIdx.x / un;
+  const KUnit ku = B.ku[u0 + u];
   const int col0 = B.ku[u0].col;
-  const int ncol = ((B.ku[u0 + un - 1].col - col0) & 0xFFFF) + 1;
+  const int ncol = ((B.ku[u0 + un - 1].col - col0) & 0xFFFF) + 1, col = (ku.col - col0) & 0xFFFF;
   if (threadIdx.x == 0) s_zmax = 0;
   __syncthreads();
-#pragma unroll
-  for (int q = 0; q < kKPer; q++) {
-    const int u = t0 + q * kPairThreads;
-    ku[q] = u < un && sl < slices ? B.ku[u0 + u] : KUnit{0, 0, 0, B.ku[u0].col, -1, -1};
-    A[q] = Bs[q] = make_float2(0.0f, 0.0f);
-    const int zw = __reduce_max_sync(0xffffffffu, (int)ku[q].nz);
-    if ((threadIdx.x & 31) == 0 && zw > 0) atomicMax(&s_zmax, zw);
-    ku[q].col = (unsigned short)(ku[q].col - col0);
-    if (u < un && sl == 0) s_col[ku[q].col] = make_short2(ku[q].nx, ku[q].ny);
-  }
+  const int zw = __reduce_max_sync(0xffffffffu, (int)ku.nz);
+  if ((threadIdx.x & 31) == 0 && zw > 0) atomicMax(&s_zmax, zw);
+  if (sl == 0) s_col[col] = make_short2(ku.nx, ku.ny);
+  float2 A = make_float2(0.0f, 0.0f), Bs = A;
   __syncthreads();
   const int nz = s_zmax + 1, ne = nz + ncol;
   const int kb = min(64, smem_bytes / (2 * ne * (int)sizeof(float2)));
@@ -695,52 +673,46 @@ __device__ __forceinline__ float k_item32(const DevParams& P, const DevBuffers& 
       }
     }
     __syncthreads();
-    if (sl < slices)
-#pragma unroll
-      for (int q = 0; q < kKPer; q++)
-        if (t0 + q * kPairThreads < un)
-          for (int it = sl; it < nt; it += slices) {
-            const float2 xy = s_xy[it * ncol + ku[q].col], ez = s_z[it * nz + ku[q].nz];
-            A[q].x = fmaf(xy.x, ez.x, A[q].x);
-            A[q].y = fmaf(xy.y, ez.x, A[q].y);
-            Bs[q].x = fmaf(xy.x, ez.y, Bs[q].x);
-            Bs[q].y = fmaf(xy.y, ez.y, Bs[q].y);
-          }
-  }
-  if (slices > 1) {  // the slices of each (unit, sum), added in order
-    s_sum[0][threadIdx.x] = A[0].x;
-    s_sum[1][threadIdx.x] = A[0].y;
-    s_sum[2][threadIdx.x] = Bs[0].x;
-    s_sum[3][threadIdx.x] = Bs[0].y;
-    __syncthreads();
-    if (sl == 0)
-      for (int w = 1; w < slices; w++) {
-        A[0].x += s_sum[0][w * un + t0];
-        A[0].y += s_sum[1][w * un + t0];
-        Bs[0].x += s_sum[2][w * un + t0];
-        Bs[0].y += s_sum[3][w * un + t0];
+    if (sl < slices) {
+#pragma unroll 4
+      for (int it = sl; it < nt; it += slices) {
+        const float2 xy = s_xy[it * ncol + col], ez = s_z[it * nz + ku.nz];
+        A.x = fmaf(xy.x, ez.x, A.x);
+        A.y = fmaf(xy.y, ez.x, A.y);
+        Bs.x = fmaf(xy.x, ez.y, Bs.x);
+        Bs.y = fmaf(xy.y, ez.y, Bs.y);
       }
+    }
   }
+  s_sum[0][threadIdx.x] = A.x;
+  s_sum[1][threadIdx.x] = A.y;
+  s_sum[2][threadIdx.x] = Bs.x;
+  s_sum[3][threadIdx.x] = Bs.y;
+  __syncthreads();
+  // slices 0 and 1: +nz and -nz (one thread for both where there is one slice)
   float e = 0.0f;
-  if (sl == 0)
-#pragma unroll
-    for (int q = 0; q < kKPer; q++)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {  // +nz, -nz (neither, past the last unit)
-        const int k = h ? ku[q].km : ku[q].kp;
-        if (k < 0) continue;
-        const float2 ds = h ? make_float2(A[q].x + Bs[q].y, A[q].y - Bs[q].x)
-                            : make_float2(A[q].x - Bs[q].y, A[q].y + Bs[q].x);
-        double2 s = B.sk[k];
-        if (sk_pend) {
-          const double2 p = B.dsk[(size_t)sk_buf * P.n_k + k];
-          s = make_double2(s.x + p.x, s.y + p.y);
-          B.sk[k] = s;
-        }
-        B.dsk[(size_t)cur_buf * P.n_k + k] = make_double2((double)ds.x, (double)ds.y);
-        const float sx = (float)s.x, sy = (float)s.y;
-        e += (float)B.kw[k] * (2.0f * (sx * ds.x + sy * ds.y) + (ds.x * ds.x + ds.y * ds.y));
-      }
+  if (sl > 1 || sl >= slices) return e;
+  A = Bs = make_float2(0.0f, 0.0f);
+  for (int w = 0; w < slices; w++) {  // the slices of each (unit, sum), added in order
+    A.x += s_sum[0][w * un + u];
+    A.y += s_sum[1][w * un + u];
+    Bs.x += s_sum[2][w * un + u];
+    Bs.y += s_sum[3][w * un + u];
+  }
+  for (int h = sl; h < 2; h += slices > 1 ? 2 : 1) {
+    const int k = h ? ku.km : ku.kp;
+    if (k < 0) continue;
+    const float2 ds = h ? make_float2(A.x + Bs.y, A.y - Bs.x) : make_float2(A.x - Bs.y, A.y + Bs.x);
+    double2 s = B.sk[k];
+    if (sk_pend) {
+      const double2 p = B.dsk[(size_t)sk_buf * P.n_k + k];
+      s = make_double2(s.x + p.x, s.y + p.y);
+      B.sk[k] = s;
+    }
+    B.dsk[(size_t)cur_buf * P.n_k + k] = make_double2((double)ds.x, (double)ds.y);
+    const float sx = (float)s.x, sy = (float)s.y;
+    e += (float)B.kw[k] * (2.0f * (sx * ds.x + sy * ds.y) + (ds.x * ds.x + ds.y * ds.y));
+  }
   return e;
 }
 
@@ -763,13 +735,15 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
                     int n_rep, int* __restrict__ item_off, double* __restrict__ slots,
                     BatchTune tune, int* __restrict__ queue, const float4* __restrict__ htab,
                     float cut_scale, int smem_bytes) {
-  const int kItemPairs = tune.item_pairs, kUnitsPer = tune.k_tile / 2;
+  const int kItemPairs = tune.item_pairs, kUnitsPer = min(tune.k_tile / 2, kKUnitsMost);
   extern __shared__ __align__(16) unsigned char smem_all[];
   // the staging / k-table area, the h(u) table where there is one, the item counts
   unsigned char* smem = smem_all;
   float4* s_h = reinterpret_cast<float4*>(smem_all + smem_bytes);
   int* s_pref = reinterpret_cast<int*>(s_h + (htab ? kH32Bins : 0));  // [n_rep + 1]
   int* s_np = s_pref + n_rep + 1;                                     // [n_rep]
+  int* s_lo = s_np + n_rep;                                           // [n_rep]
+  int* s_m = s_lo + n_rep;                                            // [n_rep]
   if (htab)
     for (int i = threadIdx.x; i < kH32Bins; i += blockDim.x) s_h[i] = htab[i];
   __shared__ float red[2 * (kPairThreads / 32)];
@@ -783,6 +757,8 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
     const int np = (pr.use_pair || pr.use_ewald) ? pair_item_count(m, pr.n_bead, kItemPairs) : 0;
     const int nk = (pr.use_ewald && m > 0) ? (pr.n_ku + kUnitsPer - 1) / kUnitsPer : 0;
     s_np[r] = np;
+    s_lo[r] = st->b_lo;
+    s_m[r] = m;
     s_pref[r + 1] = np + nk;
   }
   __syncthreads();
@@ -828,8 +804,7 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
     const int r = lo;
     const DevParams& P = rp[r];
     const DevBuffers& B = rb[r];
-    const DevState* st = B.state;
-    const int b_lo = st->b_lo, b_hi = st->b_hi, m = b_hi - b_lo, N = P.n_bead;
+    const int b_lo = s_lo[r], m = s_m[r], b_hi = b_lo + m, N = P.n_bead;
     const int local = item - s_pref[r];
     if (local < s_np[r]) {
       float2 acc = make_float2(0.0f, 0.0f);  // LJ, real space
@@ -842,24 +817,15 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
         const int c0 = (local % n_chunk) * chunk, c1 = min(N, c0 + chunk);
         int4* s_mt = reinterpret_cast<int4*>(smem);  // trial, then current
         float* s_mq = reinterpret_cast<float*>(s_mt + 2 * kPairGroup);
-        // the table path pads the staged beads to a multiple of 4 with the
-        // last bead's current position at both places and q = 0
-        const int gn4 = tab ? (gn + 3) & ~3 : gn;
         // (the barriers at the end of the item loop: every thread is done
         // with the previous item's staging area)
-        for (int u = threadIdx.x; u < gn4; u += kPairThreads) {
-          if (u < gn) {
-            int4 t = B.ftrial[g0 + u];
-            if (tab) t.w = __float_as_int(B.fq[b_lo + g0 + u]);  // the type stays in c.w
-            s_mt[u] = t;
-            s_mt[kPairGroup + u] = B.fpos[b_lo + g0 + u];
-            s_mq[u] = B.fq[b_lo + g0 + u];
-          } else {
-            const int4 p = B.fpos[b_lo + g0 + gn - 1];
-            s_mt[u] = make_int4(p.x, p.y, p.z, __float_as_int(0.0f));
-            s_mt[kPairGroup + u] = p;
-            s_mq[u] = 0.0f;
-          }
+        for (int u = threadIdx.x; u < gn; u += kPairThreads) {
+          const float q = B.fq[b_lo + g0 + u];
+          int4 t = B.ftrial[g0 + u];
+          if (tab) t.w = __float_as_int(q);  // the type stays in c.w
+          s_mt[u] = t;
+          s_mt[kPairGroup + u] = B.fpos[b_lo + g0 + u];
+          s_mq[u] = q;
         }
         __syncthreads();
         const bool cubic = tab == 1 && P.npbc == 3 && P.f_scale[0] == P.f_scale[1] &&
@@ -871,17 +837,23 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
                     : pair_sweep<false>(P, B, s_mt, s_mq, gn, b_lo + g0, c0, c1, b_lo, b_hi);
         } else if (cs > 0.0f) {
           if (cubic)
-            acc = pair_sweep_tab<true, true, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+            acc = pair_sweep_tab<true, true, false>(P, B, s_mt, s_h, gn, chunk, c0, c1, b_lo, b_hi,
+                                                    cs);
           else if (tab == 1)
-            acc = pair_sweep_tab<false, true, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+            acc = pair_sweep_tab<false, true, false>(P, B, s_mt, s_h, gn, chunk, c0, c1, b_lo, b_hi,
+                                                     cs);
           else
-            acc = pair_sweep_tab<false, true, true>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+            acc = pair_sweep_tab<false, true, true>(P, B, s_mt, s_h, gn, chunk, c0, c1, b_lo, b_hi,
+                                                    cs);
         } else if (cubic) {
-          acc = pair_sweep_tab<true, false, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+          acc = pair_sweep_tab<true, false, false>(P, B, s_mt, s_h, gn, chunk, c0, c1, b_lo, b_hi,
+                                                   cs);
         } else if (tab == 1) {
-          acc = pair_sweep_tab<false, false, false>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+          acc = pair_sweep_tab<false, false, false>(P, B, s_mt, s_h, gn, chunk, c0, c1, b_lo, b_hi,
+                                                    cs);
         } else {
-          acc = pair_sweep_tab<false, false, true>(P, B, s_mt, s_h, gn4, c0, c1, b_lo, b_hi, cs);
+          acc = pair_sweep_tab<false, false, true>(P, B, s_mt, s_h, gn, chunk, c0, c1, b_lo, b_hi,
+                                                   cs);
         }
       } else if (tab) {
         acc = cut_scale > 0.0f ? moved_pairs_tab<true, true>(P, B, s_h, b_lo, m, cut_scale)
@@ -907,11 +879,12 @@ __global__ void __launch_bounds__(kPairThreads, kMinBlocks)
       }
     } else {
       const int u0 = (local - s_np[r]) * kUnitsPer;
-      float e = k_item32(P, B, smem, smem_bytes, u0, min(kUnitsPer, P.n_ku - u0), b_lo, b_hi,
+      const DevState* st = B.state;
+      const float e = k_item32(P, B, smem, smem_bytes, u0, min(kUnitsPer, P.n_ku - u0), b_lo, b_hi,
                          st->sk_pending, st->sk_buf, st->cur_buf);
-      e = block_sum32<kPairThreads>(e, red);
+      const float2 ek = block_sum32x2<kPairThreads>(e, 0.0f, red);
       if (threadIdx.x == 0) {
-        slots[2 * item] = (double)e;
+        slots[2 * item] = (double)ek.x;
         slots[2 * item + 1] = 0.0;
       }
     }
@@ -941,7 +914,7 @@ void launch_batch_delta32(const DevParams* rp, const DevBuffers* rb, int n_rep, 
   static bool attr = false;
   if (!attr) {
     const int most = kKAreaBytes + 2 * (kMaxKmax + 1 + kKUnitsMost) * (int)sizeof(float2) +
-                     kH32Bins * (int)sizeof(float4) + (2 * kMaxReplicas + 1) * (int)sizeof(int);
+                     kH32Bins * (int)sizeof(float4) + (4 * kMaxReplicas + 1) * (int)sizeof(int);
     cudaFuncSetAttribute(k_batch_delta32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_batch_delta32<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_batch_delta32<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
@@ -952,7 +925,7 @@ void launch_batch_delta32(const DevParams* rp, const DevBuffers* rb, int n_rep, 
   if (!htab) cut_scale = 0.0f;
   const int area = (int)smem;
   if (htab) smem += kH32Bins * sizeof(float4);
-  smem += (2 * (size_t)n_rep + 1) * sizeof(int);
+  smem += (4 * (size_t)n_rep + 1) * sizeof(int);
   if (tune.min_blocks == 4)
     k_batch_delta32<4><<<grid, kPairThreads, smem, s>>>(rp, rb, n_rep, item_off, slots, tune,
                                                         queue, htab, cut_scale, area);

@@ -1177,7 +1177,6 @@ void launch_batch_serial(const DevParams* rp, const DevBuffers* rb, const int* i
 }
 
 void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStream_t s) {
-  // (the precision form's energy change adds its blocks itself)
   k_serial64<<<1, kSerialThreads, 0, s>>>(P, B, mode, delta_blocks());
 }
 
