@@ -527,6 +527,13 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   const int sample = blockIdx.x * kSamp + (row & (kSamp - 1));
   const bool swapped = row >= kSamp;
   const bool valid = sample < n;
+  // a warp whose 32 rows are all past the last sample leaves its operands out (an MMA
+  // row depends on its own operand row alone)
+  const bool some = __any_sync(0xffffffffu, valid);
+  // the vectors read later on, towards L1
+  if (t < (int)((sizeof(MlpNet) - offsetof(MlpNet, w3) + 127) / 128))
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(net) +
+                                                 offsetof(MlpNet, w3) + 128 * t));
   // launched as a dependent of the previous kernel: the weights above were
   // staged while it ran; its results are visible after this wait
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -552,7 +559,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   }
   __syncthreads();
   const float* xrow = reinterpret_cast<const float*>(sm + kH1) + (row & (kSamp - 1)) * kIn;
-  for (int k8 = cq; k8 < kIn / 8; k8 += 4) {
+  for (int k8 = cq; some && k8 < kIn / 8; k8 += 4) {
     float v[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
@@ -586,7 +593,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     mma_commit(mb);
   }
   step(true);
-  {
+  if (some) {
     float v[32];
     tmem_ld32(trow + 32 * cq, v);
 #pragma unroll
@@ -605,7 +612,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     mma_commit(mb);
   }
   step(ok);
-  {
+  if (some) {
     float v[32];
     tmem_ld32(trow + 128 + 32 * cq, v);
     float y = 0.0f;
@@ -981,13 +988,16 @@ __global__ void k_cell_scatter(const DevParams* __restrict__ rp,
   B.cell_key[j] = k;
 }
 
-// moved beads per block: a warp per (bead, before / after); many beads per
-// block keep the per-block histogram flush (global atomics) few
-constexpr int kCellBeads = 16;
+// moved beads per block: a warp per (bead, before / after). The kernel is bound by
+// instruction issue: with 16 beads a block, the chain moves of 16 replicas of 20,000
+// beads kept a third of the SMs busy for 28 us (8 beads and a walk instead of a binary
+// search per entry: 22 us). Fewer beads a block gain nothing more and flush more
+// histograms (global atomics).
+constexpr int kCellBeads = 8;
 constexpr int kCellSplit = 1;  // warps per (bead, before / after), each a part of its entries
 constexpr int kCellWarps = 2 * kCellBeads * kCellSplit;
 
-// Block (x, r): moved beads [4x, 4x + 4) of replica r's pending surrogate
+// Block (x, r): moved beads [8x, 8x + 8) of replica r's pending surrogate
 // move. Warp (bead, channel pair): before the move (channels 0, 1) the
 // entries of the 27 cells around the bead's current position, after it
 // (channels 2, 3) around its trial position, then the cell-less list of
@@ -1008,7 +1018,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, 1)
   const int b_lo = st->b_lo, m = min(st->b_hi - b_lo, kDescMaxMoved);
   if ((int)blockIdx.x * kCellBeads >= m) return;
   __shared__ unsigned fh[kFineAll];
-  __shared__ int s_pre[kCellWarps][32], s_base[kCellWarps][32];
+  __shared__ int s_pre[kCellWarps][32], s_off[kCellWarps][32];
   for (int k = threadIdx.x; k < kFineAll; k += blockDim.x) fh[k] = 0u;
   __syncthreads();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1043,8 +1053,8 @@ __global__ void __launch_bounds__(kCellWarps * 32, 1)
     };
     // the 27 cells' entries as one list, split in kCellSplit contiguous
     // parts (one per warp of this bead and channel): lane e of a part takes
-    // its entries e, e + 32, ..., finding the cell by binary search in the
-    // inclusive prefix of the counts
+    // its entries e, e + 32, ..., walking up the inclusive prefix of the
+    // counts; four loads in flight
     int pre = cn;
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, pre, o);
@@ -1052,18 +1062,24 @@ __global__ void __launch_bounds__(kCellWarps * 32, 1)
     }
     const int total = __shfl_sync(0xffffffffu, pre, 26);
     s_pre[w][lane] = pre;
-    s_base[w][lane] = cbase;
+    s_off[w][lane] = cbase - (pre - cn);
     __syncwarp();
     if (cells) {
       const int e_lo = part * total / kCellSplit, e_hi = (part + 1) * total / kCellSplit;
-#pragma unroll 4
-      for (int e = e_lo + lane; e < e_hi; e += 32) {
-        int lo = 0, hi = 26;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (s_pre[w][mid] > e) hi = mid; else lo = mid + 1;
+      int lo = 0;
+      for (int e = e_lo + lane; e < e_hi; e += 128) {
+        int4 ent[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int f = e + 32 * k;
+          ent[k].w = -1;
+          if (f < e_hi) {
+            while (s_pre[w][lo] <= f) lo++;
+            ent[k] = B.cell_ent[s_off[w][lo] + f];
+          }
         }
-        visit(B.cell_ent[s_base[w][lo] + e - (lo ? s_pre[w][lo - 1] : 0)]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) visit(ent[k]);
       }
       const int n_extra = min(B.cell_n[nx * ny * nz], P.cell_cap);
       for (int e = part * 32 + lane; e < n_extra; e += 32 * kCellSplit) visit(B.cell_extra[e]);
@@ -1089,28 +1105,38 @@ __global__ void __launch_bounds__(kCellWarps * 32, 1)
 // One block per replica: bin k of channel c = sum_f count[c][f] *
 // round(4096 exp(-(r_f - c_k)^2 / (2 w^2))) over the fine bins within
 // 1.2 sigma (where the weight rounds to zero beyond).
-__global__ void __launch_bounds__(128) k_desc_fin(const DevBuffers* __restrict__ rb) {
+// The weight of fine bin f in descriptor bin kb depends on f - 8 kb - 4 alone, so 81
+// weights serve all of them; the counts are read once, eight loads in flight a thread.
+constexpr int kFinThreads = 128, kFinReach = 40;
+static_assert(kBinW * kFinePerSigma == 8.0f, "fine bins per descriptor bin");
+
+__global__ void __launch_bounds__(kFinThreads) k_desc_fin(const DevBuffers* __restrict__ rb) {
+  __shared__ unsigned fine[kFineAll], wt[2 * kFinReach + 1];
   // launched as a dependent of k_desc: let the inference start staging, then
   // wait for the counts
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int t = threadIdx.x;
+  if (t <= 2 * kFinReach) {
+    const float d = (t - kFinReach) * (1.0f / kFinePerSigma);
+    wt[t] = __float2uint_rn(4096.0f * expf(-0.5f / (kBinW * kBinW) * d * d));
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const DevBuffers& B = rb[blockIdx.x];
   const DevState* st = B.state;
   if (!(st->pending && st->da_active)) return;
-  const int k = threadIdx.x;
-  if (k >= kIn) return;
-  const int ch = k / kBins, kb = k % kBins;
+#pragma unroll
+  for (int i = 0; i < (kFineAll + kFinThreads - 1) / kFinThreads; i++)
+    if (t + i * kFinThreads < kFineAll) fine[t + i * kFinThreads] = B.desc_fine[t + i * kFinThreads];
+  __syncthreads();
+  if (t >= kIn) return;
+  const int ch = t / kBins, kb = t % kBins, mid = 8 * kb + 4;
   const float c = (kb + 0.5f) * kBinW;
   const int f0 = max(0, (int)((c - 1.2f) * kFinePerSigma));
   const int f1 = min(kFine - 1, (int)((c + 1.2f) * kFinePerSigma) + 1);
   unsigned v = 0u;
-  for (int f = f0; f <= f1; f++) {
-    const unsigned n = B.desc_fine[ch * kFine + f];
-    if (!n) continue;
-    const float d = f * (1.0f / kFinePerSigma) - c;
-    v += n * __float2uint_rn(4096.0f * expf(-0.5f / (kBinW * kBinW) * d * d));
-  }
-  B.desc_acc[k] = v;
+#pragma unroll 8
+  for (int f = f0; f <= f1; f++) v += fine[ch * kFine + f] * wt[f - mid + kFinReach];
+  B.desc_acc[t] = v;
 }
 
 }  // namespace
