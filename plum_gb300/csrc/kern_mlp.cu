@@ -9,10 +9,11 @@
 //   k_mlp_infer   forward on 512 threads (four per tile row, one 32-column
 //                 slice each): s per sample; with DaArgs, the
 //                 delayed-acceptance stage one of each replica's pending move
-//   k_mlp<true>   forward + backward of the mean squared error against the
+//   k_mlp_grad    forward + backward of the mean squared error against the
 //                 targets; per-tile gradients of every parameter
 //   k_mlp_reduce  per-tile gradients summed in tile order (deterministic)
 //   k_mlp_adam    Adam on the fp32 master parameters, bf16 copies refreshed
+//   k_mlp_update  the two in one launch (a training step)
 //   k_desc        descriptor of pending moves (integer Gaussian-bin sums)
 //
 // Shared-memory operands use the no-swizzle K-major layout: 8x8 core
@@ -163,50 +164,64 @@ constexpr uint32_t kH1 = 81920;        // A [128][128]; later dZ2 A [128][128]
 constexpr uint32_t kW2T = 114688;      // B [128 a][128 b]
 constexpr uint32_t kXT = 147456;       // B [96 c][128 i]
 constexpr uint32_t kH1T = 172032;      // B [128 a][128 i]
-constexpr uint32_t kRed = 204800;      // f32 [128][33]
-constexpr uint32_t kMiscT = 221696;
+constexpr uint32_t kMiscT = 204800;
 constexpr uint32_t kMiscI = 114688;
-// misc block: y[128], dy[128], tmp[128], db1[128], db2[128], dw3[128] (f32),
-// mbarrier, tensor-memory address, flag
-constexpr uint32_t kMiscBytes = 6 * 512 + 16;
+// misc block: y[128], dy[128], loss[128], per-quarter sums [4][128] (f32) or, for
+// inference, per-slice outputs [4][128]; mbarrier, tensor-memory address, flag
+constexpr uint32_t kMiscBar = 7 * 512;
+constexpr uint32_t kMiscBytes = kMiscBar + 16;
 constexpr uint32_t kSmemTrain = kMiscT + kMiscBytes;
 constexpr uint32_t kSmemInfer = kMiscI + kMiscBytes;
+// an f32 [128][129] array over W1, X and W2 while the operands there are spent
+constexpr int kRedLd = 129;
+static_assert(128 * kRedLd * 4 <= 81920, "the array ends before H1");
 static_assert(kSmemTrain <= 232448, "shared memory per CTA");
 static_assert(kW1 + 49152 >= 32768 && kX == kW1 + 24576, "dZ2^T fits over W1 and X");
 
-// column sums over the 128 rows of red[row][33] (first 32 columns), in a
-// fixed order; result in out[0..31]
-__device__ __forceinline__ void col_sum32(const float* red, float* tmp, float* out) {
-  const int t = threadIdx.x, c = t & 31, q = t >> 5;
+// Forward and backward of one tile on 512 threads: thread t takes tile row (TMEM lane)
+// t % 128 and the 32-column slice t / 128 of every 128-column epilogue. What bounds it
+// is the element-wise work (a sigmoid each for 3 x 128 x 128 values) and the 2-byte
+// transposed operand stores, so four warps share each lane quarter (65,536 samples in
+// batches of 4,096: 2.15 ms an epoch with one thread per row and separate gather, loss
+// and update launches, 1.05 ms so). Sums keep one order: an output's 128 terms one after the
+// other, a column's rows in four quarters. With idx, sample k of the tile is row idx[k]
+// of x and tgt, which may be aligned to 4 bytes only.
+constexpr int kGradThreads = 512;
+
+// thread (column, quarter)'s sum of column t % 128 over rows [32 (t / 128), + 32) of
+// red, weighted by row (or not); the quarters added in order by threads < 128
+__device__ __forceinline__ float col_sum(const float* red, const float* wrow, float* tmp) {
+  const int t = threadIdx.x, c = t & 127, q = t >> 7;
   __syncthreads();
   float s = 0.0f;
-  for (int r = q * 32; r < q * 32 + 32; r++) s += red[r * 33 + c];
-  tmp[q * 32 + c] = s;
+#pragma unroll 8
+  for (int r = q * 32; r < q * 32 + 32; r++) {
+    const float v = red[r * kRedLd + c];
+    s = __fadd_rn(s, wrow ? __fmul_rn(wrow[r], v) : v);
+  }
+  tmp[t] = s;
   __syncthreads();
-  if (t < 32) out[t] = ((tmp[t] + tmp[32 + t]) + tmp[64 + t]) + tmp[96 + t];
-  __syncthreads();
+  return t < 128 ? ((tmp[t] + tmp[128 + t]) + tmp[256 + t]) + tmp[384 + t] : 0.0f;
 }
 
-template <bool kTrain, typename TIn>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_mlp(const MlpNet* __restrict__ net, const TIn* __restrict__ x, float xscale, int n,
-          const float* __restrict__ tgt, float* __restrict__ s_out, float* __restrict__ part,
-          float inv_n, DaArgs da, int* __restrict__ err) {
+__global__ void __launch_bounds__(kGradThreads, 1)
+    k_mlp_grad(const MlpNet* __restrict__ net, const float* __restrict__ x, int n,
+               const float* __restrict__ tgt, const int* __restrict__ idx,
+               float* __restrict__ part, float inv_n, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char sm[];
   const int t = threadIdx.x, warp = t >> 5;
-  const uint32_t misc = kTrain ? kMiscT : kMiscI;
-  float* ys = reinterpret_cast<float*>(sm + misc);
+  const int row = t & 127, cq = t >> 7;
+  float* ys = reinterpret_cast<float*>(sm + kMiscT);
   float* dys = ys + 128;
-  float* tmp = ys + 256;
-  float* db1s = ys + 384;
-  float* db2s = ys + 512;
-  float* dw3s = ys + 640;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + misc + 3072);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + misc + 3080);
-  int* sflag = reinterpret_cast<int*>(sm + misc + 3084);
+  float* loss = ys + 256;
+  float* tmp = ys + 384;  // [4][128]
+  float* red = reinterpret_cast<float*>(sm);
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kMiscT + kMiscBar);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kMiscT + kMiscBar + 8);
+  int* sflag = reinterpret_cast<int*>(sm + kMiscT + kMiscBar + 12);
   const uint32_t base = smem_u32(sm);
   const uint32_t mb = smem_u32(mbar);
-  constexpr uint32_t kCols = kTrain ? 512u : 256u;
+  constexpr uint32_t kCols = 512u;
 
   if (warp == 0) {
     asm volatile(
@@ -224,56 +239,51 @@ __global__ void __launch_bounds__(kThreads, 1)
   // ---- operands: weights and the input tile
   const __nv_bfloat16* w1 = net->w1;
   const __nv_bfloat16* w2 = net->w2;
-#pragma unroll 4
-  for (int c = t; c < kHid * (kIn / 8); c += kThreads) {
-    const int row = c / (kIn / 8), k8 = c % (kIn / 8);
-    *reinterpret_cast<uint4*>(sm + kW1 + op_off(row, k8 * 8, kIn)) =
-        *reinterpret_cast<const uint4*>(w1 + row * kIn + k8 * 8);
+#pragma unroll
+  for (int c = t; c < kHid * (kIn / 8); c += kGradThreads) {
+    const int r = c / (kIn / 8), k8 = c % (kIn / 8);
+    *reinterpret_cast<uint4*>(sm + kW1 + op_off(r, k8 * 8, kIn)) =
+        *reinterpret_cast<const uint4*>(w1 + r * kIn + k8 * 8);
   }
-#pragma unroll 4
-  for (int c = t; c < kHid * (kHid / 8); c += kThreads) {
-    const int row = c / (kHid / 8), k8 = c % (kHid / 8);
-    *reinterpret_cast<uint4*>(sm + kW2 + op_off(row, k8 * 8, kHid)) =
-        *reinterpret_cast<const uint4*>(w2 + row * kHid + k8 * 8);
+#pragma unroll
+  for (int c = t; c < kHid * (kHid / 8); c += kGradThreads) {
+    const int r = c / (kHid / 8), k8 = c % (kHid / 8);
+    *reinterpret_cast<uint4*>(sm + kW2 + op_off(r, k8 * 8, kHid)) =
+        *reinterpret_cast<const uint4*>(w2 + r * kHid + k8 * 8);
   }
-  if (kTrain)
-    for (int e = t; e < kHid * kHid; e += kThreads) {
-      const int a = e % kHid, b = e / kHid;  // W2^T (a, b) = W2[b][a]
-      *reinterpret_cast<__nv_bfloat16*>(sm + kW2T + op_off(a, b, kHid)) = w2[b * kHid + a];
-    }
-  const int sample = blockIdx.x * kSamp + (t & (kSamp - 1));
-  const bool swapped = t >= kSamp;
+#pragma unroll
+  for (int c = t; c < kHid * (kHid / 8); c += kGradThreads) {  // W2^T (a, b) = W2[b][a]
+    const int a = c % kHid, b8 = c / kHid * 8;
+    __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) h[e] = w2[(b8 + e) * kHid + a];
+    *reinterpret_cast<uint4*>(sm + kW2T + op_off(a, b8, kHid)) =
+        *reinterpret_cast<const uint4*>(h);
+  }
+  const int s0 = blockIdx.x * kSamp;
+  const int sample = s0 + (row & (kSamp - 1));
+  const bool swapped = row >= kSamp;
   const bool valid = sample < n;
-  // Launched as a dependent of the previous kernel, the weights above were
-  // staged while it ran; its results are visible after this wait (a no-op
-  // for an ordinary launch).
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  {
-    // the tile's input rows, staged with coalesced 16-byte loads (rows are
-    // 384 bytes, so every row starts 16-byte aligned) into the H1 region
-    float* xs = reinterpret_cast<float*>(sm + kH1);
-    const int s0 = blockIdx.x * kSamp;
-    constexpr int kVec = kSamp * kIn / 4;
-#pragma unroll 4
-    for (int e = t; e < kVec; e += kThreads) {
-      const int row = e / (kIn / 4);
+  // the tile's input rows, staged in the H1 region
+  float* xs = reinterpret_cast<float*>(sm + kH1);
+  if (idx) {
+#pragma unroll
+    for (int e = t; e < kSamp * kIn; e += kGradThreads) {
+      const int r = e / kIn, f = e % kIn;
+      xs[e] = s0 + r < n ? x[(size_t)idx[s0 + r] * kIn + f] : 0.0f;
+    }
+  } else {  // rows are 384 bytes, so every row starts 16-byte aligned
+#pragma unroll
+    for (int e = t; e < kSamp * kIn / 4; e += kGradThreads) {
+      const int r = e / (kIn / 4);
       float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (s0 + row < n) {
-        const uint4 raw = reinterpret_cast<const uint4*>(x + (size_t)s0 * kIn)[e];
-        if constexpr (std::is_same<TIn, float>::value) {
-          v = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z),
-                          __uint_as_float(raw.w));
-        } else {  // integer descriptor sums
-          v = make_float4((float)raw.x, (float)raw.y, (float)raw.z, (float)raw.w);
-        }
-      }
-      reinterpret_cast<float4*>(xs)[e] = make_float4(v.x * xscale, v.y * xscale, v.z * xscale,
-                                                     v.w * xscale);
+      if (s0 + r < n) v = reinterpret_cast<const float4*>(x + (size_t)s0 * kIn)[e];
+      reinterpret_cast<float4*>(xs)[e] = v;
     }
   }
   __syncthreads();
-  const float* xrow = reinterpret_cast<const float*>(sm + kH1) + (t & (kSamp - 1)) * kIn;
-  for (int k8 = 0; k8 < kIn / 8; k8++) {
+  const float* xrow = xs + (row & (kSamp - 1)) * kIn;
+  for (int k8 = cq; k8 < kIn / 8; k8 += 4) {
     float v[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
@@ -281,17 +291,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int src = swapped ? (f + kIn / 2) % kIn : f;
       v[e] = valid ? (xrow[src] - net->mu[f]) * net->isd[f] : 0.0f;
     }
-    st_bf16x8(sm + kX + op_off(t, k8 * 8, kIn), v);
-    if (kTrain)
+    st_bf16x8(sm + kX + op_off(row, k8 * 8, kIn), v);
 #pragma unroll
-      for (int e = 0; e < 8; e++) st_bf16(sm + kXT + op_off(k8 * 8 + e, t, kHid), v[e]);
+    for (int e = 0; e < 8; e++) st_bf16(sm + kXT + op_off(k8 * 8 + e, row, kHid), v[e]);
   }
   proxy_fence();
   tc_before();
   __syncthreads();
   tc_after();
   const uint32_t tmem = *tslot;
-  const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+  const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  const int c0 = 32 * cq;  // this thread's columns
   uint32_t phase = 0;
   bool ok = true;
   auto step = [&](bool issue) {
@@ -311,19 +321,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     mma_commit(mb);
   }
   step(true);
-  for (int q = 0; q < 4; q++) {
+  {
     float v[32];
-    tmem_ld32(trow + 32 * q, v);
+    tmem_ld32(trow + c0, v);
 #pragma unroll
     for (int c = 0; c < 32; c++) {
-      const float z = v[c] + net->b1[32 * q + c];
+      const float z = v[c] + net->b1[c0 + c];
       v[c] = z * sigm(z);
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) st_bf16x8(sm + kH1 + op_off(t, 32 * q + 8 * j, kHid), v + 8 * j);
-    if (kTrain)
+    for (int j = 0; j < 4; j++) st_bf16x8(sm + kH1 + op_off(row, c0 + 8 * j, kHid), v + 8 * j);
 #pragma unroll
-      for (int c = 0; c < 32; c++) st_bf16(sm + kH1T + op_off(32 * q + c, t, kHid), v[c]);
+    for (int c = 0; c < 32; c++) st_bf16(sm + kH1T + op_off(c0 + c, row, kHid), v[c]);
   }
   proxy_fence();
   tc_before();
@@ -336,132 +345,119 @@ __global__ void __launch_bounds__(kThreads, 1)
     mma_commit(mb);
   }
   step(ok);
-  float y = net->b3;
-  for (int q = 0; q < 4; q++) {
-    float v[32];
-    tmem_ld32(trow + 128 + 32 * q, v);
+  float z2[32], sg[32];
+  tmem_ld32(trow + 128 + c0, z2);
 #pragma unroll
-    for (int c = 0; c < 32; c++) {
-      const float z = v[c] + net->b2[32 * q + c];
-      y += __bfloat162float(net->w3[32 * q + c]) * (z * sigm(z));
-    }
+  for (int c = 0; c < 32; c++) {
+    z2[c] = z2[c] + net->b2[c0 + c];
+    sg[c] = sigm(z2[c]);
+    red[row * kRedLd + c0 + c] = z2[c] * sg[c];
   }
-  ys[t] = y;
   __syncthreads();
-  float s = 0.0f;
-  if (t < kSamp) {
-    s = net->y_scale * (ys[t] - ys[t + kSamp]);
-    if (valid && s_out) s_out[sample] = s;
-    if (!kTrain && valid && da.sts) {
-      DevState* st = da.sts[sample];
-      if (st->pending && st->da_active) {
-        const double u1 = st->da_u1;
-        const float m = net->da_margin;
-        const float sd = s > m ? s - m : (s < -m ? s + m : 0.0f);
-        st->da_s = (double)sd;
-        st->da_skip = !(u1 < exp(-da.rp[sample].beta * (double)sd));
-      }
-    }
+  if (t < 128) {
+    float y = net->b3;
+#pragma unroll 16
+    for (int c = 0; c < kHid; c++)
+      y = fmaf(__bfloat162float(net->w3[c]), red[t * kRedLd + c], y);
+    ys[t] = y;
   }
-
-  if (kTrain) {
-    float* red = reinterpret_cast<float*>(sm + kRed);
-    float* gp = part + (size_t)blockIdx.x * kGradStride;
+  __syncthreads();
+  float* gp = part + (size_t)blockIdx.x * kGradStride;
+  if (t < 128) {
     float lossv = 0.0f;
     if (t < kSamp) {
       float g = 0.0f;
       if (valid) {
-        const float d = s - tgt[sample];
+        const float s = __fmul_rn(net->y_scale, ys[t] - ys[t + kSamp]);
+        const float d = s - tgt[idx ? idx[sample] : sample];
         g = 2.0f * d * net->y_scale * inv_n;
         lossv = d * d * inv_n;
       }
       dys[t] = g;
       dys[t + kSamp] = -g;
     }
-    __syncthreads();
-    const float dyt = dys[t];
-    // loss and db3 (zero by construction: the two orientations cancel)
-    red[t * 33] = lossv;
-    red[t * 33 + 1] = dyt;
-    for (int c = 2; c < 32; c++) red[t * 33 + c] = 0.0f;
-    col_sum32(red, tmp, db1s);  // db1s is scratch here
-    if (t == 0) {
-      gp[kNParam] = db1s[0];
-      gp[kOffB3] = db1s[1];
+    loss[t] = lossv;
+  }
+  __syncthreads();
+  // loss and db3 (zero but for rounding: the two orientations cancel)
+  if (t < 8) {
+    const float* v = t & 1 ? dys : loss;
+    float s = 0.0f;
+    for (int r = (t >> 1) * 32; r < (t >> 1) * 32 + 32; r++) s += v[r];
+    tmp[t] = s;
+  }
+  __syncwarp();
+  if (t < 2) gp[t == 0 ? kNParam : kOffB3] = ((tmp[t] + tmp[2 + t]) + tmp[4 + t]) + tmp[6 + t];
+  // dz2 = dy w3 SiLU'(z2); dW3 and db2 column sums; dz2 in both layouts
+  const float dyt = dys[row];
+  const float dw3 = col_sum(red, dys, tmp);
+#pragma unroll
+  for (int c = 0; c < 32; c++) {
+    z2[c] = dyt * __bfloat162float(net->w3[c0 + c]) * sg[c] * (1.0f + z2[c] * (1.0f - sg[c]));
+    red[row * kRedLd + c0 + c] = z2[c];
+  }
+  const float db2 = col_sum(red, nullptr, tmp);
+  if (t < 128) {
+    gp[kOffW3 + t] = dw3;
+    gp[kOffB2 + t] = db2;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) st_bf16x8(sm + kH1 + op_off(row, c0 + 8 * j, kHid), z2 + 8 * j);
+#pragma unroll
+  for (int c = 0; c < 32; c++) st_bf16(sm + kW1 + op_off(c0 + c, row, kHid), z2[c]);
+  proxy_fence();
+  tc_before();
+  __syncthreads();
+  tc_after();
+  // dh1 = dz2 W2 (B = W2^T as [a][b]);  dW2 = dz2^T h1 (A = dz2^T, B = h1^T)
+  if (t == 0 && ok) {
+    mma_tile(tmem + 256, base + kH1, base + kW2T, kHid, idesc_bf16(128, 128));
+    mma_tile(tmem + 384, base + kW1, base + kH1T, kHid, idesc_bf16(128, 128));
+    mma_commit(mb);
+  }
+  step(ok);
+  {
+    float dh[32], z1[32];
+    tmem_ld32(trow + 256 + c0, dh);
+    tmem_ld32(trow + c0, z1);
+#pragma unroll
+    for (int c = 0; c < 32; c++) {
+      const float z = z1[c] + net->b1[c0 + c];
+      const float s = sigm(z);
+      dh[c] = dh[c] * s * (1.0f + z * (1.0f - s));
+      red[row * kRedLd + c0 + c] = dh[c];
     }
-    __syncthreads();
-    // dz2 = dy w3 SiLU'(z2); dW3 and db2 column sums; dz2 in both layouts
-    for (int q = 0; q < 4; q++) {
-      float v[32], dz[32];
-      tmem_ld32(trow + 128 + 32 * q, v);
+    const float db1 = col_sum(red, nullptr, tmp);
+    if (t < 128) gp[kOffB1 + t] = db1;
 #pragma unroll
-      for (int c = 0; c < 32; c++) {
-        const int b = 32 * q + c;
-        const float z = v[c] + net->b2[b];
-        const float sg = sigm(z);
-        red[t * 33 + c] = dyt * (z * sg);
-        dz[c] = dyt * __bfloat162float(net->w3[b]) * sg * (1.0f + z * (1.0f - sg));
-      }
-      col_sum32(red, tmp, dw3s + 32 * q);
+    for (int c = 0; c < 32; c++) st_bf16(sm + kW2 + op_off(c0 + c, row, kHid), dh[c]);
+  }
+  auto put = [&](float* dst, const float* v) {
 #pragma unroll
-      for (int c = 0; c < 32; c++) red[t * 33 + c] = dz[c];
-      col_sum32(red, tmp, db2s + 32 * q);
-#pragma unroll
-      for (int j = 0; j < 4; j++) st_bf16x8(sm + kH1 + op_off(t, 32 * q + 8 * j, kHid), dz + 8 * j);
-#pragma unroll
-      for (int c = 0; c < 32; c++) st_bf16(sm + kW1 + op_off(32 * q + c, t, kHid), dz[c]);
-    }
-    proxy_fence();
-    tc_before();
-    __syncthreads();
-    tc_after();
-    // dh1 = dz2 W2 (B = W2^T as [a][b]);  dW2 = dz2^T h1 (A = dz2^T, B = h1^T)
-    if (t == 0 && ok) {
-      mma_tile(tmem + 256, base + kH1, base + kW2T, kHid, idesc_bf16(128, 128));
-      mma_tile(tmem + 384, base + kW1, base + kH1T, kHid, idesc_bf16(128, 128));
-      mma_commit(mb);
-    }
-    step(ok);
-    for (int q = 0; q < 4; q++) {
-      float dh[32], z1[32];
-      tmem_ld32(trow + 256 + 32 * q, dh);
-      tmem_ld32(trow + 32 * q, z1);
-#pragma unroll
-      for (int c = 0; c < 32; c++) {
-        const float z = z1[c] + net->b1[32 * q + c];
-        const float sg = sigm(z);
-        dh[c] = dh[c] * sg * (1.0f + z * (1.0f - sg));
-        red[t * 33 + c] = dh[c];
-      }
-      col_sum32(red, tmp, db1s + 32 * q);
-#pragma unroll
-      for (int c = 0; c < 32; c++) st_bf16(sm + kW2 + op_off(32 * q + c, t, kHid), dh[c]);
-    }
-    for (int q = 0; q < 4; q++) {
-      float v[32];
-      tmem_ld32(trow + 384 + 32 * q, v);
-#pragma unroll
-      for (int c = 0; c < 32; c++) gp[kOffW2 + t * kHid + 32 * q + c] = v[c];
-    }
-    proxy_fence();
-    tc_before();
-    __syncthreads();
-    tc_after();
-    // dW1 = dz1^T x' (A = dz1^T [a][i], B = x'^T [c][i])
-    if (t == 0 && ok) {
-      mma_tile(tmem, base + kW2, base + kXT, kHid, idesc_bf16(128, 96));
-      mma_commit(mb);
-    }
-    step(ok);
-    for (int q = 0; q < 3; q++) {
-      float v[32];
-      tmem_ld32(trow + 32 * q, v);
-#pragma unroll
-      for (int c = 0; c < 32; c++) gp[kOffW1 + t * kIn + 32 * q + c] = v[c];
-    }
-    gp[kOffB1 + t] = db1s[t];
-    gp[kOffB2 + t] = db2s[t];
-    gp[kOffW3 + t] = dw3s[t];
+    for (int j = 0; j < 8; j++)
+      reinterpret_cast<float4*>(dst)[j] =
+          make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  };
+  static_assert(kOffW1 % 4 == 0 && kOffW2 % 4 == 0 && kGradStride % 4 == 0, "16-byte stores");
+  proxy_fence();
+  tc_before();
+  __syncthreads();
+  tc_after();
+  // dW1 = dz1^T x' (A = dz1^T [a][i], B = x'^T [c][i])
+  if (t == 0 && ok) {
+    mma_tile(tmem, base + kW2, base + kXT, kHid, idesc_bf16(128, 96));
+    mma_commit(mb);
+  }
+  {
+    float v[32];
+    tmem_ld32(trow + 384 + c0, v);
+    put(gp + kOffW2 + row * kHid + c0, v);
+  }
+  step(ok);
+  if (cq < 3) {
+    float v[32];
+    tmem_ld32(trow + c0, v);
+    put(gp + kOffW1 + row * kIn + c0, v);
   }
 
   tc_before();
@@ -476,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // the 32-column slice t / 128 of every 128-column epilogue, so each lane
 // quarter's rows are shared by four warps (a warp reads only its own lane
 // quarter, 32 (warp % 4) .. +31). The per-slice partial outputs are added in
-// slice order. Same operands, layout and MMAs as k_mlp; SiLU with the fast
+// slice order. Same operands, layout and MMAs as k_mlp_grad; SiLU with the fast
 // exponential and divide (relative error ~1e-6, far below the bf16 rounding
 // of the operands).
 constexpr int kInferThreads = 512;
@@ -493,9 +489,9 @@ __global__ void __launch_bounds__(kInferThreads, 1)
   const int t = threadIdx.x, warp = t >> 5;
   const int row = t & 127, cq = t >> 7;
   float* ypart = reinterpret_cast<float*>(sm + kMiscI);  // [4 slices][128 rows]
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kMiscI + 3072);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kMiscI + 3080);
-  int* sflag = reinterpret_cast<int*>(sm + kMiscI + 3084);
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kMiscI + kMiscBar);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kMiscI + kMiscBar + 8);
+  int* sflag = reinterpret_cast<int*>(sm + kMiscI + kMiscBar + 12);
   const uint32_t base = smem_u32(sm);
   const uint32_t mb = smem_u32(mbar);
   constexpr uint32_t kCols = 256u;
@@ -647,14 +643,6 @@ __global__ void __launch_bounds__(kInferThreads, 1)
                  : "memory");
 }
 
-__global__ void k_mlp_reduce(const float* __restrict__ part, int tiles, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p > kNParam) return;
-  float s = 0.0f;
-  for (int i = 0; i < tiles; i++) s += part[(size_t)i * kGradStride + p];
-  grad[p] = s;
-}
-
 __device__ __forceinline__ void put_param(MlpNet* net, int p, float w) {
   if (p < kOffB1) net->w1[p] = __float2bfloat16_rn(w);
   else if (p < kOffW2) net->b1[p - kOffB1] = w;
@@ -664,12 +652,16 @@ __device__ __forceinline__ void put_param(MlpNet* net, int p, float w) {
   else net->b3 = w;
 }
 
-__global__ void k_mlp_adam(float* __restrict__ param, float* __restrict__ m, float* __restrict__ v,
-                           const float* __restrict__ g, float lr, float c1, float c2,
-                           MlpNet* __restrict__ net) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNParam) return;
-  const float gi = g[p];
+// parameter p's gradient (or, at kNParam, the loss) over the tiles, in tile order
+__device__ __forceinline__ float tile_sum(const float* part, int tiles, int p) {
+  float s = 0.0f;
+#pragma unroll 16
+  for (int i = 0; i < tiles; i++) s += part[(size_t)i * kGradStride + p];
+  return s;
+}
+
+__device__ __forceinline__ void adam_param(float* param, float* m, float* v, float gi, float lr,
+                                           float c1, float c2, MlpNet* net, int p) {
   const float mi = 0.9f * m[p] + 0.1f * gi;
   const float vi = 0.999f * v[p] + 0.001f * gi * gi;
   m[p] = mi;
@@ -677,6 +669,32 @@ __global__ void k_mlp_adam(float* __restrict__ param, float* __restrict__ m, flo
   const float w = param[p] - lr * (mi * c1) / (sqrtf(vi * c2) + 1e-8f);
   param[p] = w;
   put_param(net, p, w);
+}
+
+__global__ void k_mlp_reduce(const float* __restrict__ part, int tiles, float* __restrict__ grad) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p <= kNParam) grad[p] = tile_sum(part, tiles, p);
+}
+
+__global__ void k_mlp_adam(float* __restrict__ param, float* __restrict__ m, float* __restrict__ v,
+                           const float* __restrict__ g, float lr, float c1, float c2,
+                           MlpNet* __restrict__ net) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < kNParam) adam_param(param, m, v, g[p], lr, c1, c2, net, p);
+}
+
+// A training step's reduction and update in one launch; the loss goes to loss[0].
+__global__ void __launch_bounds__(128)
+    k_mlp_update(const float* __restrict__ part, int tiles, float* __restrict__ param,
+                 float* __restrict__ m, float* __restrict__ v, float lr, float c1, float c2,
+                 MlpNet* __restrict__ net, double* __restrict__ loss) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p > kNParam) return;
+  const float g = tile_sum(part, tiles, p);
+  if (p == kNParam)
+    loss[0] += (double)g;
+  else
+    adam_param(param, m, v, g, lr, c1, c2, net, p);
 }
 
 __global__ void k_mlp_pack(const float* __restrict__ param, MlpNet* __restrict__ net) {
@@ -1181,18 +1199,33 @@ void launch_mlp_infer_i(const MlpNet* net, const unsigned* x, int n, float* s_ou
   cudaLaunchKernelEx(&cfg, k_mlp_infer<unsigned>, net, x, kDescUnit, n, s_out, da, err);
 }
 
-void launch_mlp_grad(const MlpNet* net, const float* x, const float* t, int n, float* part,
-                     float* grad, int* err, cudaStream_t st) {
-  if (n <= 0) return;
+static int grad_tiles(const MlpNet* net, const float* x, const float* t, const int* idx, int n,
+                      float* part, int* err, cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
-    smem_attr((const void*)k_mlp<true, float>, kSmemTrain);
+    smem_attr((const void*)k_mlp_grad, kSmemTrain);
     attr = true;
   }
   const int tiles = (n + kSamp - 1) / kSamp;
-  k_mlp<true, float><<<tiles, kThreads, kSmemTrain, st>>>(net, x, 1.0f, n, t, nullptr, part,
-                                                          1.0f / n, DaArgs{nullptr, nullptr}, err);
+  k_mlp_grad<<<tiles, kGradThreads, kSmemTrain, st>>>(net, x, n, t, idx, part, 1.0f / n, err);
+  return tiles;
+}
+
+void launch_mlp_grad(const MlpNet* net, const float* x, const float* t, int n, float* part,
+                     float* grad, int* err, cudaStream_t st) {
+  if (n <= 0) return;
+  const int tiles = grad_tiles(net, x, t, nullptr, n, part, err, st);
   k_mlp_reduce<<<(kNParam + 1 + 255) / 256, 256, 0, st>>>(part, tiles, grad);
+}
+
+void launch_mlp_train(MlpNet* net, const float* x, const float* t, const int* idx, int n,
+                      float* part, float* param, float* m, float* v, int step, float lr,
+                      double* loss, int* err, cudaStream_t st) {
+  const int tiles = grad_tiles(net, x, t, idx, n, part, err, st);
+  const float c1 = 1.0f / (1.0f - powf(0.9f, (float)step));
+  const float c2 = 1.0f / (1.0f - powf(0.999f, (float)step));
+  k_mlp_update<<<(kNParam + 1 + 127) / 128, 128, 0, st>>>(part, tiles, param, m, v, lr, c1, c2,
+                                                          net, loss);
 }
 
 void launch_mlp_adam(float* param, float* m, float* v, const float* grad, int step, float lr,

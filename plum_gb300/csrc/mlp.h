@@ -36,7 +36,6 @@ constexpr int kBins = 24;
 constexpr int kHid = 128;
 constexpr int kRows = 128;     // rows of one tile (MMA M)
 constexpr int kSamp = 64;      // samples per tile: rows [0,64) as given, [64,128) swapped
-constexpr int kThreads = 128;  // one thread per row
 constexpr float kBinW = 0.25f;
 constexpr float kDescCut = 7.5f;
 constexpr float kDescUnit = 1.0f / 4096.0f;  // integer descriptor unit
@@ -86,6 +85,11 @@ void launch_mlp_infer_i(const MlpNet* net, const unsigned* x, int n, float* s_ou
 void launch_mlp_grad(const MlpNet* net, const float* x, const float* t, int n, float* part,
                      float* grad, int* err, cudaStream_t st);
 // Adam step on the fp32 master parameters; refreshes the bf16 copies in net.
+// A training step on the n samples idx of x and t: gradient, Adam, bf16 copies, the
+// loss added to loss[0].
+void launch_mlp_train(MlpNet* net, const float* x, const float* t, const int* idx, int n,
+                      float* part, float* param, float* m, float* v, int step, float lr,
+                      double* loss, int* err, cudaStream_t st);
 void launch_mlp_adam(float* param, float* m, float* v, const float* grad, int step, float lr,
                      MlpNet* net, cudaStream_t st);
 // fp32 parameters -> net (bf16 weights, fp32 biases).

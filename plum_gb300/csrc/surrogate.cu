@@ -66,21 +66,6 @@ int check_err(plum_surrogate* g) {
   return 0;
 }
 
-__global__ void k_gather_rows(const float* __restrict__ x, const float* __restrict__ t,
-                              const int* __restrict__ idx, int n, float* __restrict__ xo,
-                              float* __restrict__ to) {
-  const int r = blockIdx.x;
-  if (r >= n) return;
-  const int src = idx[r];
-  for (int k = threadIdx.x; k < mlp::kIn; k += blockDim.x)
-    xo[(size_t)r * mlp::kIn + k] = x[(size_t)src * mlp::kIn + k];
-  if (threadIdx.x == 0) to[r] = t[src];
-}
-
-__global__ void k_add_loss(const float* __restrict__ grad, double* __restrict__ acc) {
-  acc[0] += (double)grad[mlp::kNParam];
-}
-
 }  // namespace
 
 extern "C" {
@@ -255,11 +240,8 @@ int plum_surrogate_train(plum_surrogate* g, const float* d_x, const float* d_t, 
     SCK(cudaMemcpyAsync(g->d_idx, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice, g->s));
     SCK(cudaMemsetAsync(g->d_loss, 0, sizeof(double), g->s));
     for (long k = 0; k < steps; k++) {
-      k_gather_rows<<<(unsigned)b, 128, 0, g->s>>>(d_x, d_t, g->d_idx + k * b, (int)b, g->d_x,
-                                                   g->d_t);
-      launch_mlp_grad(g->net, g->d_x, g->d_t, (int)b, g->part, g->grad, g->d_err, g->s);
-      k_add_loss<<<1, 1, 0, g->s>>>(g->grad, g->d_loss);
-      launch_mlp_adam(g->param, g->m, g->v, g->grad, ++g->step, lr, g->net, g->s);
+      launch_mlp_train(g->net, d_x, d_t, g->d_idx + k * b, (int)b, g->part, g->param, g->m, g->v,
+                       ++g->step, lr, g->d_loss, g->d_err, g->s);
     }
     SCK(cudaGetLastError());
     double l = 0.0;
