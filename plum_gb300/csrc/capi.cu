@@ -1658,7 +1658,7 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
   const bool fp32 = c->form == PLUM_FORM_FP32;
   Cbmc32Layout G{};
   if (fp32) {
-    G = cbmc32_layout(c->P, n_trials, chain_len);
+    G = cbmc32_layout(c->P, n_trials, chain_len, charged);
     if (G.smem > cbmc32_max_smem())
       return fail(PLUM_ERR_INPUT, "too many trials or grown beads for the precision form's "
                                   "trial kernel");

@@ -332,7 +332,7 @@ struct Cbmc32Layout {
   long long chain_off, k_off, slots;
   size_t smem;
 };
-Cbmc32Layout cbmc32_layout(const DevParams& P, int n_trials, int chain_len);
+Cbmc32Layout cbmc32_layout(const DevParams& P, int n_trials, int chain_len, bool charged);
 size_t cbmc32_max_smem();
 int launch_cbmc32(const DevParams& P, const DevBuffers& B, const CbmcJob& J,
                   const Cbmc32Layout& G, int* ticket, cudaStream_t s);

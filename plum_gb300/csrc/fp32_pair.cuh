@@ -95,6 +95,28 @@ __device__ __forceinline__ float real_images32(const DevParams& P, float dx, flo
     if (r2 <= rc * rc) e = real_term32(P, r2);
     return e;
   }
+  if (P.images == 2) {
+    // r_c below every box length: an axis has at most one more image in range, the
+    // one on the other side (|d| -> L - |d|)
+    const float rc2 = rc * rc, fx = P.f_img[0] - fabsf(dx), fy = P.f_img[1] - fabsf(dy),
+                fz = P.f_img[2] - fabsf(dz);
+    const float xx = dx * dx, yy = dy * dy, zz = dz * dz;
+    const float gx = fx * fx, gy = fy * fy, gz = fz * fz;
+    const auto add = [&](float r2) {
+      if (r2 <= rc2) e += real_term32(P, r2);
+    };
+    add(xx + yy + zz);
+    add(gx + yy + zz);
+    add(xx + gy + zz);
+    add(xx + yy + gz);
+    if (P.two_axes) {
+      add(gx + gy + zz);
+      add(gx + yy + gz);
+      add(xx + gy + gz);
+      add(gx + gy + gz);
+    }
+    return e;
+  }
   for (int a = -P.real_cell[0]; a <= P.real_cell[0]; a++) {
     float x = dx + a * P.f_box[0];
     if (fabsf(x) > rc) continue;

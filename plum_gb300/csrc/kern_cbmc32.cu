@@ -253,18 +253,33 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
   }
-  for (int t = tid; t < T; t += kThreads) {
+  // eight lanes per trial add its items (one thread alone waited for each item's
+  // load: 25 of them took 9 us)
+  constexpr int kLanes = 8;
+  const int p = tid % kLanes;
+  for (int t0 = 0; t0 < T; t0 += kThreads / kLanes) {
+    const int t = t0 + tid / kLanes;
     const int g = t / kGrp, u = t - g * kGrp;
     double lj = 0.0, re = 0.0, ek = 0.0;
-    if (G.n_pair > 0)
-      for (int ch = 0; ch < G.n_chunk; ch++) {
-        const double* sl = J.part + (size_t)(g * G.n_chunk + ch) * kSlot;
-        lj += sl[2 * u];
-        re += sl[2 * u + 1];
-      }
+    if (t < T) {
+      if (G.n_pair > 0)
+#pragma unroll 4
+        for (int ch = p; ch < G.n_chunk; ch += kLanes) {
+          const double* sl = J.part + (size_t)(g * G.n_chunk + ch) * kSlot;
+          lj += sl[2 * u];
+          re += sl[2 * u + 1];
+        }
+#pragma unroll 4
+      for (int kt = p; kt < G.n_kt; kt += kLanes) ek += J.part[(size_t)G.k_off + (size_t)kt * T + t];
+    }
+    for (int o = kLanes / 2; o > 0; o >>= 1) {
+      lj += __shfl_xor_sync(0xffffffffu, lj, o);
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      ek += __shfl_xor_sync(0xffffffffu, ek, o);
+    }
+    if (p != 0 || t >= T) continue;
     lj += J.part[(size_t)G.chain_off + (size_t)g * kSlot + 2 * u];
     re += J.part[(size_t)G.chain_off + (size_t)g * kSlot + 2 * u + 1];
-    for (int kt = 0; kt < G.n_kt; kt++) ek += J.part[(size_t)G.k_off + (size_t)kt * T + t];
     const int4 a = s_tf[t], a2 = s_tf[T + t];
     const float qa = s_tq[t], qa2 = s_tq[T + t];
     const double4_32a b1 = J.b1[t];
@@ -293,10 +308,11 @@ __global__ void __launch_bounds__(kThreads)
   if (tid == 0) *ticket = 0;  // ready for the next launch on this stream
 }
 
-Cbmc32Layout cbmc32_layout(const DevParams& P, int n_trials, int chain_len) {
+Cbmc32Layout cbmc32_layout(const DevParams& P, int n_trials, int chain_len, bool charged) {
   Cbmc32Layout G{};
   G.n_grp = (n_trials + kGrp - 1) / kGrp;
-  G.n_kt = (P.use_ewald && P.n_k > 0) ? (P.n_k + kKPer - 1) / kKPer : 0;
+  // a neutral species changes no structure factor
+  G.n_kt = (charged && P.use_ewald && P.n_k > 0) ? (P.n_k + kKPer - 1) / kKPer : 0;
   const int max_chunks = std::max(1, (P.n_bead + kThreads - 1) / kThreads);
   const int want = std::max(1, (2 * 152 + G.n_grp - 1) / G.n_grp);
   int n_chunk = std::min(want, max_chunks);
