@@ -79,6 +79,9 @@ struct plum_ctx {
   DevParams* d_rp1 = nullptr;
   DevBuffers* d_rb1 = nullptr;
   double* h_out = nullptr;     // pinned
+  DevState* h_state = nullptr;     // pinned, read_state's staging
+  double4_32a* h_span = nullptr;   // pinned, the trial positions of a host move
+  int span_cap = 0, span_lo = 0, span_n = 0;
   uint32_t* d_stream = nullptr;
   long long stream_cap = 0;
   uint32_t* d_mt = nullptr;    // device mt19937 state (625 words)
@@ -329,8 +332,9 @@ int total_energy(plum_ctx* c, double* out8) {
 }
 
 int read_state(plum_ctx* c, DevState* st) {
-  CK(cudaMemcpyAsync(st, c->B.state, sizeof(DevState), cudaMemcpyDeviceToHost, c->s));
+  CK(cudaMemcpyAsync(c->h_state, c->B.state, sizeof(DevState), cudaMemcpyDeviceToHost, c->s));
   CK(cudaStreamSynchronize(c->s));
+  *st = *c->h_state;
   return PLUM_OK;
 }
 
@@ -768,11 +772,12 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
     plum_ctx_destroy(c);
     return PLUM_ERR_CUDA;
   }
-  if (cudaMallocHost(&c->h_out, 64 * sizeof(double)) != cudaSuccess) {
-    c->h_out = nullptr;
+  if (cudaMallocHost(&c->h_out, 64 * sizeof(double)) != cudaSuccess ||
+      cudaMallocHost(&c->h_state, sizeof(DevState)) != cudaSuccess) {
     plum_ctx_destroy(c);
     return fail(PLUM_ERR_CUDA, "cannot allocate pinned host memory");
   }
+  B.host_out = c->h_out + 32;
   c->h_pos.resize(nb);
   for (int i = 0; i < nb; i++)
     c->h_pos[i] = make_double4_32a(in.xyz[3 * i], in.xyz[3 * i + 1], in.xyz[3 * i + 2], in.q[i]);
@@ -825,6 +830,8 @@ int plum_ctx_destroy(plum_ctx* c) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
+  if (c->h_state) cudaFreeHost(c->h_state);
+  if (c->h_span) cudaFreeHost(c->h_span);
   if (c->h_cb) cudaFreeHost(c->h_cb);
   if (c->cb_u) cudaFreeHost(c->cb_u);
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -896,7 +903,15 @@ int plum_delta_energy(plum_ctx* c, int mol, const double* trial, const int* move
   if (lo < 0) lo = hi = b0;
   // Beads inside [lo, hi) that are not flagged keep their current position,
   // so their terms cancel exactly.
-  std::vector<double4_32a> span(hi - lo);
+  if (hi - lo > c->span_cap) {
+    if (c->h_span) cudaFreeHost(c->h_span);
+    c->h_span = nullptr;
+    c->span_cap = 0;
+    CK(cudaMallocHost(&c->h_span, sizeof(double4_32a) * c->most_len));
+    c->span_cap = c->most_len;
+  }
+  c->span_lo = lo;
+  c->span_n = hi - lo;
   for (int i = lo; i < hi; i++) {
     double4_32a p = c->h_pos[i];
     if (moved[i - b0]) {
@@ -904,22 +919,27 @@ int plum_delta_energy(plum_ctx* c, int mol, const double* trial, const int* move
       p.y = trial[3 * (i - b0) + 1];
       p.z = trial[3 * (i - b0) + 2];
     }
-    span[i - lo] = p;
+    c->h_span[i - lo] = p;
   }
-  if (hi > lo)
-    CK(cudaMemcpyAsync(c->B.trial + lo, span.data(), sizeof(double4_32a) * (hi - lo),
-                       cudaMemcpyHostToDevice, c->s));
-  launch_set_move(c->P, c->B, mol, lo, hi, c->s);
-  if (c->form == PLUM_FORM_FP32) launch_fix_trial(c->P, c->B, c->s);
+  double* res = c->B.host_out;
+  res[5] = -1.0;  // not written
+  launch_set_move(c->P, c->B, mol, lo, hi, c->h_span, c->s);
   launch_delta(c, c->B);
   launch_serial64(c->P, c->B, kModeFinish, c->s);
   CK(cudaGetLastError());
-  DevState st;
-  rc = read_state(c, &st);
-  if (rc) return rc;
-  if (st.error) return fail(st.error, "device reported an error in the energy difference");
-  out[0] = st.de, out[1] = st.de_pair, out[2] = st.de_ewald, out[3] = st.de_bond,
-  out[4] = st.de_ext;
+  CK(cudaStreamSynchronize(c->s));
+  int err = (int)res[5];
+  if (err < 0) {  // the step returned early: the state says why
+    DevState st;
+    rc = read_state(c, &st);
+    if (rc) return rc;
+    err = st.error;
+    out[0] = st.de, out[1] = st.de_pair, out[2] = st.de_ewald, out[3] = st.de_bond,
+    out[4] = st.de_ext;
+  } else {
+    for (int k = 0; k < 5; k++) out[k] = res[k];
+  }
+  if (err) return fail(err, "device reported an error in the energy difference");
   c->host_pending = true;
   return PLUM_OK;
 }
@@ -1114,13 +1134,12 @@ int plum_finalize(plum_ctx* c, int accept) {
   if (!c) return fail(PLUM_ERR_INPUT, "null context");
   if (!c->host_pending) return fail(PLUM_ERR_STATE, "no pending trial move");
   cudaSetDevice(c->device);
-  int acc = accept ? 1 : 0;
-  CK(cudaMemcpyAsync(&c->B.state->last_accept, &acc, sizeof(int), cudaMemcpyHostToDevice, c->s));
-  launch_serial64(c->P, c->B, kModeCommit, c->s);
+  launch_serial64(c->P, c->B, kModeCommit | (accept ? kModeAccept : 0), c->s);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->s));
   c->host_pending = false;
-  if (accept) c->h_pos_valid = false;
+  if (accept)  // the host copy takes the committed span
+    std::copy(c->h_span, c->h_span + c->span_n, c->h_pos.begin() + c->span_lo);
   return PLUM_OK;
 }
 

@@ -222,6 +222,7 @@ struct DevBuffers {  // all pointers: copied word-wise into shared memory by the
   double4_32a* ctrial;  // [kCands][max_len] trial positions of the candidates
   int4* cftrial;     // [kCands][max_len] their fixed-point mirror (precision form)
   double* bond_mol;  // [n_mol]
+  double* host_out;  // pinned: dE, its pair, Ewald, bond and ext parts, error of a host move
   DevState* state;
   const uint32_t* stream;
   // per-step logs (may be null)
@@ -285,12 +286,13 @@ void launch_misc_total64(const DevParams& P, const DevBuffers& B, double* out, c
 constexpr int kModeFinish = 1;   // reduce partials, compose dE
 constexpr int kModeDecide = 2;   // Metropolis draw from the stream + commit
 constexpr int kModeGen = 4;      // adopt the next move's candidate (launch_gen64 before)
-constexpr int kModeCommit = 8;   // commit/reject by state->last_accept (host decided)
+constexpr int kModeCommit = 8;   // commit/reject as the host decided: kModeAccept or not
+constexpr int kModeAccept = 16;
 void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStream_t s);
 // The next move's candidates; first: no move is pending (kCandSkip only).
 void launch_gen64(const DevParams& P, const DevBuffers& B, bool first, cudaStream_t s);
 void launch_set_move(const DevParams& P, const DevBuffers& B, int mol, int b_lo, int b_hi,
-                     cudaStream_t s);
+                     const double4_32a* span, cudaStream_t s);
 void launch_observables64(const DevParams& P, const DevBuffers& B, double* per_mol,
                           double* out5, cudaStream_t s);
 void launch_rhoz(const DevParams& P, const DevBuffers& B, double res, int n_bins, unsigned* cnt,
@@ -303,7 +305,6 @@ void launch_delta_pairs32(const DevParams& P, const DevBuffers& B, cudaStream_t 
 // the plain form's 64-bit position mirror (B.fpos64), where it has one
 void launch_fix64_all(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 void launch_fix_all(const DevParams& P, const DevBuffers& B, cudaStream_t s);
-void launch_fix_trial(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 
 // configurational-bias trial sites (kern_cbmc.cu)
 struct CbmcJob {

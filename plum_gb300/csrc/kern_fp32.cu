@@ -945,18 +945,8 @@ __global__ void k_fix_all(const DevParams P, const DevBuffers B) {
   }
 }
 
-__global__ void k_fix_trial(const DevParams P, const DevBuffers B) {
-  const DevState* st = B.state;
-  for (int i = st->b_lo + threadIdx.x; i < st->b_hi; i += blockDim.x)
-    B.ftrial[i - st->b_lo] = fix_point(P, B.trial[i], B.type[i]);
-}
-
 void launch_fix_all(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
   k_fix_all<<<(P.n_bead + 255) / 256, 256, 0, s>>>(P, B);
-}
-
-void launch_fix_trial(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
-  k_fix_trial<<<1, 256, 0, s>>>(P, B);
 }
 
 }  // namespace plum

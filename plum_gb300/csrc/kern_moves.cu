@@ -990,7 +990,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
         }
         if (d.overrun) S.error = PLUM_ERR_STREAM_DEV;
       } else {
-        acc = S.last_accept;
+        acc = mode & kModeAccept ? 1 : 0;
       }
       s_accept = acc;
       sm.s_cand = acc ? kCandAccept : (d.pos != at ? kCandReject : kCandSkip);
@@ -1100,6 +1100,14 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
     }
   }
 
+  if (mode == kModeFinish && B.host_out && threadIdx.x == 0) {
+    B.host_out[0] = S.de;
+    B.host_out[1] = S.de_pair;
+    B.host_out[2] = S.de_ewald;
+    B.host_out[3] = S.de_bond;
+    B.host_out[4] = S.de_ext;
+    B.host_out[5] = (double)S.error;
+  }
   // write the state back
   if (threadIdx.x == 0 && S.stream_pos < d.pos) S.stream_pos = d.pos;
   __syncthreads();
@@ -1180,7 +1188,10 @@ void launch_serial64(const DevParams& P, const DevBuffers& B, int mode, cudaStre
   k_serial64<<<1, kSerialThreads, 0, s>>>(P, B, mode, delta_blocks());
 }
 
-__global__ void k_set_move(const DevParams P, const DevBuffers B, int mol, int b_lo, int b_hi) {
+// span: the trial positions of [b_lo, b_hi) in pinned host memory, read from there
+// (no copy of their own ahead of the kernel).
+__global__ void k_set_move(const DevParams P, const DevBuffers B, int mol, int b_lo, int b_hi,
+                           const double4_32a* __restrict__ span) {
   if (threadIdx.x == 0) {
     DevState* st = B.state;
     st->pending = 1;
@@ -1189,14 +1200,17 @@ __global__ void k_set_move(const DevParams P, const DevBuffers B, int mol, int b
     st->b_hi = b_hi;
     st->move_type = -1;
   }
-  if (B.fpos64)
-    for (int i = b_lo + threadIdx.x; i < b_hi; i += blockDim.x)
-      B.ftrial64[i - b_lo] = fix64x4(P, B.trial[i]);
+  for (int i = threadIdx.x; i < b_hi - b_lo; i += blockDim.x) {
+    const double4_32a p = span[i];
+    B.trial[b_lo + i] = p;
+    if (B.fpos64) B.ftrial64[i] = fix64x4(P, p);
+    if (P.form) B.ftrial[i] = fix_point(P, p, B.type[b_lo + i]);
+  }
 }
 
 void launch_set_move(const DevParams& P, const DevBuffers& B, int mol, int b_lo, int b_hi,
-                     cudaStream_t s) {
-  k_set_move<<<1, 128, 0, s>>>(P, B, mol, b_lo, b_hi);
+                     const double4_32a* span, cudaStream_t s) {
+  k_set_move<<<1, 128, 0, s>>>(P, B, mol, b_lo, b_hi, span);
 }
 
 // ------------------------------------------------------------ mt19937 fill
