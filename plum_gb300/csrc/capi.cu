@@ -86,6 +86,11 @@ struct plum_ctx {
   long long stream_cap = 0;
   uint32_t* d_mt = nullptr;    // device mt19937 state (625 words)
   long long gen_len = 0;       // valid words in d_stream for plum_run
+  long long gen_pos = 0;       // the first of them not read yet
+  // Dropping the unread words (a recorded stream, a restored state) has always taken
+  // the generator to the end of a full buffer. dry_len, dry_pos: that buffer's fill
+  // and read position; gen_skip: words of it not made yet when it was dropped.
+  long long dry_len = 0, dry_pos = 0, gen_skip = 0;
   int* d_log_type = nullptr;
   int* d_log_acc = nullptr;
   double* d_log_e = nullptr;
@@ -360,13 +365,19 @@ int ensure_logs(plum_ctx* c, int n) {
   return PLUM_OK;
 }
 
+// Leaves the generator's unread words.
+void drop_stream(plum_ctx* c) {
+  c->gen_skip += (c->dry_len - c->dry_pos) - (c->gen_len - c->gen_pos);
+  c->gen_len = c->gen_pos = c->dry_len = c->dry_pos = 0;
+}
+
 int ensure_stream(plum_ctx* c, long long n) {
   if (n <= c->stream_cap) return PLUM_OK;
   cudaFree(c->d_stream);
   c->d_stream = nullptr;
   if (dalloc(&c->d_stream, (size_t)n)) return PLUM_ERR_CUDA;
   c->stream_cap = n;
-  c->gen_len = 0;
+  drop_stream(c);
   return PLUM_OK;
 }
 
@@ -1163,7 +1174,7 @@ int plum_run_moves_de(plum_ctx* c, const uint32_t* stream, long n_stream, int n_
   if (rc) return rc;
   CK(cudaMemcpyAsync(c->d_stream, stream, sizeof(uint32_t) * n_stream, cudaMemcpyHostToDevice,
                      c->s));
-  c->gen_len = 0;  // the device generator's buffer is overwritten
+  drop_stream(c);  // the device generator's buffer is overwritten
   DevState st;
   rc = read_state(c, &st);
   if (rc) return rc;
@@ -1215,7 +1226,8 @@ int plum_seed(plum_ctx* c, uint32_t seed) {
   cudaSetDevice(c->device);
   CK(cudaMemcpyAsync(c->d_mt, mt, sizeof(mt), cudaMemcpyHostToDevice, c->s));
   CK(cudaStreamSynchronize(c->s));
-  c->gen_len = 0;
+  drop_stream(c);
+  c->gen_skip = 0;
   return PLUM_OK;
 }
 
@@ -1228,8 +1240,10 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   // 2 + len (2 r + 1) with r rejected pairs per randSphere (mean 1.27).
   const int batch = 256;
   const long long per_move = 16 + 12LL * c->max_len;
-  const long long need = per_move * std::min(batch, n_moves);
-  const long long cap = std::max<long long>(4 * per_move * batch, 1 << 22);
+  // (and a few thousand words for unlikely runs of rejected pairs)
+  const long long spare = 4096, need = per_move * std::min(batch, n_moves) + spare;
+  const long long full = std::max<long long>(4 * per_move * batch, 1 << 22);
+  const long long cap = std::max(full, 4 * (per_move * batch + spare));
   int rc = ensure_stream(c, cap);
   if (rc) return rc;
   DevState st;
@@ -1252,19 +1266,33 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   CK(cudaEventRecord(c->ev0, c->s));
   int done = 0;
   while (done < n_moves) {
-    // Keep at least `need` unread words: move the unread tail to the front and
-    // generate twice that on the device (one block's work, in line with the moves:
-    // a buffer filled to the brim cost a new state's first call 5.5 ms).
+    // Keep at least `need` unread words: generate twice that on the device behind
+    // them (one block's work, in line with the moves: a buffer filled to the brim cost
+    // a new state's first call 5.5 ms). At the buffer's end the unread tail moves to
+    // the front first; it is shorter than need, a quarter of the buffer at most, and
+    // what lies before it longer, so the copy's ranges do not overlap.
+    if (c->dry_len - c->dry_pos < per_move * batch) {
+      c->dry_pos = 0;
+      c->dry_len = full;
+    }
     if (len - pos < need) {
-      long long tail = len - pos;
-      if (tail > 0)
-        CK(cudaMemcpyAsync(c->d_stream, c->d_stream + pos, sizeof(uint32_t) * tail,
-                           cudaMemcpyDeviceToDevice, c->s));
-      len = std::min(cap, tail + 2 * need);
-      launch_mt_fill(c->d_mt, c->d_stream + tail, len - tail, c->s);
+      if (len + 2 * need > cap) {
+        const long long tail = len - pos;
+        if (tail > 0)
+          CK(cudaMemcpyAsync(c->d_stream, c->d_stream + pos, sizeof(uint32_t) * tail,
+                             cudaMemcpyDeviceToDevice, c->s));
+        len = tail;
+        pos = 0;
+        st.stream_pos = 0;
+      }
+      if (c->gen_skip > 0) {
+        launch_mt_fill(c->d_mt, nullptr, c->gen_skip, c->s);
+        c->gen_skip = 0;
+        c->last_kernels++;
+      }
+      launch_mt_fill(c->d_mt, c->d_stream + len, 2 * need, c->s);
       c->last_kernels++;
-      pos = 0;
-      st.stream_pos = 0;
+      len += 2 * need;
     }
     st.stream_len = len;
     st.step = 0;
@@ -1276,6 +1304,7 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
     rc = read_state(c, &st);
     if (rc) return rc;
     if (st.error) break;
+    c->dry_pos += st.stream_pos - pos;
     pos = st.stream_pos;
     done += nb;
     c->since_recompute += nb;
@@ -1304,6 +1333,7 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
   c->last_ms = ms;
   c->gen_len = len;
+  c->gen_pos = pos;
   c->h_pos_valid = false;
   if (accepted_out) *accepted_out = st.n_accept;
   if (st.error == PLUM_ERR_STREAM_DEV) return fail(PLUM_ERR_STREAM, "device stream ran out");
@@ -1458,7 +1488,7 @@ int plum_ctx_load(plum_ctx* c, const void* buf, long size) {
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->s));
   c->h_pos_valid = true;
-  c->gen_len = 0;
+  drop_stream(c);
   return PLUM_OK;
 }
 

@@ -1229,13 +1229,14 @@ __device__ __forceinline__ uint32_t mt_twist(uint32_t a, uint32_t b, uint32_t c)
 // 4 M words at a time, 5.5 ms of a new state's first call.)
 constexpr int kMtThreads = 256, kMtLag = 227, kMtRing = 1024;
 
+// (without out, n words are skipped)
 __device__ __forceinline__ void mt_fill_body(uint32_t* state, uint32_t* out, long long n) {
   __shared__ uint32_t x[kMtRing];
   if (n <= 0) return;
   const long long idx = state[624];
   const int t = threadIdx.x;
   auto emit = [&](long long g, uint32_t y) {  // word g, tempered, if it is asked for
-    if (g < idx || g >= idx + n) return;
+    if (!out || g < idx || g >= idx + n) return;
     y ^= y >> 11;
     y ^= (y << 7) & 0x9d2c5680u;
     y ^= (y << 15) & 0xefc60000u;
