@@ -139,6 +139,11 @@ __host__ __device__ inline int k_beads(const DevParams& P) {
   return fit < 1 ? 1 : (fit > 32 ? 32 : fit);
 }
 
+// (an integer comparison: one of doubles takes the FP64 pipe)
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
 struct FixStage {
   ulonglong2 a, b, c;  // trial (x, y, z), current (x, y, z)
   double q;            // charge x lB sqrt(alpha) x table unit
@@ -199,7 +204,7 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
       for (int u = u0; u < u1; u++) {
         const ulonglong2 a = st[u].a, b = st[u].b, c = st[u].c;
         if (jm && u >= l) break;
-        if (st[u].q != q) {
+        if (!same_bits(st[u].q, q)) {
           acc = fma(q, (double)sum, acc);
           q = st[u].q;
           sum = 0;
@@ -544,7 +549,7 @@ __global__ void __launch_bounds__(kFixTile)
     for (int jj = 0; jj < jn; jj++) {
       const ulonglong2 a = so[jj].a;
       const unsigned long long z = so[jj].z;
-      if (so[jj].q != q || held == kFixFlush) {
+      if (!same_bits(so[jj].q, q) || held == kFixFlush) {
         re = fma(q, (double)sum, re);
         q = so[jj].q;
         sum = 0;
