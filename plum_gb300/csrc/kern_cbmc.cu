@@ -238,8 +238,10 @@ __global__ void __launch_bounds__(kCbThreads)
 //              trial's kw (2 S_o.e + |e|^2)
 // k_cbmc64_sum adds the blocks' sums of a trial in order and its own terms, a block
 // per trial (the last block of the sweep doing it for all took longer than the
-// launch). No split depends on the number of trials, so neither does a result. One growth step of 32 trials on 6,400 beads, r_c = 0.7 L: XXX us, 430 us
-// in three FP64 launches (27 image cells per pair, a sincos per trial and k).
+// launch). No split depends on the number of trials, so neither does a result. One
+// growth step of 32 charged trials on 6,400 beads, r_c = 0.7 L: 31 us on the device
+// and 54 us a call (430 and 477 us in three FP64 launches: 27 image cells per pair, a
+// sincos per trial and k).
 constexpr int kCb64Threads = 512, kCb64K = 128;
 
 int cbmc_blocks() { return pair_grid() / 2; }

@@ -10,8 +10,8 @@
 //                             all moved beads, which equals the reference's
 //                             pairwise PairEnergyRepl sum
 //                             (potential_ewald_coul.cc:198-225) on the same k-set
-//              Every block writes its own partial sums; the last one adds them in
-//              a fixed order, so results are run-to-run identical.
+//              Every block writes its own partial sums; the serial step adds them
+//              in a fixed order, so results are run-to-run identical.
 //  k_total64*  all i<j pairs from scratch (tile pairs)
 //  k_sk64      S(k) from scratch (k unit tile x bead group partials)
 //  k_misc64    bonds, walls, self energy, self images, sum q z
@@ -122,8 +122,8 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 // last block doing so cost 3 us per move, and three blocks per SM a second wave.
 // Pairs with both beads moved are taken once (j > i), at trial positions for both.
 //
-// A move with its serial step (kern_moves.cu): 23 us for 1,000 beads and 1,687
-// k-vectors, 24 us with image cells, 46 us for 20,000 beads and 7,812 k-vectors
+// A move with its serial step (kern_moves.cu): 21 us for 1,000 beads and 1,687
+// k-vectors, 22 us with image cells, 44 us for 20,000 beads and 7,812 k-vectors
 // (50, 94 and 130 us with FP64 pairs, k tiles x bead groups and a move generated
 // in the serial step).
 constexpr int kDeltaThreads = 512;
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kTotTile)
 // over up to 16 beads of one charge). The table is staged too, as the lanes'
 // gathers from it run at a bank's pace there and a line's pace from L1; a small
 // system's tiles are cut into `parts` of the j's instead, so that they fill the
-// SMs, and read it in place. 20,000 beads: 1.35 ms (6.2 ms in FP64).
+// SMs, and read it in place. 20,000 beads: 1.1 ms (6.2 ms in FP64).
 constexpr int kFixTile = 256;
 constexpr int kFixFlush = 16;
 struct FixOther {

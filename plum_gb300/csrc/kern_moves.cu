@@ -22,7 +22,8 @@
 // Generating a move is a chain of dependent draws, scans and FP64 arithmetic on
 // one block; as part of the serial step it stood on the critical path of every
 // move (1,000 beads: 40 us per move with it there, 30 us beside the energy
-// change; 32 replicas of 20,000 beads: the serial step 36 to 24 us).
+// change; 21 us with the shorter chains below and the energy change on one block
+// per SM. 32 replicas of 20,000 beads: the serial step 36 us, 24 us, 13 us).
 //
 // Build note: this file is compiled with -fmad=false. The draw-consuming
 // tests (randSphere's r1^2 + r2^2 > 1, the move-type and pick thresholds)
