@@ -98,11 +98,24 @@ __device__ __forceinline__ unsigned long long fix64(double x, double inv) {
   return __double2ull_rn(f * 0x1p64);
 }
 
+__device__ __forceinline__ bool finite3(double4_32a p) {
+  const int e = 0x7FF00000;  // (the exponents as integers: off the FP64 pipe)
+  return (__double2hiint(p.x) & e) != e && (__double2hiint(p.y) & e) != e &&
+         (__double2hiint(p.z) & e) != e;
+}
+
+// A bead's charge for the sums over integer fractions of its coordinates: those have
+// no NaN, so where a coordinate is not finite the charge is NaN instead, and with it
+// the bead's phases and every energy that they enter.
+__device__ __forceinline__ double charge_of(double4_32a p) {
+  return finite3(p) ? p.w : __longlong_as_double(0x7FF8000000000000ll);
+}
+
 // A bead as the plain form's 64-bit mirror holds it (cubic box).
 __device__ __forceinline__ ulonglong4_32a fix64x4(const DevParams& P, double4_32a p) {
   const double inv = P.inv_ebox[0];
   return make_ulonglong4_32a(fix64(p.x, inv), fix64(p.y, inv), fix64(p.z, inv),
-                         (unsigned long long)__double_as_longlong(p.w));
+                         (unsigned long long)__double_as_longlong(charge_of(p)));
 }
 
 __device__ __forceinline__ int4 fix_point(const DevParams& P, double4_32a p, int type) {

@@ -189,7 +189,8 @@ struct MoveCand {
   // walls, sum q dz and the molecule's bonds at the trial positions
   double ext, dmz, bond;
   double bond_old;  // the molecule's bond energy before it
-  int bonded, pad;  // the molecule has bonds
+  int bonded;     // the molecule has bonds
+  int lost;       // a trial coordinate is not finite
 };
 struct StepPlan {
   MoveCand cand[kCands];

@@ -398,6 +398,9 @@ __global__ void __launch_bounds__(kCb64Sum)
   double v[3] = {0.0, 0.0, 0.0};
   for (int b = tid; b < blocks; b += kCb64Sum)
     for (int c = 0; c < 3; c++) v[c] += J.slots[((size_t)b * J.n_trials + t) * 3 + c];
+  // a neutral species' Ewald energy is zero, or NaN with a grown bead that is not finite
+  if (!J.charged)
+    for (int i = tid; i < J.cl; i += kCb64Sum) v[1] += charge_of(J.chain[i]);
   for (int c = 0; c < 3; c++) {
     v[c] = warp_sum(v[c]);
     if ((tid & 31) == 0) s_w[tid >> 5][c] = v[c];
@@ -426,6 +429,8 @@ __global__ void __launch_bounds__(kCb64Sum)
       if (P.real_cut >= P.ebox[0])  // a bead's own images
         ew += 0.5 * (cb_real(P, b1, b1) + cb_real(P, b2, b2));
     }
+  } else if (P.use_ewald && P.n_k > 0 && pair_e < kVeryLarge) {
+    ew = v[1] + charge_of(b1);
   }
   if (P.use_ext) {
     pair_e += wall64(P, b1.z, J.type);

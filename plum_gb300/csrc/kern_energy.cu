@@ -281,7 +281,7 @@ __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B
           tx = c < 0 ? 0 : turn64(P, p.x, 0);
           ty = c < 0 ? 0 : turn64(P, p.y, 1);
           tz = c < 0 ? turn64(P, p.z, 2) : 0;
-          q = p.w;
+          q = charge_of(p);
         }
         if (c < 0) {
           const double2 e1 = turn_exp(tz);

@@ -321,7 +321,7 @@ template <class Trial>
 __device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& B, bool on, int m0,
                                           int m1, int b_lo, int b_hi, const PosView& V,
                                           const Trial& T, MoveCand& C, double* red) {
-  if (threadIdx.x == 0) C.ext_bad = 0;
+  if (threadIdx.x == 0) C.ext_bad = C.lost = 0;
   __syncthreads();
   double ext = 0.0, dmz = 0.0, bt = 0.0;
   if (on) {
@@ -333,6 +333,7 @@ __device__ __forceinline__ void move_sums(const DevParams& P, const DevBuffers& 
         if (en >= kVeryLarge) C.ext_bad = 1;  // every writer stores the same value
         ext += en - wall64(P, p.z, ty);
       }
+      if (!finite3(t)) C.lost = 1;
       dmz += t.w * (t.z - p.z);
     }
     if (P.use_bond && m1 - m0 > 1)
@@ -936,6 +937,8 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
       }
       if (!done && P.use_ewald) {
         dw = de_re + P.kpref * de_k;
+        // (fixed-point pairs and phases have no NaN)
+        if (now.lost) dw = __longlong_as_double(0x7FF8000000000000ll);
         if (P.dipole) {
           dip_t = P.dip_coef * S.mz * S.mz;
           dw += dip_t - S.dipl_cur;

@@ -1,6 +1,7 @@
 // Reciprocal-space helpers of the FP64 kernels.
 #pragma once
 
+#include "device_common.cuh"
 #include "engine.h"
 
 namespace plum {
@@ -61,7 +62,7 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 __device__ __forceinline__ void build_axis_table(const DevParams& P, double4_32a p,
                                                  int axis, double2* tab) {
   const double2 e1 = turn_exp(turn64(P, axis == 0 ? p.x : (axis == 1 ? p.y : p.z), axis));
-  double2 e = axis == 0 ? make_double2(p.w, 0.0) : make_double2(1.0, 0.0);
+  double2 e = axis == 0 ? make_double2(charge_of(p), 0.0) : make_double2(1.0, 0.0);
   double2* t = tab + P.koff[axis];
   t[0] = e;
   for (int n = 1; n <= P.kmax[axis]; n++) {
