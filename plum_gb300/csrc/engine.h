@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "fix_pair.h"
+#include "per_device.h"
 #include "real_tables.h"
 
 namespace plum {

@@ -442,12 +442,8 @@ __global__ void __launch_bounds__(kCb64Sum)
 template <int kMode>
 static void launch_one64(const DevParams& P, const DevBuffers& B, const CbmcJob& J,
                          cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_cbmc64<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kFixMaxBins * 40);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_cbmc64<kMode>, kFixMaxBins * 40);
   k_cbmc64<kMode><<<cbmc_blocks(), kCb64Threads, J.charged ? (size_t)P.fx.n_bin * 40 : 0, s>>>(
       P, B, J);
   k_cbmc64_sum<kMode><<<J.n_trials, kCb64Sum, 0, s>>>(P, B, J, cbmc_blocks());

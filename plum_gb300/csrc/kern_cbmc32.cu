@@ -333,13 +333,8 @@ size_t cbmc32_max_smem() { return kMaxSmem; }
 
 int launch_cbmc32(const DevParams& P, const DevBuffers& B, const CbmcJob& J,
                   const Cbmc32Layout& G, int* ticket, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_cbmc32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kMaxSmem) != cudaSuccess)
-      return 1;
-    attr = true;
-  }
+  static OncePerDevice once;
+  if (allow_smem(once, k_cbmc32, kMaxSmem) != cudaSuccess) return 1;
   if (G.smem > kMaxSmem) return 1;
   k_cbmc32<<<G.grid, kThreads, G.smem, s>>>(P, B, J, G, ticket);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;

@@ -408,17 +408,7 @@ __global__ void __launch_bounds__(kDeltaThreads, 1)
   }
 }
 
-static int g_pair_grid = 0;
-
-int pair_grid() {
-  if (g_pair_grid == 0) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    g_pair_grid = 2 * (sms > 0 ? sms : 152);
-  }
-  return g_pair_grid;
-}
+int pair_grid() { return 2 * device_sms(); }
 
 // One block per SM (a block takes nearly all of an SM's registers), but for the
 // SMs that the next move's candidates run on meanwhile: with a block on every SM
@@ -428,12 +418,8 @@ int delta_blocks() { return std::max(1, pair_grid() / 2 - kCands); }
 template <int kMode>
 static void launch_delta64(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
   constexpr size_t stage = kFixStage * sizeof(FixStage) + kFixMaxBins * 40;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_delta64<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         stage + kKTableBytes);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_delta64<kMode>, stage + kKTableBytes);
   // the staged moved beads and the table, then the k role's phase tables
   const size_t tab = kMode ? kFixStage * sizeof(FixStage) + (size_t)P.fx.n_bin * 40 : 0;
   const size_t k = P.use_ewald && P.n_ku > 0
@@ -603,12 +589,8 @@ static void launch_total_fix(const DevParams& P, const DevBuffers& B, double* ou
   const int parts = fix_parts(P);
   const size_t smem = (size_t)P.fx.n_bin * (2 * sizeof(FixPair64) + sizeof(FixPair32));
   if (parts == 1) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_total64_fix<kMode, true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, kFixMaxBins * 40);
-      attr = true;
-    }
+    static OncePerDevice once;
+    allow_smem(once, k_total64_fix<kMode, true>, kFixMaxBins * 40);
     k_total64_fix<kMode, true><<<n_part, kFixTile, smem, s>>>(P, B, out, parts);
   } else {
     k_total64_fix<kMode, false><<<n_part, kFixTile, 0, s>>>(P, B, out, parts);
@@ -712,11 +694,8 @@ __global__ void __launch_bounds__(256) k_sk_sum(int n_k, int groups, const doubl
 
 void launch_sk_full64(const DevParams& P, const DevBuffers& B, double2* part, cudaStream_t s) {
   if (!P.use_ewald || P.n_k == 0) return;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_sk64, cudaFuncAttributeMaxDynamicSharedMemorySize, kKTableBytes + 4096);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_sk64, kKTableBytes + 4096);
   size_t smem = (size_t)P.kchunk_sk * P.kper * sizeof(double2);
   // a group of fewer than 8 beads would spend more on its tables than its sums
   const int groups = std::max(1, std::min(sk_full_groups(P), (P.n_bead + 7) / 8));

@@ -408,26 +408,13 @@ __global__ void __launch_bounds__(kD32Threads, 1)
   }
 }
 
-static int g_grid32 = 0;
-int pair_grid32() {
-  if (g_grid32 == 0) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    g_grid32 = 4 * (sms > 0 ? sms : 152);
-  }
-  return g_grid32;
-}
+int pair_grid32() { return 4 * device_sms(); }
 
 template <int kMode>
 static void launch_delta32(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
   const size_t tab = kMode ? kD32Stage * sizeof(Stage32) + kH32Bins * sizeof(float4) : 0;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_delta32<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kKTableBytes + 4096 + (int)tab);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_delta32<kMode>, kKTableBytes + 4096 + tab);
   const size_t k = P.use_ewald && P.n_ku > 0
                        ? (size_t)k_beads32(P) * 2 * (P.kmax[2] + 1 + kD32Units) * sizeof(float2)
                        : 0;
@@ -911,15 +898,12 @@ int batch_delta_smem(const DevParams& P) {
 void launch_batch_delta32(const DevParams* rp, const DevBuffers* rb, int n_rep, int* item_off,
                           double* slots, size_t smem, BatchTune tune, int* queue,
                           const float4* htab, float cut_scale, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    const int most = kKAreaBytes + 2 * (kMaxKmax + 1 + kKUnitsMost) * (int)sizeof(float2) +
-                     kH32Bins * (int)sizeof(float4) + (4 * kMaxReplicas + 1) * (int)sizeof(int);
-    cudaFuncSetAttribute(k_batch_delta32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    cudaFuncSetAttribute(k_batch_delta32<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    cudaFuncSetAttribute(k_batch_delta32<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    attr = true;
-  }
+  static OncePerDevice once[3];
+  constexpr size_t most = kKAreaBytes + 2 * (kMaxKmax + 1 + kKUnitsMost) * sizeof(float2) +
+                          kH32Bins * sizeof(float4) + (4 * kMaxReplicas + 1) * sizeof(int);
+  allow_smem(once[0], k_batch_delta32<2>, most);
+  allow_smem(once[1], k_batch_delta32<3>, most);
+  allow_smem(once[2], k_batch_delta32<4>, most);
   const int grid = tune.grid > 0 ? tune.grid : pair_grid32();
   if (!tune.htab) htab = nullptr;
   if (!htab) cut_scale = 0.0f;

@@ -1160,18 +1160,11 @@ __global__ void __launch_bounds__(kFinThreads) k_desc_fin(const DevBuffers* __re
 }  // namespace
 
 // ------------------------------------------------------------ launches
-static void smem_attr(const void* f, int bytes) {
-  cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 void launch_mlp_infer_f(const MlpNet* net, const float* x, int n, float* s_out, int* err,
                         cudaStream_t st) {
   if (n <= 0) return;
-  static bool attr = false;
-  if (!attr) {
-    smem_attr((const void*)k_mlp_infer<float>, kSmemInfer);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_mlp_infer<float>, kSmemInfer);
   k_mlp_infer<float><<<(n + kSamp - 1) / kSamp, kInferThreads, kSmemInfer, st>>>(
       net, x, 1.0f, n, s_out, DaArgs{nullptr, nullptr}, err);
 }
@@ -1179,11 +1172,8 @@ void launch_mlp_infer_f(const MlpNet* net, const float* x, int n, float* s_out, 
 void launch_mlp_infer_i(const MlpNet* net, const unsigned* x, int n, float* s_out, DaArgs da,
                         int* err, cudaStream_t st) {
   if (n <= 0) return;
-  static bool attr = false;
-  if (!attr) {
-    smem_attr((const void*)k_mlp_infer<unsigned>, kSmemInfer);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_mlp_infer<unsigned>, kSmemInfer);
   // programmatic dependent launch: may start while the preceding kernel on
   // the stream (the descriptor kernel) still runs
   cudaLaunchConfig_t cfg = {};
@@ -1201,11 +1191,8 @@ void launch_mlp_infer_i(const MlpNet* net, const unsigned* x, int n, float* s_ou
 
 static int grad_tiles(const MlpNet* net, const float* x, const float* t, const int* idx, int n,
                       float* part, int* err, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    smem_attr((const void*)k_mlp_grad, kSmemTrain);
-    attr = true;
-  }
+  static OncePerDevice once;
+  allow_smem(once, k_mlp_grad, kSmemTrain);
   const int tiles = (n + kSamp - 1) / kSamp;
   k_mlp_grad<<<tiles, kGradThreads, kSmemTrain, st>>>(net, x, n, t, idx, part, 1.0f / n, err);
   return tiles;

@@ -298,11 +298,8 @@ void launch_slit_pressure(const SlitPressParams& S, const DevParams& P, const De
                           cudaStream_t s) {
   k_slit_pairs<<<dim3(G.tiles, G.groups), kSlitThreads, 0, s>>>(S, B, G, wall_b0, gtab, scratch);
   if (G.n2 > 0) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_slit_sk, cudaFuncAttributeMaxDynamicSharedMemorySize, kKTableBytes);
-      attr = true;
-    }
+    static OncePerDevice once;
+    allow_smem(once, k_slit_sk, kKTableBytes);
     double2* sk = reinterpret_cast<double2*>(scratch + G.sk_off);
     int* mask = reinterpret_cast<int*>(scratch + G.mask_off);
     k_slit_sk<<<dim3(G.ktiles, G.kgroups), kSlitSkThreads,
