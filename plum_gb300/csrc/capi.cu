@@ -88,9 +88,10 @@ struct plum_ctx {
   long long gen_len = 0;       // valid words in d_stream for plum_run
   long long gen_pos = 0;       // the first of them not read yet
   // Dropping the unread words (a recorded stream, a restored state) has always taken
-  // the generator to the end of a full buffer. dry_len, dry_pos: that buffer's fill
-  // and read position; gen_skip: words of it not made yet when it was dropped.
-  long long dry_len = 0, dry_pos = 0, gen_skip = 0;
+  // the generator to the end of a full buffer. dry_left: unread words of that buffer,
+  // never fewer than there are in d_stream; gen_skip: words of it not made yet when it
+  // was dropped, passed over before the next ones are made.
+  long long dry_left = 0, gen_skip = 0;
   int* d_log_type = nullptr;
   int* d_log_acc = nullptr;
   double* d_log_e = nullptr;
@@ -367,8 +368,8 @@ int ensure_logs(plum_ctx* c, int n) {
 
 // Leaves the generator's unread words.
 void drop_stream(plum_ctx* c) {
-  c->gen_skip += (c->dry_len - c->dry_pos) - (c->gen_len - c->gen_pos);
-  c->gen_len = c->gen_pos = c->dry_len = c->dry_pos = 0;
+  c->gen_skip += c->dry_left - (c->gen_len - c->gen_pos);
+  c->gen_len = c->gen_pos = c->dry_left = 0;
 }
 
 int ensure_stream(plum_ctx* c, long long n) {
@@ -1268,15 +1269,14 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   while (done < n_moves) {
     // Keep at least `need` unread words: generate twice that on the device behind
     // them (one block's work, in line with the moves: a buffer filled to the brim cost
-    // a new state's first call 5.5 ms). At the buffer's end the unread tail moves to
+    // a new state's first call 5.5 ms), but none past the end of the full buffer, which
+    // has a batch's words left itself. At the buffer's end the unread tail moves to
     // the front first; it is shorter than need, a quarter of the buffer at most, and
     // what lies before it longer, so the copy's ranges do not overlap.
-    if (c->dry_len - c->dry_pos < per_move * batch) {
-      c->dry_pos = 0;
-      c->dry_len = full;
-    }
-    if (len - pos < need) {
-      if (len + 2 * need > cap) {
+    if (c->dry_left < per_move * batch) c->dry_left = full;
+    if (len - pos < std::min(need, c->dry_left)) {
+      const long long words = std::min(2 * need, c->dry_left - (len - pos));
+      if (len + words > cap) {
         const long long tail = len - pos;
         if (tail > 0)
           CK(cudaMemcpyAsync(c->d_stream, c->d_stream + pos, sizeof(uint32_t) * tail,
@@ -1290,9 +1290,9 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
         c->gen_skip = 0;
         c->last_kernels++;
       }
-      launch_mt_fill(c->d_mt, c->d_stream + len, 2 * need, c->s);
+      launch_mt_fill(c->d_mt, c->d_stream + len, words, c->s);
       c->last_kernels++;
-      len += 2 * need;
+      len += words;
     }
     st.stream_len = len;
     st.step = 0;
@@ -1303,9 +1303,9 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
     if (rc) return rc;
     rc = read_state(c, &st);
     if (rc) return rc;
-    if (st.error) break;
-    c->dry_pos += st.stream_pos - pos;
+    c->dry_left -= st.stream_pos - pos;
     pos = st.stream_pos;
+    if (st.error) break;
     done += nb;
     c->since_recompute += nb;
     if (c->recompute_every > 0 && c->since_recompute >= c->recompute_every) {
