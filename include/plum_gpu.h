@@ -371,16 +371,16 @@ int plum_batch_last_timing(const plum_batch* batch, double* ms, long* kernels);
 int plum_batch_time_kernels(plum_batch* batch, int n_steps, double* out4);
 /* Work items of the batched energy change: (moved, other) pairs per pair
  * item (>= 1024, a multiple of 256; a pair item holds up to 32 moved beads
- * against item_pairs / 32 other beads, at least 256), k-vectors per k item
- * (64..256, or 512 / 1024: up to four per thread, the moved beads' phase
- * tables built once per item), the grid (0: 4 blocks per SM) and the register budget as
- * resident blocks per SM (2, 3 or 4). They change only the summation order
- * inside FP32 partials. */
+ * against item_pairs / 32 other beads, in steps of 64), k-vectors per k item
+ * (64..256, or 512 / 1024; two of them, at +-n_z, are one unit, and an item
+ * holds at most 256 units, so 1024 is the same as 512), the grid (0: 4 blocks
+ * per SM) and the register budget as resident blocks per SM (2, 3 or 4). They
+ * change only the summation order inside FP32 partials. */
 int plum_batch_set_tune(plum_batch* batch, int item_pairs, int k_tile, int grid,
                         int min_blocks);
 /* Times the energy-change kernel on these replicas (`steps` steps per
  * candidate, see plum_batch_time_kernels) for item sizes {4096, 8192, 16384,
- * 32768} x k tiles {128, 256, 512, 1024} x grids {2, 3, 4, 6, 8} blocks per
+ * 32768} x k tiles {128, 256, 512} x grids {2, 3, 4, 6, 8} blocks per
  * SM x register budgets {2, 3, 4} blocks per SM, keeps the fastest (then the
  * two pair loops of plum_batch_set_real_term at those sizes); out4 (may be
  * NULL) = the chosen {item_pairs,

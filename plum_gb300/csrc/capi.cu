@@ -2788,7 +2788,7 @@ int plum_batch_autotune(plum_batch* b, int steps, int* out4) {
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
   const int pairs[] = {4096, 8192, 16384, 32768};
-  const int ktiles[] = {128, 256, 512, 1024};
+  const int ktiles[] = {128, 256, 512};  // (a k item holds at most 256 units, 512 vectors)
   const int per_sm[] = {2, 3, 4, 6, 8};
   const int occ[] = {2, 3, 4};
   double best = 1e300;

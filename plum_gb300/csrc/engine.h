@@ -352,7 +352,8 @@ constexpr int kMaxReplicas = 2048;
 // Work-item sizes of the batched energy change.
 struct BatchTune {
   int item_pairs;  // (moved, other) pairs per pair item
-  int k_tile;      // k-vectors per k item (k_tile / 2 units, at most a block's threads)
+  int k_tile;      // k-vectors per k item (k_tile / 2 units, at most a block's threads:
+                   // 1024 is the same as 512)
   int grid;        // blocks (0: 4 per SM)
   int min_blocks;  // register budget: 2 or 3 resident blocks per SM
   int htab;        // real-space term from the h(u) table (1) or the erfc fit (0)
