@@ -137,6 +137,13 @@ struct plum_ctx {
 
 namespace {
 
+// An Ewald box length, and its reciprocal in two doubles.
+void set_ebox(DevParams& P, int axis, double L) {
+  P.ebox[axis] = L;
+  P.inv_ebox[axis] = 1.0 / L;
+  P.inv_ebox_lo[axis] = std::fma(-L, P.inv_ebox[axis], 1.0) / L;
+}
+
 // PotentialEwaldCoul::ReadParameters (potential_ewald_coul.cc:38-115):
 // padded z for the dipole correction, real-space cut-off and cells, k^2
 // cut-off and cells; then the half-space k-set {k : 0 < k^2 <= kc^2}.
@@ -149,8 +156,7 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
   if (!ewald_setup(in, kMaxKmax, &E, &err)) return fail(PLUM_ERR_INPUT, err);
   const double vol = E.vol;
   for (int a = 0; a < 3; a++) {
-    P.ebox[a] = E.ebox[a];
-    P.inv_ebox[a] = 1.0 / E.ebox[a];
+    set_ebox(P, a, E.ebox[a]);
     P.real_cell[a] = E.real_cell[a];
     P.kmax[a] = E.kcell[a];
     P.kunit[a] = 2 * kPiRef / E.ebox[a];
@@ -559,8 +565,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   for (int a = 0; a < 3; a++) {
     P.box[a] = in.box[a];
     P.inv_box[a] = 1.0 / in.box[a];
-    P.ebox[a] = in.box[a];
-    P.inv_ebox[a] = 1.0 / in.box[a];
+    set_ebox(P, a, in.box[a]);
   }
   P.use_pair = in.use_pair;
   P.use_ewald = in.use_ewald;

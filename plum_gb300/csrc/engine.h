@@ -55,6 +55,7 @@ struct DevParams {
   int max_len;  // beads of the longest molecule
   double box[3], inv_box[3];
   double ebox[3], inv_ebox[3];
+  double inv_ebox_lo[3];  // what 1 / ebox is rounded by (see turn64)
   int use_pair, use_ewald, use_bond, use_rigid, use_ext, dipole;
   double beta, move_size, move_prob[5];
   long long move_cum[4];  // running sums of move_prob, as bits

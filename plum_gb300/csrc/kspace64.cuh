@@ -8,13 +8,17 @@ namespace plum {
 
 // A coordinate as a 64-bit fraction of a turn: frac(w / L) 2^64, times kPi / pi
 // (the reference's phases are 2 kPi n w / L with its 12-digit kPi), so that n
-// times it, mod 2^64, is the phase of n exactly.
+// times it, mod 2^64, is the phase of n exactly. w / L is carried in two doubles:
+// rounded to one it left e^{i theta} off by 2.5e-16, n times that in its n-th power, and
+// S(k) of 20,000 beads further off (2.3e-15) than a sincos of the FP64 angle (1.9e-15).
 __device__ __forceinline__ uint64_t turn64(const DevParams& P, double w, int axis) {
   double f = w * P.inv_ebox[axis];
+  const double lo = fma(w, P.inv_ebox_lo[axis], fma(w, P.inv_ebox[axis], -f));
   double g = f - floor(f);
   if (axis < P.npbc) f = g;  // wrapped into the primary cell
   if (g >= 1.0) g = 0.0;     // a tiny negative w / L rounds up to 1
-  return __double2ull_rn(g * 0x1p64) + (uint64_t)__double2ll_rn(f * P.turn_eps);
+  return __double2ull_rn(g * 0x1p64) +
+         (uint64_t)__double2ll_rn(fma(f, P.turn_eps, lo * 0x1p64));
 }
 
 // The same of a coordinate's box fraction X (fix64; a cubic periodic box): X kPi /
