@@ -1467,6 +1467,7 @@ int plum_ctx_load(plum_ctx* c, const void* buf, long size) {
   DevState st;
   std::memcpy(&st, p, sizeof(DevState));
   st.stream_pos = st.stream_len = 0;
+  st.cell_ok = 0;  // its cell lists are not part of the snapshot
   p += sizeof(DevState);
   CK(cudaMemcpyAsync(c->B.state, &st, sizeof(DevState), cudaMemcpyHostToDevice, c->s));
   CK(cudaMemcpyAsync(c->B.pos, p, sizeof(double4_32a) * c->P.n_bead, cudaMemcpyHostToDevice,
@@ -2098,6 +2099,10 @@ int cells_alloc(plum_batch* b) {
                        b->s));
     CK(cudaMemcpyAsync(b->d_rb, b->h_rb.data(), sizeof(DevBuffers) * n, cudaMemcpyHostToDevice,
                        b->s));
+    // new lists: none is valid before its first build
+    if (words) CK(cudaMemsetAsync(b->d_cells, 0, sizeof(int) * words, b->s));
+    launch_cell_rebuild(b->d_rp, b->d_rb, n, b->max_bead, 0, b->s);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(b->s));
   }
   b->cells_built = false;

@@ -1007,7 +1007,9 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
         B.pos[i] = B.trial[i];
         if (B.fpos64) B.fpos64[i] = B.ftrial64[i - b_lo];
         if (P.form) B.fpos[i] = B.ftrial[i - b_lo];
-        if (P.cell_cap && B.cell_key) {
+        // (lists that were never built, or have overflowed, hold nothing to follow:
+        // their keys may be anything)
+        if (P.cell_cap && B.cell_key && S.cell_ok) {
           // the bead's entry follows it: rewritten in place while it stays in
           // its cell (or already is in the extra list), else marked dead and
           // the bead appended to the extra list
