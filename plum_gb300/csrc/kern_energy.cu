@@ -231,7 +231,9 @@ __device__ __forceinline__ void fix_sweep(const DevParams& P, const DevBuffers& 
 
 // dS(k), the S(k) commit and the |S|^2 change of units [u0, u1) by the k role's
 // threads. A thread takes one of up to 32 units and every slices-th moved bead (a
-// block of a small k-set has few units: their beads then spread over the lanes).
+// block of a small k-set has few units: their beads then spread over the lanes), at both
+// its places one after the other: a sum over the trial places alone is large where the
+// change is small, and its rounding stays.
 // smem, kb = k_beads: [kb][2][zn] e^{i n theta_z}, then [kb][2][kUnits] xy parts.
 template <int kMode>
 __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B,
@@ -301,8 +303,9 @@ __device__ __forceinline__ double k_role(const DevParams& P, const DevBuffers& B
       }
       role_sync(1, kKThreads);
       if (sl < slices)
-        for (int it = sl; it < nt; it += slices)
-          unit_add(s_xy[it * kUnits + col], s_z[(size_t)it * zn + nz], A, Bs);
+        for (int it = 2 * sl; it < nt; it += 2 * slices)
+          for (int h = 0; h < 2; h++)
+            unit_add(s_xy[(it + h) * kUnits + col], s_z[(size_t)(it + h) * zn + nz], A, Bs);
     }
     s_sum[0][threadIdx.x] = A.x;
     s_sum[1][threadIdx.x] = A.y;

@@ -143,7 +143,7 @@ __device__ __forceinline__ float tab_eval(const DevParams& P, const TabPair& K, 
     return tab_diff<kCut, true>(K, s_h, r);
   }
   const float2 xx = sq2(dx), yy = sq2(dy), zz = sq2(dz);
-  const float2 r = add3(xx, yy, zz);
+  const float2 r = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, zz));  // (LJ's: two roundings less)
   if (fminf(r.x, r.y) < K.ljlim) acc_lj += lj32(P, k, r.x) - lj32(P, k, r.y);
   float h = tab_diff<kCut, true>(K, s_h, r);
   const float2 fx = sq2(flip2(K.bx, dx)), fy = sq2(flip2(K.by, dy)), fz = sq2(flip2(K.bz, dz));
@@ -292,13 +292,15 @@ __device__ __forceinline__ float k_role32(const DevParams& P, const DevBuffers& 
       }
       role_sync(1, kD32K);
       if (sl < slices)
-        for (int it = sl; it < nt; it += slices) {
-          const float2 xy = s_xy[it * kD32Units + col], ez = s_z[(size_t)it * zn + nz];
-          A.x = fmaf(xy.x, ez.x, A.x);
-          A.y = fmaf(xy.y, ez.x, A.y);
-          Bs.x = fmaf(xy.x, ez.y, Bs.x);
-          Bs.y = fmaf(xy.y, ez.y, Bs.y);
-        }
+        for (int b = 2 * sl; b < nt; b += 2 * slices)
+#pragma unroll
+          for (int it = b; it < b + 2; it++) {  // both places of a bead (see k_item32)
+            const float2 xy = s_xy[it * kD32Units + col], ez = s_z[(size_t)it * zn + nz];
+            A.x = fmaf(xy.x, ez.x, A.x);
+            A.y = fmaf(xy.y, ez.x, A.y);
+            Bs.x = fmaf(xy.x, ez.y, Bs.x);
+            Bs.y = fmaf(xy.y, ez.y, Bs.y);
+          }
     }
     s_sum[0][threadIdx.x] = A.x;
     s_sum[1][threadIdx.x] = A.y;
@@ -614,7 +616,10 @@ void build_h32_table(float4* out, double scale, double cut) {
 constexpr int kKUnitsMost = kPairThreads;  // most k units of a k item
 
 // dS(k), the S(k) commit and the |S|^2 change of units [u0, u0 + un), at most
-// kKUnitsMost. A thread takes one unit and every slices-th moved bead. smem:
+// kKUnitsMost. A thread takes one unit and every slices-th moved bead, at its trial and
+// its current place (the two nearly cancel: dealt out to different threads, as every
+// other entry, they left partial sums of the trial places alone, whose rounding put the
+// energy change off by 3.6 times as much in a bulk and 7 times in a slab). smem:
 // e^{i nz theta_z} of as many moved beads (trial and current) as fit, then their xy
 // parts per (nx, ny) column, every entry one thread's, from its exact integer phase.
 // (A vector's phase as a product of three table entries, the tables built by six
@@ -661,14 +666,16 @@ __device__ __forceinline__ float k_item32(const DevParams& P, const DevBuffers& 
     }
     __syncthreads();
     if (sl < slices) {
-#pragma unroll 4
-      for (int it = sl; it < nt; it += slices) {
-        const float2 xy = s_xy[it * ncol + col], ez = s_z[it * nz + ku.nz];
-        A.x = fmaf(xy.x, ez.x, A.x);
-        A.y = fmaf(xy.y, ez.x, A.y);
-        Bs.x = fmaf(xy.x, ez.y, Bs.x);
-        Bs.y = fmaf(xy.y, ez.y, Bs.y);
-      }
+#pragma unroll 2
+      for (int b = 2 * sl; b < nt; b += 2 * slices)
+#pragma unroll
+        for (int it = b; it < b + 2; it++) {
+          const float2 xy = s_xy[it * ncol + col], ez = s_z[it * nz + ku.nz];
+          A.x = fmaf(xy.x, ez.x, A.x);
+          A.y = fmaf(xy.y, ez.x, A.y);
+          Bs.x = fmaf(xy.x, ez.y, Bs.x);
+          Bs.y = fmaf(xy.y, ez.y, Bs.y);
+        }
     }
   }
   s_sum[0][threadIdx.x] = A.x;
