@@ -334,7 +334,7 @@ int enqueue_total(plum_ctx* c, cudaStream_t s, double* drift) {
 }
 
 int total_energy(plum_ctx* c, double* out8) {
-  cudaSetDevice(c->device);
+  use_device(c->device);
   enqueue_total(c, c->s, nullptr);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double) * 8, cudaMemcpyDeviceToHost, c->s));
@@ -692,7 +692,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   P.f_lB = (float)P.lB;
   c->recompute_every = form == PLUM_FORM_FP32 ? 10000 : 0;
   // Device state.
-  if (cudaSetDevice(device) != cudaSuccess) {
+  if (use_device(device) != cudaSuccess) {
     delete c;
     return fail(PLUM_ERR_CUDA, "cannot select CUDA device " + std::to_string(device));
   }
@@ -831,7 +831,7 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
 
 int plum_ctx_destroy(plum_ctx* c) {
   if (!c) return PLUM_OK;
-  cudaSetDevice(c->device);
+  use_device(c->device);
   if (c->s) cudaStreamSynchronize(c->s);
   void* ptrs[] = {c->B.pos,      c->B.trial,   c->B.type,  c->B.mol_start, c->B.chain_ids,
                   c->B.ion_ids,  c->B.kn,      c->B.kw,    c->B.sk,        c->B.dsk,
@@ -894,7 +894,7 @@ int plum_total_energy(plum_ctx* c, double* out) {
 int plum_energies(const plum_ctx* cc, double* out) {
   plum_ctx* c = const_cast<plum_ctx*>(cc);
   if (!c || !out) return fail(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   DevState st;
   int rc = read_state(c, &st);
   if (rc) return rc;
@@ -907,7 +907,7 @@ int plum_delta_energy(plum_ctx* c, int mol, const double* trial, const int* move
   if (!c || !trial || !moved || !out) return fail(PLUM_ERR_INPUT, "null argument");
   if (mol < 0 || mol >= c->P.n_mol) return fail(PLUM_ERR_INPUT, "molecule index out of range");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is already pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = refresh_host_pos(c);
   if (rc) return rc;
   const int b0 = c->in.mol_start[mol], b1 = c->in.mol_start[mol + 1];
@@ -1092,7 +1092,7 @@ int plum_append_molecules(plum_ctx* c, int n_mols, const int* sizes, const doubl
     if (type[k] < 0 || type[k] >= c->P.n_type || !std::isfinite(xyz[3 * k]) ||
         !std::isfinite(xyz[3 * k + 1]) || !std::isfinite(xyz[3 * k + 2]))
       return fail(PLUM_ERR_INPUT, "bad bead type or position");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = refresh_host_pos(c);
   if (rc) return rc;
   Input& in = c->in;
@@ -1110,7 +1110,7 @@ int plum_erase_molecules(plum_ctx* c, int first, int count) {
   if (!c || first < 0 || count <= 0 || first + count > c->in.n_mol)
     return fail(PLUM_ERR_INPUT, "molecule range out of bounds");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = refresh_host_pos(c);
   if (rc) return rc;
   Input& in = c->in;
@@ -1127,7 +1127,7 @@ int plum_erase_molecules(plum_ctx* c, int first, int count) {
 int plum_move_descriptor(plum_ctx* c, double* out) {
   if (!c || !out) return fail(PLUM_ERR_INPUT, "null argument");
   if (!c->host_pending) return fail(PLUM_ERR_STATE, "no pending trial move");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = ensure_desc(c);
   if (rc) return rc;
   DevBuffers B = c->B;
@@ -1150,7 +1150,7 @@ int plum_move_descriptor(plum_ctx* c, double* out) {
 int plum_finalize(plum_ctx* c, int accept) {
   if (!c) return fail(PLUM_ERR_INPUT, "null context");
   if (!c->host_pending) return fail(PLUM_ERR_STATE, "no pending trial move");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   launch_serial64(c->P, c->B, kModeCommit | (accept ? kModeAccept : 0), c->s);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->s));
@@ -1174,7 +1174,7 @@ int plum_run_moves_de(plum_ctx* c, const uint32_t* stream, long n_stream, int n_
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
   if (c->in.use_gc) return fail(PLUM_ERR_INPUT, "grand-canonical steps are not run by this loop");
   if (n_moves == 0) return PLUM_OK;
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = ensure_stream(c, n_stream);
   if (!rc) rc = ensure_logs(c, n_moves);
   if (rc) return rc;
@@ -1229,7 +1229,7 @@ int plum_seed(plum_ctx* c, uint32_t seed) {
   mt[0] = seed;
   for (int i = 1; i < 624; i++) mt[i] = 1812433253u * (mt[i - 1] ^ (mt[i - 1] >> 30)) + (uint32_t)i;
   mt[624] = 624;
-  cudaSetDevice(c->device);
+  use_device(c->device);
   CK(cudaMemcpyAsync(c->d_mt, mt, sizeof(mt), cudaMemcpyHostToDevice, c->s));
   CK(cudaStreamSynchronize(c->s));
   drop_stream(c);
@@ -1241,7 +1241,7 @@ int plum_run(plum_ctx* c, int n_moves, int* accepted_out) {
   if (!c || n_moves < 0) return fail(PLUM_ERR_INPUT, "bad argument");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
   if (c->in.use_gc) return fail(PLUM_ERR_INPUT, "grand-canonical steps are not run by this loop");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   // Draw budget per step: 5 fixed draws + the move's own; a pivot consumes
   // 2 + len (2 r + 1) with r rejected pairs per randSphere (mean 1.27).
   const int batch = 256;
@@ -1375,7 +1375,7 @@ int plum_time_kernels(plum_ctx* c, int n_moves, double* out2) {
 int plum_get_positions(const plum_ctx* cc, double* xyz) {
   plum_ctx* c = const_cast<plum_ctx*>(cc);
   if (!c || !xyz) return fail(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = refresh_host_pos(c);
   if (rc) return rc;
   for (int i = 0; i < c->P.n_bead; i++) {
@@ -1389,7 +1389,7 @@ int plum_get_positions(const plum_ctx* cc, double* xyz) {
 int plum_set_positions(plum_ctx* c, const double* xyz) {
   if (!c || !xyz) return fail(PLUM_ERR_INPUT, "null argument");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = refresh_host_pos(c);
   if (rc) return rc;
   for (int i = 0; i < c->P.n_bead; i++) {
@@ -1423,7 +1423,7 @@ int plum_ctx_save(const plum_ctx* cc, void* buf, long size) {
   plum_ctx* c = const_cast<plum_ctx*>(cc);
   if (!c || !buf || size < (long)snap_bytes(c)) return fail(PLUM_ERR_INPUT, "bad argument");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   unsigned char* p = static_cast<unsigned char*>(buf);
   const int head[5] = {kSnapMagic, c->P.n_bead, c->P.n_k, c->P.n_mol, c->form};
   std::memcpy(p, head, sizeof(head));
@@ -1459,7 +1459,7 @@ int plum_ctx_load(plum_ctx* c, const void* buf, long size) {
   if (head[0] != kSnapMagic || head[1] != c->P.n_bead || head[2] != c->P.n_k ||
       head[3] != c->P.n_mol || head[4] != c->form || size < (long)snap_bytes(c))
     return fail(PLUM_ERR_INPUT, "the snapshot belongs to another system or form");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   p += sizeof(head);
   CK(cudaStreamSynchronize(c->s));
   // the snapshot replaces the device state, the generator's stream cursor
@@ -1502,7 +1502,7 @@ int plum_structure_factor(const plum_ctx* cc, double* sk_out, int* kn_out) {
   plum_ctx* c = const_cast<plum_ctx*>(cc);
   if (!c) return fail(PLUM_ERR_INPUT, "null context");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   const int nk = c->P.use_ewald ? c->P.n_k : 0;
   if (nk == 0) return PLUM_OK;
   if (kn_out) {
@@ -1536,7 +1536,7 @@ int plum_structure_factor(const plum_ctx* cc, double* sk_out, int* kn_out) {
 int plum_observables(const plum_ctx* cc, double* out) {
   plum_ctx* c = const_cast<plum_ctx*>(cc);
   if (!c || !out) return fail(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   launch_observables64(c->P, c->B, c->d_obs_per, c->d_out + 32, c->s);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(c->h_out, c->d_out + 32, sizeof(double) * 5, cudaMemcpyDeviceToHost, c->s));
@@ -1553,7 +1553,7 @@ int plum_chain_observables(const plum_ctx* cc, double* out, int cap, int* n_chai
   for (int m = 0; m < in.n_mol; m++) n += in.mol_start[m + 1] - in.mol_start[m] > 1;
   if (n_chains) *n_chains = n;
   if (cap == 0) return PLUM_OK;
-  cudaSetDevice(c->device);
+  use_device(c->device);
   launch_observables64(c->P, c->B, c->d_obs_per, c->d_out + 32, c->s);
   CK(cudaGetLastError());
   std::vector<double> per(5 * (size_t)in.n_mol);
@@ -1576,7 +1576,7 @@ int plum_rhoz(const plum_ctx* cc, double* out, int cap, int* n_bins) {
   if (n_bins) *n_bins = nb;
   if (cap == 0) return PLUM_OK;
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   launch_rhoz(c->P, c->B, kRhoZRes, nb, c->d_rhoz, c->s);
   CK(cudaGetLastError());
   std::vector<unsigned> cnt(3 * (size_t)nb);
@@ -1592,7 +1592,7 @@ int plum_rhoz(const plum_ctx* cc, double* out, int cap, int* n_bins) {
 int plum_pressure_slit(plum_ctx* c, double* out6) {
   if (!c || !out6) return fail(PLUM_ERR_INPUT, "null argument");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   const Input& in = c->in;
   const DevParams& P = c->P;
   SlitPressParams S{};
@@ -1709,7 +1709,7 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
     return fail(PLUM_ERR_INPUT, "a charged species needs trial counterions");
   if (chain_len > 0 && !chain) return fail(PLUM_ERR_INPUT, "missing grown chain");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   const bool fp32 = c->form == PLUM_FORM_FP32;
   Cbmc32Layout G{};
   if (fp32) {
@@ -1851,7 +1851,7 @@ int plum_collect_surrogate_data(plum_ctx* c, int n_moves, long cap, float* d_des
   if (!c || n_moves < 0 || cap <= 0 || cap > (1L << 31) - 1 || !d_desc || !d_de)
     return fail(PLUM_ERR_INPUT, "bad argument");
   if (c->host_pending) return fail(PLUM_ERR_STATE, "a trial move is pending");
-  cudaSetDevice(c->device);
+  use_device(c->device);
   int rc = ensure_desc(c);
   if (rc) return rc;
   DevState st;
@@ -1915,7 +1915,7 @@ int plum_cbmc_trials_noalloc(plum_ctx* c, int n_trials, const double* d_b1, cons
   }
   int type = 0;
   while (type < (int)in.type_names.size() && in.type_names[type] != in.gc_symbol) type++;
-  if (cudaSetDevice(c->device) != cudaSuccess) {
+  if (use_device(c->device) != cudaSuccess) {
     say("plum_cbmc_trials_noalloc: cannot select the context's device");
     return PLUM_ERR_CUDA;
   }
@@ -1940,7 +1940,7 @@ int plum_drift(const plum_ctx* c, double* out) {
 }
 
 int plum_probe_peaks(int device, double* fp32_tflops, double* fp64_tflops) {
-  if (cudaSetDevice(device) != cudaSuccess) return fail(PLUM_ERR_CUDA, "cannot select device");
+  if (use_device(device) != cudaSuccess) return fail(PLUM_ERR_CUDA, "cannot select device");
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   float* o32 = nullptr;
@@ -2262,7 +2262,7 @@ extern "C" {
 
 int plum_batch_energies(plum_batch* b, double* out) {
   if (!b || !out) return fail(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   const int R = (int)b->reps.size();
   // one gather launch and one copy for all replicas
   launch_gather_energies(b->d_sts, R, b->d_energies, b->s);
@@ -2282,7 +2282,7 @@ int plum_batch_set_recompute(plum_batch* b, long every) {
 
 int plum_batch_drift(plum_batch* b, double* out, long* count, double* ms) {
   if (!b || !out) return fail(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   const int R = (int)b->reps.size();
   CK(cudaMemcpyAsync(out, b->d_drift, sizeof(double) * 6 * R, cudaMemcpyDeviceToHost, b->s));
   CK(cudaStreamSynchronize(b->s));
@@ -2293,7 +2293,7 @@ int plum_batch_drift(plum_batch* b, double* out, long* count, double* ms) {
 
 int plum_batch_destroy(plum_batch* b) {
   if (!b) return PLUM_OK;
-  cudaSetDevice(b->device);
+  use_device(b->device);
   if (b->s) cudaStreamSynchronize(b->s);
   for (plum_ctx* c : b->reps) plum_ctx_destroy(c);
   void* ptrs[] = {b->d_cells, b->d_queue, b->d_slots2, b->d_rp,    b->d_rb,  b->d_item_off, b->d_slots, b->d_states, b->d_outs,
@@ -2343,7 +2343,7 @@ int plum_batch_create(int n, const char* const* dirs, const char* const* runins,
     }
     b->reps.push_back(c);
   }
-  cudaSetDevice(device);
+  use_device(device);
   if (cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->s2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
@@ -2541,7 +2541,7 @@ int plum_batch_seed_each(plum_batch* b, const uint32_t* seeds) {
 
 int plum_batch_run(plum_batch* b, int n_steps, long* accepted_out) {
   if (!b || n_steps < 0) return fail(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   const int R = (int)b->reps.size();
   std::vector<int> need(R);
   std::vector<long long> pos(R), len(R);
@@ -2618,7 +2618,7 @@ int plum_batch_run(plum_batch* b, int n_steps, long* accepted_out) {
 
 int plum_batch_time_kernels(plum_batch* b, int n_steps, double* out4) {
   if (!b || n_steps <= 0 || !out4) return fail(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   const int R = (int)b->reps.size();
   // the stream words these steps need (as plum_batch_run refills them)
   launch_gather_states(b->d_sts, R, b->d_gather, b->s);
@@ -2721,7 +2721,7 @@ int plum_batch_set_tune(plum_batch* b, int item_pairs, int k_tile, int grid, int
 
 int plum_batch_descriptors(plum_batch* b, float* out) {
   if (!b || !out) return fail(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   const size_t n = (size_t)mlp::kIn * b->reps.size();
   std::vector<unsigned> h(n);
   CK(cudaMemcpyAsync(h.data(), b->d_desc, sizeof(unsigned) * n, cudaMemcpyDeviceToHost, b->s));
@@ -2732,7 +2732,7 @@ int plum_batch_descriptors(plum_batch* b, float* out) {
 
 int plum_batch_cell_stats(plum_batch* b, int* out4) {
   if (!b || !out4) return fail(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   int with = 0, ok = 0, most = 0, cap = 0;
   std::vector<DevBuffers> hb(b->reps.size());
   std::vector<DevParams> hp(b->reps.size());
@@ -2773,7 +2773,7 @@ int plum_batch_set_groups(plum_batch* b, int groups) {
 
 int plum_batch_set_cell_cap(plum_batch* b, int cap) {
   if (!b || cap < 1 || cap > (1 << 20)) return fail(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   if (!b->cell_moved) return PLUM_OK;
   for (auto& P : b->h_rp)
     if (P.cell_cap) P.cell_cap = cap;
@@ -2877,7 +2877,7 @@ int plum_batch_set_surrogate(plum_batch* b, const plum_surrogate* sg) {
   if (!b) return fail(PLUM_ERR_INPUT, "null batch");
   if (sg && sg->device != b->device)
     return fail(PLUM_ERR_INPUT, "the surrogate lives on another device");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   if (sg) CK(cudaStreamSynchronize(sg->s));
   for (plum_ctx* c : b->reps) {
     DevState st;
@@ -2900,7 +2900,7 @@ int plum_batch_set_surrogate(plum_batch* b, const plum_surrogate* sg) {
 
 int plum_batch_da_stats(plum_batch* b, long* out3) {
   if (!b || !out3) return fail(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(b->device);
+  use_device(b->device);
   out3[0] = out3[1] = out3[2] = 0;
   int e = 0;
   CK(cudaMemcpy(&e, b->d_err, sizeof(int), cudaMemcpyDeviceToHost));

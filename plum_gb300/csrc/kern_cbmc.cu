@@ -373,6 +373,8 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
         }
         if (J.charged)
           re = fma(p1.w * __longlong_as_double((long long)o.w) * unit, (double)v + h * hs, re);
+        else if (own)  // a neutral species': zero, or NaN where it is not finite
+          re += __longlong_as_double((long long)o.w);
       }
       s_red[0][id] = lj;
       s_red[1][id] = re;
@@ -398,9 +400,6 @@ __global__ void __launch_bounds__(kCb64Sum)
   double v[3] = {0.0, 0.0, 0.0};
   for (int b = tid; b < blocks; b += kCb64Sum)
     for (int c = 0; c < 3; c++) v[c] += J.slots[((size_t)b * J.n_trials + t) * 3 + c];
-  // a neutral species' Ewald energy is zero, or NaN with a grown bead that is not finite
-  if (!J.charged)
-    for (int i = tid; i < J.cl; i += kCb64Sum) v[1] += charge_of(J.chain[i]);
   for (int c = 0; c < 3; c++) {
     v[c] = warp_sum(v[c]);
     if ((tid & 31) == 0) s_w[tid >> 5][c] = v[c];

@@ -75,7 +75,7 @@ int plum_surrogate_nparams(void) { return mlp::kNParam; }
 int plum_surrogate_create(int device, unsigned long long seed, plum_surrogate** out) {
   if (!out) return plum::fail_msg(PLUM_ERR_INPUT, "null argument");
   *out = nullptr;
-  if (cudaSetDevice(device) != cudaSuccess)
+  if (use_device(device) != cudaSuccess)
     return plum::fail_msg(PLUM_ERR_CUDA, "cannot select the device");
   plum_surrogate* g = new plum_surrogate();
   g->device = device;
@@ -119,7 +119,7 @@ int plum_surrogate_create(int device, unsigned long long seed, plum_surrogate** 
 
 int plum_surrogate_destroy(plum_surrogate* g) {
   if (!g) return PLUM_OK;
-  cudaSetDevice(g->device);
+  use_device(g->device);
   if (g->s) cudaStreamSynchronize(g->s);
   void* ptrs[] = {g->net, g->param, g->m,   g->v,    g->grad, g->d_err,
                   g->d_loss, g->d_x, g->d_t, g->d_s, g->part, g->d_idx};
@@ -132,7 +132,7 @@ int plum_surrogate_destroy(plum_surrogate* g) {
 
 int plum_surrogate_set_params(plum_surrogate* g, const float* params) {
   if (!g || !params) return plum::fail_msg(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   SCK(cudaMemcpyAsync(g->param, params, sizeof(float) * mlp::kNParam, cudaMemcpyHostToDevice,
                       g->s));
   launch_mlp_pack(g->param, g->net, g->s);
@@ -143,7 +143,7 @@ int plum_surrogate_set_params(plum_surrogate* g, const float* params) {
 
 int plum_surrogate_get_params(const plum_surrogate* g, float* params) {
   if (!g || !params) return plum::fail_msg(PLUM_ERR_INPUT, "null argument");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   SCK(cudaMemcpyAsync(params, g->param, sizeof(float) * mlp::kNParam, cudaMemcpyDeviceToHost,
                       g->s));
   SCK(cudaStreamSynchronize(g->s));
@@ -152,7 +152,7 @@ int plum_surrogate_get_params(const plum_surrogate* g, float* params) {
 
 int plum_surrogate_set_norm(plum_surrogate* g, const float* mu, const float* isd, float y_scale) {
   if (!g || !mu || !isd || !(y_scale > 0.0f)) return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   for (int k = 0; k < mlp::kIn; k++)
     if (!std::isfinite(mu[k]) || !std::isfinite(isd[k]))
       return plum::fail_msg(PLUM_ERR_INPUT, "non-finite normalisation");
@@ -169,7 +169,7 @@ int plum_surrogate_set_norm(plum_surrogate* g, const float* mu, const float* isd
 
 int plum_surrogate_set_margin(plum_surrogate* g, float margin) {
   if (!g || !(margin >= 0.0f)) return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   SCK(cudaMemcpyAsync(reinterpret_cast<char*>(g->net) + offsetof(MlpNet, da_margin), &margin,
                       sizeof(float), cudaMemcpyHostToDevice, g->s));
   SCK(cudaStreamSynchronize(g->s));
@@ -180,7 +180,7 @@ int plum_surrogate_predict(plum_surrogate* g, const float* x, long n, float* s_o
   if (!g || n < 0 || (n > 0 && (!x || !s_out))) return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
   if (n == 0) return PLUM_OK;
   if (n > (1L << 30) / mlp::kIn) return plum::fail_msg(PLUM_ERR_INPUT, "too many samples");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   if (ensure_cap(g, n)) return PLUM_ERR_CUDA;
   SCK(cudaMemcpyAsync(g->d_x, x, sizeof(float) * mlp::kIn * n, cudaMemcpyHostToDevice, g->s));
   launch_mlp_infer_f(g->net, g->d_x, (int)n, g->d_s, g->d_err, g->s);
@@ -193,7 +193,7 @@ int plum_surrogate_predict_device(plum_surrogate* g, const float* d_x, long n, f
   if (!g || n < 0 || (n > 0 && (!d_x || !d_s))) return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
   if (n == 0) return PLUM_OK;
   if (n > (1L << 30) / mlp::kIn) return plum::fail_msg(PLUM_ERR_INPUT, "too many samples");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   launch_mlp_infer_f(g->net, d_x, (int)n, d_s, g->d_err, g->s);
   SCK(cudaGetLastError());
   return check_err(g);
@@ -203,7 +203,7 @@ int plum_surrogate_grad(plum_surrogate* g, const float* x, const float* t, long 
                         float* grad_out) {
   if (!g || n <= 0 || !x || !t || !grad_out) return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
   if (n > (1L << 30) / mlp::kIn) return plum::fail_msg(PLUM_ERR_INPUT, "too many samples");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   if (ensure_cap(g, n)) return PLUM_ERR_CUDA;
   SCK(cudaMemcpyAsync(g->d_x, x, sizeof(float) * mlp::kIn * n, cudaMemcpyHostToDevice, g->s));
   SCK(cudaMemcpyAsync(g->d_t, t, sizeof(float) * n, cudaMemcpyHostToDevice, g->s));
@@ -219,7 +219,7 @@ int plum_surrogate_train(plum_surrogate* g, const float* d_x, const float* d_t, 
   if (!g || !d_x || !d_t || n <= 0 || batch <= 0 || epochs < 0 || !(lr > 0.0f))
     return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
   if (n > (1L << 31) - 1 || batch > (1 << 20)) return plum::fail_msg(PLUM_ERR_INPUT, "too large");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   const long b = std::min<long>(batch, n);
   if (ensure_cap(g, b)) return PLUM_ERR_CUDA;
   if (g->idx_cap < n) {
@@ -255,7 +255,7 @@ int plum_surrogate_train(plum_surrogate* g, const float* d_x, const float* d_t, 
 
 int plum_surrogate_adam_step(plum_surrogate* g, const float* grad, float lr) {
   if (!g || !grad || !(lr > 0.0f)) return plum::fail_msg(PLUM_ERR_INPUT, "bad argument");
-  cudaSetDevice(g->device);
+  use_device(g->device);
   SCK(cudaMemcpyAsync(g->grad, grad, sizeof(float) * mlp::kNParam, cudaMemcpyHostToDevice, g->s));
   launch_mlp_adam(g->param, g->m, g->v, g->grad, ++g->step, lr, g->net, g->s);
   SCK(cudaGetLastError());

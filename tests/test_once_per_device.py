@@ -26,6 +26,8 @@ def test_every_launcher_uses_it():
         with open(path) as f:
             text = f.read()
         assert "cudaFuncSetAttribute" not in text, path
+        # a call's device is selected, and known, through one function
+        assert "cudaSetDevice" not in text and "cudaGetDevice(" not in text, path
         # no other state of a device in a function's or a file's static flag
         assert not re.search(r"static (bool|int) \w+ = (false|0);", text), path
         assert len(re.findall(r"\bOncePerDevice (\w+)", text)) <= len(
