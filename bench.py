@@ -60,9 +60,10 @@ sys.path.insert(0, ROOT)
 METRIC = "MC moves/s and Rg-decorrelated samples/s: plain FP64 vs chosen form, 1 GB300"
 
 # DRAM bytes per evaluated move of the batched energy-change kernel on this
-# workload: dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture
-# (64 replicas, every move evaluated: 44 MB per launch of 64 moves)
-TRAFFIC_PER_EXACT_MOVE = 44.0e6 / 64
+# workload: dram__bytes_read.sum + dram__bytes_write.sum, mean of four launches
+# under ncu (64 replicas, every move evaluated: 43.7 MB per launch of 64 moves;
+# profiles/energy_and_step_kernels.md)
+TRAFFIC_PER_EXACT_MOVE = 43.7e6 / 64
 
 
 def mt19937_stream(seed: int, n: int):

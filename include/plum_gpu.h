@@ -387,8 +387,8 @@ int plum_batch_set_tune(plum_batch* batch, int item_pairs, int k_tile, int grid,
  * k_tile, grid, min_blocks}. */
 int plum_batch_autotune(plum_batch* batch, int steps, int* out4);
 /* The pair loop of the batched energy change. table = 1 (the default where
- * it applies): for LJ + Ewald replicas whose real cut-off is at most half
- * the box, the table of h(u) = erfc(sqrt u)/sqrt u (cubic pieces, 32 per
+ * it applies): for LJ + Ewald replicas whose real cut-off is below every box
+ * length (a second image per axis where it is past half of one), the table of h(u) = erfc(sqrt u)/sqrt u (cubic pieces, 32 per
  * octave of u, about 1e-7 relative below u = 4; erfc(sqrt(alpha) r)/r =
  * sqrt(alpha) h(alpha r^2)) staged in shared memory and the trial and current
  * evaluations of a pair done together, branch-free. table = 0: the loop of

@@ -140,10 +140,10 @@ struct DevState {
   int moves_left;
   int n_accept;
   int n_nonfinite;   // steps whose dE was NaN/Inf (rejected, as in the reference)
-  // pending move's sums, reduced by the last block of the delta kernel
+  // pending move's sums: the serial step's, of the energy change's block sums or items
   double red_lj, red_re, red_k;
   // S(k) commit of an accepted move is applied by the next delta kernel's
-  // k tiles: dsk[sk_buf] is pending while sk_pending; the delta kernel writes
+  // k units: dsk[sk_buf] is pending while sk_pending; the delta kernel writes
   // the new dS(k) into dsk[cur_buf]
   int sk_pending, sk_buf, cur_buf;
   // delayed acceptance (surrogate stage one before the exact energy change):

@@ -12,7 +12,9 @@
 //     multiply-add), so e^{i k.r} = sincospi(phase * 2^-31) has no FP32
 //     range-reduction error.
 // In the slab geometry z is not wrapped (|dz| < H < L_z,Ewald / 2), so the same
-// subtraction gives the raw dz the reference uses (GetDistVector, npbc = 2).
+// subtraction gives the raw dz the reference uses (GetDistVector, npbc = 2). That needs
+// the Ewald box that the dipole correction pads: in a slab without it (L_z,Ewald = H)
+// the nearest image across the walls is taken, for LJ too.
 //
 // Per-thread and per-block sums are FP32; blocks are added in FP64 by the
 // serial kernel.
@@ -721,7 +723,7 @@ __device__ __forceinline__ float k_item32(const DevParams& P, const DevBuffers& 
 // result does not depend on which block took which item.
 // The item sizes, the grid and the register budget (kMinBlocks resident
 // blocks per SM) are run-time choices (BatchTune, picked by
-// plum_batch_autotune); defaults: 4096 pairs per item, 128-vector k tiles,
+// plum_batch_autotune); defaults: 4096 pairs per item, 64 units per k item,
 // 4 blocks per SM, 2 resident.
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kPairThreads, kMinBlocks)

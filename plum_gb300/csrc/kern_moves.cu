@@ -919,7 +919,7 @@ __device__ __forceinline__ void serial_body(const DevParams& P, const DevBuffers
     if (threadIdx.x == 0) {
       const double ext = now.ext, dmz = now.dmz, bt = now.bond;
       const int ext_bad = now.ext_bad;
-      // the delta kernel applied any pending S(k) commit if it ran k tiles
+      // the delta kernel applied any pending S(k) commit if it ran k units
       if (P.use_ewald && b_hi > b_lo) S.sk_pending = 0;
       const double de_lj = S.red_lj, de_re = S.red_re, de_k = b_hi > b_lo ? S.red_k : 0.0;
       double de = 0.0, dp = 0.0, dx = 0.0, dw = 0.0, db = 0.0;

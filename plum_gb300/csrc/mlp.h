@@ -84,12 +84,12 @@ void launch_mlp_infer_i(const MlpNet* net, const unsigned* x, int n, float* s_ou
 // [kNParam + 1] (the last entry is the loss).
 void launch_mlp_grad(const MlpNet* net, const float* x, const float* t, int n, float* part,
                      float* grad, int* err, cudaStream_t st);
-// Adam step on the fp32 master parameters; refreshes the bf16 copies in net.
 // A training step on the n samples idx of x and t: gradient, Adam, bf16 copies, the
 // loss added to loss[0].
 void launch_mlp_train(MlpNet* net, const float* x, const float* t, const int* idx, int n,
                       float* part, float* param, float* m, float* v, int step, float lr,
                       double* loss, int* err, cudaStream_t st);
+// Adam step on the fp32 master parameters; refreshes the bf16 copies in net.
 void launch_mlp_adam(float* param, float* m, float* v, const float* grad, int step, float lr,
                      MlpNet* net, cudaStream_t st);
 // fp32 parameters -> net (bf16 weights, fp32 biases).
