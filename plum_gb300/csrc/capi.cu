@@ -144,6 +144,10 @@ void set_ebox(DevParams& P, int axis, double L) {
   P.inv_ebox_lo[axis] = std::fma(-L, P.inv_ebox[axis], 1.0) / L;
 }
 
+// A slab's z is not wrapped, and its beads may be further apart than half the Ewald box:
+// no dipole correction pads it (or there is no Ewald term, and the box stands for it).
+bool unpadded_slab(const DevParams& P) { return P.npbc == 2 && P.ebox[2] < 2.0 * P.box[2]; }
+
 // PotentialEwaldCoul::ReadParameters (potential_ewald_coul.cc:38-115):
 // padded z for the dipole correction, real-space cut-off and cells, k^2
 // cut-off and cells; then the half-space k-set {k : 0 < k^2 <= kc^2}.
@@ -170,7 +174,9 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
   P.kchunk_sk = std::max(1, std::min(32, kKTableBytes / row));
   const double rc = E.real_cut;
   P.real_cut = rc;
-  P.single_image = rc <= 0.5 * E.ebox[0] && rc <= 0.5 * E.ebox[1] && rc <= 0.5 * E.ebox[2];
+  // (one image is enough only where the differences are wrapped or short along z)
+  P.single_image = rc <= 0.5 * E.ebox[0] && rc <= 0.5 * E.ebox[1] && rc <= 0.5 * E.ebox[2] &&
+                   !unpadded_slab(P);
   // the tabulated real-space term: one image, or at most two on each axis (r_c below
   // every box length; the further one stays above the table's lower end)
   bool two = true;
@@ -178,7 +184,7 @@ int setup_ewald(plum_ctx* c, std::vector<short4>* kn, std::vector<double>* kw,
     P.f_img[a] = rc > 0.5 * E.ebox[a] ? (float)E.ebox[a] : 2.0f * kNoImage;
     two = two && rc < E.ebox[a] && in.alpha * 0.25 * E.ebox[a] * E.ebox[a] >= std::ldexp(1.0, kH32ELo);
   }
-  P.images = P.single_image ? 1 : (two ? 2 : 0);
+  P.images = P.single_image ? 1 : (two && !unpadded_slab(P) ? 2 : 0);
   P.two_axes = 0;
   for (int a = 0; a < 3; a++) {
     const double La = E.ebox[a], Lb = E.ebox[(a + 1) % 3];
@@ -664,11 +670,13 @@ static int create_ctx(plum_ctx* c, int form, int device, plum_ctx** out) {
   }
   // Precision-form constants: fixed point in units of the Ewald box.
   P.form = form;
+  P.z_turns = unpadded_slab(P) ? 2u : 1u;
   for (int a = 0; a < 3; a++) {
-    P.f_scale[a] = (float)(P.ebox[a] / 4294967296.0);
+    const double span = a == 2 ? P.z_turns * P.ebox[a] : P.ebox[a];  // of 2^32 units
+    P.f_scale[a] = (float)(span / 4294967296.0);
     P.same_wrap = (a == 0 ? 1 : P.same_wrap) &&
                   (a >= P.npbc || (P.box[a] == P.ebox[a] && P.inv_box[a] == P.inv_ebox[a]));
-    P.inv_fix[a] = 4294967296.0 / P.ebox[a];
+    P.inv_fix[a] = 4294967296.0 / span;
     P.f_box[a] = (float)P.ebox[a];
   }
   // the largest LJ (or hard-sphere bound) cut-off over the type pairs in

@@ -56,6 +56,10 @@ struct DevParams {
   double box[3], inv_box[3];
   double ebox[3], inv_ebox[3];
   double inv_ebox_lo[3];  // what 1 / ebox is rounded by (see turn64)
+  // Ewald boxes along z that the 2^32 fixed-point units cover: 2 in a slab whose Ewald
+  // box is not padded (z is not wrapped, and |dz| may pass half of it), so that a
+  // difference is still the raw one and phases count twice the turns; else 1.
+  unsigned z_turns, pad_z;
   int use_pair, use_ewald, use_bond, use_rigid, use_ext, dipole;
   double beta, move_size, move_prob[5];
   long long move_cum[4];  // running sums of move_prob, as bits

@@ -60,9 +60,9 @@ __device__ __forceinline__ float real_only(const DevParams& P, int4 a, float qa,
 }
 
 // q e^{ik.r} from the fixed-point coordinates (integer phase, wrapped mod 2^32)
-__device__ __forceinline__ float2 cis_q(short4 k, int4 f, float q) {
+__device__ __forceinline__ float2 cis_q(const DevParams& P, short4 k, int4 f, float q) {
   const unsigned ph = (unsigned)(int)k.x * (unsigned)f.x + (unsigned)(int)k.y * (unsigned)f.y +
-                      (unsigned)(int)k.z * (unsigned)f.z;
+                      (unsigned)(int)k.z * P.z_turns * (unsigned)f.z;
   float s, c;
   sincospif((float)(int)ph * 4.6566128730773926e-10f, &s, &c);  // * 2^-31
   return make_float2(q * c, q * s);
@@ -180,16 +180,16 @@ __global__ void __launch_bounds__(kThreads)
       }
       float ax = 0.0f, ay = 0.0f;
       for (int j = J.ex_lo; j < J.ex_hi; j++) {
-        const float2 e = cis_q(kv, B.fpos[j], B.fq[j]);
+        const float2 e = cis_q(P, kv, B.fpos[j], B.fq[j]);
         ax -= e.x;
         ay -= e.y;
       }
       for (int i = 0; i < cl; i++) {
-        float2 e = cis_q(kv, s_cf[i], s_cq[i]);
+        float2 e = cis_q(P, kv, s_cf[i], s_cq[i]);
         ax += e.x;
         ay += e.y;
         if (J.charged) {
-          e = cis_q(kv, s_cf[cl + i], s_cq[cl + i]);
+          e = cis_q(P, kv, s_cf[cl + i], s_cq[cl + i]);
           ax += e.x;
           ay += e.y;
         }
@@ -200,9 +200,9 @@ __global__ void __launch_bounds__(kThreads)
     for (int t = 0; t < T; t++) {
       float c = 0.0f;
       if (mine) {
-        float2 e = cis_q(kv, s_tf[t], s_tq[t]);
+        float2 e = cis_q(P, kv, s_tf[t], s_tq[t]);
         if (J.charged) {
-          const float2 e2 = cis_q(kv, s_tf[T + t], s_tq[T + t]);
+          const float2 e2 = cis_q(P, kv, s_tf[T + t], s_tq[T + t]);
           e.x += e2.x;
           e.y += e2.y;
         }

@@ -12,9 +12,8 @@
 //     multiply-add), so e^{i k.r} = sincospi(phase * 2^-31) has no FP32
 //     range-reduction error.
 // In the slab geometry z is not wrapped (|dz| < H < L_z,Ewald / 2), so the same
-// subtraction gives the raw dz the reference uses (GetDistVector, npbc = 2). That needs
-// the Ewald box that the dipole correction pads: in a slab without it (L_z,Ewald = H)
-// the nearest image across the walls is taken, for LJ too.
+// subtraction gives the raw dz the reference uses (GetDistVector, npbc = 2). Where no
+// dipole correction pads that box, z covers two of it (DevParams::z_turns).
 //
 // Per-thread and per-block sums are FP32; blocks are added in FP64 by the
 // serial kernel.
@@ -283,7 +282,7 @@ __device__ __forceinline__ float k_role32(const DevParams& P, const DevBuffers& 
         const int bead = g0 + (it >> 1);
         const int4 f = (it & 1) ? B.fpos[bead] : B.ftrial[bead - b_lo];
         if (c <= zmax) {
-          s_z[(size_t)it * zn + c] = turn32((unsigned)f.z * (unsigned)c);
+          s_z[(size_t)it * zn + c] = turn32((unsigned)f.z * (P.z_turns * (unsigned)c));
         } else {
           const short2 kc = s_col[c - zmax - 1];
           const float2 v = turn32((unsigned)f.x * (unsigned)(int)kc.x +
@@ -657,7 +656,7 @@ __device__ __forceinline__ float k_item32(const DevParams& P, const DevBuffers& 
       const int bead = g0 + (it >> 1);
       const int4 f = (it & 1) ? B.fpos[bead] : B.ftrial[bead - b_lo];
       if (c < nz) {
-        s_z[it * nz + c] = turn32((unsigned)f.z * (unsigned)c);
+        s_z[it * nz + c] = turn32((unsigned)f.z * (P.z_turns * (unsigned)c));
       } else {
         const short2 kc = s_col[c - nz];
         const float2 v = turn32((unsigned)f.x * (unsigned)(int)kc.x +
