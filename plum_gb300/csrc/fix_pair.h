@@ -15,9 +15,9 @@
 // 2e-16, which is 5e-13, 2e-12 and (image cells) 7e-11 of h there, against 1e-15 of h
 // from the FP64 polynomial. The Horner steps truncate, so most of that has a sign
 // (low); charges of both signs cancel it. Whole results, against 64-bit sums and with
-// FP64 pairs in brackets: a 20,000-bead energy is off by 2.9e-15 of it (2.7e-15), the
-// energies of a 1,000-bead run by 1e-16 to 6e-16 (1e-16 to 5e-16), growth steps by
-// 3e-17 (3e-17).
+// FP64 pairs in brackets: a 20,000-bead frame (energies and S(k)) is off by 2.7e-15
+// (2.7e-15), the energies of a 1,000-bead run by 1e-16 to 6e-16 (3e-16 to 8e-16),
+// growth steps by 3e-17 (3e-17).
 //
 // Units. X = frac(x / L) 2^64 (fix64), d = X_b - X_a as a signed 64-bit number
 // is the minimum-image difference. With shift = 0 (r_c <= L / 2) S = |d|^2 /
