@@ -1768,11 +1768,14 @@ static int cbmc_prepare(plum_ctx* c, int n_trials, const double* b1, const doubl
   };
   put(b1, n_trials, q1);
   put(chain, chain_len, q1);
+  CbmcJob J;
   if (charged) {
     put(b2, n_trials, q2);
     put(chain_ci, chain_len, q2);
+  } else {
+    for (int i = 0; i < 3 * chain_len; i++)
+      if (!std::isfinite(chain[i])) J.lost = 1;
   }
-  CbmcJob J;
   J.n_trials = n_trials;
   J.charged = charged;
   J.cl = chain_len;

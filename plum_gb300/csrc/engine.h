@@ -325,6 +325,7 @@ struct CbmcJob {
   double* part;                     // [n_trials][groups][2] scratch
   double* u;                        // [n_trials] result
   double* slots;                    // [cbmc_blocks()][n_trials][3] block sums
+  int lost = 0;                     // a neutral species: a grown bead is not finite
 };
 constexpr int kCbmcGroups = 64;  // most that cbmc_groups returns
 int cbmc_groups(const DevParams& P);

@@ -373,8 +373,6 @@ __global__ void __launch_bounds__(kCb64Threads, 1)
         }
         if (J.charged)
           re = fma(p1.w * __longlong_as_double((long long)o.w) * unit, (double)v + h * hs, re);
-        else if (own)  // a neutral species': zero, or NaN where it is not finite
-          re += __longlong_as_double((long long)o.w);
       }
       s_red[0][id] = lj;
       s_red[1][id] = re;
@@ -429,7 +427,8 @@ __global__ void __launch_bounds__(kCb64Sum)
         ew += 0.5 * (cb_real(P, b1, b1) + cb_real(P, b2, b2));
     }
   } else if (P.use_ewald && P.n_k > 0 && pair_e < kVeryLarge) {
-    ew = v[1] + charge_of(b1);
+    // a neutral species' is zero, or NaN where it or a grown bead is not finite
+    ew = J.lost ? __longlong_as_double(0x7FF8000000000000ll) : charge_of(b1);
   }
   if (P.use_ext) {
     pair_e += wall64(P, b1.z, J.type);
